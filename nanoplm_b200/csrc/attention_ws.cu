@@ -225,7 +225,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = warp_index();
   const int lane = tid & 31;
   const int T = args.T, H = args.H;
   const int HD = H * FA_D;
@@ -267,7 +267,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(WS_REGS_LIGHT));
   if (warp == WS_LOADER_WARP) {
     // ------------------------------------------------------------------ loader
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t qc = 0, kc = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -305,7 +305,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     // probabilities are late does not hold back the other tile's next score tile), and the issue
     // work of a step (12 instructions per tile) is spread over two schedulers. Descriptors of a
     // tile are formed once; a step inside a tile only adds to the 14-bit address field.
-    if (lane == 0) {
+    if (elect_one()) {
       const int i = warp - WS_MMA_WARP;
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, 0, 1);
@@ -395,7 +395,6 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     const int w = args.window;
     uint32_t s_cnt = 0, pv_cnt = 0;
     bool ok = true;
-    const bool st_issuer = quarter == 0 && lane == 0;     // issues this warpgroup's output stores
     // geometry and key range of an item's rows are loaded one item ahead (a global load at an item
     // boundary cost 1 000 - 4 500 cycles inside this kernel)
     WsGeoRaw raw_n = ws_geo_load(args, blockIdx.x / H);
@@ -584,7 +583,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
       if constexpr (PTMEM) {
         // The output tile leaves through this warpgroup's 16 KB of the (otherwise unused) P area and one
         // TMA store: the warpgroup goes on to its next item while the copy engine writes the rows.
-        if (st_issuer && ok) tma_store_wait_read<0>();     // the previous item's store has read the tile
+        if (quarter == 0 && elect_one() && ok) tma_store_wait_read<0>();   // the previous item's store has read the tile
         ok = wg_barrier_and(1 + i, ok);                    // (a warp that gives up says so here)
         if (!ok) break;
         tc_fence_after();
@@ -607,7 +606,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         tc_fence_before();
         fence_proxy_async_smem();
         wg_barrier(1 + i);
-        if (st_issuer) {                                   // rows past the end of the batch are clipped
+        if (quarter == 0 && elect_one()) {                 // rows past the end of the batch are clipped
           tma_store_2d(&tmO, sPi, h * FA_D, g.t0 + i * FA_T);
           tma_store_commit();
         }
@@ -642,7 +641,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         args.lse[static_cast<size_t>(h) * T + row] = l_run > 0.f ? m_used * args.scale + __logf(l_run) : 0.f;
       WS_TRACE(quarter == 0, 1 + i, 5);
     }
-    if (PTMEM && st_issuer) tma_store_wait<0>();   // the stores are complete before the CTA gives up its shared memory
+    if (PTMEM && quarter == 0 && elect_one()) tma_store_wait<0>();   // the stores are complete before the CTA gives up its shared memory
     if (!ok && lane == 0 && *abort_flag == 0) {
       atomicExch(args.status, ST_TIMEOUT_TMEM_FULL);
       *abort_flag = 1;
@@ -813,7 +812,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   using Cfg = WsBwdCfg<NWG, DQ>;
   constexpr int CPT = Cfg::CPT;
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = warp_index();
   const int lane = tid & 31;
   const int T = args.T, H = args.H;
   const int HD = H * FA_D;
@@ -869,7 +868,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const bool issuer = warp == Cfg::DRAIN_WARP && lane == 0;
+    const bool issuer_warp = warp == Cfg::DRAIN_WARP;     // its elected thread issues the bulk copies
     uint32_t c_g = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -879,7 +878,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         ok = mbar_wait(g_done, c_g & 1u);
         ++c_g;
         // the previous tile's reduce-adds have finished reading the staging tile
-        if (issuer) tma_store_wait_read<0>();
+        if (issuer_warp && elect_one()) tma_store_wait_read<0>();
         // barrier over the warpgroup that also agrees on going on: all four warps leave together (a warp
         // that stayed behind would leave the others at the second barrier below for ever)
         ok = wg_barrier_and(1, ok && *abort_flag == 0);
@@ -905,7 +904,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         }
         fence_proxy_async_smem();
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (issuer) {
+        if (issuer_warp && elect_one()) {
           const int q0 = g.q_lo + j * FA_T;
           tma_reduce_add_2d(&tmDQ, sDQ, h * FA_D, q0);
           tma_reduce_add_2d(&tmDQ, sDQ + FA_TILE_BYTES, h * FA_D + 32, q0);
@@ -919,7 +918,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
       // at a time (channel e and its rotation partner e + 32), scaled and rotated back (dK), packed to
       // bf16 into the two halves of the staging area laid out as TMA boxes, then two TMA stores into
       // dqkv. The compute warpgroups are already working on the next item meanwhile.
-      if (issuer) tma_store_wait_read<0>();
+      if (issuer_warp && elect_one()) tma_store_wait_read<0>();
       asm volatile("bar.sync 1, 128;" ::: "memory");
       {
         const int krow = g.kv0 + r;
@@ -988,7 +987,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
       }
       fence_proxy_async_smem();
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (issuer) {
+      if (issuer_warp && elect_one()) {
         if constexpr (QST) {
           tma_store_2d(&tmOUT, sDQ, h * FA_D, g.kv0);
         } else {
@@ -998,7 +997,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         tma_store_commit();
       }
     }
-    if (issuer) tma_store_wait<0>();            // the adds are complete before the CTA gives up its shared memory
+    if (issuer_warp && elect_one()) tma_store_wait<0>();            // the adds are complete before the CTA gives up its shared memory
     if (!ok && lane == 0 && *abort_flag == 0) {
       atomicExch(args.status, ST_TIMEOUT_TMEM_FULL);
       *abort_flag = 1;
@@ -1007,7 +1006,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_LIGHT));   // all four warps of the warpgroup
   if (warp == Cfg::LOADER_WARP) {
     // ------------------------------------------------------------------ loader
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t ic = 0, qc = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++ic) {
@@ -1044,7 +1043,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         *abort_flag = 1;
       }
     }
-  } else if (lane == 0) {
+  } else if (elect_one()) {
     // ------------------------------------------------------------------ MMA issuers
     // Three issuing threads, one per kind of product, so that a step's 24 - 32 instructions do not
     // queue behind one thread: A issues S = Q K^T and dP = dO V^T of the NEXT step as soon as the

@@ -115,7 +115,7 @@ struct WorkItem {
 // columns beyond the tensor are clipped by the TMA unit.
 __device__ __forceinline__ void stage_store_bf16(uint8_t* stage, int& toggle, const CUtensorMap* tm,
                                                  const uint32_t (&packed)[32], int x, int y, int lane) {
-  if (lane == 0) tma_store_wait_read<1>();
+  if (elect_one()) tma_store_wait_read<1>();
   __syncwarp();
   uint8_t* buf = stage + toggle * 4096;
   toggle ^= 1;
@@ -126,7 +126,7 @@ __device__ __forceinline__ void stage_store_bf16(uint8_t* stage, int& toggle, co
   }
   fence_proxy_async_smem();
   __syncwarp();
-  if (lane == 0) {
+  if (elect_one()) {
     tma_store_2d(tm, buf, x, y);
     tma_store_commit();
   }
@@ -157,7 +157,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   const int M = args.M, N = args.N, K = args.K;
@@ -281,7 +281,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -393,7 +393,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && (!PAIR || rank == 0)) {
+    if ((!PAIR || rank == 0) && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(PAIR ? 2 * BM : BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       // arrive-on-completion of everything issued so far; in a pair both CTAs are notified
       auto commit = [&](uint64_t* bar) {
@@ -638,7 +638,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if constexpr (EPI == EPI_ADD) {
             // residual tile of chunk 0 (issued before the accumulator wait would be even better;
             // the tile is already in L2 in the encoder, where the residual is the block input)
-            if (lane == 0 && rows_in && n0 < N) {
+            if (rows_in && n0 < N && elect_one()) {
               tma_store_wait_read<0>();
               mbar_arrive_expect_tx(&res_bar[quarter * 2 + stage_toggle], 4096);
               tma_load_2d(stage + stage_toggle * 4096, &tmR, &res_bar[quarter * 2 + stage_toggle], n0, y0);
@@ -670,7 +670,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if constexpr (EPI == EPI_ADD) {
               const int buf = stage_toggle;
               // prefetch the residual of the next chunk into the other buffer
-              if (lane == 0 && rows_in && c + 1 < NCH && x + 64 < N) {
+              if (rows_in && c + 1 < NCH && x + 64 < N && elect_one()) {
                 tma_store_wait_read<0>();
                 mbar_arrive_expect_tx(&res_bar[quarter * 2 + (buf ^ 1)], 4096);
                 tma_load_2d(stage + (buf ^ 1) * 4096, &tmR, &res_bar[quarter * 2 + (buf ^ 1)], x + 64, y0);
@@ -706,7 +706,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {
+                if (elect_one()) {
                   tma_store_2d(&tmC, ob, x, y0);
                   tma_store_commit();
                 }
@@ -882,7 +882,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
     if constexpr (TMA_EPI) {
-      if (lane == 0) tma_store_wait<0>();
+      if (elect_one()) tma_store_wait<0>();
       __syncwarp();
     }
   }
