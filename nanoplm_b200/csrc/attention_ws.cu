@@ -805,7 +805,8 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   uint64_t* g_done = pds_ready + 1;                // dV, dK, dQ of a step have finished
   uint64_t* dq_free = g_done + 1;                  // the dQ tile has been read back
   uint64_t* acc_free = dq_free + 1;                // dK / dV of the previous item have been read back
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
+  uint64_t* item_done = acc_free + 1;              // the item's last products have finished (modes without DQ)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(item_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   constexpr bool DQ = MODE == BWD_KV_DQ, QST = MODE == BWD_Q;
@@ -833,6 +834,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     mbar_init(g_done, DQ ? 2 : 1);           // issuer B, and C when both run (query-stationary: C alone)
     mbar_init(dq_free, (Cfg::DRAIN_WG || QST) ? 4 : NWG * 4);   // the warps that read dQ back
     mbar_init(acc_free, Cfg::DRAIN_WG ? 4 : 8);   // the warps that read dK / dV back
+    mbar_init(item_done, 1);                      // issuer B (query-stationary: C)
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -874,6 +876,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const int h = item % H;
       const WsBwdGeo g = ws_bwd_geometry(args, item / H);
+      if constexpr (DQ) {
       for (int j = 0; j < g.n_q; ++j) {
         ok = mbar_wait(g_done, c_g & 1u);
         ++c_g;
@@ -884,7 +887,6 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         ok = wg_barrier_and(1, ok && *abort_flag == 0);
         if (!ok) break;
         tc_fence_after();
-        if constexpr (DQ) {
 #pragma unroll
         for (int hlf = 0; hlf < 2; ++hlf) {     // 32 channels at a time: this warpgroup runs on few registers
           uint32_t v[32];
@@ -910,7 +912,15 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
           tma_reduce_add_2d(&tmDQ, sDQ + FA_TILE_BYTES, h * FA_D + 32, q0);
           tma_store_commit();
         }
-        }
+      }
+      } else if (g.n_q > 0) {
+        // Without dQ nothing in a step waits for this warpgroup, so it may not follow g_done: two of its phases
+        // could pass unseen while the previous item is being stored. item_done completes once per item, and
+        // the next item's first product waits for this warpgroup (acc_free, dq_free).
+        ok = mbar_wait(item_done, c_g & 1u);
+        ++c_g;
+        ok = wg_barrier_and(1, ok && *abort_flag == 0);
+        tc_fence_after();
       }
       if (!ok) break;
       // ---- the item's dK and dV: the last products have finished (the wait above covered them). This
@@ -1113,6 +1123,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
           for (int k = 0; k < FA_T / 16; ++k)   // dK[kv][d] += dS^T[kv][q] Q[q][d]
             umma_bf16(tdK, dST + k * 128, dQ0 + k * 128, idesc_g, (j > 0 || k > 0) ? 1u : 0u);
           umma_commit(g_done);                 // with issuer C when dQ is formed here
+          if (!DQ && j == g.n_q - 1) umma_commit(item_done);
           umma_commit(&qdo_empty[st]);
           WS_TRACE(true, 3, 3);
         }
@@ -1160,6 +1171,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
           for (int k = 0; k < FA_T / 16; ++k)
             umma_bf16_ts(tdQ, tdS + k * 8, dKr + k * 128, idesc_dq, (j > 0 || k > 0) ? 1u : 0u);
           umma_commit(g_done);
+          if (j == g.n_q - 1) umma_commit(item_done);
           umma_commit(&qdo_empty[st]);     // with issuer A
         }
         if (!ok) break;
