@@ -13,8 +13,8 @@
 // Replaces the cuBLAS calls behind nn.Linear in the reference
 // (src/nanoplm/pretraining/models/modern_bert/modeling.py:281-302,340,366,559).
 //
-// Warp roles (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer,
-// warps 2..5 = epilogue (each owns the TMEM lane quarter warp_idx % 4).
+// Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2.. = epilogue (four, or eight
+// on CTA pairs; a warp reads the TMEM lane quarter warp_idx % 4, two of a quarter split the columns).
 #include "common.cuh"
 
 namespace nplm {
@@ -22,7 +22,6 @@ namespace nplm {
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int GEMM_THREADS = 192;
 
 enum : int {
   EPI_STORE = 0,       // C(bf16) = acc
@@ -47,15 +46,26 @@ enum : int {
 // of A and half of B, which cuts the L2 -> shared-memory traffic per FLOP by a third.
 // STAGED: the epilogue goes through shared memory (TMA stores); kernels that write straight from
 // registers (fp32 outputs, the direct epilogue) spend that room on one more pipeline stage.
-template <int BN, bool PAIR = false, bool STAGED = true>
+// Epilogue warps: one per TMEM lane quarter, or two that split the columns. A 128 x 256 tile with K = 1024
+// leaves the epilogue about 8 200 cycles. The forms that read a second operand or tables need more than that on
+// four warps: 55 424 rows, SwiGLU backward 356 -> 277 us, RoPE 322 -> 288, delta 120 -> 107 with eight. The
+// others fit, and lose more by the operand stage that eight warps' staging takes (SwiGLU 385 -> 405 us, store
+// 264 -> 275).
+template <bool PAIR, bool STAGED, int EPI>
+constexpr int EPI_WARPS_OF =
+    (PAIR && STAGED && (EPI == EPI_ROPE || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD)) ? 8 : 4;
+
+template <int BN, bool PAIR = false, bool STAGED = true, int EPI_WARPS_ = 4>
 struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = PAIR ? (STAGED ? 6 : 7) : ((BN == 256) ? 4 : (STAGED ? 6 : 7));
-  static constexpr int BAR_BYTES = 256;
-  // epilogue staging: 4 warps x 2 buffers x (32 rows x 128 B), written swizzled, read by TMA stores
-  static constexpr int EPI_BYTES = STAGED ? 4 * 2 * 4096 : 0;
+  static constexpr int STAGES = PAIR ? (STAGED ? (EPI_WARPS_ == 8 ? 5 : 6) : 7) : ((BN == 256) ? 4 : (STAGED ? 6 : 7));
+  static constexpr int BAR_BYTES = 512;
+  static constexpr int EPI_WARPS = EPI_WARPS_;
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  // epilogue staging: 2 buffers x (32 rows x 128 B) per warp, written swizzled, read by TMA stores
+  static constexpr int EPI_BYTES = STAGED ? EPI_WARPS * 2 * 4096 : 0;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + BAR_BYTES + 1024;  // + alignment slack
 };
 
@@ -132,12 +142,29 @@ __device__ __forceinline__ void stage_store_bf16(uint8_t* stage, int& toggle, co
   }
 }
 
+// Same, into the buffer that held this chunk's second operand (no other buffer is touched).
+__device__ __forceinline__ void stage_store_inplace(uint8_t* buf, const CUtensorMap* tm, const uint32_t (&packed)[32],
+                                                    int x, int y, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+        make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+  }
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (elect_one()) {
+    tma_store_2d(tm, buf, x, y);
+    tma_store_commit();
+  }
+}
+
 template <int BN, bool A_MN, bool B_MN, int EPI, bool TMA_EPI, bool PAIR = false>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(GemmSmem<BN, PAIR, TMA_EPI, EPI_WARPS_OF<PAIR, TMA_EPI, EPI>>::THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR,
                  const GemmArgs args) {
-  using S = GemmSmem<BN, PAIR, TMA_EPI>;
+  using S = GemmSmem<BN, PAIR, TMA_EPI, EPI_WARPS_OF<PAIR, TMA_EPI, EPI>>;
   // CTA pair: rank 0 issues the MMAs, both CTAs load operands and run their own epilogue
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
   const int work_first = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
@@ -153,8 +180,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* empty_bar = bars + STAGES;
   uint64_t* tfull_bar = bars + 2 * STAGES;
   uint64_t* tempty_bar = bars + 2 * STAGES + 2;
-  uint64_t* res_bar = bars + 2 * STAGES + 4;  // [4 warps][2 buffers], residual tiles (EPI_ADD)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 12);
+  uint64_t* res_bar = bars + 2 * STAGES + 4;  // [epilogue warps][2 buffers]: the epilogue's second operand
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + 2 * S::EPI_WARPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = warp_index();
@@ -240,9 +267,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], PAIR ? 8 : 4);   // epilogue warps of both CTAs release rank 0's accumulator
+      // the epilogue warps of both CTAs of a pair release rank 0's accumulator
+      mbar_init(&tempty_bar[a], (PAIR ? 2 : 1) * S::EPI_WARPS);
     }
-    for (int i = 0; i < 8; ++i) mbar_init(&res_bar[i], 1);
+    for (int i = 0; i < 2 * S::EPI_WARPS; ++i) mbar_init(&res_bar[i], 1);
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -485,11 +513,39 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     int acc = 0;
     uint32_t acc_phase = 0;
     int stage_toggle = 0;       // which of this warp's two staging buffers is next
-    uint32_t res_phase = 0;     // parity bits of this warp's two residual barriers
+    uint32_t res_phase = 0;     // parity bits of this warp's two operand barriers
+    const int ew = warp - 2;                        // 0 .. EPI_WARPS - 1
+    constexpr int NCHW = TILE_N / 64 / (S::EPI_WARPS / 4);   // 64-column chunks of a tile per warp
+    const int c0 = (ew >> 2) * NCHW, c1 = c0 + NCHW;
+    uint8_t* stage = epi_stage + ew * 8192;
+    // One thread copies a [32][64] tile of the epilogue's second operand (tmR) into a staging buffer, once the
+    // stores issued from this warp's buffers have read them. Called by the whole warp.
+    auto operand_load = [&](int buf, int x, int y) {
+      if (elect_one()) {
+        tma_store_wait_read<0>();
+        mbar_arrive_expect_tx(&res_bar[ew * 2 + buf], 4096);
+        tma_load_2d(stage + buf * 4096, &tmR, &res_bar[ew * 2 + buf], x, y);
+      }
+      __syncwarp();
+    };
+    auto operand_wait = [&](int buf) {
+      const bool got = mbar_wait(&res_bar[ew * 2 + buf], (res_phase >> buf) & 1u);
+      res_phase ^= 1u << buf;
+      return got;
+    };
     for (int w = w_begin; w < total_work; w += w_step) {
       WorkItem it;
       if (!decode(w, it)) continue;
       const int m0 = it.m0, n0 = it.n0;
+      if constexpr (TMA_EPI && (EPI == EPI_ADD || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD)) {
+        // the second operand does not depend on the product: its first tiles travel while the MMAs run
+        const int y0 = m0 + quarter * 32, x0 = n0 + c0 * 64;
+        if (y0 < M && x0 < N) {
+          operand_load(0, x0, y0);
+          if constexpr (EPI == EPI_SWIGLU_BWD) operand_load(1, N + x0, y0);
+          else if (NCHW > 1 && x0 + 64 < N) operand_load(1, x0 + 64, y0);
+        }
+      }
       if (!mbar_wait(&tfull_bar[acc], acc_phase)) {
         if (lane == 0) atomicExch(args.status, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
@@ -501,14 +557,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
 
       if constexpr (TMA_EPI) {
-        // ---- shared-memory staged epilogue, 64 output columns per step, one TMA store each
-        uint8_t* stage = epi_stage + quarter * 8192;
+        // ---- shared-memory staged epilogue, 64 output columns per step, one TMA store each. This warp's
+        // chunks are [c0, c1): all of the tile's with four warps, one half of them with eight.
         const int y0 = m0 + quarter * 32;
         const bool rows_in = y0 < M;
+        auto chunk_in = [&](int c) { return rows_in && n0 + c * 64 < n_extent; };
         if constexpr (EPI == EPI_SWIGLU) {
-          constexpr int NCH = BN / 2 / 64;
 #pragma unroll 1
-          for (int c = 0; c < NCH; ++c) {
+          for (int c = c0; c < c1; ++c) {
             uint32_t pv[32], pg[32], po[32];
 #pragma unroll
             for (int hlf = 0; hlf < 2; ++hlf) {
@@ -528,13 +584,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                                                gr.y / (1.0f + __expf(-gr.y)) * vr.y);
               }
             }
-            if (c == NCH - 1) {
+            if (c == c1 - 1) {
               tc_fence_before();
               __syncwarp();
               if (lane == 0) release_acc(acc);
             }
             const int x = n0 + c * 64;
-            if (rows_in && x < n_extent) {
+            if (chunk_in(c)) {
               stage_store_bf16(stage, stage_toggle, &tmC, po, x, y0, lane);
               if (args.R != nullptr) {
                 stage_store_bf16(stage, stage_toggle, &tmR, pv, x, y0, lane);
@@ -543,18 +599,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
           }
         } else if constexpr (EPI == EPI_STORE_DELTA) {
-          constexpr int NCH = BN / 64;
-          const __nv_bfloat16* orow = args.R + static_cast<size_t>(row_ok ? row : 0) * args.ldr;
 #pragma unroll 1
-          for (int c = 0; c < NCH; ++c) {
-            const int x = n0 + c * 64;
-            const bool active = rows_in && x < N;
-            uint4 ov[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ov[j] = make_uint4(0, 0, 0, 0);
-            if (active && row_ok) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) ov[j] = __ldg(reinterpret_cast<const uint4*>(orow + x) + j);
+          for (int c = c0; c < c1; ++c) {
+            const int x = n0 + c * 64, buf = (c - c0) & 1;
+            const bool active = chunk_in(c);
+            uint8_t* rb = stage + buf * 4096;
+            if (active && !operand_wait(buf)) {
+              if (lane == 0) atomicExch(args.status, ST_TIMEOUT_MISC);
             }
             uint32_t packed[32];
             float dot = 0.f;
@@ -563,90 +614,106 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               uint32_t d[32];
               tmem_ld32(taddr + c * 64 + hlf * 32, d);
               tmem_ld_wait();
-              if (c == NCH - 1 && hlf == 1) {
+              if (c == c1 - 1 && hlf == 1) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) release_acc(acc);
               }
 #pragma unroll
-              for (int e = 0; e < 16; ++e) {
-                const int q = hlf * 16 + e;
-                const uint32_t pk = pack_bf16x2(__uint_as_float(d[2 * e]), __uint_as_float(d[2 * e + 1]));
-                packed[q] = pk;
-                const float2 g2 = unpack_bf16x2(pk);
-                const float2 o2 = unpack_bf16x2(reinterpret_cast<const uint32_t*>(&ov[q >> 2])[q & 3]);
-                dot += g2.x * o2.x + g2.y * o2.y;
+              for (int j = 0; j < 4; ++j) {
+                const uint4 ov = *reinterpret_cast<const uint4*>(rb + lane * 128 + (((hlf * 4 + j) ^ (lane & 7)) << 4));
+                const uint32_t* ow = reinterpret_cast<const uint32_t*>(&ov);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const int e = j * 4 + u;
+                  const uint32_t pk = pack_bf16x2(__uint_as_float(d[2 * e]), __uint_as_float(d[2 * e + 1]));
+                  packed[hlf * 16 + e] = pk;
+                  const float2 g2 = unpack_bf16x2(pk);
+                  const float2 o2 = unpack_bf16x2(ow[u]);
+                  dot += g2.x * o2.x + g2.y * o2.y;
+                }
               }
             }
             if (active) {
-              stage_store_bf16(stage, stage_toggle, &tmC, packed, x, y0, lane);
+              stage_store_inplace(rb, &tmC, packed, x, y0, lane);
               if (row_ok) args.delta[static_cast<size_t>(x >> 6) * M + row] = dot;
+              if (c + 2 < c1 && chunk_in(c + 2)) operand_load(buf, x + 128, y0);
             }
           }
         } else if constexpr (EPI == EPI_SWIGLU_BWD) {
-          constexpr int NCH = BN / 64;
-          const __nv_bfloat16* prow = args.R + static_cast<size_t>(row_ok ? row : 0) * args.ldr;
 #pragma unroll 1
-          for (int c = 0; c < NCH; ++c) {
+          for (int c = c0; c < c1; ++c) {
             const int x = n0 + c * 64;
-            const bool active = rows_in && x < N;
-            // this lane's 64 value and 64 gate pre-activations: in flight while the accumulator loads
-            uint4 vv[8], gg[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              vv[j] = make_uint4(0, 0, 0, 0);
-              gg[j] = make_uint4(0, 0, 0, 0);
+            const bool active = chunk_in(c);
+            // buffer 0: this chunk's value pre-activations, buffer 1: its gates; overwritten by their gradients
+            if (active) {
+              const bool got0 = operand_wait(0), got1 = operand_wait(1);
+              if (!(got0 && got1) && lane == 0) atomicExch(args.status, ST_TIMEOUT_MISC);
             }
-            if (active && row_ok) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                vv[j] = __ldg(reinterpret_cast<const uint4*>(prow + x) + j);
-                gg[j] = __ldg(reinterpret_cast<const uint4*>(prow + N + x) + j);
-              }
-            }
-            uint32_t dvp[32], dgp[32];
 #pragma unroll
             for (int hlf = 0; hlf < 2; ++hlf) {
               uint32_t d[32];
               tmem_ld32(taddr + c * 64 + hlf * 32, d);
               tmem_ld_wait();
-              if (c == NCH - 1 && hlf == 1) {
+              if (c == c1 - 1 && hlf == 1) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) release_acc(acc);
               }
+              if (active) {
 #pragma unroll
-              for (int e = 0; e < 16; ++e) {
-                const int q = hlf * 16 + e;   // bf16 pair index inside the 64-column chunk
-                const uint32_t vraw = reinterpret_cast<const uint32_t*>(&vv[q >> 2])[q & 3];
-                const uint32_t graw = reinterpret_cast<const uint32_t*>(&gg[q >> 2])[q & 3];
-                const float2 v2 = unpack_bf16x2(vraw), g2 = unpack_bf16x2(graw);
-                const float d0 = __uint_as_float(d[2 * e]), d1 = __uint_as_float(d[2 * e + 1]);
-                const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
-                dvp[q] = pack_bf16x2(d0 * g2.x * s0, d1 * g2.y * s1);
-                dgp[q] = pack_bf16x2(d0 * v2.x * s0 * (1.f + g2.x * (1.f - s0)),
-                                     d1 * v2.y * s1 * (1.f + g2.y * (1.f - s1)));
+                for (int j = 0; j < 4; ++j) {
+                  uint4* vp = reinterpret_cast<uint4*>(stage + lane * 128 + (((hlf * 4 + j) ^ (lane & 7)) << 4));
+                  uint4* gp = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(vp) + 4096);
+                  uint4 vv = *vp, gg = *gp;
+                  uint32_t* vw = reinterpret_cast<uint32_t*>(&vv);
+                  uint32_t* gw = reinterpret_cast<uint32_t*>(&gg);
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) {
+                    const int e = j * 4 + u;
+                    const float2 v2 = unpack_bf16x2(vw[u]), g2 = unpack_bf16x2(gw[u]);
+                    const float d0 = __uint_as_float(d[2 * e]), d1 = __uint_as_float(d[2 * e + 1]);
+                    const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
+                    vw[u] = pack_bf16x2(d0 * g2.x * s0, d1 * g2.y * s1);
+                    gw[u] = pack_bf16x2(d0 * v2.x * s0 * (1.f + g2.x * (1.f - s0)),
+                                        d1 * v2.y * s1 * (1.f + g2.y * (1.f - s1)));
+                  }
+                  *vp = vv;
+                  *gp = gg;
+                }
               }
             }
             if (active) {
-              stage_store_bf16(stage, stage_toggle, &tmC, dvp, x, y0, lane);
-              stage_store_bf16(stage, stage_toggle, &tmC, dgp, N + x, y0, lane);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (elect_one()) {
+                tma_store_2d(&tmC, stage, x, y0);
+                tma_store_2d(&tmC, stage + 4096, N + x, y0);
+                tma_store_commit();
+              }
+              if (c + 1 < c1 && chunk_in(c + 1)) {
+                operand_load(0, x + 64, y0);
+                operand_load(1, N + x + 64, y0);
+              }
             }
           }
         } else {
-          constexpr int NCH = BN / 64;
-          if constexpr (EPI == EPI_ADD) {
-            // residual tile of chunk 0 (issued before the accumulator wait would be even better;
-            // the tile is already in L2 in the encoder, where the residual is the block input)
-            if (rows_in && n0 < N && elect_one()) {
-              tma_store_wait_read<0>();
-              mbar_arrive_expect_tx(&res_bar[quarter * 2 + stage_toggle], 4096);
-              tma_load_2d(stage + stage_toggle * 4096, &tmR, &res_bar[quarter * 2 + stage_toggle], n0, y0);
+          float rc[EPI == EPI_ROPE ? 32 : 1], rs[EPI == EPI_ROPE ? 32 : 1];
+          if constexpr (EPI == EPI_ROPE) {
+            // cos / sin of this lane's row, once per tile: all chunks (heads) of the tile use them
+            if (rows_in && n0 + c0 * 64 < args.rope_cols) {
+              const int pos = row_ok ? args.rope_pos[row] : 0;
+              const float4* cp = reinterpret_cast<const float4*>(args.rope_cos + static_cast<size_t>(pos) * 32);
+              const float4* sp = reinterpret_cast<const float4*>(args.rope_sin + static_cast<size_t>(pos) * 32);
+#pragma unroll
+              for (int q4 = 0; q4 < 8; ++q4) {
+                *reinterpret_cast<float4*>(rc + 4 * q4) = __ldg(cp + q4);
+                *reinterpret_cast<float4*>(rs + 4 * q4) = __ldg(sp + q4);
+              }
             }
-            __syncwarp();
           }
 #pragma unroll 1
-          for (int c = 0; c < NCH; ++c) {
+          for (int c = c0; c < c1; ++c) {
             uint32_t packed[32];
             float f[64];
             {
@@ -660,57 +727,32 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 f[32 + e] = __uint_as_float(r1[e]);
               }
             }
-            if (c == NCH - 1) {
+            if (c == c1 - 1) {
               tc_fence_before();
               __syncwarp();
               if (lane == 0) release_acc(acc);
             }
             const int x = n0 + c * 64;
-            const bool active = rows_in && x < N;
+            const bool active = chunk_in(c);
             if constexpr (EPI == EPI_ADD) {
-              const int buf = stage_toggle;
-              // prefetch the residual of the next chunk into the other buffer
-              if (rows_in && c + 1 < NCH && x + 64 < N && elect_one()) {
-                tma_store_wait_read<0>();
-                mbar_arrive_expect_tx(&res_bar[quarter * 2 + (buf ^ 1)], 4096);
-                tma_load_2d(stage + (buf ^ 1) * 4096, &tmR, &res_bar[quarter * 2 + (buf ^ 1)], x + 64, y0);
-              }
               if (active) {
-                const bool got = mbar_wait(&res_bar[quarter * 2 + buf], (res_phase >> buf) & 1u);
-                res_phase ^= (1u << buf);
-                if (!got) {
+                const int buf = (c - c0) & 1;
+                uint8_t* rb = stage + buf * 4096;
+                if (!operand_wait(buf)) {
                   if (lane == 0) atomicExch(args.status, ST_TIMEOUT_MISC);
-                } else {
-                  uint8_t* rb = stage + buf * 4096;
-#pragma unroll
-                  for (int j = 0; j < 8; ++j) {
-                    const uint4 rv = *reinterpret_cast<const uint4*>(rb + lane * 128 + ((j ^ (lane & 7)) << 4));
-                    const uint32_t* rr = reinterpret_cast<const uint32_t*>(&rv);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                      const float2 t = unpack_bf16x2(rr[e]);
-                      f[j * 8 + 2 * e] += t.x;
-                      f[j * 8 + 2 * e + 1] += t.y;
-                    }
-                  }
                 }
-#pragma unroll
-                for (int e = 0; e < 32; ++e) packed[e] = pack_bf16x2(f[2 * e], f[2 * e + 1]);
-                // in-place: the buffer that held the residual now holds the result
-                __syncwarp();
-                uint8_t* ob = stage + buf * 4096;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                  *reinterpret_cast<uint4*>(ob + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                      make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+                  const uint4 rv = *reinterpret_cast<const uint4*>(rb + lane * 128 + ((j ^ (lane & 7)) << 4));
+                  const uint32_t* rr = reinterpret_cast<const uint32_t*>(&rv);
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) {
+                    const float2 t = unpack_bf16x2(rr[e]);
+                    packed[j * 4 + e] = pack_bf16x2(f[j * 8 + 2 * e] + t.x, f[j * 8 + 2 * e + 1] + t.y);
+                  }
                 }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (elect_one()) {
-                  tma_store_2d(&tmC, ob, x, y0);
-                  tma_store_commit();
-                }
-                stage_toggle ^= 1;
+                stage_store_inplace(rb, &tmC, packed, x, y0, lane);
+                if (c + 2 < c1 && chunk_in(c + 2)) operand_load(buf, x + 128, y0);
               }
             } else if constexpr (EPI == EPI_GELU) {
               if (active) {
@@ -730,21 +772,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if constexpr (EPI == EPI_ROPE) {
                   if (x < args.rope_cols) {
                     // this thread holds one whole head (64 channels) of its row: rotate-half RoPE
-                    const int rr = y0 + lane;
-                    const int pos = rr < M ? args.rope_pos[rr] : 0;
-                    const float4* cp = reinterpret_cast<const float4*>(args.rope_cos + static_cast<size_t>(pos) * 32);
-                    const float4* sp = reinterpret_cast<const float4*>(args.rope_sin + static_cast<size_t>(pos) * 32);
 #pragma unroll
-                    for (int q4 = 0; q4 < 8; ++q4) {
-                      const float4 c4 = cp[q4], s4 = sp[q4];
-                      const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                      for (int u = 0; u < 4; ++u) {
-                        const int e = q4 * 4 + u;
-                        const float a = f[e], b = f[e + 32];
-                        f[e] = a * cc[u] - b * ss[u];
-                        f[e + 32] = b * cc[u] + a * ss[u];
-                      }
+                    for (int e = 0; e < 32; ++e) {
+                      const float a = f[e], b = f[e + 32];
+                      f[e] = a * rc[e] - b * rs[e];
+                      f[e + 32] = b * rc[e] + a * rs[e];
                     }
                   }
                 }
@@ -986,16 +1018,16 @@ static int launch_impl(const GemmMaps& maps, const GemmArgs& args, int max_ctas,
                       const_cast<CUtensorMap*>(&maps.C), const_cast<CUtensorMap*>(&maps.R),
                       const_cast<GemmArgs*>(&args)};
     return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(grid),
-                                                        dim3(GEMM_THREADS), params, S::TOTAL, stream));
+                                                        dim3(S::THREADS), params, S::TOTAL, stream));
   }
-  kern<<<grid, GEMM_THREADS, S::TOTAL, stream>>>(tmA, tmB, maps.C, maps.R, args);
+  kern<<<grid, S::THREADS, S::TOTAL, stream>>>(tmA, tmB, maps.C, maps.R, args);
   return static_cast<int>(cudaGetLastError());
 }
 
 // CTA-pair form (BN = 256 only): clusters of two CTAs, one 256 x 256 work item per cluster and step.
 template <bool A_MN, bool B_MN, int EPI, bool TMA_EPI>
 static int launch_pair_impl(const GemmMaps& maps, const GemmArgs& args, cudaStream_t stream) {
-  using S = GemmSmem<256, true, TMA_EPI>;
+  using S = GemmSmem<256, true, TMA_EPI, EPI_WARPS_OF<true, TMA_EPI, EPI>>;
   auto kern = gemm_bf16_kernel<256, A_MN, B_MN, EPI, TMA_EPI, true>;
   static bool configured_on[nplm::MAX_DEVICES];
   const int dev_slot = nplm::current_device_slot();
@@ -1016,7 +1048,7 @@ static int launch_pair_impl(const GemmMaps& maps, const GemmArgs& args, cudaStre
   if (pairs <= 0) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.blockDim = dim3(S::THREADS);
   cfg.dynamicSmemBytes = S::TOTAL;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -1031,7 +1063,7 @@ static int launch_pair_impl(const GemmMaps& maps, const GemmArgs& args, cudaStre
 
 template <bool A_MN, bool B_MN, int EPI>
 static int launch_pair(const GemmMaps& maps, const GemmArgs& args, cudaStream_t stream) {
-  if constexpr (EPI == EPI_ROPE) {
+  if constexpr (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD || EPI == EPI_STORE_DELTA) {
     return launch_pair_impl<A_MN, B_MN, EPI, true>(maps, args, stream);
   } else {
     if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_GELU || EPI == EPI_SWIGLU) {
@@ -1043,7 +1075,7 @@ static int launch_pair(const GemmMaps& maps, const GemmArgs& args, cudaStream_t 
 
 template <int BN, bool A_MN, bool B_MN, int EPI>
 static int launch(const GemmMaps& maps, const GemmArgs& args, int max_ctas, cudaStream_t stream) {
-  if constexpr (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD || EPI == EPI_STORE_DELTA) {
+  if constexpr (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD) {
     return launch_impl<BN, A_MN, B_MN, EPI, true>(maps, args, max_ctas, stream);
   } else {
     if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_GELU || EPI == EPI_SWIGLU) {
@@ -1124,7 +1156,7 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   const uint64_t b_rows_mnmajor = grp.mode == 1 ? static_cast<uint64_t>(grp.b_group_rows) * grp.groups : K;
 
   const bool pair = grp.pair && bn == 256 && grp.mode == 0 && grp.ag_world <= 1 && max_ctas == 0 &&
-                    !(a_mn && !b_mn) && epi != EPI_SWIGLU_BWD && epi != EPI_STORE_DELTA;
+                    !(a_mn && !b_mn);
   GemmMaps maps;
   CUtensorMap& tmA = maps.A;
   CUtensorMap& tmB = maps.B;
@@ -1152,9 +1184,9 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
     const int out_cols = epi == EPI_SWIGLU ? N / 2 : (epi == EPI_SWIGLU_BWD ? 2 * N : N);
     rc = make_map_2d(&maps.C, C, out_cols, M, ldc, 64, 32, 2);
     if (rc) return rc;
-    if (R != nullptr && epi != EPI_SWIGLU_BWD && epi != EPI_STORE_DELTA) {
+    if (R != nullptr) {
       if ((reinterpret_cast<uintptr_t>(R) & 15) || (ldr % 8)) return -3;
-      rc = make_map_2d(&maps.R, R, N, M, ldr, 64, 32, 2);
+      rc = make_map_2d(&maps.R, R, epi == EPI_SWIGLU_BWD ? 2 * N : N, M, ldr, 64, 32, 2);
       if (rc) return rc;
     }
   }
@@ -1235,6 +1267,12 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
       if (epi == EPI_SWIGLU) return launch_pair<false, false, EPI_SWIGLU>(maps, args, stream);
       return launch_pair<false, false, EPI_ROPE>(maps, args, stream);
     }
+    if (epi == EPI_STORE_DELTA)
+      return b_mn ? launch_pair<false, true, EPI_STORE_DELTA>(maps, args, stream)
+                  : launch_pair<false, false, EPI_STORE_DELTA>(maps, args, stream);
+    if (epi == EPI_SWIGLU_BWD)
+      return b_mn ? launch_pair<false, true, EPI_SWIGLU_BWD>(maps, args, stream)
+                  : launch_pair<false, false, EPI_SWIGLU_BWD>(maps, args, stream);
     if (!a_mn && !b_mn) { NPLM_DISPATCH_PAIR(false, false) }
     else if (!a_mn && b_mn) { NPLM_DISPATCH_PAIR(false, true) }
     else { NPLM_DISPATCH_PAIR(true, true) }
@@ -1254,10 +1292,6 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   if (epi == EPI_ROPE) {
     if (bn == 256) return launch<256, false, false, EPI_ROPE>(maps, args, max_ctas, stream);
     return launch<128, false, false, EPI_ROPE>(maps, args, max_ctas, stream);
-  }
-  if (epi == EPI_STORE_DELTA) {
-    if (b_mn) return launch<256, false, true, EPI_STORE_DELTA>(maps, args, max_ctas, stream);
-    return launch<256, false, false, EPI_STORE_DELTA>(maps, args, max_ctas, stream);
   }
   if (epi == EPI_SWIGLU_BWD) {
     if (bn != 256) return -6;
@@ -1307,6 +1341,7 @@ extern "C" int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const
                                     int N, int K, int lda, int ldb, int ldc, int ldr, int b_mn, int* status,
                                     cudaStream_t stream) {
   GroupSpec g;
+  g.pair = true;
   g.delta = delta;
   return gemm_entry(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, 0, b_mn, EPI_STORE_DELTA, 1, 256, 0, 0, nullptr,
                     nullptr, nullptr, 0, status, stream, g);
