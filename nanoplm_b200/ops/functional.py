@@ -49,19 +49,15 @@ def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
     T, N = dy2.shape
     Kd = x2.shape[1]
     if N % 64 == 0 and Kd % 64 == 0:
-        # pair=None: single-CTA tiles unless K.set_gemm_pair_default(True). In isolation the CTA-pair
-        # form is within +-5 % of them on these shapes; inside a training step both run at the rate
-        # the power cap allows.
-        pair = None
         if _has_main_grad(w):
             K.gemm(dy2, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=w.main_grad,
-                   splits=K.wgrad_splits(N, Kd, T), pair=pair)
+                   splits=K.wgrad_splits(N, Kd, T))
             if _WGRAD_READY[0] is not None:
                 _WGRAD_READY[0](w)
             return None
         acc = torch.zeros((N, Kd), dtype=torch.float32, device=w.device)
         K.gemm(dy2, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=acc,
-               splits=K.wgrad_splits(N, Kd, T), pair=pair)
+               splits=K.wgrad_splits(N, Kd, T))
         return acc.to(w.dtype)
     if Kd % 64 == 0 and N < 256 and dy2.is_cuda and dy2.dtype == BF and x2.dtype == BF:
         # narrow outputs (the 2n + n^2 coefficient projection of a hyper-connection site, a router):
@@ -92,7 +88,7 @@ def _param_grad(p, g32: torch.Tensor):
 # ------------------------------------------------------------------------------------- linear
 class _LinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, bias, residual, act, rope=None):
+    def forward(ctx, x, w, bias, residual, act, rope=None, train=True):
         x2 = x.reshape(-1, x.shape[-1])
         if not (x2.stride(1) == 1 and x2.stride(0) % 8 == 0):
             x2 = x2.contiguous()
@@ -100,13 +96,15 @@ class _LinearFn(torch.autograd.Function):
         if rope is not None:
             y = K.gemm(x2, w, epi=K.EPI_ROPE, rope=rope)
         elif act in ("gelu", "relu"):
-            # the pre-activation is only kept when a backward pass will need it
-            need_pre = ctx.needs_input_grad[0] or ctx.needs_input_grad[1]
+            # the pre-activation is only kept when a backward pass will need it (`needs_input_grad` says what
+            # requires a gradient, also where gradients are off: `train` carries the mode of the caller)
+            need_pre = train and (ctx.needs_input_grad[0] or ctx.needs_input_grad[1])
             pre = torch.empty((x2.shape[0], w.shape[0]), dtype=BF, device=x.device) if need_pre else None
             y = K.gemm(x2, w, epi=K.EPI_GELU if act == "gelu" else K.EPI_RELU, aux=pre)
         elif act == "swiglu":
-            pre = torch.empty((x2.shape[0], w.shape[0]), dtype=BF, device=x.device)
-            y = K.gemm(x2, w, epi=K.EPI_SWIGLU, aux=pre, pair=True)   # CTA pairs: +4 % in isolation
+            if train:
+                pre = torch.empty((x2.shape[0], w.shape[0]), dtype=BF, device=x.device)
+            y = K.gemm(x2, w, epi=K.EPI_SWIGLU, aux=pre)
         elif residual is not None:
             y = K.gemm(x2, w, epi=K.EPI_ADD, aux=residual.reshape(-1, w.shape[0]))
         else:
@@ -141,7 +139,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = _param_grad(ctx.bias_ref, dpre.float().sum(0))
         dres = dy if ctx.has_res else None
-        return dx, dw, db, dres, None, None
+        return dx, dw, db, dres, None, None, None
 
 
 class _SwiGLUMLPFn(torch.autograd.Function):
@@ -150,12 +148,12 @@ class _SwiGLUMLPFn(torch.autograd.Function):
     of the GEMM that produces dL/dh (no separate SwiGLU-backward pass over [T, 3I] elements)."""
 
     @staticmethod
-    def forward(ctx, x, w_in, w_out, residual):
+    def forward(ctx, x, w_in, w_out, residual, train):
         x2 = x.reshape(-1, x.shape[-1])
         if not (x2.stride(1) == 1 and x2.stride(0) % 8 == 0):
             x2 = x2.contiguous()
-        pre = torch.empty((x2.shape[0], w_in.shape[0]), dtype=BF, device=x.device)
-        h = K.gemm(x2, w_in, epi=K.EPI_SWIGLU, aux=pre, pair=True)
+        pre = torch.empty((x2.shape[0], w_in.shape[0]), dtype=BF, device=x.device) if train else None
+        h = K.gemm(x2, w_in, epi=K.EPI_SWIGLU, aux=pre)
         if residual is not None:
             y = K.gemm(h, w_out, epi=K.EPI_ADD, aux=residual.reshape(-1, w_out.shape[0]))
         else:
@@ -175,7 +173,7 @@ class _SwiGLUMLPFn(torch.autograd.Function):
         dw_out = _wgrad(dy2, h, w_out) if ctx.needs_input_grad[2] else None
         dw_in = _wgrad(dpre, x2, w_in) if ctx.needs_input_grad[1] else None
         dx = _as_shape(K.gemm(dpre, w_in, b_mn=True), ctx.x_shape) if ctx.needs_input_grad[0] else None
-        return dx, dw_in, dw_out, (dy if ctx.has_res else None)
+        return dx, dw_in, dw_out, (dy if ctx.has_res else None), None
 
 
 def mlp_swiglu(x, w_in, w_out, residual=None):
@@ -184,7 +182,7 @@ def mlp_swiglu(x, w_in, w_out, residual=None):
     inter = w_out.shape[1]
     if (x.is_cuda and x.dtype == BF and not _FP8_STATE["enabled"] and inter % 64 == 0 and w_in.shape[0] == 2 * inter
             and w_in.shape[1] % 64 == 0 and w_out.shape[0] % 64 == 0):
-        return _SwiGLUMLPFn.apply(x, w_in, w_out, residual)
+        return _SwiGLUMLPFn.apply(x, w_in, w_out, residual, torch.is_grad_enabled())
     return linear(linear(x, w_in, act="swiglu"), w_out, residual=residual)
 
 
@@ -228,7 +226,7 @@ def linear(x, w, bias=None, residual=None, act: str | None = None):
             if act == "swiglu" and bias is not None:
                 y = _LinearFn.apply(x, w, bias, None, None)
                 return swiglu(y)
-            return _LinearFn.apply(x, w, bias, residual, act)
+            return _LinearFn.apply(x, w, bias, residual, act, None, torch.is_grad_enabled())
     y = F.linear(x, w, bias)
     if act == "gelu":
         y = F.gelu(y)
