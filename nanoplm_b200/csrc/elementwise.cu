@@ -1084,6 +1084,54 @@ extern "C" int nplm_act_bwd(const void* pre, const void* dout, void* dpre, long 
   return static_cast<int>(cudaGetLastError());
 }
 
+// out[b][c] = mean over rows cu[b] .. cu[b + 1] - drop_last of x[row][c] (bf16 in, fp32 sums and result; no rows: NaN,
+// as an empty mean is). A block takes 64 channels of one sequence: 8 threads cover a 128-byte line of a row, 32
+// row groups walk the sequence, so one protein still fills C / 64 blocks. Bound by reading x once (2 C bytes a
+// token); what it replaces is a reduction, a count and two copies per sequence (13.5 + 3.5 + 3.2 + 2.9 us each
+// and as many launches and host synchronisations).
+namespace nplm {
+__global__ void __launch_bounds__(256)
+segment_mean_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ cu, float* __restrict__ out,
+                    int C, int drop_last) {
+  __shared__ float part[32][64];
+  const int b = blockIdx.x, g = threadIdx.x >> 3, l = threadIdx.x & 7;
+  const int c = blockIdx.y * 64 + l * 8;
+  const int lo = cu[b], hi = cu[b + 1] - drop_last;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (c < C) {
+    for (int r = lo + g; r < hi; r += 32) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * C + c));
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&u);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 t = unpack_bf16x2(w[e]);
+        acc[2 * e] += t.x;
+        acc[2 * e + 1] += t.y;
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) part[g][l * 8 + e] = acc[e];
+  __syncthreads();
+  const int col = blockIdx.y * 64 + threadIdx.x;
+  if (threadIdx.x < 64 && col < C) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) s += part[i][threadIdx.x];
+    out[static_cast<size_t>(b) * C + col] = s / static_cast<float>(max(hi - lo, 0));
+  }
+}
+}  // namespace nplm
+
+extern "C" int nplm_segment_mean(const void* x, const int* cu, float* out, int B, int C, int drop_last,
+                                 cudaStream_t st) {
+  if (B <= 0) return 0;
+  if ((C % 8) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
+  nplm::segment_mean_kernel<<<dim3(B, (C + 63) / 64), 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x), cu, out,
+                                                                    C, drop_last);
+  return static_cast<int>(cudaGetLastError());
+}
+
 extern "C" int nplm_gather_rows(const void* src, const int* idx, void* dst, int n, int C,
                                 cudaStream_t st) {
   if (n <= 0) return 0;

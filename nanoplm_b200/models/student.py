@@ -7,6 +7,7 @@ from __future__ import annotations
 from pathlib import Path
 from typing import Optional
 
+import numpy as np
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -15,6 +16,7 @@ from nanoplm_b200.config.schema import StudentConfig
 from nanoplm_b200.data.tokenizer import StudentTokenizer
 from nanoplm_b200.models.encoder import (BatchContext, EncoderModel, Linear, Norm,
                                          position_ids_from_cu_seqlens)
+from nanoplm_b200.ops import kernels as K
 
 
 class ProtX(EncoderModel):
@@ -96,6 +98,32 @@ class ProtX(EncoderModel):
         groups["total"] = sum(groups.values())
         return groups
 
+    def _embeds_packed(self, device: torch.device) -> bool:
+        """Whether embed_sequences may hand the model flat ids: bf16 on a GPU, and nothing that observes the padded
+        call (a forward of a subclass, hooks on this module)."""
+        w = self.final_norm.weight
+        return (device.type == "cuda" and w.dtype == torch.bfloat16 and w.shape[0] % 8 == 0
+                and type(self).forward is ProtX.forward and not self._forward_hooks and not self._forward_pre_hooks)
+
+    def _embed_packed(self, ids: torch.Tensor, mask: torch.Tensor, device):
+        """(hidden states [T, C] of the real tokens, device cu_seqlens, host lengths) of a padded host batch. The
+        padding is dropped on the host, where the lengths are known: ids, positions and offsets go over in one
+        copy from pinned memory and nothing waits for the device."""
+        lens = mask.sum(dim=1).numpy()
+        T, B = int(lens.sum()), len(lens)
+        Tp = (T + 3) // 4 * 4                                  # every part starts on 16 bytes
+        host = torch.empty(2 * Tp + B + 1, dtype=torch.int32, pin_memory=True)
+        buf = host.numpy()
+        cu = np.zeros(B + 1, np.int32)
+        np.cumsum(lens, out=cu[1:])
+        buf[:T] = ids.numpy()[mask.numpy().astype(bool)]
+        buf[Tp:Tp + T] = np.arange(T, dtype=np.int32) - np.repeat(cu[:-1], lens)
+        buf[2 * Tp:] = cu
+        dev = host.to(device, non_blocking=True)
+        cu_dev = dev[2 * Tp:]
+        h = self(dev[:T], cu_seqlens=cu_dev, position_ids=dev[Tp:Tp + T])["last_hidden_state"]
+        return h, cu_dev, lens.tolist()
+
     @torch.no_grad()
     def embed_sequences(self, sequences: list[str], batch_size: int = 16, per_token: bool = False,
                         device: Optional[torch.device] = None) -> list[torch.Tensor]:
@@ -103,14 +131,45 @@ class ProtX(EncoderModel):
         device = device or next(self.parameters()).device
         was_training = self.training
         self.eval()
-        out = []
+        packed = self._embeds_packed(torch.device(device))
+        out, waiting, rows = [], [], 0
+
+        def collect():
+            """One copy to the host for all results that wait on the device; every sequence gets its own tensor."""
+            nonlocal rows
+            if waiting:
+                host = torch.cat([t for t, _ in waiting]).cpu()
+                lens = [n for _, ns in waiting for n in ns]
+                for part in host.split(lens):
+                    out.append(part.float() if per_token else part[0].clone())
+                waiting.clear()
+                rows = 0
+
         for i in range(0, len(sequences), batch_size):
             enc = self.tokenizer(sequences[i:i + batch_size], padding=True, return_tensors="pt")
-            ids, mask = enc["input_ids"].to(device), enc["attention_mask"].to(device)
+            ids, mask = enc["input_ids"], enc["attention_mask"]
+            # the real tokens first, at least one, then padding
+            if (packed and not ids.is_cuda and bool(mask[:, 0].all())
+                    and bool((mask[:, :-1] >= mask[:, 1:]).all())):
+                h, cu, lens = self._embed_packed(ids, mask, device)
+                if per_token:       # the residues' rows, without the trailing </s> of every sequence
+                    keep = torch.cat([torch.arange(e - n, e - 1) for n, e in zip(lens, np.cumsum(lens).tolist())])
+                    h = h[keep.to(device)]
+                    waiting.append((h, [n - 1 for n in lens]))
+                else:
+                    h = K.segment_mean(h, cu, drop_last=1)
+                    waiting.append((h, [1] * len(lens)))
+                rows += h.shape[0]
+                if rows >= 65536:   # bounds what waits on the device
+                    collect()
+                continue
+            collect()
+            ids, mask = ids.to(device), mask.to(device)
             h = self(ids, mask)["last_hidden_state"].float()
             for b in range(ids.shape[0]):
                 n = int(mask[b].sum()) - 1          # drop the trailing </s>
                 out.append(h[b, :n].cpu() if per_token else h[b, :n].mean(0).cpu())
+        collect()
         self.train(was_training)
         return out
 

@@ -326,6 +326,21 @@ def scatter_rows_(dst: torch.Tensor, idx: torch.Tensor, src: torch.Tensor) -> to
     return dst
 
 
+def segment_mean(x: torch.Tensor, cu: torch.Tensor, drop_last: int = 0) -> torch.Tensor:
+    """fp32 [B, C]: mean of x's rows cu[b] .. cu[b + 1] - drop_last (x bf16 [T, C] contiguous, cu int32 [B + 1])."""
+    _chk(x, _BF16, "x")
+    _chk(cu, torch.int32, "cu")
+    if x.dim() != 2 or not x.is_contiguous() or not cu.is_contiguous():
+        raise ValueError("x must be a contiguous [T, C] tensor and cu contiguous")
+    B, C = cu.numel() - 1, x.shape[1]
+    out = torch.empty((B, C), dtype=torch.float32, device=x.device)
+    rc = lib("elementwise").nplm_segment_mean(ptr(x), ptr(cu), ptr(out), c_int(B), c_int(C), c_int(int(drop_last)),
+                                              stream_ptr())
+    check_rc(rc, "segment_mean")
+    count_launch()
+    return out
+
+
 # --------------------------------------------------------------------------- cross entropy
 def ce_fwd(h, W, bias, labels, inv_count, want_logits=False):
     n, C = h.shape
