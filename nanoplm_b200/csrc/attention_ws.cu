@@ -87,27 +87,11 @@ constexpr int WS_FWD_SMEM = WS_OFF_BAR + 512;
 
 // Key-tile geometry of one work item: query tiles i = 0, 1 cover tokens [t0 + 128 i, +128); the
 // item walks key tiles j = 0 .. n-1 starting at kv_lo, and tile i takes part in j in [a[i], b[i]).
-// three-input maximum and packed two-lane fp32 arithmetic (sm_100): half the instructions of the
-// scalar forms in the softmax loops
+// three-input maximum (sm_100): half the instructions of the scalar form in the softmax loops
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(d)
-      : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)),
-        "l"(*reinterpret_cast<uint64_t*>(&c)));
-  return *reinterpret_cast<float2*>(&d);
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;"
-      : "=l"(d)
-      : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
-  return *reinterpret_cast<float2*>(&d);
 }
 
 // Named barrier `id` over 128 threads (one warpgroup) with an AND over everybody's predicate: the

@@ -11,8 +11,8 @@
 // scale[kb * row_blocks + r / 128] for block-scaled ones (128 x 128). value = q * scale.
 //
 // GEMM. C[M,N] (+)= sum_kb (A_kb * sa[.,kb]) (B_kb * sb[.,kb])^T. One pipeline stage holds one
-// 128-wide K block of A (128 rows) and B (128 rows) as 128-byte swizzled rows; the MMA warp issues
-// four kind::f8f6f4 UMMAs (K = 32 each) per stage into one of four TMEM buffers and the eight
+// 128-wide K block of A (128 rows) and B (256 or 128 rows) as 128-byte swizzled rows; the MMA warp issues
+// four kind::f8f6f4 UMMAs (K = 32 each) per stage into one of the TMEM buffers and the eight
 // epilogue warps read each partial product, multiply by the scales of that K block and add it to
 // fp32 registers ("promotion"), so the scales never have to be folded into 8-bit data.
 #include <cuda_fp8.h>
@@ -165,21 +165,117 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, ui
   }
 }
 
+// ------------------------------------------------------------------ both forms of an operand in one pass
+// x bf16 [R][K] (R, K multiples of 128) -> what quant_rows_kernel and quant_tile_kernel<true, false> give, bit for
+// bit: qr [R][K] with scales sr[(k/128) * R + r], qt [K][R] with scales st[(r/128) * K + k]. Bound by memory: 2
+// bytes read and 2 written an element, against 6 for the two kernels. A warp holds 16 rows x 128 columns of
+// the tile in registers (a lane four columns, so a row is one 256-byte request): row maxima by warp reduction, column
+// maxima through shared memory; the transposed bytes cross the block in shared memory (16-byte chunks swizzled so that
+// neither side conflicts) and leave as whole 128-byte lines.
+__global__ void __launch_bounds__(256)
+quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, uint8_t* __restrict__ qr,
+                  float* __restrict__ sr, uint8_t* __restrict__ qt, float* __restrict__ st) {
+  __shared__ __align__(16) uint8_t tile[128 * 128];
+  __shared__ float cmax[8][128];
+  const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  uint2 v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    v[i] = __ldg(reinterpret_cast<const uint2*>(x + static_cast<size_t>(r0 + w * 16 + i) * ldx + k0 + 4 * l));
+  float cm[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float2 a = unpack_bf16x2(v[i].x), b = unpack_bf16x2(v[i].y);
+    const float m[4] = {fabsf(a.x), fabsf(a.y), fabsf(b.x), fabsf(b.y)};
+    float rm = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      cm[j] = fmaxf(cm[j], m[j]);
+      rm = fmaxf(rm, m[j]);
+    }
+    // magnitudes order like their bit patterns
+    rm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rm)));
+    const float s = fmaxf(rm, 1e-12f) / E4M3_MAX;
+    const float inv = 1.f / s;
+    *reinterpret_cast<uint32_t*>(qr + static_cast<size_t>(r0 + w * 16 + i) * K + k0 + 4 * l) =
+        pack_e4m3x4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
+    if (l == i) sr[static_cast<size_t>(blockIdx.x) * R + r0 + w * 16 + i] = s;
+  }
+  *reinterpret_cast<float4*>(&cmax[w][4 * l]) = make_float4(cm[0], cm[1], cm[2], cm[3]);
+  __syncthreads();
+  if (threadIdx.x < 128) {
+    float m = cmax[0][threadIdx.x];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) m = fmaxf(m, cmax[j][threadIdx.x]);
+    const float s = fmaxf(m, 1e-12f) / E4M3_MAX;
+    cmax[0][threadIdx.x] = s;
+    st[static_cast<size_t>(blockIdx.y) * K + k0 + threadIdx.x] = s;
+  }
+  __syncthreads();
+  const float4 s4 = *reinterpret_cast<const float4*>(&cmax[0][4 * l]);
+  const float ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t pk[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float f[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 t = unpack_bf16x2(j < 2 ? v[q * 4 + u].x : v[q * 4 + u].y);
+        f[u] = ((j & 1) ? t.y : t.x) / ss[j];
+      }
+      pk[q] = pack_e4m3x4(f[0], f[1], f[2], f[3]);
+    }
+    *reinterpret_cast<uint4*>(tile + (4 * l + j) * 128 + ((w ^ (l & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = threadIdx.x; i < 128 * 8; i += 256) {
+    const int col = i >> 3, c = i & 7;
+    *reinterpret_cast<uint4*>(qt + static_cast<size_t>(k0 + col) * R + r0 + c * 16) =
+        *reinterpret_cast<const uint4*>(tile + col * 128 + ((c ^ ((col >> 2) & 7)) << 4));
+  }
+}
+
 // ------------------------------------------------------------------ GEMM
-constexpr int F8_BM = 128, F8_BN = 128, F8_BK = 128;  // BK in elements = bytes
-constexpr int F8_STAGES = 6;
-constexpr int F8_ACC = 4;  // TMEM partial-product buffers (4 x 128 columns = all of TMEM)
-constexpr int F8_STAGE_BYTES = (F8_BM + F8_BN) * F8_BK;  // 32 KB
-constexpr int F8_THREADS = 320;  // TMA warp, MMA warp, 8 epilogue warps (2 per TMEM lane quarter)
-constexpr int F8_SMEM = F8_STAGES * F8_STAGE_BYTES + 256 + 1024;
+constexpr int F8_BM = 128, F8_BK = 128;  // BK in elements = bytes
+// Warpgroup 0: TMA warp, MMA warp, two idle warps, 40 registers a thread. Warpgroups 1 and 2: 8 epilogue warps (2 per
+// TMEM lane quarter), which hold 128 sums a thread: at the 168 registers an even split gives they spilled inside
+// the promotion loop (6 100 cycles per K block of a weight gradient instead of under 1 000).
+constexpr int F8_THREADS = 384;
+constexpr int F8_REGS_LAUNCH = 168, F8_REGS_LIGHT = 40, F8_REGS_HEAVY = 232;
+static_assert(128 * F8_REGS_LIGHT + 256 * F8_REGS_HEAVY <= F8_THREADS * F8_REGS_LAUNCH,
+              "setmaxnreg.inc would wait forever for registers the CTA does not own");
+
+// 256-wide tiles: a K block is 512 cycles of MMAs, and every epilogue warp has those 512 cycles for its 128
+// columns (128 packed multiply-adds or 256, plus the TMEM reads), so the promotion of one block hides behind the
+// products of the next (two TMEM buffers). 128-wide tiles load 4/3 of the bytes per FLOP and were bound by that
+// and by the serial wait -> read -> add -> release chain. They remain for narrow outputs and for weight shards
+// that do not hold whole 256-row tiles.
+template <int BN>
+struct F8Cfg {
+  static constexpr int ACC = 512 / BN;                             // TMEM partial-product buffers (all of TMEM)
+  static constexpr int STAGE_BYTES = (F8_BM + BN) * F8_BK;
+  static constexpr int STAGES = BN == 256 ? 3 : 5;
+  static constexpr int HC = BN / 2;                                // columns per epilogue thread
+  // 8 warps x 2 output tiles of 32 rows x 128 B. The CTAs finish their tiles together and their stores leave at the
+  // rate L2 takes them; with the whole bf16 tile staged the warps go on to the next one meanwhile (K = 1024: the
+  // stores took 4 200 of 13 600 cycles a tile with half of that and a fourth operand stage)
+  static constexpr int OFF_EPI = STAGES * STAGE_BYTES;
+  static constexpr int OFF_SB = OFF_EPI + 8 * 8192;                // [2][BN] scales of B (row-scaled form)
+  static constexpr int OFF_BAR = OFF_SB + 2 * BN * 4;
+  static constexpr int SMEM = OFF_BAR + 256;
+};
 
 struct Fp8Args {
-  void* C;
   const float* sa;   // [KB][M]
   const float* sb;   // [KB][N] (b_block == 0) or [KB][ceil(N/128)] (b_block == 1)
   int M, N, K, ldc;
   int b_block;
-  int out_mode;      // 0: bf16 store, 1: fp32 store, 2: fp32 atomic add
+  int out_mode;      // 0: bf16 store, 1: fp32 store, 2: fp32 reduce-add (all through tmC)
+  int splits;        // out_mode 2: the K blocks of a tile are cut into this many work items
   int* status;
   // All-gather mode (ag_world > 1, block-scaled B only): B's rows and the matching scale columns
   // are sharded over the ranks. The epilogue warps of all CTAs first copy the other ranks' e4m3
@@ -203,45 +299,58 @@ __device__ __forceinline__ bool f8_wait_shard(const Fp8Args& args, int shard, un
   return true;
 }
 
+template <int BN, bool B_BLOCK>
 __global__ void __launch_bounds__(F8_THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const Fp8Args args) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + F8_STAGES * F8_STAGE_BYTES);
+                const __grid_constant__ CUtensorMap tmC, const Fp8Args args) {
+  using C8 = F8Cfg<BN>;
+  constexpr int STAGES = C8::STAGES, ACC = C8::ACC, HC = C8::HC;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1024-byte aligned base
+    if (threadIdx.x == 0) atomicExch(args.status, ST_BAD_ARG);
+    return;
+  }
+  float* sb_tile = reinterpret_cast<float*>(smem + C8::OFF_SB);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C8::OFF_BAR);
   uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + F8_STAGES;
-  uint64_t* tfull_bar = bars + 2 * F8_STAGES;
-  uint64_t* tempty_bar = bars + 2 * F8_STAGES + F8_ACC;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * F8_STAGES + 2 * F8_ACC);
+  uint64_t* empty_bar = bars + STAGES;
+  uint64_t* tfull_bar = bars + 2 * STAGES;
+  uint64_t* tempty_bar = bars + 2 * STAGES + ACC;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * ACC);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int M = args.M, N = args.N;
-  const int num_m = (M + F8_BM - 1) / F8_BM, num_n = (N + F8_BN - 1) / F8_BN;
+  const int num_m = (M + F8_BM - 1) / F8_BM, num_n = (N + BN - 1) / BN;
   const int KB = args.K / F8_BK;
-  const int total = num_m * num_n;
-  // work item -> tile origin (all-gather mode: shard by shard, the local one first)
-  auto tile_of = [&](int w, int& m0, int& n0) {
+  const int n_blocks = (N + 127) / 128;      // columns of a block-scaled B's scale table
+  const int kb_per = (KB + args.splits - 1) / args.splits;
+  const int total = num_m * num_n * args.splits;
+  // work item -> tile origin and K blocks (all-gather mode: shard by shard, the local one first). Tiles run
+  // fastest: the items of one wave walk the same K blocks and share operand panels through L2
+  auto tile_of = [&](int w, int& m0, int& n0, int& kb0, int& kb1) {
+    const int tiles = num_m * num_n;
+    const int split = w / tiles, t = w % tiles;
+    kb0 = split * kb_per;
+    kb1 = min(KB, kb0 + kb_per);
     if (args.ag_world > 1) {
-      const int n_per = args.ag_rows / F8_BN;
+      const int n_per = args.ag_rows / BN;
       const int per_shard = num_m * n_per;
-      const int shard = (args.ag_rank + w / per_shard) % args.ag_world;
-      const int rem = w % per_shard;
+      const int shard = (args.ag_rank + t / per_shard) % args.ag_world;
+      const int rem = t % per_shard;
       m0 = (rem / n_per) * F8_BM;
-      n0 = shard * args.ag_rows + (rem % n_per) * F8_BN;
+      n0 = shard * args.ag_rows + (rem % n_per) * BN;
     } else {
-      m0 = (w / num_n) * F8_BM;
-      n0 = (w % num_n) * F8_BN;
+      m0 = (t / num_n) * F8_BM;
+      n0 = (t % num_n) * BN;
     }
   };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < F8_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
-    for (int a = 0; a < F8_ACC; ++a) {
+    for (int a = 0; a < ACC; ++a) {
       mbar_init(&tfull_bar[a], 1);
       mbar_init(&tempty_bar[a], 8);
     }
@@ -249,9 +358,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     fence_proxy_async_smem();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+    tma_prefetch_desc(&tmC);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, F8_ACC * F8_BN);
+    tmem_alloc(tmem_slot, ACC * BN);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -259,6 +369,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(F8_REGS_LIGHT));
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
@@ -266,8 +378,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       bool ok = true;
       uint32_t ag_seen = 0;
       for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-        int m0, n0;
-        tile_of(w, m0, n0);
+        int m0, n0, kb0, kb1;
+        tile_of(w, m0, n0, kb0, kb1);
         if (args.ag_world > 1) {
           const int shard = n0 / args.ag_rows;
           if (shard != args.ag_rank && !((ag_seen >> shard) & 1u)) {
@@ -280,18 +392,18 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             fence_proxy_async_global();
           }
         }
-        for (int kb = 0; kb < KB; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
             atomicExch(args.status, ST_TIMEOUT_EMPTY);
             ok = false;
             break;
           }
-          uint8_t* sa = smem + stage * F8_STAGE_BYTES;
+          uint8_t* sa = smem + stage * C8::STAGE_BYTES;
           uint8_t* sb = sa + F8_BM * F8_BK;
-          mbar_arrive_expect_tx(&full_bar[stage], F8_STAGE_BYTES);
+          mbar_arrive_expect_tx(&full_bar[stage], C8::STAGE_BYTES);
           tma_load_2d(sa, &tmA, &full_bar[stage], kb * F8_BK, m0);
           tma_load_2d(sb, &tmB, &full_bar[stage], kb * F8_BK, n0);
-          if (++stage == F8_STAGES) {
+          if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
@@ -300,14 +412,16 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc_e4m3(F8_BM, F8_BN);
+      constexpr uint32_t idesc = make_idesc_e4m3(F8_BM, BN);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-        for (int kb = 0; kb < KB; ++kb) {
+        int m0, n0, kb0, kb1;
+        tile_of(w, m0, n0, kb0, kb1);
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1)) {
             atomicExch(args.status, ST_TIMEOUT_TMEM_EMPTY);
             ok = false;
@@ -319,38 +433,41 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * F8_STAGE_BYTES);
+          const uint32_t sa = smem_u32(smem + stage * C8::STAGE_BYTES);
           const uint32_t sb = sa + F8_BM * F8_BK;
-          const uint32_t d_tmem = tmem_base + acc * F8_BN;
+          const uint32_t d_tmem = tmem_base + acc * BN;
 #pragma unroll
           for (int k = 0; k < F8_BK / 32; ++k)
             umma_f8(d_tmem, make_smem_desc(sa + k * 32, 16, 1024), make_smem_desc(sb + k * 32, 16, 1024),
                     idesc, k > 0 ? 1u : 0u);
           umma_commit(&empty_bar[stage]);
           umma_commit(&tfull_bar[acc]);
-          if (++stage == F8_STAGES) {
+          if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
-          if (++acc == F8_ACC) {
+          if (++acc == ACC) {
             acc = 0;
             acc_phase ^= 1;
           }
         }
       }
     }
+  }
   } else {
-    // warp w owns TMEM lanes 32 * (w % 4) .. +31 (hardware rule) and the column half (w - 2) / 4
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(F8_REGS_HEAVY));
+    // warp w owns TMEM lanes 32 * (w % 4) .. +31 (hardware rule) and the column half (w - 4) / 4
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;
-    constexpr int HC = F8_BN / 2;  // 64 columns per thread
+    const int half = (warp - 4) >> 2;
+    const int et = threadIdx.x - 128;  // 0..255 over the eight epilogue warps
+    uint8_t* stage_out = smem + C8::OFF_EPI + (warp - 4) * 8192;
+    int toggle = 0;                      // which of this warp's two staging tiles is next
     uint32_t ag_seen = 0;
     if (args.ag_world > 1) {
-      const int et = threadIdx.x - 64;  // 0..255 over the eight epilogue warps
       const long long shard_vecs = static_cast<long long>(args.ag_rows) * args.K / 16;
       const long long per_cta = (shard_vecs + gridDim.x - 1) / gridDim.x;
       const long long v0 = per_cta * blockIdx.x, v1 = min(shard_vecs, v0 + per_cta);
-      const int nb_all = num_n, nb_shard = args.ag_rows / F8_BN;
+      const int nb_shard = args.ag_rows / 128;
       for (int d = 1; d < args.ag_world; ++d) {
         const int shard = (args.ag_rank + d) % args.ag_world;
         const uint4* src = reinterpret_cast<const uint4*>(args.ag_src[shard]);
@@ -358,7 +475,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         for (long long v = v0 + et; v < v1; v += 256) dst[v] = src[v];
         if (blockIdx.x == 0) {   // the scale columns of this shard, every K block
           for (int i = et; i < KB * nb_shard; i += 256) {
-            const int idx = (i / nb_shard) * nb_all + shard * nb_shard + (i % nb_shard);
+            const int idx = (i / nb_shard) * n_blocks + shard * nb_shard + (i % nb_shard);
             args.ag_sdst[idx] = args.ag_ssrc[shard][idx];
           }
         }
@@ -369,10 +486,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
     int acc = 0;
     uint32_t acc_phase = 0;
+    uint32_t it = 0;          // K blocks so far: the scale buffers alternate across work items too
     bool ok = true;
-    for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-      int m0, n0;
-      tile_of(w, m0, n0);
+    // (with a row-scaled B a warp whose wait ran out goes on to the barriers the other warps need)
+    for (int w = blockIdx.x; w < total && (ok || !B_BLOCK); w += gridDim.x) {
+      int m0, n0, kb0, kb1;
+      tile_of(w, m0, n0, kb0, kb1);
       if (args.ag_world > 1) {
         const int shard = n0 / args.ag_rows;
         if (shard != args.ag_rank && !((ag_seen >> shard) & 1u)) {
@@ -384,98 +503,133 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           ag_seen |= 1u << shard;
         }
       }
-      n0 += half * HC;
+      const int nh = n0 + half * HC;            // first of this thread's columns
       const int row = m0 + quarter * 32 + lane;
       const bool row_ok = row < M;
-      float c[HC];
+      const int nb = min(nh >> 7, n_blocks - 1);
+      float2 c[HC / 2];
 #pragma unroll
-      for (int j = 0; j < HC; ++j) c[j] = 0.f;
-      // scales of K block 0; those of block kb + 1 are fetched while block kb is being awaited
-      float sa_n = row_ok ? args.sa[row] : 0.f;
-      float sb_n = args.b_block ? __ldcg(args.sb + (n0 >> 7)) : 0.f;
-      for (int kb = 0; kb < KB; ++kb) {
+      for (int j = 0; j < HC / 2; ++j) c[j] = make_float2(0.f, 0.f);
+      // Scales of the item's first K block; those of block kb + 1 are fetched while block kb is being awaited (two
+      // or four blocks ahead measured no faster). Row-scaled B: thread et carries the scale of tile column et (BN =
+      // 128: the first 128 threads) to shared memory, where every thread reads the scales of its columns.
+      const bool sb_mine = !B_BLOCK && et < BN && n0 + et < N;
+      float sa_n = row_ok ? args.sa[static_cast<size_t>(kb0) * M + row] : 0.f;
+      float sb_n = B_BLOCK ? __ldcg(args.sb + static_cast<size_t>(kb0) * n_blocks + nb)
+                           : (sb_mine ? __ldg(args.sb + static_cast<size_t>(kb0) * N + n0 + et) : 0.f);
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const float sa = sa_n;
         const float sblk = sb_n * sa;
-        if (kb + 1 < KB) {
-          sa_n = row_ok ? args.sa[static_cast<size_t>(kb + 1) * M + row] : 0.f;
-          if (args.b_block) sb_n = __ldcg(args.sb + static_cast<size_t>(kb + 1) * num_n + (n0 >> 7));
+        float* sb_cur = sb_tile + (it & 1) * BN;
+        if (!B_BLOCK) {
+          // the buffer's readers (two blocks ago) are behind the barrier of the block in between
+          if (et < BN) sb_cur[et] = sb_n;
+          asm volatile("bar.sync 1, 256;" ::: "memory");
         }
-        if (!mbar_wait(&tfull_bar[acc], acc_phase)) {
+        if (kb + 1 < kb1) {
+          sa_n = row_ok ? args.sa[static_cast<size_t>(kb + 1) * M + row] : 0.f;
+          if (B_BLOCK) sb_n = __ldcg(args.sb + static_cast<size_t>(kb + 1) * n_blocks + nb);
+          else sb_n = sb_mine ? __ldg(args.sb + static_cast<size_t>(kb + 1) * N + n0 + et) : 0.f;
+        }
+        if (ok && !mbar_wait(&tfull_bar[acc], acc_phase)) {
           if (lane == 0) atomicExch(args.status, ST_TIMEOUT_TMEM_FULL);
           ok = false;
-          break;
+        }
+        if (!ok) {
+          if (B_BLOCK) break;
+          continue;
         }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + acc * F8_BN + half * HC + (static_cast<uint32_t>(quarter * 32) << 16);
-        uint32_t r0[32], r1[32];
-        tmem_ld32(taddr, r0);
-        tmem_ld32(taddr + 32, r1);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty_bar[acc]);
-        if (args.b_block) {
+        const uint32_t taddr = tmem_base + acc * BN + half * HC + (static_cast<uint32_t>(quarter * 32) << 16);
+        const float2 sa2 = make_float2(sa, sa), sblk2 = make_float2(sblk, sblk);
+        // Reading the partial products (128 KB a block) takes 1 024 cycles, tensor memory gives about 128 bytes a
+        // clock and SM: that, not the MMAs, bounds this kernel (without the arithmetic 224 us for 55 424 x 1024 x
+        // 4096). So the next 32 columns are on their way while these are scaled and added.
+        uint32_t r[2][32];
+        tmem_ld32(taddr, r[0]);
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            c[e] = fmaf(__uint_as_float(r0[e]), sblk, c[e]);
-            c[32 + e] = fmaf(__uint_as_float(r1[e]), sblk, c[32 + e]);
+        for (int q = 0; q < HC / 32; ++q) {
+          tmem_ld_wait();
+          if (q + 1 < HC / 32) {
+            tmem_ld32(taddr + (q + 1) * 32, r[(q + 1) & 1]);
+          } else {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty_bar[acc]);
           }
-        } else {
+          const uint32_t (&v)[32] = r[q & 1];
+          if (B_BLOCK) {
 #pragma unroll
-          const float4* sbp = reinterpret_cast<const float4*>(args.sb + static_cast<size_t>(kb) * N + n0);
+            for (int e = 0; e < 16; ++e)
+              c[q * 16 + e] = fma2(make_float2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])), sblk2,
+                                   c[q * 16 + e]);
+          } else {
+            const float4* sp = reinterpret_cast<const float4*>(sb_cur + half * HC + q * 32);
 #pragma unroll
-          for (int e4 = 0; e4 < HC / 4; ++e4) {
-            const float4 s4 = (n0 + e4 * 4 < N) ? __ldg(sbp + e4) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float ss[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int e = e4 * 4 + u;
-              const float p = __uint_as_float(e < 32 ? r0[e] : r1[e - 32]) * sa;
-              c[e] = fmaf(p, ss[u], c[e]);
+            for (int e4 = 0; e4 < 8; ++e4) {
+              const float4 s4 = sp[e4];
+              const int e = e4 * 2;
+              c[q * 16 + e] = fma2(mul2(make_float2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])), sa2),
+                                   make_float2(s4.x, s4.y), c[q * 16 + e]);
+              c[q * 16 + e + 1] =
+                  fma2(mul2(make_float2(__uint_as_float(v[2 * e + 2]), __uint_as_float(v[2 * e + 3])), sa2),
+                       make_float2(s4.z, s4.w), c[q * 16 + e + 1]);
             }
           }
         }
-        if (++acc == F8_ACC) {
+        if (++acc == ACC) {
           acc = 0;
           acc_phase ^= 1;
         }
       }
-      if (!ok) break;
-      if (row_ok) {
-        if (args.out_mode == 0) {
-          __nv_bfloat16* Cb = reinterpret_cast<__nv_bfloat16*>(args.C) + static_cast<size_t>(row) * args.ldc + n0;
+      if (!ok) continue;
+      // 128 bytes of every row at a time (64 bf16 or 32 fp32 columns) through this warp's staging tile and one TMA
+      // store or reduce-add; rows and columns past the end are clipped by the tensor map. (Adds issued from the
+      // registers touch 32 rows an instruction: a fifth of a weight gradient's time.)
+      const int y0 = m0 + quarter * 32;
+      const bool bf = args.out_mode == 0;
 #pragma unroll
-          for (int j = 0; j < HC; j += 8) {
-            if (n0 + j < N) {
-              uint4 o;
-              uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+      for (int q = 0; q < HC / 32; ++q) {
+        if (bf && q >= HC / 64) break;
+        const int x = nh + q * (bf ? 64 : 32);
+        if (y0 < M && x < N) {
+          if (elect_one()) tma_store_wait_read<1>();
+          __syncwarp();
+          uint8_t* tile_out = stage_out + toggle * 4096;
+          toggle ^= 1;
 #pragma unroll
-              for (int e = 0; e < 4; ++e) ow[e] = pack_bf16x2(c[j + 2 * e], c[j + 2 * e + 1]);
-              *reinterpret_cast<uint4*>(Cb + j) = o;
+          for (int j = 0; j < 8; ++j) {
+            uint4 o;
+            if (bf) {
+              const float2* v = c + (q % (HC / 64)) * 32 + j * 4;
+              o = make_uint4(pack_bf16x2(v[0].x, v[0].y), pack_bf16x2(v[1].x, v[1].y), pack_bf16x2(v[2].x, v[2].y),
+                             pack_bf16x2(v[3].x, v[3].y));
+            } else {
+              const float2* v = c + q * 16 + j * 2;
+              o = make_uint4(__float_as_uint(v[0].x), __float_as_uint(v[0].y), __float_as_uint(v[1].x),
+                             __float_as_uint(v[1].y));
             }
+            *reinterpret_cast<uint4*>(tile_out + lane * 128 + ((j ^ (lane & 7)) << 4)) = o;
           }
-        } else {
-          float* Cf = reinterpret_cast<float*>(args.C) + static_cast<size_t>(row) * args.ldc + n0;
-#pragma unroll
-          for (int j = 0; j < HC; j += 4) {
-            if (n0 + j < N) {
-              const float4 v = make_float4(c[j], c[j + 1], c[j + 2], c[j + 3]);
-              if (args.out_mode == 2)
-                atomicAdd(reinterpret_cast<float4*>(Cf + j), v);
-              else
-                *reinterpret_cast<float4*>(Cf + j) = v;
-            }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (elect_one()) {
+            if (args.out_mode == 2) tma_reduce_add_2d(&tmC, tile_out, x, y0);
+            else tma_store_2d(&tmC, tile_out, x, y0);
+            tma_store_commit();
           }
         }
       }
     }
+    if (elect_one()) tma_store_wait<0>();
+    __syncwarp();
   }
 
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, F8_ACC * F8_BN);
+    tmem_dealloc(tmem_base, ACC * BN);
   }
 }
 
@@ -496,18 +650,88 @@ static EncodeTiledFn8 f8_encode_fn() {
   return fn;
 }
 
-// uint8 [rows][K] row-major, box 128 bytes x 128 rows, 128-byte swizzle
-static int f8_make_map(CUtensorMap* map, const void* base, uint64_t K, uint64_t rows) {
+// uint8 [rows][K] row-major, box 128 bytes x box_rows rows, 128-byte swizzle
+static int f8_make_map(CUtensorMap* map, const void* base, uint64_t K, uint64_t rows, uint32_t box_rows) {
   EncodeTiledFn8 fn = f8_encode_fn();
   if (fn == nullptr) return -1;
   cuuint64_t dims[2] = {K, rows};
   cuuint64_t strides[1] = {K};
-  cuuint32_t box[2] = {128, 128};
+  cuuint32_t box[2] = {128, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -2;
+}
+
+// bf16 or fp32 [rows][cols] output, boxes of 32 rows x 128 bytes
+static int f8_make_out_map(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, uint64_t ld, bool bf16) {
+  EncodeTiledFn8 fn = f8_encode_fn();
+  if (fn == nullptr) return -1;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * (bf16 ? 2 : 4)};
+  cuuint32_t box[2] = {bf16 ? 64u : 32u, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims,
+                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -2;
+}
+
+// Work items a tile is cut into when the output is accumulated (weight gradients: few tiles, a long contraction
+// over tokens): the smallest number that fills the last wave of SMs best, at least 16 K blocks (2 048 tokens) each.
+// 55 424 tokens: a 1024 x 1024 gradient is 32 tiles, i.e. 116 of 148 SMs idle without it.
+static int f8_splits(int tiles, int kb, int sms) {
+  int best = 1;
+  double best_eff = 0.0;
+  for (int s = 1; s <= 9 && (s == 1 || kb / s >= 16); ++s) {
+    const int work = tiles * s;
+    const double eff = static_cast<double>(work) / (static_cast<double>((work + sms - 1) / sms) * sms);
+    if (eff > best_eff + 0.02) {
+      best = s;
+      best_eff = eff;
+    }
+  }
+  return best;
+}
+
+template <int BN, bool B_BLOCK>
+static int f8_launch_form(const void* A, const void* B, void* C, Fp8Args& args, bool coop, cudaStream_t stream) {
+  CUtensorMap tmA, tmB, tmC;
+  int rc = f8_make_map(&tmA, A, args.K, args.M, F8_BM);
+  if (rc) return rc;
+  rc = f8_make_map(&tmB, B, args.K, args.N, BN);
+  if (rc) return rc;
+  rc = f8_make_out_map(&tmC, C, args.N, args.M, args.ldc, args.out_mode == 0);
+  if (rc) return rc;
+  static bool configured_on[nplm::MAX_DEVICES];
+  const int dev_slot = nplm::current_device_slot();
+  if (dev_slot < 0) return -4;
+  bool& configured = configured_on[dev_slot];
+  if (!configured) {
+    NPLM_CUDA_CHECK(
+        cudaFuncSetAttribute(gemm_fp8_kernel<BN, B_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, F8Cfg<BN>::SMEM));
+    configured = true;
+  }
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_slot);
+  const int tiles = ((args.M + F8_BM - 1) / F8_BM) * ((args.N + BN - 1) / BN);
+  args.splits = args.out_mode == 2 ? f8_splits(tiles, args.K / F8_BK, sms) : 1;
+  const int total = tiles * args.splits;
+  const int grid = total < sms ? total : sms;
+  if (coop) {
+    void* params[] = {&tmA, &tmB, &tmC, &args};
+    return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(gemm_fp8_kernel<BN, B_BLOCK>), dim3(grid),
+                                                        dim3(F8_THREADS), params, F8Cfg<BN>::SMEM, stream));
+  }
+  gemm_fp8_kernel<BN, B_BLOCK><<<grid, F8_THREADS, F8Cfg<BN>::SMEM, stream>>>(tmA, tmB, tmC, args);
+  return static_cast<int>(cudaGetLastError());
+}
+
+template <int BN>
+static int f8_launch(const void* A, const void* B, void* C, Fp8Args& args, bool coop, cudaStream_t stream) {
+  return args.b_block ? f8_launch_form<BN, true>(A, B, C, args, coop, stream)
+                      : f8_launch_form<BN, false>(A, B, C, args, coop, stream);
 }
 
 static int f8_grid(long long threads_needed, int block) {
@@ -552,6 +776,18 @@ extern "C" int nplm_fp8_quant_tile(const void* x, int R, int K, int ldx, int tra
   return static_cast<int>(cudaGetLastError());
 }
 
+// Row form and transposed row form of x bf16 [R][K] in one pass, R and K multiples of 128; see quant_dual_kernel.
+extern "C" int nplm_fp8_quant_dual(const void* x, int R, int K, int ldx, void* qr, float* sr, void* qt, float* st,
+                                   cudaStream_t stream) {
+  if (R <= 0 || K <= 0) return 0;
+  if ((K % 128) || (R % 128) || (ldx % 4) || (reinterpret_cast<uintptr_t>(x) & 7)) return -3;
+  if (R / 128 > 65535) return -3;
+  quant_dual_kernel<<<dim3(K / 128, R / 128), 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx,
+                                                                reinterpret_cast<uint8_t*>(qr), sr,
+                                                                reinterpret_cast<uint8_t*>(qt), st);
+  return static_cast<int>(cudaGetLastError());
+}
+
 // C[M][N] (+)= (A * sa) (B * sb)^T, A e4m3 [M][K], B e4m3 [N][K] (both K-major, K % 128 == 0).
 // sa fp32 [K/128][M]; sb fp32 [K/128][N] (b_block = 0) or [K/128][ceil(N/128)] (b_block = 1).
 // out_mode 0: bf16 C; 1: fp32 C; 2: fp32 C accumulated with atomics.
@@ -559,24 +795,12 @@ extern "C" int nplm_gemm_fp8(const void* A, const void* B, void* C, const float*
                              int M, int N, int K, int ldc, int b_block, int out_mode, int* status,
                              cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((K % 128) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
+  if ((K % 128) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
+      (reinterpret_cast<uintptr_t>(C) & 15))
+    return -3;
   if (out_mode == 0 ? ((N % 8) || (ldc % 8)) : ((N % 4) || (ldc % 4))) return -5;
   if (!b_block && (N % 4)) return -5;
-  CUtensorMap tmA, tmB;
-  int rc = f8_make_map(&tmA, A, K, M);
-  if (rc) return rc;
-  rc = f8_make_map(&tmB, B, K, N);
-  if (rc) return rc;
-  static bool configured_on[nplm::MAX_DEVICES];
-  const int dev_slot = nplm::current_device_slot();
-  if (dev_slot < 0) return -4;
-  bool& configured = configured_on[dev_slot];
-  if (!configured) {
-    NPLM_CUDA_CHECK(cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F8_SMEM));
-    configured = true;
-  }
   Fp8Args args;
-  args.C = C;
   args.sa = sa;
   args.sb = sb;
   args.M = M;
@@ -596,13 +820,7 @@ extern "C" int nplm_gemm_fp8(const void* A, const void* B, void* C, const float*
     args.ag_src[r] = nullptr;
     args.ag_ssrc[r] = nullptr;
   }
-  const int total = ((M + F8_BM - 1) / F8_BM) * ((N + F8_BN - 1) / F8_BN);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = total < sms ? total : sms;
-  gemm_fp8_kernel<<<grid, F8_THREADS, F8_SMEM, stream>>>(tmA, tmB, args);
-  return static_cast<int>(cudaGetLastError());
+  return N > 128 ? f8_launch<256>(A, B, C, args, false, stream) : f8_launch<128>(A, B, C, args, false, stream);
 }
 
 // All-gather fused into the fp8 GEMM. b_ptrs[r] / sb_ptrs[r]: rank r's full-size e4m3 weight buffer
@@ -613,25 +831,11 @@ extern "C" int nplm_gemm_fp8_ag(const void* A, void* const* b_ptrs, void* C, con
                                 void* const* sb_ptrs, int M, int N, int K, int ldc, int out_mode,
                                 int rank, int world, unsigned* flags, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (world < 2 || world > 8 || rank < 0 || rank >= world || (N % world) || ((N / world) % F8_BN) ||
+  if (world < 2 || world > 8 || rank < 0 || rank >= world || (N % world) || ((N / world) % 128) ||
       (K % 128) || flags == nullptr)
     return -10;
   if (out_mode == 0 ? ((N % 8) || (ldc % 8)) : ((N % 4) || (ldc % 4))) return -5;
-  CUtensorMap tmA, tmB;
-  int rc = f8_make_map(&tmA, A, K, M);
-  if (rc) return rc;
-  rc = f8_make_map(&tmB, b_ptrs[rank], K, N);
-  if (rc) return rc;
-  static bool configured_on[nplm::MAX_DEVICES];
-  const int dev_slot = nplm::current_device_slot();
-  if (dev_slot < 0) return -4;
-  bool& configured = configured_on[dev_slot];
-  if (!configured) {
-    NPLM_CUDA_CHECK(cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F8_SMEM));
-    configured = true;
-  }
   Fp8Args args;
-  args.C = C;
   args.sa = sa;
   args.sb = reinterpret_cast<const float*>(sb_ptrs[rank]);
   args.M = M;
@@ -653,12 +857,6 @@ extern "C" int nplm_gemm_fp8_ag(const void* A, void* const* b_ptrs, void* C, con
     args.ag_ssrc[r] = r < world ? reinterpret_cast<const float*>(sb_ptrs[r]) : nullptr;
   }
   NPLM_CUDA_CHECK(cudaMemsetAsync(flags, 0, 8 * sizeof(unsigned), stream));
-  const int total = ((M + F8_BM - 1) / F8_BM) * (N / F8_BN);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = total < sms ? total : sms;
-  void* params[] = {&tmA, &tmB, &args};
-  return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(gemm_fp8_kernel), dim3(grid),
-                                                      dim3(F8_THREADS), params, F8_SMEM, stream));
+  return args.ag_rows % 256 == 0 ? f8_launch<256>(A, b_ptrs[rank], C, args, true, stream)
+                                 : f8_launch<128>(A, b_ptrs[rank], C, args, true, stream);
 }

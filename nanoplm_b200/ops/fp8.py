@@ -79,6 +79,22 @@ def quant_tile(x: torch.Tensor, transpose: bool, block: bool) -> Quantized:
     return Quantized(q, s, block)
 
 
+def quant_dual(x: torch.Tensor) -> tuple[Quantized, Quantized]:
+    """(quant_rows(x), quant_tile(x, transpose=True, block=False)) in one pass over x bf16 [R, K], both multiples
+    of 128."""
+    R, K = x.shape
+    if x.stride(1) != 1 or x.stride(0) % 4 or x.data_ptr() % 8:
+        x = x.contiguous()
+    dev = x.device
+    qr, sr = torch.empty((R, K), dtype=torch.uint8, device=dev), torch.empty((K // 128, R), dtype=torch.float32, device=dev)
+    qt, st = torch.empty((K, R), dtype=torch.uint8, device=dev), torch.empty((R // 128, K), dtype=torch.float32, device=dev)
+    rc = lib("fp8").nplm_fp8_quant_dual(ptr(x), c_int(R), c_int(K), c_int(x.stride(0)), ptr(qr), ptr(sr), ptr(qt),
+                                        ptr(st), stream_ptr())
+    check_rc(rc, "fp8_quant_dual")
+    count_launch()
+    return Quantized(qr, sr, False), Quantized(qt, st, False)
+
+
 def gemm_fp8(a: Quantized, b: Quantized, *, out: torch.Tensor | None = None, out_dtype=_BF16,
              accumulate: bool = False) -> torch.Tensor:
     """C[M,N] (+)= deq(a) deq(b)^T. a: row-scaled [M,K]; b: row- or block-scaled [N,K]."""
@@ -149,15 +165,25 @@ def supported(x: torch.Tensor, w: torch.Tensor) -> bool:
             and w.shape[1] % 128 == 0)
 
 
+def _dual_rows(T: int) -> bool:
+    """Token counts for which the weight gradient runs on e4m3 operands (whole 128-token scale blocks)."""
+    return T % 128 == 0 and T // 128 <= 65535
+
+
 class _Fp8LinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w):
+    def forward(ctx, x, w, train):
         from .functional import _as_shape
         x2 = x.reshape(-1, x.shape[-1])
-        qx = quant_rows(x2)
         qw, _ = _quantized_weight(w)
+        ctx.dual = train and ctx.needs_input_grad[1] and _dual_rows(x2.shape[0])
+        if ctx.dual:      # the weight gradient's form of x comes from the same pass; x itself need not be kept
+            qx, qx_t = quant_dual(x2)
+            ctx.save_for_backward(qx_t.q, qx_t.scale, w)
+        else:
+            qx = quant_rows(x2)
+            ctx.save_for_backward(x2, w)
         y = gemm_fp8(qx, qw)
-        ctx.save_for_backward(x2, w)
         ctx.w_ref = w
         ctx.shape = x.shape
         return _as_shape(y, (*x.shape[:-1], w.shape[0]))
@@ -165,30 +191,33 @@ class _Fp8LinearFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         from .functional import _as_shape, _has_main_grad, _wgrad
-        x2, w = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        dx = dw = None
+        dx = dw = qdy = qdy_t = None
+        if ctx.dual:
+            qx_t, sx_t, w = ctx.saved_tensors
+            if ctx.needs_input_grad[0]:
+                qdy, qdy_t = quant_dual(dy2)
+            else:
+                qdy_t = quant_tile(dy2, transpose=True, block=False)
+        elif ctx.needs_input_grad[0]:
+            qdy = quant_rows(dy2)
         if ctx.needs_input_grad[0]:
             _, qwt = _quantized_weight(ctx.w_ref)
-            dx = _as_shape(gemm_fp8(quant_rows(dy2), qwt), ctx.shape)
-        if ctx.needs_input_grad[1]:
-            T = x2.shape[0]
-            if T % 128 == 0:
-                # dW[N,K] = dY^T X: both operands transposed to token-contiguous payloads
-                qdy_t = quant_tile(dy2, transpose=True, block=False)
-                qx_t = quant_tile(x2, transpose=True, block=False)
-                p = ctx.w_ref
-                if _has_main_grad(p):
-                    gemm_fp8(qdy_t, qx_t, out=p.main_grad.view(w.shape), accumulate=True)
-                else:
-                    dw = gemm_fp8(qdy_t, qx_t, out_dtype=torch.float32).to(w.dtype)
+            dx = _as_shape(gemm_fp8(qdy, qwt), ctx.shape)
+        if ctx.dual:
+            # dW[N,K] = dY^T X: both operands as token-contiguous payloads
+            p, qx = ctx.w_ref, Quantized(qx_t, sx_t, False)
+            if _has_main_grad(p):
+                gemm_fp8(qdy_t, qx, out=p.main_grad.view(w.shape), accumulate=True)
             else:
-                dw = _wgrad(dy2, x2, ctx.w_ref)
-        return dx, dw
+                dw = gemm_fp8(qdy_t, qx, out_dtype=torch.float32).to(w.dtype)
+        elif ctx.needs_input_grad[1]:
+            dw = _wgrad(dy2, ctx.saved_tensors[0], ctx.w_ref)
+        return dx, dw, None
 
 
 def fp8_linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """y = x W^T with e4m3 operands (no bias)."""
-    return _Fp8LinearFn.apply(x, w)
+    return _Fp8LinearFn.apply(x, w, torch.is_grad_enabled())
