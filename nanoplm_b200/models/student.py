@@ -129,8 +129,11 @@ class ProtX(EncoderModel):
                         device: Optional[torch.device] = None) -> list[torch.Tensor]:
         """Mean-pooled (EOS excluded) or per-token embeddings for raw sequences."""
         device = device or next(self.parameters()).device
-        was_training = self.training
-        self.eval()
+        # (walking all modules to set a flag that is set already costs more than several layers' launches)
+        was_training = any(m.training for m in self.modules())
+        restore = self.training
+        if was_training:
+            self.eval()
         packed = self._embeds_packed(torch.device(device))
         out, waiting, rows = [], [], 0
 
@@ -170,7 +173,8 @@ class ProtX(EncoderModel):
                 n = int(mask[b].sum()) - 1          # drop the trailing </s>
                 out.append(h[b, :n].cpu() if per_token else h[b, :n].mean(0).cpu())
         collect()
-        self.train(was_training)
+        if was_training:
+            self.train(restore)
         return out
 
 

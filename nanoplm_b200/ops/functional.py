@@ -16,6 +16,7 @@ from __future__ import annotations
 import math
 
 import torch
+import torch.autograd.forward_ad as _fwd_ad
 import torch.nn.functional as F
 
 from . import kernels as K
@@ -83,6 +84,25 @@ def _param_grad(p, g32: torch.Tensor):
         p.main_grad.add_(g32.view_as(p.main_grad))
         return None
     return g32.to(p.dtype).view_as(p)
+
+
+class _NoGradCtx:
+    """Context of a forward that no backward follows."""
+    needs_input_grad = (False,) * 16
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    def mark_non_differentiable(self, *tensors):
+        pass
+
+
+def _call(fn, *args):
+    """fn.apply(*args); where gradients are off (and no forward-mode level or function transform is active, which
+    have to see the Function) its forward directly: the dispatch of a Function costs more than most of its bodies."""
+    if torch.is_grad_enabled() or _fwd_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
+        return fn.apply(*args)
+    return fn.forward(_NoGradCtx(), *args)
 
 
 # ------------------------------------------------------------------------------------- linear
@@ -182,7 +202,7 @@ def mlp_swiglu(x, w_in, w_out, residual=None):
     inter = w_out.shape[1]
     if (x.is_cuda and x.dtype == BF and not _FP8_STATE["enabled"] and inter % 64 == 0 and w_in.shape[0] == 2 * inter
             and w_in.shape[1] % 64 == 0 and w_out.shape[0] % 64 == 0):
-        return _SwiGLUMLPFn.apply(x, w_in, w_out, residual, torch.is_grad_enabled())
+        return _call(_SwiGLUMLPFn, x, w_in, w_out, residual, torch.is_grad_enabled())
     return linear(linear(x, w_in, act="swiglu"), w_out, residual=residual)
 
 
@@ -190,7 +210,7 @@ def linear_rope(x, w, pos, cos, sin, rope_cols: int):
     """QKV projection with the rotary embedding of q and k applied in the GEMM epilogue (CUDA,
     head_dim 64). The result equals rope_qkv(linear(x, w)); its gradient w.r.t. the un-rotated
     projection is obtained by passing rope=(pos, cos, sin) to attention_varlen."""
-    return _LinearFn.apply(x, w, None, None, None, (pos, cos, sin, rope_cols))
+    return _call(_LinearFn, x, w, None, None, None, (pos, cos, sin, rope_cols))
 
 
 _FP8_STATE = {"enabled": False}
@@ -224,9 +244,9 @@ def linear(x, w, bias=None, residual=None, act: str | None = None):
     if x.is_cuda:
         if w.shape[1] % 8 == 0 and w.shape[0] % 8 == 0 and x.dtype == BF:
             if act == "swiglu" and bias is not None:
-                y = _LinearFn.apply(x, w, bias, None, None)
+                y = _call(_LinearFn, x, w, bias, None, None)
                 return swiglu(y)
-            return _LinearFn.apply(x, w, bias, residual, act, None, torch.is_grad_enabled())
+            return _call(_LinearFn, x, w, bias, residual, act, None, torch.is_grad_enabled())
     y = F.linear(x, w, bias)
     if act == "gelu":
         y = F.gelu(y)
@@ -257,7 +277,7 @@ class _SwigluFn(torch.autograd.Function):
 def swiglu(pre):
     """pre = [value | gate] -> silu(gate) * value (reference: modeling.py:301-302)."""
     if pre.is_cuda and pre.dtype == BF:
-        return _SwigluFn.apply(pre)
+        return _call(_SwigluFn, pre)
     v, g = pre.chunk(2, dim=-1)
     return F.silu(g) * v
 
@@ -278,7 +298,7 @@ class _ActFn(torch.autograd.Function):
 
 def activation(x, name: str):
     if x.is_cuda and x.dtype == BF and x.numel() % 8 == 0 and name in ("gelu", "relu", "silu"):
-        return _ActFn.apply(x, name)
+        return _call(_ActFn, x, name)
     return {"gelu": F.gelu, "relu": F.relu, "silu": F.silu, "tanh": torch.tanh}[name](x)
 
 
@@ -289,7 +309,7 @@ class _NormFn(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        y, mean, rstd = K.norm_fwd(x2, w, eps, rms=rms)
+        y, mean, rstd = K.norm_fwd(x2, w, eps, rms=rms, stats=any(ctx.needs_input_grad))
         ctx.save_for_backward(x2, w, mean, rstd)
         ctx.rms = rms
         ctx.shape = x.shape
@@ -315,7 +335,7 @@ class _NormResFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps, rms):
         x2 = x if x.is_contiguous() else x.contiguous()
-        y, mean, rstd = K.norm_fwd(x2, w, eps, rms=rms)
+        y, mean, rstd = K.norm_fwd(x2, w, eps, rms=rms, stats=any(ctx.needs_input_grad))
         ctx.save_for_backward(x2, w, mean, rstd)
         ctx.rms = rms
         return y, x2.view_as(x2)
@@ -339,14 +359,14 @@ class _NormResFn(torch.autograd.Function):
 def norm_residual(x, w, eps: float = 1e-5, rms: bool = False):
     """Returns (norm(x), x) — see _NormResFn. x is a flat [T, C] activation."""
     if x.is_cuda and x.dtype == BF and x.dim() == 2 and x.shape[-1] % 8 == 0 and x.shape[-1] <= 4096:
-        return _NormResFn.apply(x, w, eps, rms)
+        return _call(_NormResFn, x, w, eps, rms)
     return norm(x, w, eps, rms), x
 
 
 def norm(x, w, eps: float = 1e-5, rms: bool = False):
     """LayerNorm without bias (reference encoder norms) or RMSNorm (T5LayerNorm) over the last dim."""
     if x.is_cuda and x.dtype == BF and x.shape[-1] % 8 == 0 and x.shape[-1] <= 4096:
-        return _NormFn.apply(x, w, eps, rms)
+        return _call(_NormFn, x, w, eps, rms)
     xf = x.float()
     if rms:
         y = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
@@ -361,7 +381,7 @@ class _EmbedNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, ids, table, w, eps, rms):
         ids32 = ids.to(torch.int32).contiguous()
-        y, mean, rstd = K.norm_fwd(table, w, eps, rms=rms, ids=ids32)
+        y, mean, rstd = K.norm_fwd(table, w, eps, rms=rms, ids=ids32, stats=any(ctx.needs_input_grad))
         ctx.save_for_backward(ids32, table, w, mean, rstd)
         ctx.rms = rms
         return y
@@ -380,7 +400,7 @@ class _EmbedNormFn(torch.autograd.Function):
 def embed_norm(ids, table, w, eps: float = 1e-5, rms: bool = False):
     """norm(table[ids]) for flat ids (reference: modeling.py:222-223)."""
     if table.is_cuda and table.dtype == BF and table.shape[1] % 8 == 0 and table.shape[1] <= 4096:
-        return _EmbedNormFn.apply(ids, table, w, eps, rms)
+        return _call(_EmbedNormFn, ids, table, w, eps, rms)
     return norm(F.embedding(ids.long(), table), w, eps, rms)
 
 
@@ -482,7 +502,7 @@ def attention_out_proj(qkv, w_out, residual, seq_start, seq_end, H: int, D: int,
     bias-free projection run as one autograd node (fused backward); otherwise the two separate ops."""
     if (qkv.is_cuda and qkv.dtype == BF and D == 64 and qkv.dim() == 2 and not _FP8_STATE["enabled"]
             and w_out.shape[1] == H * D and w_out.shape[0] % 8 == 0):
-        return _AttnOutFn.apply(qkv, w_out, residual, seq_start, seq_end, H, D, window, scale, rope)
+        return _call(_AttnOutFn, qkv, w_out, residual, seq_start, seq_end, H, D, window, scale, rope)
     return linear(attention_varlen(qkv, seq_start, seq_end, H, D, window, scale, rope=rope), w_out,
                   residual=residual)
 
@@ -507,7 +527,7 @@ def attention_varlen(qkv, seq_start, seq_end, H: int, D: int, window: int, scale
     rope=(pos, cos, sin) (CUDA only) declares that q / k were rotated by linear_rope: the backward
     then returns the gradient of the un-rotated projection."""
     if qkv.is_cuda and qkv.dtype == BF and D == 64:
-        return _AttnFn.apply(qkv, seq_start, seq_end, H, D, window, scale, rope)
+        return _call(_AttnFn, qkv, seq_start, seq_end, H, D, window, scale, rope)
     if rope is not None:
         raise ValueError("fused rope backward is only available on the CUDA kernels")
     T = qkv.shape[0]

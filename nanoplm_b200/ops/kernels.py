@@ -10,7 +10,7 @@ from ctypes import c_float, c_int, c_longlong
 import torch
 
 from . import _lib
-from ._lib import check_rc, count_launch, lib, ptr, status_word, stream_ptr
+from ._lib import check_rc, count_launch, lib, ptr, raw_stream, status_word, stream_ptr, typed
 
 EPI_STORE, EPI_ADD, EPI_ATOMIC_F32, EPI_GELU, EPI_STORE_F32, EPI_SWIGLU, EPI_ROPE, EPI_RELU = 0, 1, 2, 3, 4, 5, 6, 7
 # acc = dL/dh of h = silu(gate) * value; aux = the [value | gate] pre-activations (2N wide);
@@ -25,6 +25,11 @@ def _chk(t: torch.Tensor, dtype, name: str) -> None:
         raise ValueError(f"{name} must be a CUDA tensor")
     if t.dtype != dtype:
         raise ValueError(f"{name} must be {dtype}, got {t.dtype}")
+
+
+def _dp(t: torch.Tensor | None):
+    """Device address for a `typed` call; None is the null pointer."""
+    return None if t is None else t.data_ptr()
 
 
 def _rowmajor(t: torch.Tensor, name: str) -> int:
@@ -125,20 +130,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         pair = _GEMM_PAIR_DEFAULT[0]
         if pair is None:
             pair = not f32_out
+    aux_p = aux.data_ptr() if aux is not None else None
+    rope_p = (r_pos.data_ptr(), r_cos.data_ptr(), r_sin.data_ptr()) if r_pos is not None else (None, None, None)
     if pair and bn == 256 and max_ctas == 0 and not (a_mn and not b_mn):
-        rc = lib("gemm_tcgen05").nplm_gemm_bf16_pair(
-            ptr(a), ptr(b), ptr(out), ptr(aux), c_int(M), c_int(N), c_int(K), c_int(lda), c_int(ldb),
-            c_int(ldc), c_int(ldr), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi), c_int(splits),
-            c_int(int(direct_epilogue)), ptr(r_pos), ptr(r_cos), ptr(r_sin),
-            c_int(int(r_cols)), ptr(status_word(a.device)), stream_ptr())
+        rc = typed("gemm_tcgen05", "nplm_gemm_bf16_pair", "pppp" + "i" * 12 + "pppipp")(
+            a.data_ptr(), b.data_ptr(), out.data_ptr(), aux_p, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, splits,
+            direct_epilogue, *rope_p, r_cols, status_word(a.device).data_ptr(), raw_stream())
         check_rc(rc, "gemm_bf16_pair")
         count_launch()
         return out
-    rc = lib("gemm_tcgen05").nplm_gemm_bf16(
-        ptr(a), ptr(b), ptr(out), ptr(aux), c_int(M), c_int(N), c_int(K), c_int(lda), c_int(ldb),
-        c_int(ldc), c_int(ldr), c_int(int(a_mn)), c_int(int(b_mn)), c_int(epi), c_int(splits),
-        c_int(bn), c_int(max_ctas), c_int(int(direct_epilogue)), ptr(r_pos), ptr(r_cos), ptr(r_sin),
-        c_int(int(r_cols)), ptr(status_word(a.device)), stream_ptr())
+    rc = typed("gemm_tcgen05", "nplm_gemm_bf16", "pppp" + "i" * 14 + "pppipp")(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), aux_p, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, splits, bn,
+        max_ctas, direct_epilogue, *rope_p, r_cols, status_word(a.device).data_ptr(), raw_stream())
     check_rc(rc, "gemm_bf16")
     count_launch()
     return out
@@ -207,10 +210,10 @@ def wgrad_splits(n_out: int, k_in: int, tokens: int, bn: int = 256, sms: int = 1
 
 # --------------------------------------------------------------------------- norms
 def norm_fwd(x: torch.Tensor, w: torch.Tensor | None, eps: float, rms: bool = False,
-             ids: torch.Tensor | None = None):
+             ids: torch.Tensor | None = None, stats: bool = True):
     """LayerNorm (no bias) / RMSNorm over the last dim. With ids, rows are table[ids] (embedding).
 
-    Returns (y, mean, rstd); mean is None for RMSNorm.
+    Returns (y, mean, rstd); mean is None for RMSNorm, both are with stats=False (no backward pass to come).
     """
     _chk(x, _BF16, "x")
     C = x.shape[-1]
@@ -223,11 +226,10 @@ def norm_fwd(x: torch.Tensor, w: torch.Tensor | None, eps: float, rms: bool = Fa
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     y = torch.empty((T, C), dtype=_BF16, device=x.device)
-    mean = None if rms else torch.empty(T, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-    rc = lib("elementwise").nplm_norm_fwd(ptr(x2), ptr(ids), ptr(w), ptr(y), ptr(mean), ptr(rstd),
-                                          c_int(T), c_int(C), c_float(eps), c_int(int(rms)),
-                                          stream_ptr())
+    mean = None if rms or not stats else torch.empty(T, dtype=torch.float32, device=x.device)
+    rstd = torch.empty(T, dtype=torch.float32, device=x.device) if stats else None
+    rc = typed("elementwise", "nplm_norm_fwd", "ppppppiifip")(
+        x2.data_ptr(), _dp(ids), _dp(w), y.data_ptr(), _dp(mean), _dp(rstd), T, C, eps, rms, raw_stream())
     check_rc(rc, "norm_fwd")
     count_launch()
     return y, mean, rstd
@@ -244,9 +246,9 @@ def norm_bwd(dy, x, w, mean, rstd, *, rms=False, dres=None, dw=None, ids=None, d
         dy2 = dy2.contiguous()
     dx = None if ids is not None else torch.empty((T, C), dtype=_BF16, device=dy.device)
     V = x.shape[0] if ids is not None else 0
-    rc = lib("elementwise").nplm_norm_bwd(
-        ptr(dy2), ptr(x), ptr(ids), ptr(w), ptr(mean), ptr(rstd), ptr(dres), ptr(dx), ptr(dw),
-        ptr(dtable), c_int(T), c_int(C), c_int(V), c_int(int(rms)), stream_ptr())
+    rc = typed("elementwise", "nplm_norm_bwd", "pppppppppp" + "iiiip")(
+        dy2.data_ptr(), x.data_ptr(), _dp(ids), _dp(w), _dp(mean), _dp(rstd), _dp(dres), _dp(dx), _dp(dw),
+        _dp(dtable), T, C, V, rms, raw_stream())
     check_rc(rc, "norm_bwd")
     count_launch()
     return dx
@@ -465,9 +467,9 @@ def fa_fwd(qkv, seq_start, seq_end, H, D, window, scale, impl: str | None = None
     out = torch.empty((T, H * D), dtype=_BF16, device=qkv.device)
     lse = torch.empty((H, T), dtype=torch.float32, device=qkv.device)
     if (impl or _FA_IMPL[0]) == "ws":
-        rc = lib("attention_ws").nplm_fa_fwd_ws(ptr(qkv), ptr(out), ptr(lse), ptr(seq_start), ptr(seq_end),
-                                                c_int(T), c_int(H), c_int(D), c_int(window), c_float(scale),
-                                                c_int(max_ctas), ptr(status_word(qkv.device)), stream_ptr())
+        rc = typed("attention_ws", "nplm_fa_fwd_ws", "pppppiiiifipp")(
+            qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), T, H, D, window,
+            scale, max_ctas, status_word(qkv.device).data_ptr(), raw_stream())
     else:
         rc = lib("attention").nplm_fa_fwd(ptr(qkv), ptr(out), ptr(lse), ptr(seq_start), ptr(seq_end),
                                           c_int(T), c_int(H), c_int(D), c_int(window), c_float(scale),
@@ -491,10 +493,9 @@ def gemm_dgrad_delta(dy: torch.Tensor, w: torch.Tensor, o: torch.Tensor, delta: 
     if N % 64 or tuple(o.shape) != (M, N) or tuple(delta.shape) != (N // 64, M) or not delta.is_contiguous():
         raise ValueError("o must be [M, N], delta [N / 64, M] contiguous, N a multiple of 64")
     out = torch.empty((M, N), dtype=_BF16, device=dy.device)
-    rc = lib("gemm_tcgen05").nplm_gemm_bf16_delta(
-        ptr(dy), ptr(w), ptr(out), ptr(o), ptr(delta), c_int(M), c_int(N), c_int(Kd), c_int(_rowmajor(dy, "dy")),
-        c_int(_rowmajor(w, "w")), c_int(N), c_int(_rowmajor(o, "o")), c_int(1), ptr(status_word(dy.device)),
-        stream_ptr())
+    rc = typed("gemm_tcgen05", "nplm_gemm_bf16_delta", "ppppp" + "iiiiiiii" + "pp")(
+        dy.data_ptr(), w.data_ptr(), out.data_ptr(), o.data_ptr(), delta.data_ptr(), M, N, Kd, _rowmajor(dy, "dy"),
+        _rowmajor(w, "w"), N, _rowmajor(o, "o"), 1, status_word(dy.device).data_ptr(), raw_stream())
     check_rc(rc, "gemm_bf16_delta")
     count_launch()
     return out
@@ -530,12 +531,10 @@ def fa_bwd(qkv, out, dout, lse, seq_start, seq_end, H, D, window, scale, dq_acc=
     if delta_ready:
         out = None
     if use_ws:
-        rc = lib("attention_ws").nplm_fa_bwd_ws_mode(ptr(qkv), ptr(out), ptr(dout), ptr(lse), ptr(dqkv),
-                                                     ptr(dq_acc), ptr(delta), ptr(seq_start), ptr(seq_end),
-                                                     c_int(T), c_int(H), c_int(D), c_int(window), c_float(scale),
-                                                     ptr(r_pos), ptr(r_cos), ptr(r_sin), c_int(max_ctas),
-                                                     c_int(3 if det else -1),
-                                                     ptr(status_word(qkv.device)), stream_ptr())
+        rc = typed("attention_ws", "nplm_fa_bwd_ws_mode", "ppppppppp" + "iiiif" + "pppii" + "pp")(
+            qkv.data_ptr(), _dp(out), dout.data_ptr(), lse.data_ptr(), dqkv.data_ptr(), _dp(dq_acc), delta.data_ptr(),
+            seq_start.data_ptr(), seq_end.data_ptr(), T, H, D, window, scale, _dp(r_pos), _dp(r_cos), _dp(r_sin),
+            max_ctas, 3 if det else -1, status_word(qkv.device).data_ptr(), raw_stream())
     else:
         rc = lib("attention").nplm_fa_bwd_rope(ptr(qkv), ptr(out), ptr(dout), ptr(lse), ptr(dqkv),
                                                ptr(dq_acc), ptr(delta), ptr(seq_start), ptr(seq_end),
