@@ -193,18 +193,22 @@ def gemm_ag(a: torch.Tensor, b_full: torch.Tensor, b_ptrs, rank: int, world: int
 
 
 def wgrad_splits(n_out: int, k_in: int, tokens: int, bn: int = 256, sms: int = 148) -> int:
-    """Split-K factor for a weight-gradient GEMM [n_out, k_in] reduced over `tokens`: the smallest
-    factor (<= 4) whose work items fill the last wave of `sms` CTAs best."""
+    """Split-K factor for a weight-gradient GEMM [n_out, k_in] reduced over `tokens`.
+
+    A work item of kb 64-token blocks costs kb + 25 block times (pipeline fill, atomic epilogue, and what its
+    additions take from the others); the factor with the least waves * cost wins. The 25 fits measurements from both
+    ends: 55 424 tokens, 4096 x 1024 (128 tiles) 377 us unsplit, 405 us in 8; 3072 x 1024 (96 tiles) 400 us unsplit, 331 in
+    3, 342 in 6; 1024 x 1024 (32 tiles) 121 us in 4, 118 in 9. Small outputs are what gains over filling a wave with
+    at most 4 items a tile: 17 000 tokens, 512 x 512 (8 tiles) 33.1 -> 19.4 us."""
     tiles = ((n_out + 127) // 128) * ((k_in + bn - 1) // bn)
     kb = (tokens + 63) // 64
-    best, best_eff = 1, 0.0
-    for s in range(1, 5):
-        if s > 1 and kb // s < 16:
+    best, best_cost = 1, None
+    for s in range(1, 17):
+        if s > 1 and kb // s < 4:
             break
-        work = tiles * s
-        eff = work / (((work + sms - 1) // sms) * sms)
-        if eff > best_eff + 0.02:
-            best, best_eff = s, eff
+        cost = -(-tiles * s // sms) * (-(-kb // s) + 25)
+        if best_cost is None or cost < 0.98 * best_cost:
+            best, best_cost = s, cost
     return best
 
 
