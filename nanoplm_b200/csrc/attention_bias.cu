@@ -8,15 +8,17 @@
 // bucketed relative_attention_bias, shared by all layers). bias is a per-head table indexed by
 // the relative position (key - query), built once per forward on the host side of the model.
 //
-// Same tiling as the training forward in attention.cu: the flat token axis (batch x padded
-// length) is cut into 128-token tiles; operands are [128 rows][64 bf16] swizzled tiles loaded by
-// TMA (two per operand for head_dim 128), S = Q K^T and O_part = P V run on tcgen05 with fp32
-// accumulators in TMEM, the online softmax runs one thread per query row.
+// Persistent and warp-specialised: a CTA per SM walks (256-query pair of tiles, head) items. Two softmax warpgroups, one per
+// 128-query tile, a thread per query row; one MMA-issuing warp per tile; one loader warp. The flat token axis (batch
+// x padded length) is tiled regardless of sequence boundaries, every row masks keys outside its own range. Keys
+// are consumed 64 at a time: the two tiles' scores (2 x 64 columns), bf16 probabilities (2 x 32) and outputs (2 x 128 for
+// head_dim 128) then all have their own tensor-memory columns, so the score product of a step runs while the previous
+// step's softmax and output product do, and a tile's chain hides behind the other's. The bias row of a thread is
+// read from a per-item table in shared memory (neighbouring lanes read neighbouring words).
 //
-// Keys are consumed KC at a time: 128 for head_dim 64; 64 for head_dim 128, which keeps a CTA at
-// 112 KB of shared memory and 192 TMEM columns so that two CTAs share an SM (the kernel is bound
-// by the latency of its MMA -> softmax -> MMA chain, so the second CTA nearly doubles throughput).
-// The bias table is read through the read-only cache instead of shared memory for the same reason.
+// The kernel it replaces ran one chain of MMA -> softmax -> MMA per CTA with the output in registers and two passes over the
+// scores, two CTAs an SM: 551 us for the teacher's layer (17 000 tokens, 32 heads of 128, sequences of 21 - 512),
+// 243 us now.
 #include "common.cuh"
 
 namespace nplm {
@@ -30,7 +32,6 @@ __device__ __forceinline__ uint32_t ab_swz(int r, int chunk) {
 }
 
 struct AbArgs {
-  __nv_bfloat16* out;    // [T][H*D]
   const int* seq_start;  // [T]
   const int* seq_end;    // [T]
   const float* bias;     // [H][2*S-1], index = key - query + S - 1
@@ -39,270 +40,450 @@ struct AbArgs {
   int* status;
 };
 
-template <int D, int KC>
-constexpr int ab_smem_bytes() {
-  // Q + 2 K + 2 V + P + barriers
-  return (D / 64) * AB_TILE + 4 * (D / 64) * (KC * 128) + AB_T * KC * 2 + 256;
+constexpr int AB_KC = 64;                       // keys per step
+constexpr int AB_THREADS = 384;                 // warps 0-3, 4-7: softmax of tile 0 / 1; 8: loader; 9, 10: MMA; 11: idle
+constexpr int AB_LOADER_WARP = 8, AB_MMA_WARP = 9;
+constexpr int AB_TAB = 2304;                    // floats of a tile's bias table: key ranges up to 2 176 keys
+
+template <int D>
+struct AbCfg {
+  static constexpr int NA = D / 64;                       // 64-column atoms per operand tile
+  static constexpr int Q_TILE = NA * AB_TILE;             // [atom][128 rows][128 B]
+  static constexpr int KA = AB_KC * 128;                  // bytes of one K / V atom
+  static constexpr int KV_TILE = NA * KA;                 // [atom][64 rows][128 B]
+  static constexpr int STAGES = D == 128 ? 2 : 4;
+  static constexpr int OFF_Q = 0;                         // [2 buffers][2 tiles]; a tile's buffer stages its output
+  static constexpr int OFF_K = OFF_Q + 4 * Q_TILE;
+  static constexpr int OFF_V = OFF_K + STAGES * KV_TILE;
+  static constexpr int OFF_TAB = OFF_V + STAGES * KV_TILE;
+  static constexpr int OFF_BAR = OFF_TAB + 2 * AB_TAB * 4;
+  static constexpr int SMEM = OFF_BAR + 512;
+};
+
+// Key range of an item and the steps [a, b) in which each tile takes part; lo / hi: union over the tile's rows.
+struct AbGeo {
+  int kv_lo, n;
+  int a[2], b[2];
+};
+
+// Computed by a whole warp: 16 coalesced loads, four warp reductions.
+__device__ __forceinline__ AbGeo ab_geometry(const AbArgs& args, int pair, int lane) {
+  const int t0 = pair * 2 * AB_T, T = args.T;
+  int lo[2], hi[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    lo[i] = 0x7fffffff;
+    hi[i] = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = t0 + i * AB_T + k * 32 + lane;
+      if (row < T) {
+        const int s = __ldg(args.seq_start + row), e = __ldg(args.seq_end + row);
+        if (e > s) {
+          lo[i] = min(lo[i], s);
+          hi[i] = max(hi[i], e);
+        }
+      }
+    }
+    lo[i] = __reduce_min_sync(0xffffffffu, lo[i]);
+    hi[i] = __reduce_max_sync(0xffffffffu, hi[i]);
+  }
+  AbGeo g;
+  g.kv_lo = min(lo[0], lo[1]);
+  const int kv_hi = max(hi[0], hi[1]);
+  g.n = kv_hi > g.kv_lo ? (kv_hi - g.kv_lo + AB_KC - 1) / AB_KC : 0;
+  if (g.n == 0) g.kv_lo = 0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    g.a[i] = g.b[i] = 0;
+    if (hi[i] > lo[i]) {
+      g.a[i] = (lo[i] - g.kv_lo) / AB_KC;
+      g.b[i] = (hi[i] - g.kv_lo + AB_KC - 1) / AB_KC;
+    }
+  }
+  return g;
 }
 
-template <int D, int KC>
-__global__ void __launch_bounds__(128, 2)
-fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmKV,
-                   const AbArgs args) {
-  constexpr int NA = D / 64;              // 64-column atoms per operand tile
-  constexpr int QB = NA * AB_TILE;        // bytes of the Q tile (128 rows)
-  constexpr int KA = KC * 128;            // bytes of one K / V atom (KC rows x 64 columns)
-  constexpr int OP = NA * KA;             // bytes of one K / V tile
-  constexpr int PB = AB_T * KC * 2;       // bytes of the P tile (KC / 64 atoms of [128][128 B])
+// barrier over one softmax warpgroup with an AND over everybody's predicate
+__device__ __forceinline__ bool ab_barrier_and(int id, bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q, o;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "bar.red.and.pred o, %1, 128, q;\n\t"
+      "selp.u32 %0, 1, 0, o;\n\t"
+      "}"
+      : "=r"(r)
+      : "r"(id), "r"(static_cast<uint32_t>(p))
+      : "memory");
+  return r != 0;
+}
+
+template <int D>
+__global__ void __launch_bounds__(AB_THREADS, 1)
+fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
+                   const __grid_constant__ CUtensorMap tmO, const AbArgs args) {
+  using C = AbCfg<D>;
+  constexpr int NA = C::NA, STAGES = C::STAGES;
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {
     if (threadIdx.x == 0) atomicExch(args.status, ST_BAD_ARG);
     return;
   }
-  uint8_t* sQ = smem;
-  uint8_t* sK = smem + QB;            // 2 buffers
-  uint8_t* sV = smem + QB + 2 * OP;   // 2 buffers
-  uint8_t* sP = smem + QB + 4 * OP;   // [KC / 64 key blocks][128 rows][128 B]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + QB + 4 * OP + PB);
-  uint64_t* bar_q = bars;
-  uint64_t* bar_kv = bars + 1;  // [2]
-  uint64_t* bar_s = bars + 3;
-  uint64_t* bar_o = bars + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
+  uint8_t* sQ = smem + C::OFF_Q;
+  uint8_t* sK = smem + C::OFF_K;
+  uint8_t* sV = smem + C::OFF_V;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
+  uint64_t* q_full = bars;                  // [2]
+  uint64_t* q_empty = q_full + 2;           // [2] both warpgroups: their output has left the buffer
+  uint64_t* k_full = q_empty + 2;           // [STAGES]
+  uint64_t* k_empty = k_full + STAGES;      // both MMA issuers
+  uint64_t* v_full = k_empty + STAGES;
+  uint64_t* v_empty = v_full + STAGES;
+  uint64_t* s_full = v_empty + STAGES;      // [2] per tile: scores of a step are in TMEM
+  uint64_t* s_free = s_full + 2;            // the warpgroup holds them in registers
+  uint64_t* p_ready = s_free + 2;           // probabilities are in TMEM
+  uint64_t* pv_done = p_ready + 2;          // the step's output product has finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const float* g_bias = args.bias + static_cast<size_t>(blockIdx.y) * (2 * args.S - 1);
 
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5;
-  const int T = args.T, H = args.H, S = args.S;
-  const int t0 = blockIdx.x * AB_T;
-  const int h = blockIdx.y;
-  const int HD = H * D;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
+  const int T = args.T, H = args.H, HD = H * D;
+  const int n_items = ((T + 2 * AB_T - 1) / (2 * AB_T)) * H;
 
   if (tid == 0) {
-    mbar_init(bar_q, 1);
-    mbar_init(&bar_kv[0], 1);
-    mbar_init(&bar_kv[1], 1);
-    mbar_init(bar_s, 1);
-    mbar_init(bar_o, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 2);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_free[i], 4);
+      mbar_init(&p_ready[i], 4);
+      mbar_init(&pv_done[i], 1);
+    }
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(&k_full[i], 1);
+      mbar_init(&k_empty[i], 2);
+      mbar_init(&v_full[i], 1);
+      mbar_init(&v_empty[i], 2);
+    }
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
-    tma_prefetch_desc(&tmQKV);
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmKV);
+    tma_prefetch_desc(&tmO);
   }
-  if (warp == 1) {
+  if (warp == AB_MMA_WARP) {
     __syncwarp();
-    tmem_alloc(tmem_slot, 256);
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tS = tmem_base;        // KC columns
-  const uint32_t tO = tmem_base + 128;  // D columns
+  // columns: S0 [0,64), S1 [64,128), P0 [128,160), P1 [160,192), O0 [256,256+D), O1 [384,384+D)
 
-  const int row = t0 + tid;
-  const bool row_ok = row < T;
-  int lo = 0, hi = 0;
-  if (row_ok) {
-    lo = args.seq_start[row];
-    hi = args.seq_end[row];
-  }
-  const int last = min(t0 + AB_T - 1, T - 1);
-  // key range of the tile: union over its rows (rows of one padded sequence share a range; a tile
-  // may span several sequences)
-  int kv_lo = args.seq_start[t0], kv_hi = args.seq_end[last];
-  {
-    int* s_rng = reinterpret_cast<int*>(bars + 6);  // [lo, hi]
-    if (tid == 0) {
-      s_rng[0] = kv_lo;
-      s_rng[1] = kv_hi;
-    }
-    __syncthreads();
-    if (row_ok) {
-      atomicMin(&s_rng[0], lo);
-      atomicMax(&s_rng[1], hi);
-    }
-    __syncthreads();
-    kv_lo = s_rng[0];
-    kv_hi = s_rng[1];
-  }
-  const int n_kv = kv_hi > kv_lo ? (kv_hi - kv_lo + KC - 1) / KC : 0;
-
-  constexpr uint32_t idesc_s = make_idesc_bf16(128, KC, 0, 0);
-  constexpr uint32_t idesc_o = make_idesc_bf16(128, D, 0, 1);
-  const int colQ = h * D, colK = HD + h * D, colV = 2 * HD + h * D;
-
-  auto load_q = [&](uint8_t* dst, uint64_t* bar, int col, int r0) {
+  if (warp == AB_LOADER_WARP) {
+    // ------------------------------------------------------------------ loader
+    uint32_t qc = 0, kc = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++qc) {
+      const int h = item % H, pair = item / H;
+      const AbGeo g = ab_geometry(args, pair, lane);
+      if (elect_one()) {
+        const int colQ = h * D, colK = HD + h * D, colV = 2 * HD + h * D;
+        const uint32_t qb = qc & 1u;
+        const int t0 = pair * 2 * AB_T;
+        if (!mbar_wait(&q_empty[qb], ((qc >> 1) & 1u) ^ 1u)) ok = false;
+        if (ok) {
+          const int nq = t0 + AB_T < T ? 2 : 1;
+          mbar_arrive_expect_tx(&q_full[qb], nq * C::Q_TILE);
+          for (int i = 0; i < nq; ++i)
 #pragma unroll
-    for (int a = 0; a < NA; ++a) tma_load_2d(dst + a * AB_TILE, &tmQKV, bar, col + a * 64, r0);
-  };
-  auto load_tile = [&](uint8_t* dst, uint64_t* bar, int col, int r0) {   // KC rows
-#pragma unroll
-    for (int a = 0; a < NA; ++a) tma_load_2d(dst + a * KA, &tmKV, bar, col + a * 64, r0);
-  };
-  auto issue_s = [&](int buf) {
-    const uint32_t qa = smem_u32(sQ), ka = smem_u32(sK + buf * OP);
-#pragma unroll
-    for (int k = 0; k < D / 16; ++k)
-      umma_bf16(tS, make_smem_desc(qa + (k >> 2) * AB_TILE + (k & 3) * 32, 16, 1024),
-                make_smem_desc(ka + (k >> 2) * KA + (k & 3) * 32, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
-    umma_commit(bar_s);
-  };
-
-  if (tid == 0 && n_kv > 0) {
-    mbar_arrive_expect_tx(bar_q, QB);
-    load_q(sQ, bar_q, colQ, t0);
-    mbar_arrive_expect_tx(&bar_kv[0], 2 * OP);
-    load_tile(sK, &bar_kv[0], colK, kv_lo);
-    load_tile(sV, &bar_kv[0], colV, kv_lo);
-    if (mbar_wait(bar_q, 0) && mbar_wait(&bar_kv[0], 0)) {
-      tc_fence_after();
-      issue_s(0);
-    } else {
-      atomicExch(args.status, ST_TIMEOUT_FULL);
-      *abort_flag = 1;
-    }
-  }
-  __syncwarp();
-
-  const float sl2 = args.scale * AB_LOG2E;
-  const int boff = S - 1 - row;  // bias index = key + boff
-  float m_run = -1e30f, l_run = 0.f;
-  float o[D];
-#pragma unroll
-  for (int e = 0; e < D; ++e) o[e] = 0.f;
-  const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
-
-  bool alive = true;
-  for (int j = 0; j < n_kv && alive; ++j) {
-    const int buf = j & 1;
-    const int kv0 = kv_lo + j * KC;
-    if (tid == 0 && j + 1 < n_kv) {
-      mbar_arrive_expect_tx(&bar_kv[buf ^ 1], 2 * OP);
-      load_tile(sK + (buf ^ 1) * OP, &bar_kv[buf ^ 1], colK, kv0 + KC);
-      load_tile(sV + (buf ^ 1) * OP, &bar_kv[buf ^ 1], colV, kv0 + KC);
-    }
-    __syncwarp();
-    bool ok = mbar_wait(bar_s, j & 1);
-    ok = __syncthreads_and(ok && *abort_flag == 0);
-    if (!ok) {
-      if (tid == 0) atomicExch(args.status, ST_TIMEOUT_TMEM_FULL);
-      alive = false;
-      break;
-    }
-    tc_fence_after();
-
-    // pass 1: row maximum of scale * s + bias over the valid keys (log2 domain)
-    float tmax = -1e30f;
-#pragma unroll 1
-    for (int c = 0; c < KC; c += 32) {
-      uint32_t r[32];
-      tmem_ld32(tS + lane_addr + c, r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int e = 0; e < 32; ++e) {
-        const int col = kv0 + c + e;
-        if (col >= lo && col < hi)
-          tmax = fmaxf(tmax, fmaf(__uint_as_float(r[e]), sl2, __ldg(g_bias + col + boff) * AB_LOG2E));
-      }
-    }
-    const float m_new = fmaxf(m_run, tmax);
-    const float alpha = exp2f(m_run - m_new);
-    float psum = 0.f;
-    // pass 2: probabilities -> bf16 -> swizzled shared memory
-#pragma unroll 1
-    for (int c = 0; c < KC; c += 32) {
-      uint32_t r[32];
-      tmem_ld32(tS + lane_addr + c, r);
-      tmem_ld_wait();
-      uint32_t packed[16];
-#pragma unroll
-      for (int e = 0; e < 32; e += 2) {
-        float p[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int col = kv0 + c + e + u;
-          p[u] = 0.f;
-          if (col >= lo && col < hi)
-            p[u] = exp2f(fmaf(__uint_as_float(r[e + u]), sl2, __ldg(g_bias + col + boff) * AB_LOG2E) - m_new);
+            for (int x = 0; x < NA; ++x)
+              tma_load_2d(sQ + (qb * 2 + i) * C::Q_TILE + x * AB_TILE, &tmQ, &q_full[qb], colQ + x * 64, t0 + i * AB_T);
         }
-        psum += p[0] + p[1];
-        packed[e >> 1] = pack_bf16x2(p[0], p[1]);
-      }
-      uint8_t* blk = sP + (c >> 6) * AB_TILE;
-      const int chunk0 = ((c >> 5) & 1) * 4;
+        uint32_t k = kc;
+        for (int j = 0; j < g.n && ok; ++j, ++k) {
+          const uint32_t st = k % STAGES, ph = (k / STAGES) & 1u;
+          const int kv0 = g.kv_lo + j * AB_KC;
+          if (!mbar_wait(&k_empty[st], ph ^ 1u)) { ok = false; break; }
+          mbar_arrive_expect_tx(&k_full[st], C::KV_TILE);
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<uint4*>(blk + ab_swz(tid, chunk0 + q)) =
-            make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-    }
-    l_run = l_run * alpha + psum;
-    m_run = m_new;
+          for (int x = 0; x < NA; ++x)
+            tma_load_2d(sK + st * C::KV_TILE + x * C::KA, &tmKV, &k_full[st], colK + x * 64, kv0);
+          if (!mbar_wait(&v_empty[st], ph ^ 1u)) { ok = false; break; }
+          mbar_arrive_expect_tx(&v_full[st], C::KV_TILE);
 #pragma unroll
-    for (int e = 0; e < D; ++e) o[e] *= alpha;
-
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after();
-      const uint32_t pa = smem_u32(sP), va = smem_u32(sV + buf * OP);
-#pragma unroll
-      for (int k = 0; k < KC / 16; ++k)
-        umma_bf16(tO, make_smem_desc(pa + (k >> 2) * AB_TILE + (k & 3) * 32, 16, 1024),
-                  make_smem_desc(va + k * 2048, KA, 1024), idesc_o, k > 0 ? 1u : 0u);
-      umma_commit(bar_o);
-      if (j + 1 < n_kv) {
-        if (mbar_wait(&bar_kv[buf ^ 1], ((j + 1) >> 1) & 1)) {
-          tc_fence_after();
-          issue_s(buf ^ 1);
-        } else {
-          atomicExch(args.status, ST_TIMEOUT_FULL);
+          for (int x = 0; x < NA; ++x)
+            tma_load_2d(sV + st * C::KV_TILE + x * C::KA, &tmKV, &v_full[st], colV + x * 64, kv0);
+        }
+        if (!ok && *abort_flag == 0) {
+          atomicExch(args.status, ST_TIMEOUT_EMPTY);
           *abort_flag = 1;
         }
+        if (*abort_flag) ok = false;
       }
+      ok = __all_sync(0xffffffffu, ok);
+      kc += g.n;
     }
+  } else if (warp == AB_MMA_WARP || warp == AB_MMA_WARP + 1) {
+    // ------------------------------------------------------------------ MMA issuers, one per query tile
+    const int i = warp - AB_MMA_WARP;
+    constexpr uint32_t idesc_s = make_idesc_bf16(128, AB_KC, 0, 0);
+    constexpr uint32_t idesc_o = make_idesc_bf16(128, D, 0, 1);
+    const uint32_t tS = tmem_base + i * 64, tP = tmem_base + 128 + i * 32, tO = tmem_base + 256 + i * 128;
+    uint32_t qc = 0, kc = 0, s_cnt = 0, p_cnt = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++qc) {
+      const AbGeo g = ab_geometry(args, item / H, lane);
+      const int ja = i ? g.a[1] : g.a[0], jb = i ? g.b[1] : g.b[0];
+      if (elect_one()) {
+        int why = ST_TIMEOUT_FULL;
+        uint32_t sc = s_cnt, pc = p_cnt;
+        const uint32_t qb = qc & 1u;
+        if (!mbar_wait(&q_full[qb], (qc >> 1) & 1u)) ok = false;
+        const uint32_t qa = smem_u32(sQ + (qb * 2 + i) * C::Q_TILE);
+        for (int j = 0; j <= g.n && ok; ++j) {
+          if (j < g.n) {   // scores of step j
+            const uint32_t st = (kc + j) % STAGES, ph = ((kc + j) / STAGES) & 1u;
+            if (!mbar_wait(&k_full[st], ph)) { ok = false; break; }
+            if (j >= ja && j < jb) {
+              if (!mbar_wait(&s_free[i], (sc & 1u) ^ 1u)) { ok = false; why = ST_TIMEOUT_TMEM_EMPTY; break; }
+              tc_fence_after();
+              const uint32_t ka = smem_u32(sK + st * C::KV_TILE);
+#pragma unroll
+              for (int k = 0; k < D / 16; ++k)
+                umma_bf16(tS, make_smem_desc(qa + (k >> 2) * AB_TILE + (k & 3) * 32, 16, 1024),
+                          make_smem_desc(ka + (k >> 2) * C::KA + (k & 3) * 32, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
+              umma_commit(&s_full[i]);
+              ++sc;
+            }
+            umma_commit(&k_empty[st]);     // by both issuers
+          }
+          if (j >= 1) {    // output product of step j - 1
+            const int jj = j - 1;
+            const uint32_t st = (kc + jj) % STAGES, ph = ((kc + jj) / STAGES) & 1u;
+            if (!mbar_wait(&v_full[st], ph)) { ok = false; break; }
+            if (jj >= ja && jj < jb) {
+              if (!mbar_wait(&p_ready[i], pc & 1u)) { ok = false; why = ST_TIMEOUT_MISC; break; }
+              tc_fence_after();
+              const uint32_t va = smem_u32(sV + st * C::KV_TILE);
+#pragma unroll
+              for (int k = 0; k < AB_KC / 16; ++k)   // P: 8 columns per 16 keys; V (MN-major): 16 key rows = 2048 bytes
+                umma_bf16_ts(tO, tP + k * 8, make_smem_desc(va + k * 2048, C::KA, 1024), idesc_o,
+                             (jj > ja || k > 0) ? 1u : 0u);
+              umma_commit(&pv_done[i]);
+              ++pc;
+            }
+            umma_commit(&v_empty[st]);
+          }
+        }
+        if (!ok && *abort_flag == 0) {
+          atomicExch(args.status, why);
+          *abort_flag = 1;
+        }
+        if (*abort_flag) ok = false;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      kc += g.n;
+      s_cnt += jb - ja;
+      p_cnt += jb - ja;
+    }
+  } else if (warp < 8) {
+    // ------------------------------------------------------------------ softmax warpgroups
+    const int i = warp >> 2;
+    const int quarter = warp & 3;
+    const int rl = quarter * 32 + lane;                // row inside the tile
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t tS = tmem_base + i * 64 + lane_addr, tP = tmem_base + 128 + i * 32 + lane_addr;
+    const uint32_t tO = tmem_base + 256 + i * 128 + lane_addr;
+    float* tab = reinterpret_cast<float*>(smem + C::OFF_TAB) + i * AB_TAB;
+    const float sl2 = args.scale * AB_LOG2E;
+    const int S = args.S;
+    uint32_t qc = 0, s_cnt = 0, pv_cnt = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++qc) {
+      const int h = item % H, pair = item / H;
+      const AbGeo g = ab_geometry(args, pair, lane);
+      const int ja = i ? g.a[1] : g.a[0], jb = i ? g.b[1] : g.b[0];
+      const int row0 = pair * 2 * AB_T + i * AB_T;
+      const int row = row0 + rl;
+      int lo = 0, hi = 0;
+      if (row < T) {
+        lo = __ldg(args.seq_start + row);
+        hi = __ldg(args.seq_end + row);
+      }
+      const float* gb = args.bias + static_cast<size_t>(h) * (2 * S - 1);
+      // tab[t] = bias of (key - row) = kbase - (row0 + 127) + t: thread rl finds key kbase + u at tab[u + 127 - rl].
+      // Entries outside the table belong to keys of other sequences and are masked.
+      const int kbase = g.kv_lo + ja * AB_KC;
+      const int len = (jb - ja) * AB_KC + 127;
+      const bool in_smem = len <= AB_TAB;
+      if (in_smem) {
+        const int first = kbase - row0 - 127 + S - 1;
+        for (int t = rl; t < len; t += 128) {
+          const int x = first + t;
+          tab[t] = (x >= 0 && x < 2 * S - 1) ? __ldg(gb + x) * AB_LOG2E : 0.f;
+        }
+      }
+      ok = ab_barrier_and(1 + i, *abort_flag == 0);
+      if (!ok) break;
+      float m_used = -1e30f, l_run = 0.f;
+      for (int j = ja; j < jb; ++j) {
+        const int kv0 = g.kv_lo + j * AB_KC;
+        ok = mbar_wait(&s_full[i], s_cnt & 1u);
+        ++s_cnt;
+        ok = __all_sync(0xffffffffu, ok && *abort_flag == 0);
+        if (!ok) break;
+        tc_fence_after();
+        const bool none = __all_sync(0xffffffffu, kv0 >= hi || kv0 + AB_KC <= lo);   // no row of the warp sees the block
+        uint32_t r[AB_KC];
+        if (!none) {
+          tmem_ld32(tS, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+          tmem_ld32(tS + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+          tmem_ld_wait();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[i]);   // the score tile may be overwritten
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (!none) {
+          const bool inside = kv0 >= lo && kv0 + AB_KC <= hi;
+          uint64_t bits = ~0ull;                  // bit e: key kv0 + e lies inside the row's range
+          if (!inside) {
+            const int x = max(lo - kv0, 0), y = min(hi - kv0, AB_KC);
+            bits = y > x ? (~0ull >> (64 - (y - x))) << x : 0ull;
+          }
+          if (in_smem) {
+            const float* tb = tab + (j - ja) * AB_KC + 127 - rl;
+#pragma unroll
+            for (int e = 0; e < AB_KC; ++e) r[e] = __float_as_uint(fmaf(__uint_as_float(r[e]), sl2, tb[e]));
+          } else {
+            const float* tb = gb + (kv0 - row + S - 1);
+#pragma unroll
+            for (int e = 0; e < AB_KC; ++e)
+              if ((bits >> e) & 1ull) r[e] = __float_as_uint(fmaf(__uint_as_float(r[e]), sl2, __ldg(tb + e) * AB_LOG2E));
+          }
+          if (!__all_sync(0xffffffffu, inside)) {
+#pragma unroll
+            for (int e = 0; e < AB_KC; ++e)
+              if (!((bits >> e) & 1ull)) r[e] = 0xff800000u;
+          }
+#pragma unroll
+          for (int e = 0; e < AB_KC; ++e) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(r[e]));
+        }
+        const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+        // the running maximum is only moved when a row has grown by 2^8: probabilities stay below 2^8, and most steps
+        // leave the output accumulator alone
+        const bool grow = __any_sync(0xffffffffu, m_new - m_used > 8.f);
+        float alpha = 1.f;
+        if (grow) {
+          alpha = exp2f(m_used - m_new);
+          m_used = m_new;
+        }
+        if (j > ja) {
+          // the previous output product has finished: P may be overwritten and O rescaled
+          ok = mbar_wait(&pv_done[i], pv_cnt & 1u);
+          ++pv_cnt;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+          if (grow) {
+#pragma unroll
+            for (int c = 0; c < D; c += 32) {
+              uint32_t o[32];
+              tmem_ld32(tO + c, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+              tmem_st32(tO + c, o);
+            }
+            tmem_st_wait();
+          }
+        }
+        float ps[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t pk[32];
+        if (!none) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            const float p0 = exp2f(__uint_as_float(r[2 * c]) - m_used), p1 = exp2f(__uint_as_float(r[2 * c + 1]) - m_used);
+            ps[c & 3] += p0 + p1;
+            pk[c] = pack_bf16x2(p0, p1);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) pk[c] = 0u;
+        }
+        tmem_st32(tP, pk);
+        tmem_st_wait();
+        l_run = l_run * alpha + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[i]);
+      }
+      if (ok && jb > ja) {
+        ok = mbar_wait(&pv_done[i], pv_cnt & 1u);   // the item's last output product
+        ++pv_cnt;
+      }
+      // the output leaves through this tile's Q buffer, which the finished score products no longer read
+      const uint32_t qb = qc & 1u;
+      ok = ab_barrier_and(1 + i, ok && *abort_flag == 0);
+      if (!ok) break;
+      tc_fence_after();
+      if (row0 < T) {
+        uint8_t* so = sQ + (qb * 2 + i) * C::Q_TILE;
+        const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+#pragma unroll
+        for (int c = 0; c < D; c += 32) {
+          uint32_t o[32];
+          if (jb > ja) {
+            tmem_ld32(tO + c, o);
+            tmem_ld_wait();
+          } else {
+            // no key for any row of the tile; the loads of Q still have to have landed before the buffer is written
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = 0u;
+            if (c == 0 && !mbar_wait(&q_full[qb], (qc >> 1) & 1u) && lane == 0) atomicExch(args.status, ST_TIMEOUT_FULL);
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e += 8) {
+            uint4 u;
+            uint32_t* p = reinterpret_cast<uint32_t*>(&u);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              p[q] = pack_bf16x2(__uint_as_float(o[e + 2 * q]) * inv, __uint_as_float(o[e + 2 * q + 1]) * inv);
+            *reinterpret_cast<uint4*>(so + (c >> 6) * AB_TILE + ab_swz(rl, ((c & 63) + e) >> 3)) = u;
+          }
+        }
+        tc_fence_before();
+        fence_proxy_async_smem();
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + i) : "memory");
+        if (quarter == 0 && elect_one()) {            // rows past the end of the batch are clipped
+#pragma unroll
+          for (int x = 0; x < NA; ++x) tma_store_2d(&tmO, so + x * AB_TILE, h * D + x * 64, row0);
+          tma_store_commit();
+          tma_store_wait_read<0>();
+        }
+      }
+      if (quarter == 0 && elect_one()) mbar_arrive(&q_empty[qb]);
+    }
+    if (quarter == 0 && elect_one()) tma_store_wait<0>();
     __syncwarp();
-    ok = mbar_wait(bar_o, j & 1);
-    ok = __syncthreads_and(ok && *abort_flag == 0);
-    if (!ok) {
-      if (tid == 0) atomicExch(args.status, ST_TIMEOUT_TMEM_FULL);
-      alive = false;
-      break;
-    }
-    tc_fence_after();
-#pragma unroll
-    for (int c = 0; c < D; c += 32) {
-      uint32_t r[32];
-      tmem_ld32(tO + lane_addr + c, r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int e = 0; e < 32; ++e) o[c + e] += __uint_as_float(r[e]);
-    }
-    tc_fence_before();
-  }
-
-  if (row_ok && alive) {
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-    __nv_bfloat16* dst = args.out + static_cast<size_t>(row) * HD + h * D;
-#pragma unroll
-    for (int e = 0; e < D; e += 8) {
-      uint4 u;
-      uint32_t* p = reinterpret_cast<uint32_t*>(&u);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) p[q] = pack_bf16x2(o[e + 2 * q] * inv, o[e + 2 * q + 1] * inv);
-      *reinterpret_cast<uint4*>(dst + e) = u;
+    if (!ok && lane == 0 && *abort_flag == 0) {
+      atomicExch(args.status, ST_TIMEOUT_TMEM_FULL);
+      *abort_flag = 1;
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == AB_MMA_WARP) {
     tc_fence_after();
     __syncwarp();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -323,19 +504,22 @@ static AbEncodeFn ab_encode_fn() {
   return fn;
 }
 
-template <int D, int KC>
-static int ab_launch(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const AbArgs& a, cudaStream_t st) {
-  constexpr int smem = ab_smem_bytes<D, KC>();
+template <int D>
+static int ab_launch(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const CUtensorMap& tmO, const AbArgs& a,
+                     cudaStream_t st) {
+  constexpr int smem = AbCfg<D>::SMEM;
   static bool configured_on[nplm::MAX_DEVICES];
   const int dev_slot = nplm::current_device_slot();
   if (dev_slot < 0) return -4;
   bool& configured = configured_on[dev_slot];
   if (!configured) {
-    NPLM_CUDA_CHECK(cudaFuncSetAttribute(fa_bias_fwd_kernel<D, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NPLM_CUDA_CHECK(cudaFuncSetAttribute(fa_bias_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured = true;
   }
-  dim3 grid((a.T + AB_T - 1) / AB_T, a.H);
-  fa_bias_fwd_kernel<D, KC><<<grid, 128, smem, st>>>(tmQ, tmKV, a);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_slot);
+  const int n_items = ((a.T + 2 * AB_T - 1) / (2 * AB_T)) * a.H;
+  fa_bias_fwd_kernel<D><<<n_items < sms ? n_items : sms, AB_THREADS, smem, st>>>(tmQ, tmKV, tmO, a);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -349,25 +533,22 @@ extern "C" int nplm_fa_bias_fwd(const void* qkv, void* out, const int* seq_start
                                 cudaStream_t st) {
   if (T <= 0) return 0;
   if ((D != 64 && D != 128) || S < 1 || (reinterpret_cast<uintptr_t>(qkv) & 15)) return -3;
+  if ((reinterpret_cast<uintptr_t>(out) & 15) || H <= 0) return -3;
   AbEncodeFn fn = ab_encode_fn();
   if (fn == nullptr) return -1;
-  CUtensorMap tmQ, tmKV;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(3) * H * D, static_cast<cuuint64_t>(T)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(3) * H * D * 2};
-  cuuint32_t estr[2] = {1, 1};
-  const cuuint32_t kc = D == 64 ? 128 : 64;     // key rows per K / V box
-  cuuint32_t box_q[2] = {64, AB_T};
-  cuuint32_t box_kv[2] = {64, kc};
-  if (fn(&tmQ, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(qkv), dims, strides, box_q, estr,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return -2;
-  if (fn(&tmKV, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(qkv), dims, strides, box_kv, estr,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return -2;
+  auto make = [&](CUtensorMap* map, const void* base, uint64_t cols, uint32_t rows) {
+    cuuint64_t dims[2] = {cols, static_cast<cuuint64_t>(T)};
+    cuuint64_t strides[1] = {cols * 2};
+    cuuint32_t estr[2] = {1, 1};
+    cuuint32_t box[2] = {64, rows};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  CUtensorMap tmQ, tmKV, tmO;
+  const uint64_t cols = static_cast<uint64_t>(H) * D;
+  if (!make(&tmQ, qkv, 3 * cols, AB_T) || !make(&tmKV, qkv, 3 * cols, AB_KC) || !make(&tmO, out, cols, AB_T)) return -2;
   AbArgs a;
-  a.out = reinterpret_cast<__nv_bfloat16*>(out);
   a.seq_start = seq_start;
   a.seq_end = seq_end;
   a.bias = bias;
@@ -376,5 +557,5 @@ extern "C" int nplm_fa_bias_fwd(const void* qkv, void* out, const int* seq_start
   a.S = S;
   a.scale = scale;
   a.status = status;
-  return D == 64 ? ab_launch<64, 128>(tmQ, tmKV, a, st) : ab_launch<128, 64>(tmQ, tmKV, a, st);
+  return D == 64 ? ab_launch<64>(tmQ, tmKV, tmO, a, st) : ab_launch<128>(tmQ, tmKV, tmO, a, st);
 }

@@ -8,7 +8,7 @@ Module / parameter names equal HF `T5EncoderModel` (`shared`, `encoder.block.N.l
 benchmarks and offline machines use `random_init=True`. The reference wraps HF's implementation and
 torch.compile (src/nanoplm/distillation/models/teacher/prott5.py:14-70); here the linear layers run
 on the tcgen05 GEMM (ReLU and residual adds fused where the epilogue allows) and the norms on the
-RMSNorm kernel. The bias-added attention uses PyTorch SDPA (a library call).
+RMSNorm kernel. The bias-added attention runs in csrc/attention_bias.cu; on the CPU it is PyTorch SDPA.
 """
 from __future__ import annotations
 
