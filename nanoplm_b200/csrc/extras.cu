@@ -47,11 +47,14 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
 
 constexpr int MAX_KS = 9;
 
-// flip = 0: forward (tap k reads t + k - r);  flip = 1: input gradient (tap k reads t - (k - r))
+// flip = 0: forward (tap k reads t + k - r);  flip = 1: input gradient (tap k reads t - (k - r));
+// residual: the input itself is added (y = x + conv(x), dx = dy + conv^T(dy)): one more on the centre tap, which always
+// lies inside the token's own sequence.
 __global__ void __launch_bounds__(256)
 dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
               const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
-              const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int KS, int flip) {
+              const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int KS, int flip,
+              int residual) {
   const int vec = C >> 3;
   const int r = KS >> 1;
   const long long total = static_cast<long long>(T) * vec;
@@ -73,7 +76,8 @@ dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       float xv[8];
       ld8(x + static_cast<size_t>(src) * C + c, xv);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += xv[e] * __bfloat162float(w[(c + e) * KS + k]);
+      for (int e = 0; e < 8; ++e)
+        acc[e] += xv[e] * (__bfloat162float(w[(c + e) * KS + k]) + (residual && k == r ? 1.f : 0.f));
     }
     st8(y + static_cast<size_t>(t) * C + c, acc);
   }
@@ -88,7 +92,8 @@ template <int KS>
 __global__ void __launch_bounds__(256)
 dwconv_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
-                   const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip) {
+                   const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip,
+                   int residual) {
   constexpr int R = KS / 2;
   const int vec = C >> 3;
   const int n_tb = (T + DW_TT - 1) / DW_TT;
@@ -116,6 +121,10 @@ dwconv_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
       for (int e = 0; e < 8; ++e)
 #pragma unroll
         for (int k = 0; k < KS; ++k) wt[k][e] = __bfloat162float(wl[e * KS + (flip ? KS - 1 - k : k)]);
+      if (residual) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) wt[R][e] += 1.f;
+      }
     }
     float acc[DW_TT][8];
     int lo[DW_TT], hi[DW_TT];
@@ -504,7 +513,7 @@ static int grid_for(long long work, int threads) {
 using namespace nplm;
 
 extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const int* s_start,
-                           const int* s_end, void* y, int T, int C, int KS, int flip, cudaStream_t st) {
+                           const int* s_end, void* y, int T, int C, int KS, int flip, int residual, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || KS < 1 || KS > MAX_KS || !(KS & 1)) return -3;
   const bool aligned = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
@@ -513,7 +522,8 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
 #define NPLM_DWCONV(KS_)                                                                                   \
   dwconv_tile_kernel<KS_><<<grid, 256, 0, st>>>(                                                           \
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),                \
-      reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip)
+      reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip,     \
+      residual)
     switch (KS) {
       case 3: NPLM_DWCONV(3); break;
       case 5: NPLM_DWCONV(5); break;
@@ -526,7 +536,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
   dwconv_kernel<<<grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
       reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C,
-      KS, flip);
+      KS, flip, residual);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -691,6 +701,23 @@ namespace nplm {
 
 constexpr int MHC_MAX_ITERS = 8;
 
+// The static parts a [N], b [N], r [N*N] and scales s [3] of a site as fp32, read from fp32 or bf16 parameters.
+template <int N, typename P>
+struct MhcStatic {
+  float a[N], b[N], r[N * N], s[3];
+  __device__ __forceinline__ MhcStatic(const P* pa, const P* pb, const P* pr, const P* ps) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      a[i] = static_cast<float>(pa[i]);
+      b[i] = static_cast<float>(pb[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N * N; ++i) r[i] = static_cast<float>(pr[i]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s[i] = static_cast<float>(ps[i]);
+  }
+};
+
 template <int N>
 __device__ __forceinline__ void mhc_coef_forward(const float (&d)[2 * N + N * N], const float* a, const float* b,
                                                  const float* r, const float* s, int iters,
@@ -748,19 +775,19 @@ __device__ __forceinline__ void mhc_coef_forward(const float (&d)[2 * N + N * N]
   }
 }
 
-template <int N>
+template <int N, typename P>
 __global__ void __launch_bounds__(128)
-mhc_coef_fwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restrict__ a,
-                    const float* __restrict__ b, const float* __restrict__ r, const float* __restrict__ s,
-                    int iters, int T, float* __restrict__ alpha_out, float* __restrict__ beta_out,
+mhc_coef_fwd_kernel(const __nv_bfloat16* __restrict__ pre, const P* __restrict__ pa, const P* __restrict__ pb,
+                    const P* __restrict__ pr, const P* __restrict__ ps, int iters, int T, float* __restrict__ alpha_out, float* __restrict__ beta_out,
                     float* __restrict__ R_out) {
   constexpr int M = 2 * N + N * N;
+  const MhcStatic<N, P> st(pa, pb, pr, ps);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
     float d[M];
 #pragma unroll
     for (int i = 0; i < M; ++i) d[i] = tanhf(__bfloat162float(pre[static_cast<size_t>(t) * M + i]));
     float alpha[N], beta[N], x[N * N];
-    mhc_coef_forward<N>(d, a, b, r, s, iters, alpha, beta, x, nullptr);
+    mhc_coef_forward<N>(d, st.a, st.b, st.r, st.s, iters, alpha, beta, x, nullptr);
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       alpha_out[t * N + i] = alpha[i];
@@ -771,16 +798,16 @@ mhc_coef_fwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restri
   }
 }
 
-template <int N>
+template <int N, typename P>
 __global__ void __launch_bounds__(128)
-mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restrict__ a,
-                    const float* __restrict__ b, const float* __restrict__ r, const float* __restrict__ s,
-                    int iters, int T, const float* __restrict__ dalpha, const float* __restrict__ dbeta,
+mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const P* __restrict__ pa, const P* __restrict__ pb,
+                    const P* __restrict__ pr, const P* __restrict__ ps, int iters, int T, const float* __restrict__ dalpha, const float* __restrict__ dbeta,
                     const float* __restrict__ dR, __nv_bfloat16* __restrict__ dpre,
                     float* __restrict__ da, float* __restrict__ db, float* __restrict__ dr,
                     float* __restrict__ ds) {
   constexpr int M = 2 * N + N * N;
   static_assert(M + 3 <= 32, "parameter gradients are reduced with one value per lane");
+  const MhcStatic<N, P> st(pa, pb, pr, ps);
   // per-thread sums of the parameter gradients: [da (N) | db (N) | dr (N*N) | ds (3)]
   float acc[32];
 #pragma unroll
@@ -796,7 +823,7 @@ mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restri
       for (int i = 0; i < M; ++i) d[i] = tanhf(__bfloat162float(pre[static_cast<size_t>(t) * M + i]));
       float alpha[N], beta[N], x[N * N];
       float hist[2 * MHC_MAX_ITERS * N * N];
-      mhc_coef_forward<N>(d, a, b, r, s, iters, alpha, beta, x, hist);
+      mhc_coef_forward<N>(d, st.a, st.b, st.r, st.s, iters, alpha, beta, x, hist);
       float gd[M];   // gradient w.r.t. d (tanh output)
       // alpha = softmax(u): du = alpha * (dalpha - sum alpha * dalpha)
       float dot = 0.f;
@@ -807,7 +834,7 @@ mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restri
         const float du = alpha[i] * (dalpha[t * N + i] - dot);
         acc[i] += du;
         acc[2 * N + N * N] += du * d[i];
-        gd[i] = du * s[0];
+        gd[i] = du * st.s[0];
       }
       // beta = 2 sigmoid(v): dv = dbeta * beta * (1 - beta / 2)
 #pragma unroll
@@ -815,7 +842,7 @@ mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restri
         const float dv = dbeta[t * N + i] * beta[i] * (1.f - 0.5f * beta[i]);
         acc[N + i] += dv;
         acc[2 * N + N * N + 1] += dv * d[N + i];
-        gd[N + i] = dv * s[1];
+        gd[N + i] = dv * st.s[1];
       }
       // R = exp(x_final): dx = dR * R, then back through the half-steps
       float g[N * N];
@@ -845,7 +872,7 @@ mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restri
       for (int i = 0; i < N * N; ++i) {
         acc[2 * N + i] += g[i];
         acc[2 * N + N * N + 2] += g[i] * d[2 * N + i];
-        gd[2 * N + i] = g[i] * s[2];
+        gd[2 * N + i] = g[i] * st.s[2];
       }
 #pragma unroll
       for (int i = 0; i < M; ++i)
@@ -862,39 +889,54 @@ mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const float* __restri
 
 }  // namespace nplm
 
-extern "C" int nplm_mhc_coef_fwd(const void* pre, const float* a, const float* b, const float* r,
-                                 const float* s, int iters, int T, int n, float* alpha, float* beta,
-                                 float* R, cudaStream_t st) {
+namespace nplm {
+template <int N, typename P>
+static void mhc_coef_fwd_launch(const __nv_bfloat16* pre, const void* a, const void* b, const void* r, const void* s,
+                                int iters, int T, float* alpha, float* beta, float* R, int blocks, cudaStream_t st) {
+  mhc_coef_fwd_kernel<N, P><<<blocks, 128, 0, st>>>(pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
+                                                    reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters,
+                                                    T, alpha, beta, R);
+}
+template <int N, typename P>
+static void mhc_coef_bwd_launch(const __nv_bfloat16* pre, const void* a, const void* b, const void* r, const void* s,
+                                int iters, int T, const float* dalpha, const float* dbeta, const float* dR,
+                                __nv_bfloat16* dpre, float* da, float* db, float* dr, float* ds, int blocks,
+                                cudaStream_t st) {
+  mhc_coef_bwd_kernel<N, P><<<blocks, 128, 0, st>>>(pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
+                                                    reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters,
+                                                    T, dalpha, dbeta, dR, dpre, da, db, dr, ds);
+}
+}  // namespace nplm
+
+// a, b, r, s: the site's parameters, all fp32 (param_bf16 = 0) or all bf16 (1).
+extern "C" int nplm_mhc_coef_fwd(const void* pre, const void* a, const void* b, const void* r, const void* s,
+                                 int param_bf16, int iters, int T, int n, float* alpha, float* beta, float* R,
+                                 cudaStream_t st) {
   if (T <= 0) return 0;
   if (n != 4 && n != 2) return -3;
   if (iters < 1 || iters > nplm::MHC_MAX_ITERS) return -3;
   int blocks = (T + 127) / 128;
   if (blocks > 148 * 8) blocks = 148 * 8;
   const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(pre);
-  if (n == 4)
-    nplm::mhc_coef_fwd_kernel<4><<<blocks, 128, 0, st>>>(p, a, b, r, s, iters, T, alpha, beta, R);
-  else
-    nplm::mhc_coef_fwd_kernel<2><<<blocks, 128, 0, st>>>(p, a, b, r, s, iters, T, alpha, beta, R);
+  auto go = n == 4 ? (param_bf16 ? nplm::mhc_coef_fwd_launch<4, __nv_bfloat16> : nplm::mhc_coef_fwd_launch<4, float>)
+                   : (param_bf16 ? nplm::mhc_coef_fwd_launch<2, __nv_bfloat16> : nplm::mhc_coef_fwd_launch<2, float>);
+  go(p, a, b, r, s, iters, T, alpha, beta, R, blocks, st);
   return static_cast<int>(cudaGetLastError());
 }
 
-// da / db / dr / ds are accumulated (callers pass zeroed or running fp32 buffers)
-extern "C" int nplm_mhc_coef_bwd(const void* pre, const float* a, const float* b, const float* r,
-                                 const float* s, int iters, int T, int n, const float* dalpha,
-                                 const float* dbeta, const float* dR, void* dpre, float* da, float* db,
-                                 float* dr, float* ds, cudaStream_t st) {
+// da / db / dr / ds (fp32) are accumulated: callers pass zeroed or running buffers.
+extern "C" int nplm_mhc_coef_bwd(const void* pre, const void* a, const void* b, const void* r, const void* s,
+                                 int param_bf16, int iters, int T, int n, const float* dalpha, const float* dbeta,
+                                 const float* dR, void* dpre, float* da, float* db, float* dr, float* ds,
+                                 cudaStream_t st) {
   if (T <= 0) return 0;
   if (n != 4 && n != 2) return -3;
   if (iters < 1 || iters > nplm::MHC_MAX_ITERS) return -3;
   int blocks = (T + 127) / 128;
   if (blocks > 148 * 4) blocks = 148 * 4;
   const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(pre);
-  __nv_bfloat16* dp = reinterpret_cast<__nv_bfloat16*>(dpre);
-  if (n == 4)
-    nplm::mhc_coef_bwd_kernel<4><<<blocks, 128, 0, st>>>(p, a, b, r, s, iters, T, dalpha, dbeta, dR, dp, da, db,
-                                                         dr, ds);
-  else
-    nplm::mhc_coef_bwd_kernel<2><<<blocks, 128, 0, st>>>(p, a, b, r, s, iters, T, dalpha, dbeta, dR, dp, da, db,
-                                                         dr, ds);
+  auto go = n == 4 ? (param_bf16 ? nplm::mhc_coef_bwd_launch<4, __nv_bfloat16> : nplm::mhc_coef_bwd_launch<4, float>)
+                   : (param_bf16 ? nplm::mhc_coef_bwd_launch<2, __nv_bfloat16> : nplm::mhc_coef_bwd_launch<2, float>);
+  go(p, a, b, r, s, iters, T, dalpha, dbeta, dR, reinterpret_cast<__nv_bfloat16*>(dpre), da, db, dr, ds, blocks, st);
   return static_cast<int>(cudaGetLastError());
 }

@@ -1128,7 +1128,7 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
       (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(C) & 15))
     return -3;
-  if (a_mn && (M % 64)) return -4;
+  if (a_mn && (M % 8)) return -4;     // (columns past M are read as zeros, rows past M of C are not written)
   if (b_mn && (N % 64)) return -4;
   if (epi == EPI_SWIGLU && (b_mn || (N % 2) || ((N / 2) % 8))) return -4;
   if ((epi == EPI_ATOMIC_F32 || epi == EPI_STORE_F32) ? (N % 4 || ldc % 4) : (N % 8 || ldc % 8))

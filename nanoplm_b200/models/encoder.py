@@ -159,7 +159,7 @@ class EncoderLayer(nn.Module):
         if not normed:
             h = self.attn_norm(h)
         if self.conv is not None:
-            h = h + self.conv(h, ctx)
+            h = self.conv(h, ctx, residual=True)      # h + conv(h)
         return self.attn(h, ctx, window, rope, residual=residual)
 
     def forward(self, x, ctx: BatchContext, window: int, rope: tuple):

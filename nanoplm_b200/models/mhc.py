@@ -138,27 +138,33 @@ class _CoefFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, pre, a, b, r, s, iters, n):
         pre = pre.contiguous()
-        a32, b32, r32, s32 = (t.detach().float().contiguous() for t in (a, b, r, s))
-        alpha, beta, R = K.mhc_coef_fwd(pre, a32, b32, r32, s32, iters, n)
-        ctx.save_for_backward(pre, a32, b32, r32, s32)
+        params = tuple(t.detach() for t in (a, b, r, s))
+        if {t.dtype for t in params} != {torch.bfloat16} or not all(t.is_contiguous() for t in params):
+            params = tuple(t.float().contiguous() for t in params)
+        alpha, beta, R = K.mhc_coef_fwd(pre, *params, iters, n)
+        ctx.save_for_backward(pre, *params)
         ctx.iters, ctx.n = iters, n
         ctx.refs = (a, b, r, s)
         return alpha, beta, R
 
     @staticmethod
     def backward(ctx, dalpha, dbeta, dR):
-        from nanoplm_b200.ops.functional import _param_grad
-        pre, a32, b32, r32, s32 = ctx.saved_tensors
+        from nanoplm_b200.ops.functional import _has_main_grad, _param_grad
+        pre, *params = ctx.saved_tensors
         n, dev = ctx.n, pre.device
         T = pre.shape[0]
         zeros = lambda *shape: torch.zeros(shape, dtype=torch.float32, device=dev)
         dalpha = dalpha.float().contiguous() if dalpha is not None else zeros(T, n)
         dbeta = dbeta.float().contiguous() if dbeta is not None else zeros(T, n)
         dR = dR.float().contiguous() if dR is not None else zeros(T, n, n)
-        da, db, dr, ds = zeros(n), zeros(n), zeros(n, n), zeros(3)
-        dpre = K.mhc_coef_bwd(pre, a32, b32, r32, s32, ctx.iters, n, dalpha, dbeta, dR, da, db, dr, ds)
-        a, b, r, s = ctx.refs
-        return dpre, _param_grad(a, da), _param_grad(b, db), _param_grad(r, dr), _param_grad(s, ds), None, None
+        # the kernel adds to what it is given: the parameters' running gradients where they have them
+        direct = all(_has_main_grad(p) and p.main_grad.dtype == torch.float32 and p.main_grad.is_contiguous()
+                     for p in ctx.refs)
+        grads = tuple(p.main_grad if direct else zeros(*p.shape) for p in ctx.refs)
+        dpre = K.mhc_coef_bwd(pre, *params, ctx.iters, n, dalpha, dbeta, dR, *grads)
+        if direct:
+            return dpre, None, None, None, None, None, None
+        return (dpre, *(_param_grad(p, g) for p, g in zip(ctx.refs, grads)), None, None)
 
 
 class HyperConnection(nn.Module):

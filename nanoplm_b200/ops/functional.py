@@ -49,29 +49,21 @@ def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
     """dW[N,K] = dy2[T,N]^T x2[T,K]; accumulates into w.main_grad or returns a bf16 gradient."""
     T, N = dy2.shape
     Kd = x2.shape[1]
-    if N % 64 == 0 and Kd % 64 == 0:
-        if _has_main_grad(w):
+    # widths below a tile are fine too (a hyper-connection site's 2n + n^2 coefficients): 8-aligned rows for TMA
+    tiled = N % 64 == 0
+    narrow = not tiled and N % 8 == 0 and dy2.is_cuda and dy2.dtype == BF and x2.dtype == BF and dy2.data_ptr() % 16 == 0
+    if (tiled or narrow) and Kd % 64 == 0:
+        if _has_main_grad(w) and (tiled or w.main_grad.data_ptr() % 16 == 0):
             K.gemm(dy2, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=w.main_grad,
                    splits=K.wgrad_splits(N, Kd, T))
-            if _WGRAD_READY[0] is not None:
+            if tiled and _WGRAD_READY[0] is not None:
                 _WGRAD_READY[0](w)
             return None
         acc = torch.zeros((N, Kd), dtype=torch.float32, device=w.device)
         K.gemm(dy2, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=acc,
                splits=K.wgrad_splits(N, Kd, T))
-        return acc.to(w.dtype)
-    if Kd % 64 == 0 and N < 256 and dy2.is_cuda and dy2.dtype == BF and x2.dtype == BF:
-        # narrow outputs (the 2n + n^2 coefficient projection of a hyper-connection site, a router):
-        # pad the output columns to a whole 64 so the tensor-core kernel applies instead of an fp32
-        # library GEMM over fp32 copies of both operands
-        Np = (N + 63) // 64 * 64
-        dyp = torch.zeros((T, Np), dtype=BF, device=dy2.device)
-        dyp[:, :N] = dy2
-        acc = torch.zeros((Np, Kd), dtype=torch.float32, device=w.device)
-        K.gemm(dyp, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=acc, splits=K.wgrad_splits(Np, Kd, T))
-        g = acc[:N]
-    else:
-        g = dy2.float().t() @ x2.float()
+        return _param_grad(w, acc)
+    g = dy2.float().t() @ x2.float()
     if _has_main_grad(w):
         w.main_grad.add_(g)
         return None

@@ -576,12 +576,13 @@ def check_status() -> None:
 
 
 # --------------------------------------------------------------------------- conv / mHC
-def dwconv(x, w, bias, seq_start, seq_end, flip=False):
+def dwconv(x, w, bias, seq_start, seq_end, flip=False, residual=False):
+    """Varlen depthwise convolution (flip: its input gradient); residual adds the input itself."""
     T, C = x.shape
     KS = w.shape[1]
     y = torch.empty_like(x)
     rc = lib("extras").nplm_dwconv(ptr(x), ptr(w), ptr(bias), ptr(seq_start), ptr(seq_end), ptr(y), c_int(T),
-                                   c_int(C), c_int(KS), c_int(int(flip)), stream_ptr())
+                                   c_int(C), c_int(KS), c_int(int(flip)), c_int(int(residual)), stream_ptr())
     check_rc(rc, "dwconv")
     count_launch()
     return y
@@ -657,16 +658,24 @@ def mhc_bwd(X, y, R, alpha, beta, dXn, dh, want_dx: bool = True):
 
 
 # --------------------------------------------------------------------------- device-side MLM masking
+def _coef_bf16(*params) -> int:
+    """1 when the parameters are all bf16, 0 when all fp32."""
+    kinds = {p.dtype for p in params}
+    if kinds not in ({_BF16}, {torch.float32}) or not all(p.is_contiguous() for p in params):
+        raise ValueError("the static parameters must be contiguous and of one type, fp32 or bf16")
+    return int(kinds == {_BF16})
+
+
 def mhc_coef_fwd(pre, a, b, r, s, iters: int, n: int):
     """Raw coefficient projections pre bf16 [T, 2n+n*n] -> (alpha [T,n], beta [T,n], R [T,n,n]) fp32.
-    a, b [n], r [n,n], s [3]: fp32 static parts and dynamic scales."""
+    a, b [n], r [n,n], s [3]: static parts and dynamic scales, all fp32 or all bf16, contiguous."""
     _chk(pre, _BF16, "pre")
     T = pre.shape[0]
     dev = pre.device
     alpha = torch.empty((T, n), dtype=torch.float32, device=dev)
     beta = torch.empty((T, n), dtype=torch.float32, device=dev)
     R = torch.empty((T, n, n), dtype=torch.float32, device=dev)
-    rc = lib("extras").nplm_mhc_coef_fwd(ptr(pre), ptr(a), ptr(b), ptr(r), ptr(s), c_int(iters), c_int(T),
+    rc = lib("extras").nplm_mhc_coef_fwd(ptr(pre), ptr(a), ptr(b), ptr(r), ptr(s), c_int(_coef_bf16(a, b, r, s)), c_int(iters), c_int(T),
                                          c_int(n), ptr(alpha), ptr(beta), ptr(R), stream_ptr())
     check_rc(rc, "mhc_coef_fwd")
     count_launch()
@@ -677,7 +686,7 @@ def mhc_coef_bwd(pre, a, b, r, s, iters: int, n: int, dalpha, dbeta, dR, da, db,
     """Backward of mhc_coef_fwd. Returns dpre (bf16); da, db, dr, ds (fp32) are accumulated in place."""
     T = pre.shape[0]
     dpre = torch.empty_like(pre)
-    rc = lib("extras").nplm_mhc_coef_bwd(ptr(pre), ptr(a), ptr(b), ptr(r), ptr(s), c_int(iters), c_int(T),
+    rc = lib("extras").nplm_mhc_coef_bwd(ptr(pre), ptr(a), ptr(b), ptr(r), ptr(s), c_int(_coef_bf16(a, b, r, s)), c_int(iters), c_int(T),
                                          c_int(n), ptr(dalpha), ptr(dbeta), ptr(dR), ptr(dpre), ptr(da), ptr(db),
                                          ptr(dr), ptr(ds), stream_ptr())
     check_rc(rc, "mhc_coef_bwd")

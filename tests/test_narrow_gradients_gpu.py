@@ -1,0 +1,80 @@
+"""Weight gradients narrower than a tile, the residual form of the depthwise convolution, and coefficient parameters
+read in bf16 with their gradients added in place."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("N", [8, 24, 40, 72, 136])
+@pytest.mark.parametrize("T,Kd", [(64, 64), (333, 192), (5000, 768)])
+@pytest.mark.parametrize("main_grad", [False, True])
+def test_narrow_weight_gradient(N, T, Kd, main_grad, cuda_status):
+    from nanoplm_b200.ops.functional import _wgrad
+    g = torch.Generator(device="cuda").manual_seed(N + T)
+    dy = torch.randn(T, N, device="cuda", generator=g).to(BF)
+    x = torch.randn(T, Kd, device="cuda", generator=g).to(BF)
+    w = torch.nn.Parameter(torch.zeros(N, Kd, device="cuda", dtype=BF))
+    want = dy.double().t() @ x.double()
+    mag = dy.double().abs().t() @ x.double().abs()
+    if main_grad:
+        w.main_grad = torch.ones(N, Kd, device="cuda")
+        assert _wgrad(dy, x, w) is None
+        # fp32 sums of T products
+        assert ((w.main_grad.double() - 1 - want).abs() <= mag * T * 2 ** -24 + 1e-5).all()
+    else:
+        got = _wgrad(dy, x, w)
+        assert got.dtype == BF
+        assert ((got.double() - want).abs() <= mag * T * 2 ** -24 + want.abs() * 2 ** -8 + 1e-5).all()
+
+
+@pytest.mark.parametrize("KS", [3, 7, 9, 1])
+@pytest.mark.parametrize("lens", [[1, 2, 3], [40, 7, 129]])
+def test_residual_convolution(KS, lens, cuda_status):
+    from nanoplm_b200.models.conv import dwconv_reference, dwconv_varlen
+    from nanoplm_b200.ops import functional as ops
+    T, C = sum(lens), 64
+    cu = torch.tensor([0, *lens]).cumsum(0).to(torch.int32).cuda()
+    ss, se = ops.seq_bounds(cu, T)
+    g = torch.Generator(device="cuda").manual_seed(KS)
+    x = torch.randn(T, C, device="cuda", generator=g).to(BF).requires_grad_(True)
+    w = (torch.randn(C, KS, device="cuda", generator=g) * 0.3).to(BF).requires_grad_(True)
+    gy = torch.randn(T, C, device="cuda", generator=g).to(BF)
+    y = dwconv_varlen(x, w, None, ss, se, residual=True)
+    y.backward(gy)
+    xr, wr = x.detach().float().requires_grad_(True), w.detach().float().requires_grad_(True)
+    ref = xr + dwconv_reference(xr, wr, None, ss, se)
+    ref.backward(gy.float())
+    # fp32 sums of at most ten terms, one bf16 rounding
+    assert torch.allclose(y.float(), ref, rtol=2 ** -8, atol=1e-4)
+    assert torch.allclose(x.grad.float(), xr.grad, rtol=2 ** -8, atol=1e-4)
+    assert torch.allclose(w.grad.float(), wr.grad, rtol=2 ** -7, atol=1e-3)
+
+
+@pytest.mark.parametrize("n", [2, 4])
+def test_coefficient_parameters_in_bf16(n, cuda_status):
+    from nanoplm_b200.models.mhc import _CoefFn
+    g = torch.Generator(device="cuda").manual_seed(n)
+    T = 300
+    pre = torch.randn(T, 2 * n + n * n, device="cuda", generator=g).to(BF)
+    params = [torch.nn.Parameter(torch.randn(*s, device="cuda", generator=g).to(BF)) for s in ((n,), (n,), (n, n), (3,))]
+    outs = []
+    for kind in ("bf16", "fp32", "main_grad"):
+        ps = [torch.nn.Parameter(p.detach().float() if kind == "fp32" else p.detach().clone()) for p in params]
+        if kind == "main_grad":
+            for p in ps:
+                p.main_grad = torch.ones(p.shape, device="cuda")
+        x = pre.clone().requires_grad_(True)
+        alpha, beta, R = _CoefFn.apply(x, *ps, 5, n)
+        (alpha.square().sum() + beta.square().sum() + (R * R).sum()).backward()
+        grads = [(p.main_grad - 1) if kind == "main_grad" else p.grad.float() for p in ps]
+        outs.append((alpha, beta, R, x.grad, grads))
+    for o in outs[1:]:
+        for a, b in zip(o[:4], outs[1][:4]):
+            assert torch.equal(a, b)                      # the same fp32 values enter
+    for a, b in zip(outs[0][4], outs[1][4]):
+        assert torch.allclose(a, b, rtol=2 ** -8, atol=1e-3)        # returned in bf16
+    for a, b in zip(outs[2][4], outs[1][4]):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-3)           # atomics in another order
