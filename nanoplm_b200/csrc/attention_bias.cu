@@ -541,9 +541,11 @@ extern "C" int nplm_fa_bias_fwd(const void* qkv, void* out, const int* seq_start
     cuuint64_t strides[1] = {cols * 2};
     cuuint32_t estr[2] = {1, 1};
     cuuint32_t box[2] = {64, rows};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return nplm::with_context([&] {
+             return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+           }) == CUDA_SUCCESS;
   };
   CUtensorMap tmQ, tmKV, tmO;
   const uint64_t cols = static_cast<uint64_t>(H) * D;

@@ -1527,9 +1527,9 @@ static int ws_make_map_f32(CUtensorMap* map, const void* base, uint64_t cols, ui
   cuuint64_t strides[1] = {cols * 4};
   cuuint32_t box[2] = {32, FA_T};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides,
+  CUresult r = nplm::with_context([&] { return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
@@ -1540,9 +1540,9 @@ static int ws_make_map(CUtensorMap* map, const void* base, uint64_t cols, uint64
   cuuint64_t strides[1] = {cols * 2};
   cuuint32_t box[2] = {FA_D, FA_T};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
+  CUresult r = nplm::with_context([&] { return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 

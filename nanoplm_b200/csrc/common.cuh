@@ -540,6 +540,18 @@ namespace nplm {
 // Per-function attributes (cudaFuncSetAttribute) apply to the current device only, so one-time
 // set-up is tracked per device ordinal. Returns the slot of the current device or -1.
 constexpr int MAX_DEVICES = 64;
+// Runs a driver call that needs the thread's context. A thread that has made no runtime call yet (the autograd engine's,
+// when its first operation is one of these kernels) has none: cudaSetDevice makes the device's primary context current.
+template <typename Call>
+inline CUresult with_context(Call call) {
+  CUresult r = call();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    int d = 0;
+    if (cudaGetDevice(&d) == cudaSuccess && cudaSetDevice(d) == cudaSuccess) r = call();
+  }
+  return r;
+}
+
 inline int current_device_slot() {
   int d = 0;
   if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= MAX_DEVICES) return -1;

@@ -658,9 +658,9 @@ static int f8_make_map(CUtensorMap* map, const void* base, uint64_t K, uint64_t 
   cuuint64_t strides[1] = {K};
   cuuint32_t box[2] = {128, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = nplm::with_context([&] { return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
@@ -672,9 +672,9 @@ static int f8_make_out_map(CUtensorMap* map, void* base, uint64_t cols, uint64_t
   cuuint64_t strides[1] = {ld * (bf16 ? 2 : 4)};
   cuuint32_t box[2] = {bf16 ? 64u : 32u, 32};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims,
+  CUresult r = nplm::with_context([&] { return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims,
                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 

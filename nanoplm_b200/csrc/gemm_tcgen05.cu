@@ -965,9 +965,9 @@ static int make_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint6
   cuuint32_t estr[2] = {1, 1};
   CUtensorMapDataType dt =
       elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-  CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = nplm::with_context([&] { return fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
