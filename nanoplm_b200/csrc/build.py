@@ -102,7 +102,7 @@ def build_one(name: str, verbose: bool = False, force: bool = False) -> Path:
     return _locked_build(out, digest, cmd, name, verbose, force)
 
 
-HOST_SOURCES = ["packer.cpp"]
+HOST_SOURCES = ["packer.cpp", "layer.cpp"]
 
 
 def build_host(name: str, force: bool = False) -> Path:

@@ -1,0 +1,215 @@
+// Host-side launch sequences of one plain encoder layer (pre-norm, rotary attention, SwiGLU MLP, no biases): all
+// kernels of a layer's forward pass from one call, and all of its backward pass from another.
+//
+// The kernels and their order are those of the op-by-op path (nanoplm_b200/models/encoder.py: EncoderLayer); what
+// this saves is the interpreter between them: a launch from Python costs 15 - 20 us (wrapper, checks, allocation, autograd
+// node), the same launch from here 4. A layer has 7 launches forward and 14 backward, so calls whose kernels take
+// less than that (single proteins, small batches, small models) were bound by the interpreter.
+//
+// The kernels live in other shared objects; nplm_layer_init receives their entry points once. Every function
+// returns 0, or the first non-zero code of a launch.
+#include <cstddef>
+#include <cstdint>
+
+namespace {
+
+typedef int (*GemmFn)(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int,
+                      int, int, int, const int*, const float*, const float*, int, int*, void*);
+typedef int (*GemmPairFn)(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int,
+                          int, int, const int*, const float*, const float*, int, int*, void*);
+typedef int (*DeltaFn)(const void*, const void*, void*, const void*, float*, int, int, int, int, int, int, int, int, int*,
+                       void*);
+typedef int (*NormFwdFn)(const void*, const int*, const void*, void*, float*, float*, int, int, float, int, void*);
+typedef int (*NormBwdFn)(const void*, const void*, const int*, const void*, const float*, const float*, const void*, void*,
+                         float*, float*, int, int, int, int, void*);
+typedef int (*FaFwdFn)(const void*, void*, float*, const int*, const int*, int, int, int, int, float, int, int*, void*);
+typedef int (*FaBwdFn)(const void*, const void*, const void*, const float*, void*, float*, float*, const int*, const int*,
+                       int, int, int, int, float, const int*, const float*, const float*, int, int, int*, void*);
+
+struct Entry {
+  GemmFn gemm;
+  GemmPairFn pair;
+  DeltaFn delta;
+  NormFwdFn norm_fwd;
+  NormBwdFn norm_bwd;
+  FaFwdFn fa_fwd;
+  FaBwdFn fa_bwd;
+};
+Entry fn;
+
+enum { EPI_STORE = 0, EPI_ADD = 1, EPI_ATOMIC_F32 = 2, EPI_SWIGLU = 5, EPI_ROPE = 6, EPI_SWIGLU_BWD = 8 };
+
+typedef unsigned char u8;
+
+struct Cut {   // consecutive 256-byte aligned parts of one allocation
+  u8* base;
+  size_t at = 0;
+  explicit Cut(void* p) : base(static_cast<u8*>(p)) {}
+  u8* take(size_t bytes) {
+    u8* p = base + at;
+    at += (bytes + 255) & ~static_cast<size_t>(255);
+    return p;
+  }
+};
+
+// What a forward pass leaves for the backward pass, in one allocation.
+struct Saved {
+  void *h1, *qkv, *o, *x1, *h2, *pre, *hs;
+  float *mean1, *rstd1, *lse, *mean2, *rstd2;
+  size_t bytes;
+  Saved(void* buf, long long T, long long C, long long I, long long H, bool norm1, bool train) {
+    Cut c(buf);
+    const size_t t = static_cast<size_t>(T);
+    h1 = norm1 ? c.take(t * C * 2) : nullptr;
+    mean1 = norm1 && train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
+    rstd1 = norm1 && train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
+    qkv = c.take(t * 3 * H * 64 * 2);
+    o = c.take(t * H * 64 * 2);
+    lse = reinterpret_cast<float*>(c.take(t * H * 4));
+    x1 = c.take(t * C * 2);
+    mean2 = train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
+    rstd2 = train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
+    h2 = c.take(t * C * 2);
+    pre = train ? c.take(t * 2 * I * 2) : nullptr;
+    hs = c.take(t * I * 2);
+    bytes = c.at;
+  }
+};
+
+// Scratch of a backward pass. The pre-activation gradients are dead once the MLP's part is done and the attention's
+// tensors take their place.
+struct Scratch {
+  void *dpre, *dh, *dx1, *d_o, *dqkv;
+  float *delta, *dq;
+  size_t bytes;
+  Scratch(void* buf, long long T, long long C, long long I, long long H) {
+    const size_t t = static_cast<size_t>(T);
+    Cut c(buf);
+    dh = c.take(t * C * 2);
+    dx1 = c.take(t * C * 2);
+    const size_t shared = c.at;
+    dpre = c.take(t * 2 * I * 2);
+    Cut a(buf);
+    a.at = shared;
+    d_o = a.take(t * H * 64 * 2);
+    delta = reinterpret_cast<float*>(a.take(t * H * 4));
+    dq = reinterpret_cast<float*>(a.take(t * H * 64 * 4));
+    dqkv = a.take(t * 3 * H * 64 * 2);
+    bytes = c.at > a.at ? c.at : a.at;
+  }
+};
+
+struct Call {
+  int* status;
+  void* stream;
+  // bf16 output: CTA pairs on 256-wide tiles, as ops.kernels.gemm chooses by default
+  int out(const void* A, const void* B, void* Cp, const void* R, int M, int N, int K, int ldb, int ldc, int ldr, int b_mn,
+          int epi, const int* pos = nullptr, const float* cosp = nullptr, const float* sinp = nullptr,
+          int rope_cols = 0) const {
+    if (N >= 256 || epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD)
+      return fn.pair(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, 0, pos, cosp, sinp, rope_cols, status, stream);
+    return fn.gemm(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, 128, 0, 0, pos, cosp, sinp, rope_cols, status,
+                   stream);
+  }
+  // fp32 C[N][K] += dy[T][N]^T x[T][K]
+  int wgrad(const void* dy, const void* x, float* g, int T, int N, int K, int splits) const {
+    return fn.gemm(dy, x, g, nullptr, N, K, T, N, K, K, 0, 1, 1, EPI_ATOMIC_F32, splits, K >= 256 ? 256 : 128, 0, 0, nullptr,
+                   nullptr, nullptr, 0, status, stream);
+  }
+};
+
+template <typename P>
+P* ptr(const long long* a, int i) {
+  return reinterpret_cast<P*>(static_cast<intptr_t>(a[i]));
+}
+
+#define TRY(call)              \
+  do {                         \
+    const int rc_ = (call);    \
+    if (rc_ != 0) return rc_;  \
+  } while (0)
+
+}  // namespace
+
+extern "C" void nplm_layer_init(void* const* f) {
+  fn.gemm = reinterpret_cast<GemmFn>(f[0]);
+  fn.pair = reinterpret_cast<GemmPairFn>(f[1]);
+  fn.delta = reinterpret_cast<DeltaFn>(f[2]);
+  fn.norm_fwd = reinterpret_cast<NormFwdFn>(f[3]);
+  fn.norm_bwd = reinterpret_cast<NormBwdFn>(f[4]);
+  fn.fa_fwd = reinterpret_cast<FaFwdFn>(f[5]);
+  fn.fa_bwd = reinterpret_cast<FaBwdFn>(f[6]);
+}
+
+// Bytes of the forward pass's buffer (backward = 0) or of the backward pass's scratch (1).
+extern "C" long long nplm_layer_bytes(long long T, long long C, long long I, long long H, int norm1, int train,
+                                      int backward) {
+  return static_cast<long long>(backward ? Scratch(nullptr, T, C, I, H).bytes
+                                         : Saved(nullptr, T, C, I, H, norm1 != 0, train != 0).bytes);
+}
+
+// a: T, C, I, H, window, norm1, rms, train, then addresses: x, w_qkv, w_o, w_in, w_out, n1, n2, seq_start, seq_end,
+// pos, cos, sin, buffer, y, status, stream
+extern "C" int nplm_layer_fwd(const long long* a, double eps1, double eps2, double scale) {
+  const int T = static_cast<int>(a[0]), C = static_cast<int>(a[1]), I = static_cast<int>(a[2]), H = static_cast<int>(a[3]);
+  const int window = static_cast<int>(a[4]), rms = static_cast<int>(a[6]);
+  const bool norm1 = a[5] != 0, train = a[7] != 0;
+  const int HD = H * 64;
+  if (T <= 0) return 0;
+  const void *x = ptr<void>(a, 8), *wqkv = ptr<void>(a, 9), *wo = ptr<void>(a, 10), *win = ptr<void>(a, 11),
+             *wout = ptr<void>(a, 12), *n1 = ptr<void>(a, 13), *n2 = ptr<void>(a, 14);
+  const int *ss = ptr<int>(a, 15), *se = ptr<int>(a, 16), *pos = ptr<int>(a, 17);
+  const float *cosp = ptr<float>(a, 18), *sinp = ptr<float>(a, 19);
+  const Saved s(ptr<void>(a, 20), T, C, I, H, norm1, train);
+  void* y = ptr<void>(a, 21);
+  const Call k{ptr<int>(a, 22), ptr<void>(a, 23)};
+  if (norm1)
+    TRY(fn.norm_fwd(x, nullptr, n1, s.h1, rms ? nullptr : s.mean1, s.rstd1, T, C, static_cast<float>(eps1), rms, k.stream));
+  const void* h1 = norm1 ? s.h1 : x;
+  TRY(k.out(h1, wqkv, s.qkv, nullptr, T, 3 * HD, C, C, 3 * HD, 0, 0, EPI_ROPE, pos, cosp, sinp, 2 * HD));
+  TRY(fn.fa_fwd(s.qkv, s.o, s.lse, ss, se, T, H, 64, window, static_cast<float>(scale), 0, k.status, k.stream));
+  TRY(k.out(s.o, wo, s.x1, x, T, C, HD, HD, C, C, 0, EPI_ADD));
+  TRY(fn.norm_fwd(s.x1, nullptr, n2, s.h2, rms ? nullptr : s.mean2, s.rstd2, T, C, static_cast<float>(eps2), rms, k.stream));
+  TRY(k.out(s.h2, win, s.hs, s.pre, T, 2 * I, C, C, I, s.pre != nullptr ? 2 * I : 0, 0, EPI_SWIGLU));
+  return k.out(s.hs, wout, y, s.x1, T, C, I, I, C, C, 0, EPI_ADD);
+}
+
+// a: as nplm_layer_fwd with y = the incoming gradient dy, then addresses: dx, scratch, the fp32 gradients of w_qkv, w_o,
+// w_in, w_out, n1, n2 (added to), then the split factors of the four weight gradients and the attention mode
+// (-1 default, 3 reproducible)
+extern "C" int nplm_layer_bwd(const long long* a, double scale) {
+  const int T = static_cast<int>(a[0]), C = static_cast<int>(a[1]), I = static_cast<int>(a[2]), H = static_cast<int>(a[3]);
+  const int window = static_cast<int>(a[4]), rms = static_cast<int>(a[6]);
+  const bool norm1 = a[5] != 0;
+  const int HD = H * 64;
+  if (T <= 0) return 0;
+  const void *x = ptr<void>(a, 8), *wqkv = ptr<void>(a, 9), *wo = ptr<void>(a, 10), *win = ptr<void>(a, 11),
+             *wout = ptr<void>(a, 12), *n1 = ptr<void>(a, 13), *n2 = ptr<void>(a, 14);
+  const int *ss = ptr<int>(a, 15), *se = ptr<int>(a, 16), *pos = ptr<int>(a, 17);
+  const float *cosp = ptr<float>(a, 18), *sinp = ptr<float>(a, 19);
+  const Saved s(ptr<void>(a, 20), T, C, I, H, norm1, true);
+  const void* dy = ptr<void>(a, 21);
+  const Call k{ptr<int>(a, 22), ptr<void>(a, 23)};
+  void* dx = ptr<void>(a, 24);
+  const Scratch d(ptr<void>(a, 25), T, C, I, H);
+  float *g_qkv = ptr<float>(a, 26), *g_o = ptr<float>(a, 27), *g_in = ptr<float>(a, 28), *g_out = ptr<float>(a, 29),
+        *g_n1 = ptr<float>(a, 30), *g_n2 = ptr<float>(a, 31);
+  const int mode = static_cast<int>(a[36]);
+  // MLP
+  TRY(k.out(dy, wout, d.dpre, s.pre, T, I, C, I, 2 * I, 2 * I, 1, EPI_SWIGLU_BWD));
+  TRY(k.wgrad(dy, s.hs, g_out, T, C, I, static_cast<int>(a[35])));
+  TRY(k.wgrad(d.dpre, s.h2, g_in, T, 2 * I, C, static_cast<int>(a[34])));
+  TRY(k.out(d.dpre, win, d.dh, nullptr, T, C, 2 * I, C, C, 0, 1, EPI_STORE));
+  TRY(fn.norm_bwd(d.dh, s.x1, nullptr, n2, rms ? nullptr : s.mean2, s.rstd2, dy, d.dx1, g_n2, nullptr, T, C, 0, rms,
+                  k.stream));
+  // attention
+  TRY(fn.delta(d.dx1, wo, d.d_o, s.o, d.delta, T, HD, C, C, HD, HD, HD, 1, k.status, k.stream));
+  TRY(k.wgrad(d.dx1, s.o, g_o, T, C, HD, static_cast<int>(a[33])));
+  TRY(fn.fa_bwd(s.qkv, nullptr, d.d_o, s.lse, d.dqkv, mode == 3 ? nullptr : d.dq, d.delta, ss, se, T, H, 64, window,
+                static_cast<float>(scale), pos, cosp, sinp, 0, mode, k.status, k.stream));
+  TRY(k.wgrad(d.dqkv, norm1 ? s.h1 : x, g_qkv, T, 3 * HD, C, static_cast<int>(a[32])));
+  if (!norm1)   // the layer input enters the projection and the residual: both gradients in one epilogue
+    return k.out(d.dqkv, wqkv, dx, d.dx1, T, C, 3 * HD, C, C, C, 1, EPI_ADD);
+  TRY(k.out(d.dqkv, wqkv, d.dh, nullptr, T, C, 3 * HD, C, C, 0, 1, EPI_STORE));
+  return fn.norm_bwd(d.dh, x, nullptr, n1, rms ? nullptr : s.mean1, s.rstd1, d.dx1, dx, g_n1, nullptr, T, C, 0, rms, k.stream);
+}

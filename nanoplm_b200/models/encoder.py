@@ -23,6 +23,7 @@ import torch.nn.functional as F
 
 from nanoplm_b200.config.schema import ModelConfig
 from nanoplm_b200.ops import functional as ops
+from nanoplm_b200.ops import layer as native_layer
 
 
 class Linear(nn.Module):
@@ -162,9 +163,21 @@ class EncoderLayer(nn.Module):
             h = self.conv(h, ctx, residual=True)      # h + conv(h)
         return self.attn(h, ctx, window, rope, residual=residual)
 
+    def _plain(self) -> bool:
+        """The parts are the ones this class was built with, and none of the optional blocks is there."""
+        a, m = self.attn, self.mlp
+        return (self.conv is None and type(a) is Attention and type(m) is MLP and type(self.mlp_norm) is Norm
+                and type(self.attn_norm) is (nn.Identity if self.layer_idx == 0 else Norm)
+                and type(a.Wqkv) is Linear and type(a.Wo) is Linear and type(m.Wi) is Linear and type(m.Wo) is Linear)
+
     def forward(self, x, ctx: BatchContext, window: int, rope: tuple):
         aux = None
         if self.mhc_attn is None:
+            if x.is_cuda and self._plain():
+                y = native_layer.run(self.attn, self.mlp, None if self.layer_idx == 0 else self.attn_norm, self.mlp_norm,
+                                     x, ctx, window, rope)
+                if y is not None:
+                    return y, None
             if isinstance(self.attn_norm, Norm):
                 h, skip = self.attn_norm.with_residual(x)
                 x = self._attn_branch(h, ctx, window, rope, residual=skip, normed=True)
