@@ -123,7 +123,8 @@ __device__ __forceinline__ uint32_t act_bf16x2(uint32_t pre) {
 
 struct WorkItem {
   int m0, n0, kb0, kb1, b_row;
-  long long c_off;
+  long long c_off;   // group_mode 2: where this group's output starts, in elements and in rows
+  int c_row;
 };
 
 // Writes 32 rows x 64 bf16 columns held by one warp (lane = row, packed[0..31] = the 64 values of
@@ -219,6 +220,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   auto decode = [&](int w, WorkItem& it) -> bool {
     it.b_row = 0;
     it.c_off = 0;
+    it.c_row = 0;
     if (args.group_mode == 2) {
       const int per = num_m * num_n;
       const int g = w / per, tile = w % per;
@@ -227,6 +229,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       it.kb0 = args.group_off[g] / BK;
       it.kb1 = args.group_off[g + 1] / BK;
       it.c_off = static_cast<long long>(g) * args.c_group_stride;
+      it.c_row = g * M;
       return it.kb0 < it.kb1;
     }
     if (stream_k) {
@@ -569,7 +572,41 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int y0 = m0 + quarter * 32;
         const bool rows_in = y0 < M;
         auto chunk_in = [&](int c) { return rows_in && n0 + c * 64 < n_extent; };
-        if constexpr (EPI == EPI_SWIGLU) {
+        if constexpr (EPI == EPI_ATOMIC_F32 || EPI == EPI_STORE_F32) {
+          // 32 fp32 columns (128 bytes a row) at a time through a staging buffer and one TMA reduce-add or store. Added
+          // from registers (16 bytes from each of 32 rows an instruction) a 128 x 256 tile took about 8 us, all of it
+          // exposed where a CTA has one tile (8 704 tokens: 4096 x 1024 66.8 -> 55.3 us, 1024 x 1024 25.2 -> 18.8; 55 424
+          // tokens: 3072 x 1024 249.7 -> 239.9)
+#pragma unroll 1
+          for (int c = 0; c < BN / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld32(taddr + c * 32, r);
+            tmem_ld_wait();
+            if (c == BN / 32 - 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) release_acc(acc);
+            }
+            const int x = n0 + c * 32;
+            if (rows_in && x < N) {
+              if (elect_one()) tma_store_wait_read<1>();
+              __syncwarp();
+              uint8_t* buf = stage + stage_toggle * 4096;
+              stage_toggle ^= 1;
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                    make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (elect_one()) {
+                if constexpr (EPI == EPI_ATOMIC_F32) tma_reduce_add_2d(&tmC, buf, x, y0 + it.c_row);
+                else tma_store_2d(&tmC, buf, x, y0 + it.c_row);
+                tma_store_commit();
+              }
+            }
+          }
+        } else if constexpr (EPI == EPI_SWIGLU) {
 #pragma unroll 1
           for (int c = c0; c < c1; ++c) {
             uint32_t pv[32], pg[32], po[32];
@@ -956,7 +993,7 @@ static EncodeTiledFn get_encode_fn() {
 // 2-D bf16 tensor map, 128-byte swizzle. inner = contiguous extent, outer = rows.
 static int make_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
                        uint64_t row_stride_elems, uint32_t box_inner, uint32_t box_outer,
-                       int elem_bytes) {
+                       int elem_bytes) {   // 2: bf16, 4: fp32
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return -1;
   cuuint64_t dims[2] = {inner, outer};
@@ -964,7 +1001,7 @@ static int make_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint6
   cuuint32_t box[2] = {box_inner, box_outer};
   cuuint32_t estr[2] = {1, 1};
   CUtensorMapDataType dt =
-      elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+      elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   CUresult r = nplm::with_context([&] { return fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
@@ -1069,7 +1106,8 @@ static int launch_pair(const GemmMaps& maps, const GemmArgs& args, cudaStream_t 
   if constexpr (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD || EPI == EPI_STORE_DELTA) {
     return launch_pair_impl<A_MN, B_MN, EPI, true>(maps, args, stream);
   } else {
-    if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_GELU || EPI == EPI_RELU || EPI == EPI_SWIGLU) {
+    if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_GELU || EPI == EPI_RELU || EPI == EPI_SWIGLU ||
+                  EPI == EPI_ATOMIC_F32 || EPI == EPI_STORE_F32) {
       if (maps.tma_epi) return launch_pair_impl<A_MN, B_MN, EPI, true>(maps, args, stream);
     }
     return launch_pair_impl<A_MN, B_MN, EPI, false>(maps, args, stream);
@@ -1081,7 +1119,8 @@ static int launch(const GemmMaps& maps, const GemmArgs& args, int max_ctas, cuda
   if constexpr (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD) {
     return launch_impl<BN, A_MN, B_MN, EPI, true>(maps, args, max_ctas, stream);
   } else {
-    if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_GELU || EPI == EPI_RELU || EPI == EPI_SWIGLU) {
+    if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_GELU || EPI == EPI_RELU || EPI == EPI_SWIGLU ||
+                  EPI == EPI_ATOMIC_F32 || EPI == EPI_STORE_F32) {
       if (maps.tma_epi) return launch_impl<BN, A_MN, B_MN, EPI, true>(maps, args, max_ctas, stream);
     }
     return launch_impl<BN, A_MN, B_MN, EPI, false>(maps, args, max_ctas, stream);
@@ -1172,13 +1211,20 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
     rc = make_map_2d(&tmB, B, N, b_rows_mnmajor, ldb, 64, BK, 2);
   if (rc) return rc;
   // staged (TMA store) epilogue for the bf16 outputs; maps C / R describe [32 rows][64 cols] boxes
+  const bool f32_out = epi == EPI_ATOMIC_F32 || epi == EPI_STORE_F32;
+  // fp32 outputs leave in boxes of 32 rows x 32 columns; those of all groups form one tall matrix, whose boxes must not
+  // reach into the next group
+  const bool f32_tma = f32_out && (grp.mode != 2 || (M % 32 == 0 && grp.c_group_stride == static_cast<long long>(M) * ldc));
   maps.tma_epi = !direct_epilogue &&
-                 (epi == EPI_STORE || epi == EPI_ADD || epi == EPI_GELU || epi == EPI_RELU || epi == EPI_SWIGLU ||
+                 (f32_tma || epi == EPI_STORE || epi == EPI_ADD || epi == EPI_GELU || epi == EPI_RELU || epi == EPI_SWIGLU ||
                   epi == EPI_ROPE || epi == EPI_SWIGLU_BWD || epi == EPI_STORE_DELTA) &&
                  !(epi == EPI_ADD && (R == nullptr || (reinterpret_cast<uintptr_t>(R) & 15) || (ldr % 8)));
   maps.C = tmA;
   maps.R = tmA;
-  if (maps.tma_epi) {
+  if (maps.tma_epi && f32_out) {
+    rc = make_map_2d(&maps.C, C, N, static_cast<uint64_t>(M) * (grp.mode == 2 ? grp.groups : 1), ldc, 32, 32, 4);
+    if (rc) return rc;
+  } else if (maps.tma_epi) {
     const int out_cols = epi == EPI_SWIGLU ? N / 2 : (epi == EPI_SWIGLU_BWD ? 2 * N : N);
     rc = make_map_2d(&maps.C, C, out_cols, M, ldc, 64, 32, 2);
     if (rc) return rc;

@@ -199,7 +199,8 @@ def wgrad_splits(n_out: int, k_in: int, tokens: int, bn: int = 256, sms: int = 1
     additions take from the others); the factor with the least waves * cost wins. The 25 fits measurements from both
     ends: 55 424 tokens, 4096 x 1024 (128 tiles) 377 us unsplit, 405 us in 8; 3072 x 1024 (96 tiles) 400 us unsplit, 331 in
     3, 342 in 6; 1024 x 1024 (32 tiles) 121 us in 4, 118 in 9. Small outputs are what gains over filling a wave with
-    at most 4 items a tile: 17 000 tokens, 512 x 512 (8 tiles) 33.1 -> 19.4 us."""
+    at most 4 items a tile: 17 000 tokens, 512 x 512 (8 tiles) 33.1 -> 19.4 us.
+    (Taken before the additions went through TMA; with them the same factors are the best or within 4 % of it.)"""
     tiles = ((n_out + 127) // 128) * ((k_in + bn - 1) // bn)
     kb = (tokens + 63) // 64
     best, best_cost = 1, None
