@@ -124,11 +124,9 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                 const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                 float* __restrict__ dw, float* __restrict__ dtable, int T, int C, int rms) {
-  extern __shared__ float sm_dw[];  // [C]
+  __shared__ __align__(16) float sm_dw[8][256];  // one 256-channel chunk of every warp's sums
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < C; i += blockDim.x) sm_dw[i] = 0.f;
-  __syncthreads();
 
   float acc[CHUNKS][8];
 #pragma unroll
@@ -216,16 +214,24 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
     }
   }
   if (dw) {
+    // The warps' sums meet in shared memory chunk by chunk and without atomics (fp32 adds there are compare-and-swap
+    // loops, and all eight warps wanted the same words: 8 704 x 1024 21.3 -> 15.6 us, 55 424 x
+    // 1024 91.7 -> 85.9)
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
-      const int i = c * 256 + lane * 8;
+      if (c) __syncthreads();
+      float4* mine = reinterpret_cast<float4*>(&sm_dw[threadIdx.x >> 5][lane * 8]);
+      mine[0] = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+      mine[1] = make_float4(acc[c][4], acc[c][5], acc[c][6], acc[c][7]);
+      __syncthreads();
+      const int i = c * 256 + threadIdx.x;
       if (i < C) {
+        float sum = 0.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) atomicAdd(&sm_dw[i + e], acc[c][e]);
+        for (int j = 0; j < 8; ++j) sum += sm_dw[j][threadIdx.x];
+        atomicAdd(&dw[i], sum);
       }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < C; i += blockDim.x) atomicAdd(&dw[i], sm_dw[i]);
   }
 }
 
@@ -1028,7 +1034,7 @@ extern "C" int nplm_norm_bwd(const void* dy, const void* x, const int* ids, cons
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 2) blocks = 148 * 2;   // more blocks only add contention on the dw atomics
 #define CALL(N_)                                                                              \
-  norm_bwd_kernel<N_><<<blocks, 256, C * sizeof(float), st>>>(                                \
+  norm_bwd_kernel<N_><<<blocks, 256, 0, st>>>(                                                \
       reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x),  \
       ids, reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd,                             \
       reinterpret_cast<const __nv_bfloat16*>(dres), reinterpret_cast<__nv_bfloat16*>(dx), dw, \
