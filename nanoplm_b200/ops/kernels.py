@@ -402,6 +402,21 @@ def muon_momentum_(g, m, offsets, numel: int, upd, usq, sumsq, grad_scale: float
     count_launch()
 
 
+def transpose_scale(x: torch.Tensor, scale: torch.Tensor | None = None) -> torch.Tensor:
+    """[B, C, R] = x[B, R, C] transposed, times scale[b] (bf16 [B]) where given; x bf16 contiguous, R and C multiples
+    of 64."""
+    _chk(x, _BF16, "x")
+    B, R, C = x.shape
+    if not x.is_contiguous() or (scale is not None and (scale.dtype != _BF16 or scale.numel() != B
+                                                        or not scale.is_contiguous())):
+        raise ValueError("x must be contiguous and scale a contiguous bf16 [B]")
+    y = torch.empty((B, C, R), dtype=_BF16, device=x.device)
+    rc = lib("elementwise").nplm_transpose_scale(ptr(x), ptr(scale), ptr(y), c_int(B), c_int(R), c_int(C), stream_ptr())
+    check_rc(rc, "transpose_scale")
+    count_launch()
+    return y
+
+
 def muon_apply_(p, p_bf16, offsets, numel: int, O, lr: float, wd: float, cautious: bool) -> None:
     """p[offsets[i] : +numel] -= lr * (wd-term + O[i]) for the bf16 stack O [n, numel]; also
     writes the bf16 copy of the parameters."""

@@ -102,13 +102,21 @@ def orthogonalize_batched(G: torch.Tensor, coeffs=NS_QUINTIC, eps: float = 1e-7,
     dt = torch.bfloat16 if G.is_cuda else torch.float32
     X = G.to(dt)
     transposed = X.shape[1] > X.shape[2]
-    if transposed:
-        X = X.transpose(1, 2).contiguous()
     nrm = X.float().flatten(1).norm(dim=1) if sumsq is None else sumsq.float().sqrt()
     inv = (1.0 / (nrm * 1.01 + eps)).to(dt)[:, None, None]
+    # tall stacks: transposed and scaled in one pass by this package's kernel where whole 64 x 64 tiles allow
+    tiled = (transposed and X.is_cuda and X.is_contiguous() and X.shape[1] % 64 == 0 and X.shape[2] % 64 == 0
+             and X.shape[0] <= 65535 and X.data_ptr() % 16 == 0)
+    scaled = False
+    if tiled and X.shape[2] % 128 == 0:             # the grouped path below
+        from nanoplm_b200.ops import kernels as K
+        X, scaled = K.transpose_scale(X, inv.reshape(-1)), True
+    elif transposed:
+        X = X.transpose(1, 2).contiguous()
     grouped = _grouped_ok(X)
     if grouped:
-        X = X.mul_(inv) if (X.data_ptr() != G.data_ptr() or sumsq is not None) else X * inv
+        if not scaled:
+            X = X.mul_(inv) if (X.data_ptr() != G.data_ptr() or sumsq is not None) else X * inv
         for a, b, c in coeffs:
             A = _bmm_nt(X, X, grouped)                          # X X^T, symmetric [B, m, m]
             Ac = A * c
@@ -122,6 +130,9 @@ def orthogonalize_batched(G: torch.Tensor, coeffs=NS_QUINTIC, eps: float = 1e-7,
             A = _bmm_nt(X, X, grouped)
             Bm = torch.add(A * b, _bmm_nt(A, A, grouped), alpha=c)
             X = torch.add(_bmm_nn(Bm, X, grouped), X, alpha=a)
+    if tiled and X.is_contiguous():
+        from nanoplm_b200.ops import kernels as K
+        return K.transpose_scale(X)
     if transposed:
         X = X.transpose(1, 2).contiguous()
     return X
