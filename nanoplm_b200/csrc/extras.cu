@@ -47,14 +47,11 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
 
 constexpr int MAX_KS = 9;
 
-// flip = 0: forward (tap k reads t + k - r);  flip = 1: input gradient (tap k reads t - (k - r));
-// residual: the input itself is added (y = x + conv(x), dx = dy + conv^T(dy)): one more on the centre tap, which always
-// lies inside the token's own sequence.
+// flip = 0: forward (tap k reads t + k - r);  flip = 1: input gradient (tap k reads t - (k - r))
 __global__ void __launch_bounds__(256)
 dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
               const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
-              const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int KS, int flip,
-              int residual) {
+              const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int KS, int flip) {
   const int vec = C >> 3;
   const int r = KS >> 1;
   const long long total = static_cast<long long>(T) * vec;
@@ -76,8 +73,7 @@ dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       float xv[8];
       ld8(x + static_cast<size_t>(src) * C + c, xv);
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
-        acc[e] += xv[e] * (__bfloat162float(w[(c + e) * KS + k]) + (residual && k == r ? 1.f : 0.f));
+      for (int e = 0; e < 8; ++e) acc[e] += xv[e] * __bfloat162float(w[(c + e) * KS + k]);
     }
     st8(y + static_cast<size_t>(t) * C + c, acc);
   }
@@ -92,8 +88,7 @@ template <int KS>
 __global__ void __launch_bounds__(256)
 dwconv_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
-                   const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip,
-                   int residual) {
+                   const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip) {
   constexpr int R = KS / 2;
   const int vec = C >> 3;
   const int n_tb = (T + DW_TT - 1) / DW_TT;
@@ -121,10 +116,6 @@ dwconv_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
       for (int e = 0; e < 8; ++e)
 #pragma unroll
         for (int k = 0; k < KS; ++k) wt[k][e] = __bfloat162float(wl[e * KS + (flip ? KS - 1 - k : k)]);
-      if (residual) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) wt[R][e] += 1.f;
-      }
     }
     float acc[DW_TT][8];
     int lo[DW_TT], hi[DW_TT];
@@ -513,7 +504,7 @@ static int grid_for(long long work, int threads) {
 using namespace nplm;
 
 extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const int* s_start,
-                           const int* s_end, void* y, int T, int C, int KS, int flip, int residual, cudaStream_t st) {
+                           const int* s_end, void* y, int T, int C, int KS, int flip, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || KS < 1 || KS > MAX_KS || !(KS & 1)) return -3;
   const bool aligned = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
@@ -522,8 +513,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
 #define NPLM_DWCONV(KS_)                                                                                   \
   dwconv_tile_kernel<KS_><<<grid, 256, 0, st>>>(                                                           \
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),                \
-      reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip,     \
-      residual)
+      reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip)
     switch (KS) {
       case 3: NPLM_DWCONV(3); break;
       case 5: NPLM_DWCONV(5); break;
@@ -536,7 +526,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
   dwconv_kernel<<<grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
       reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C,
-      KS, flip, residual);
+      KS, flip);
   return static_cast<int>(cudaGetLastError());
 }
 

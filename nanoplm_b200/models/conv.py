@@ -31,19 +31,18 @@ def dwconv_reference(x, w, bias, seq_start, seq_end):
 
 class _DWConvFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, bias, ss, se, residual):
+    def forward(ctx, x, w, bias, ss, se):
         x = x.contiguous()
         ctx.save_for_backward(x, w, ss, se)
         ctx.bias_ref = bias
         ctx.w_ref = w
-        ctx.residual = residual
-        return K.dwconv(x, w.contiguous(), bias, ss, se, residual=residual)
+        return K.dwconv(x, w.contiguous(), bias, ss, se)
 
     @staticmethod
     def backward(ctx, dy):
         x, w, ss, se = ctx.saved_tensors
         dy = dy.contiguous()
-        dx = K.dwconv(dy, w.contiguous(), None, ss, se, flip=True, residual=ctx.residual)
+        dx = K.dwconv(dy, w.contiguous(), None, ss, se, flip=True)
         bias = ctx.bias_ref
         dw = w.main_grad if _has_main_grad(w) else torch.zeros(w.shape, dtype=torch.float32, device=w.device)
         db = None
@@ -52,15 +51,13 @@ class _DWConvFn(torch.autograd.Function):
         K.dwconv_bwd_w(x, dy, ss, se, dw, db)
         gw = None if _has_main_grad(w) else dw.to(w.dtype)
         gb = None if (bias is None or _has_main_grad(bias)) else db.to(bias.dtype)
-        return dx, gw, gb, None, None, None
+        return dx, gw, gb, None, None
 
 
-def dwconv_varlen(x, w, bias, seq_start, seq_end, residual: bool = False):
-    """conv(x), or x + conv(x): on the GPU the sum is one more on the centre tap, in both directions."""
+def dwconv_varlen(x, w, bias, seq_start, seq_end):
     if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and w.shape[1] <= 9:
-        return _DWConvFn.apply(x, w, bias, seq_start, seq_end, residual)
-    y = dwconv_reference(x, w, bias, seq_start, seq_end)
-    return x + y if residual else y
+        return _DWConvFn.apply(x, w, bias, seq_start, seq_end)
+    return dwconv_reference(x, w, bias, seq_start, seq_end)
 
 
 class VarlenDepthwiseConv(nn.Module):
@@ -72,5 +69,5 @@ class VarlenDepthwiseConv(nn.Module):
         self.weight = nn.Parameter(w)
         self.bias = nn.Parameter(torch.zeros(channels)) if bias else None
 
-    def forward(self, x, ctx, residual: bool = False):
-        return dwconv_varlen(x, self.weight, self.bias, ctx.seq_start, ctx.seq_end, residual)
+    def forward(self, x, ctx):
+        return dwconv_varlen(x, self.weight, self.bias, ctx.seq_start, ctx.seq_end)

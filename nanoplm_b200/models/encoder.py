@@ -160,7 +160,7 @@ class EncoderLayer(nn.Module):
         if not normed:
             h = self.attn_norm(h)
         if self.conv is not None:
-            h = self.conv(h, ctx, residual=True)      # h + conv(h)
+            h = h + self.conv(h, ctx)
         return self.attn(h, ctx, window, rope, residual=residual)
 
     def _plain(self) -> bool:

@@ -592,13 +592,12 @@ def check_status() -> None:
 
 
 # --------------------------------------------------------------------------- conv / mHC
-def dwconv(x, w, bias, seq_start, seq_end, flip=False, residual=False):
-    """Varlen depthwise convolution (flip: its input gradient); residual adds the input itself."""
+def dwconv(x, w, bias, seq_start, seq_end, flip=False):
     T, C = x.shape
     KS = w.shape[1]
     y = torch.empty_like(x)
     rc = lib("extras").nplm_dwconv(ptr(x), ptr(w), ptr(bias), ptr(seq_start), ptr(seq_end), ptr(y), c_int(T),
-                                   c_int(C), c_int(KS), c_int(int(flip)), c_int(int(residual)), stream_ptr())
+                                   c_int(C), c_int(KS), c_int(int(flip)), stream_ptr())
     check_rc(rc, "dwconv")
     count_launch()
     return y
