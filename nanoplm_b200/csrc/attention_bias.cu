@@ -136,7 +136,9 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint8_t* sV = smem + C::OFF_V;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint64_t* q_full = bars;                  // [2]
-  uint64_t* q_empty = q_full + 2;           // [2] both warpgroups: their output has left the buffer
+  // [2] every consumer (both warpgroups, whose output leaves through the buffer, and both MMA issuers) gives a buffer
+  // back once per item, and only after it has seen that item's q_full: nobody can be two items behind or ahead
+  uint64_t* q_empty = q_full + 2;
   uint64_t* k_full = q_empty + 2;           // [STAGES]
   uint64_t* k_empty = k_full + STAGES;      // both MMA issuers
   uint64_t* v_full = k_empty + STAGES;
@@ -155,7 +157,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&q_full[i], 1);
-      mbar_init(&q_empty[i], 2);
+      mbar_init(&q_empty[i], 4);
       mbar_init(&s_full[i], 1);
       mbar_init(&s_free[i], 4);
       mbar_init(&p_ready[i], 4);
@@ -281,6 +283,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             umma_commit(&v_empty[st]);
           }
         }
+        if (ok) mbar_arrive(&q_empty[qb]);   // (the warpgroup waits for the products that read the buffer)
         if (!ok && *abort_flag == 0) {
           atomicExch(args.status, why);
           *abort_flag = 1;
@@ -428,8 +431,11 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         ok = mbar_wait(&pv_done[i], pv_cnt & 1u);   // the item's last output product
         ++pv_cnt;
       }
-      // the output leaves through this tile's Q buffer, which the finished score products no longer read
+      // The output leaves through this tile's Q buffer, which the finished score products no longer read. A tile without
+      // keys or rows has waited for no product: the loads of Q have to have landed before the buffer is written, and
+      // before it is given back (an early arrival would count for the item that the buffer still holds)
       const uint32_t qb = qc & 1u;
+      ok = ok && mbar_wait(&q_full[qb], (qc >> 1) & 1u);
       ok = ab_barrier_and(1 + i, ok && *abort_flag == 0);
       if (!ok) break;
       tc_fence_after();
@@ -443,10 +449,8 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tmem_ld32(tO + c, o);
             tmem_ld_wait();
           } else {
-            // no key for any row of the tile; the loads of Q still have to have landed before the buffer is written
 #pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] = 0u;
-            if (c == 0 && !mbar_wait(&q_full[qb], (qc >> 1) & 1u) && lane == 0) atomicExch(args.status, ST_TIMEOUT_FULL);
+            for (int e = 0; e < 32; ++e) o[e] = 0u;   // no key for any row of the tile
           }
 #pragma unroll
           for (int e = 0; e < 32; e += 8) {

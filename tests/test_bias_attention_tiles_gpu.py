@@ -56,3 +56,17 @@ def test_many_items_per_block(cuda_status):
     start = torch.cat([torch.full((n,), a) for n, a in zip(lens, cu)]).to(torch.int32).cuda()
     end = torch.cat([torch.full((n,), b) for n, b in zip(lens, cu[1:])]).to(torch.int32).cuda()
     _check(128, 16, 512, start, end, seed=9)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("empty", [False, True])
+def test_buffers_are_given_back_in_order(D, empty, cuda_status):
+    """Several items a block, among them some whose second tile has no rows (a last pair of 100) and, with `empty`, runs
+    of items without keys: these wait for no product and may not run ahead of the buffers they share."""
+    T, S = 20 * 256 + 100, 256
+    start = torch.arange(T, dtype=torch.int32) // S * S
+    end = (start + S).clamp(max=T)
+    if empty:
+        end[1024:3072] = start[1024:3072]
+    for seed in range(3):
+        _check(D, 32, S, start.cuda(), end.cuda(), seed=seed)
