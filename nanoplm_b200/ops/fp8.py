@@ -220,4 +220,5 @@ class _Fp8LinearFn(torch.autograd.Function):
 
 def fp8_linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """y = x W^T with e4m3 operands (no bias)."""
-    return _Fp8LinearFn.apply(x, w, torch.is_grad_enabled())
+    from .functional import _keeps
+    return _Fp8LinearFn.apply(x, w, _keeps())

@@ -89,12 +89,23 @@ class _NoGradCtx:
         pass
 
 
+def functions_observed() -> bool:
+    """Somebody has to see the autograd Functions themselves: a forward-mode level, a function transform, or a tracer
+    (which records a Function as a call to replay, but of its body only the allocations that the kernels fill)."""
+    return _fwd_ad._current_level >= 0 or torch._C._is_tracing() or torch._C._are_functorch_transforms_active()
+
+
 def _call(fn, *args):
-    """fn.apply(*args); where gradients are off (and no forward-mode level or function transform is active, which
-    have to see the Function) its forward directly: the dispatch of a Function costs more than most of its bodies."""
-    if torch.is_grad_enabled() or _fwd_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
+    """fn.apply(*args); where gradients are off and nobody observes the Functions, its forward directly: the dispatch
+    of a Function costs more than most of its bodies."""
+    if torch.is_grad_enabled() or functions_observed():
         return fn.apply(*args)
     return fn.forward(_NoGradCtx(), *args)
+
+
+def _keeps() -> bool:
+    """Whether a forward pass has to keep what a backward pass would need. A traced call is replayed in either mode."""
+    return torch.is_grad_enabled() or torch._C._is_tracing()
 
 
 # ------------------------------------------------------------------------------------- linear
@@ -194,7 +205,7 @@ def mlp_swiglu(x, w_in, w_out, residual=None):
     inter = w_out.shape[1]
     if (x.is_cuda and x.dtype == BF and not _FP8_STATE["enabled"] and inter % 64 == 0 and w_in.shape[0] == 2 * inter
             and w_in.shape[1] % 64 == 0 and w_out.shape[0] % 64 == 0):
-        return _call(_SwiGLUMLPFn, x, w_in, w_out, residual, torch.is_grad_enabled())
+        return _call(_SwiGLUMLPFn, x, w_in, w_out, residual, _keeps())
     return linear(linear(x, w_in, act="swiglu"), w_out, residual=residual)
 
 
@@ -238,7 +249,7 @@ def linear(x, w, bias=None, residual=None, act: str | None = None):
             if act == "swiglu" and bias is not None:
                 y = _call(_LinearFn, x, w, bias, None, None)
                 return swiglu(y)
-            return _call(_LinearFn, x, w, bias, residual, act, None, torch.is_grad_enabled())
+            return _call(_LinearFn, x, w, bias, residual, act, None, _keeps())
     y = F.linear(x, w, bias)
     if act == "gelu":
         y = F.gelu(y)

@@ -2,16 +2,16 @@
 same order as the op-by-op path of `EncoderLayer`, without the interpreter between the launches.
 
 `run` returns None when the call is not the plain case; the caller then goes op by op. Plain means: bf16 on a GPU, head
-dimension 64, SwiGLU, no biases, dropout, convolution, hyper-connections or experts, no hooks on the parts, no weights
-that are gathered on use, default kernel choices; and either gradients are off, or every parameter is trained into a
-running fp32 gradient (`main_grad`) and nobody waits for single weight gradients."""
+dimension 64, SwiGLU, no biases, dropout, convolution, hyper-connections or experts, no hooks on the parts, no tracer,
+forward-mode level or function transform, no weights that are gathered on use, default kernel choices; and either
+gradients are off, or every parameter is trained into a running fp32 gradient (`main_grad`) and nobody waits for single
+weight gradients."""
 from __future__ import annotations
 
 import ctypes
 from functools import lru_cache
 
 import torch
-import torch.autograd.forward_ad as _fwd_ad
 import torch.nn.modules.module as _mod
 
 from . import functional as F_
@@ -102,6 +102,8 @@ def _ok_weight(w, rows: int, cols: int) -> bool:
 
 def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
     """attn, mlp, norm2: the layer's Attention, MLP and Norm; norm1: its Norm or None (first layer). Returns y or None."""
+    if F_.functions_observed():     # before anything else: a tracer also sees the sizes that the checks below look at
+        return None
     wqkv, wo, win, wout = attn.Wqkv, attn.Wo, mlp.Wi, mlp.Wo
     if not (x.dtype == BF and x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.data_ptr() % 16 == 0
             and x.shape[0] > 0 and attn.head_dim == 64 and mlp.swiglu and not (mlp.p_drop > 0.0 and mlp.training)
@@ -137,8 +139,6 @@ def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
                 and all(p.requires_grad and _main_grad_ok(p) for p in params if p is not None)):
             return None
         return _LayerFn.apply(x, *params, geo, meta)
-    if _fwd_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():
-        return None
     return _forward(x, params, geo, meta, False)[0]
 
 
