@@ -174,8 +174,7 @@ class EncoderLayer(nn.Module):
         aux = None
         if self.mhc_attn is None:
             if x.is_cuda and self._plain():
-                y = native_layer.run(self.attn, self.mlp, None if self.layer_idx == 0 else self.attn_norm, self.mlp_norm,
-                                     x, ctx, window, rope)
+                y = native_layer.run(self.attn, self.mlp, self.attn_norm, self.mlp_norm, x, ctx, window, rope)
                 if y is not None:
                     return y, None
             if isinstance(self.attn_norm, Norm):

@@ -91,8 +91,9 @@ class _LayerFn(torch.autograd.Function):
 
 
 def _quiet(m) -> bool:
-    """No hooks of any kind on a module whose call would be passed by."""
-    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+    """No hooks of any kind on a module whose call would be passed by, and no forward of the instance's own."""
+    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or "forward" in m.__dict__)
 
 
 def _ok_weight(w, rows: int, cols: int) -> bool:
@@ -101,7 +102,8 @@ def _ok_weight(w, rows: int, cols: int) -> bool:
 
 
 def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
-    """attn, mlp, norm2: the layer's Attention, MLP and Norm; norm1: its Norm or None (first layer). Returns y or None."""
+    """attn, mlp, norm2: the layer's Attention, MLP and Norm; norm1: its Norm, or an Identity (first layer). Returns y
+    or None."""
     if F_.functions_observed():     # before anything else: a tracer also sees the sizes that the checks below look at
         return None
     wqkv, wo, win, wout = attn.Wqkv, attn.Wo, mlp.Wi, mlp.Wo
@@ -110,14 +112,14 @@ def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
             and not F_.fp8_enabled() and K._FA_IMPL[0] == "ws" and K._GEMM_PAIR_DEFAULT[0] is None
             and type(x) is torch.Tensor):
         return None
-    parts = (attn, mlp, wqkv, wo, win, wout, norm2)
+    parts = (attn, mlp, wqkv, wo, win, wout, norm1, norm2)
     if (any(l.bias is not None for l in (wqkv, wo, win, wout, norm2)) or not all(map(_quiet, parts))
             or _mod._has_any_global_hook()):
         return None
     C, HD, I = x.shape[1], attn.num_heads * 64, wout.weight.shape[1]
     n1 = None
-    if norm1 is not None:
-        if norm1.bias is not None or not _quiet(norm1) or norm1.rms != norm2.rms:
+    if type(norm1) is not torch.nn.Identity:
+        if norm1.bias is not None or norm1.rms != norm2.rms:
             return None
         n1 = norm1.weight
     params = (wqkv.weight, wo.weight, win.weight, wout.weight, n1, norm2.weight)
@@ -133,7 +135,7 @@ def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
         return None
     geo = (ctx.seq_start, ctx.seq_end, pos, cos, sin)
     meta = (I, attn.num_heads, window, int(n1 is not None), int(norm2.rms),
-            norm1.eps if norm1 is not None else 0.0, norm2.eps, attn.scale)
+            norm1.eps if n1 is not None else 0.0, norm2.eps, attn.scale)
     if torch.is_grad_enabled():
         if not (x.requires_grad and F_._WGRAD_READY[0] is None
                 and all(p.requires_grad and _main_grad_ok(p) for p in params if p is not None)):

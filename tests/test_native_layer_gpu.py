@@ -95,3 +95,39 @@ def test_layer_falls_back(cuda_status, monkeypatch):
         layer(x, ctx, 64, rope)
     finally:
         K.set_attention_impl("ws")
+
+
+@pytest.mark.parametrize("idx", [0, 1])
+@pytest.mark.parametrize("grad", [False, True])
+def test_every_part_that_is_called_op_by_op_is_observed(idx, grad, cuda_status):
+    """Hooks, backward hooks and a forward of the instance's own on each part in turn: they run, as op by op."""
+    layer, ctx, rope = _layer(128, 128, idx), _context([50, 20]), _rope()
+    for p in layer.parameters():
+        p.main_grad = torch.zeros(p.shape, device="cuda")
+    x = torch.randn(70, 128, device="cuda").to(BF).requires_grad_(grad)
+    seen = []
+
+    def call():
+        with torch.set_grad_enabled(grad):
+            y, _ = layer(x, ctx, 64, rope)
+        if grad:
+            y.sum().backward()
+
+    # (the linear layers' weights and the norms' residual form are used without a call of these modules)
+    called = [layer.attn, layer.mlp] + ([layer.attn_norm] if idx == 0 else [])
+    for m in called:
+        for add in (lambda: m.register_forward_hook(lambda *a: seen.append(1)),
+                    lambda: m.register_forward_pre_hook(lambda *a: seen.append(1))):
+            h = add()
+            call()
+            assert seen.pop() and not seen
+            h.remove()
+        m.forward = lambda *a, f=m.forward, **k: (seen.append(1), f(*a, **k))[1]
+        call()
+        del m.forward
+        assert seen.pop() and not seen
+        if grad:
+            h = m.register_full_backward_hook(lambda *a: seen.append(1))
+            call()
+            assert seen.pop() and not seen
+            h.remove()
