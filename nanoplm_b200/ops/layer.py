@@ -63,7 +63,7 @@ class _LayerFn(torch.autograd.Function):
         y, buf = _forward(x, params, geo, meta, True)
         ctx.save_for_backward(x, buf, *params, *geo)
         ctx.meta = meta
-        ctx.refs = params[:4]
+        ctx.refs = params       # saved-tensor hooks may give back copies, which do not carry the running gradients
         return y
 
     @staticmethod
@@ -76,7 +76,7 @@ class _LayerFn(torch.autograd.Function):
         h = _native()
         dx = torch.empty_like(x)
         scratch = torch.empty(h.nplm_layer_bytes(T, C, I, H, norm1, 1, 1), dtype=torch.uint8, device=x.device)
-        grads = [p.main_grad.data_ptr() if p is not None else 0 for p in params]
+        grads = [p.main_grad.data_ptr() if p is not None else 0 for p in ctx.refs]
         HD = H * 64
         a = _BwdArgs(T, C, I, H, window, norm1, rms, 1, x.data_ptr(), *[p.data_ptr() if p is not None else 0 for p in params],
                      *[g.data_ptr() for g in geo], buf.data_ptr(), dy.data_ptr(), status_word(x.device).data_ptr(),
@@ -85,7 +85,7 @@ class _LayerFn(torch.autograd.Function):
         check_rc(h.nplm_layer_bwd(a, scale), "layer_bwd")
         count_launch(12 + norm1)
         if F_._WGRAD_READY[0] is not None:      # (set after this layer's forward)
-            for p in reversed(ctx.refs):
+            for p in reversed(ctx.refs[:4]):
                 F_._WGRAD_READY[0](p)
         return dx, None, None, None, None, None, None, None, None
 
