@@ -130,8 +130,11 @@ def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
         return None
     cos, sin = rope
     pos = ctx.position_ids
-    if (pos.numel() != x.shape[0] or cos.dtype != torch.float32 or cos.shape[-1] != 32 or not cos.is_contiguous()
-            or not pos.is_contiguous()):
+    # (what is wrong here is for the op-by-op path to refuse)
+    if not (pos.numel() == x.shape[0] and all(t.dtype == torch.int32 and t.is_cuda and t.is_contiguous()
+                                              for t in (pos, ctx.seq_start, ctx.seq_end))
+            and all(t.dtype == torch.float32 and t.is_cuda and t.is_contiguous() and t.shape[-1] == 32
+                    for t in (cos, sin))):
         return None
     geo = (ctx.seq_start, ctx.seq_end, pos, cos, sin)
     meta = (I, attn.num_heads, window, int(n1 is not None), int(norm2.rms),
@@ -146,4 +149,5 @@ def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
 
 def _main_grad_ok(p) -> bool:
     g = getattr(p, "main_grad", None)
-    return g is not None and g.dtype == torch.float32 and g.is_contiguous() and g.data_ptr() % 16 == 0
+    return (g is not None and g.dtype == torch.float32 and g.is_cuda and g.shape == p.shape and g.is_contiguous()
+            and g.data_ptr() % 16 == 0)

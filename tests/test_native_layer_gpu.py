@@ -159,3 +159,24 @@ def test_saved_tensors_may_come_back_as_copies(how, cuda_status):
     assert (dx.float() - dx_h.float()).norm() <= 6e-3 * dx.float().norm()
     for n in grads:
         assert (grads[n] - grads_h[n]).norm() <= 6e-3 * grads[n].norm() and grads[n].norm() > 0, n
+
+
+def test_refusals_of_the_op_by_op_path_stay(cuda_status):
+    """Metadata of the wrong type or on the wrong device, and running gradients of the wrong shape, are errors."""
+    import copy
+    layer, ctx, rope = _layer(128, 128, 1), _context([50, 20]), _rope()
+    x = torch.randn(70, 128, device="cuda").to(BF).requires_grad_(True)
+    for p in layer.parameters():
+        p.main_grad = torch.zeros(p.shape, device="cuda")
+    for wrong in (lambda p: p.long(), lambda p: p.cpu(), lambda p: p[:69]):
+        c = copy.copy(ctx)
+        c.position_ids = wrong(ctx.position_ids)
+        for grad in (False, True):
+            with torch.set_grad_enabled(grad), pytest.raises(ValueError):
+                layer(x, c, 64, rope)
+    for cos in (rope[0].double(), rope[0].cpu(), rope[0][:, :16]):
+        with torch.no_grad(), pytest.raises(ValueError):
+            layer(x, ctx, 64, (cos, rope[1]))
+    layer.mlp.Wi.weight.main_grad = torch.zeros(128, 256, device="cuda")
+    with pytest.raises(ValueError):
+        layer(x, ctx, 64, rope)[0].sum().backward()
