@@ -159,7 +159,7 @@ class _CoefFn(torch.autograd.Function):
         dR = dR.float().contiguous() if dR is not None else zeros(T, n, n)
         # the kernel adds to what it is given: the parameters' running gradients where they have them
         direct = all(_has_main_grad(p) and p.main_grad.dtype == torch.float32 and p.main_grad.is_contiguous()
-                     for p in ctx.refs)
+                     and p.main_grad.device == dev and p.main_grad.numel() == p.numel() for p in ctx.refs)
         grads = tuple(p.main_grad if direct else zeros(*p.shape) for p in ctx.refs)
         dpre = K.mhc_coef_bwd(pre, *params, ctx.iters, n, dalpha, dbeta, dR, *grads)
         if direct:

@@ -54,3 +54,15 @@ def test_coefficient_parameters_in_bf16(n, cuda_status):
         assert torch.allclose(a, b, rtol=2 ** -8, atol=1e-3)        # returned in bf16
     for a, b in zip(outs[2][4], outs[1][4]):
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-3)           # atomics in another order
+
+
+def test_coefficient_gradients_of_the_wrong_size_are_refused(cuda_status):
+    from nanoplm_b200.models.mhc import _CoefFn
+    n, T = 4, 50
+    ps = [torch.nn.Parameter(torch.randn(*s, device="cuda").to(BF)) for s in ((n,), (n,), (n, n), (3,))]
+    for p in ps:
+        p.main_grad = torch.zeros(p.shape, device="cuda")
+    ps[2].main_grad = torch.zeros(n, device="cuda")
+    alpha, beta, R = _CoefFn.apply(torch.randn(T, 2 * n + n * n, device="cuda").to(BF).requires_grad_(True), *ps, 5, n)
+    with pytest.raises(RuntimeError):
+        (alpha.sum() + beta.sum() + R.sum()).backward()
