@@ -102,17 +102,19 @@ def orthogonalize_batched(G: torch.Tensor, coeffs=NS_QUINTIC, eps: float = 1e-7,
     dt = torch.bfloat16 if G.is_cuda else torch.float32
     X = G.to(dt)
     transposed = X.shape[1] > X.shape[2]
+    # Tall stacks with their norms at hand (the optimizer step): transposed and scaled in one pass by this package's kernel
+    # where whole 64 x 64 tiles allow. Without the norms several passes over the stack in fp32 come first and the
+    # transpose is not what such a call waits for.
+    tiled = (transposed and sumsq is not None and X.is_cuda and X.is_contiguous() and X.shape[1] % 64 == 0
+             and X.shape[2] % 64 == 0 and X.shape[0] <= 65535 and X.data_ptr() % 16 == 0)
+    scaled = tiled and X.shape[2] % 128 == 0        # the grouped path below
+    if transposed and not scaled:
+        X = X.transpose(1, 2).contiguous()
     nrm = X.float().flatten(1).norm(dim=1) if sumsq is None else sumsq.float().sqrt()
     inv = (1.0 / (nrm * 1.01 + eps)).to(dt)[:, None, None]
-    # tall stacks: transposed and scaled in one pass by this package's kernel where whole 64 x 64 tiles allow
-    tiled = (transposed and X.is_cuda and X.is_contiguous() and X.shape[1] % 64 == 0 and X.shape[2] % 64 == 0
-             and X.shape[0] <= 65535 and X.data_ptr() % 16 == 0)
-    scaled = False
-    if tiled and X.shape[2] % 128 == 0:             # the grouped path below
+    if scaled:
         from nanoplm_b200.ops import kernels as K
-        X, scaled = K.transpose_scale(X, inv.reshape(-1)), True
-    elif transposed:
-        X = X.transpose(1, 2).contiguous()
+        X = K.transpose_scale(X, inv.reshape(-1))
     grouped = _grouped_ok(X)
     if grouped:
         if not scaled:
