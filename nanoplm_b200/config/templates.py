@@ -101,7 +101,7 @@ pretraining:
   # balance_ranks: true           # equal-cost micro-batches on every rank (static packing, several GPUs)
   # shard_params: false           # shard the layers' weights over the ranks (all-gather fused into the GEMMs)
   # nvtx_ranges: false            # NVTX ranges around forward / backward / optimizer step
-  # deterministic_attention: false  # attention backward without atomics (bitwise reproducible, slower)
+  # deterministic_attention: false  # attention backward and linear weight gradients bitwise reproducible (slower)
   # hf_checkpoint_files: false    # also write model.safetensors + trainer_state.json with every checkpoint
 
 # The native pipeline (own CUDA kernels, sharded data parallelism). `use_compile` is accepted for

@@ -275,7 +275,7 @@ struct Fp8Args {
   int M, N, K, ldc;
   int b_block;
   int out_mode;      // 0: bf16 store, 1: fp32 store, 2: fp32 reduce-add (all through tmC)
-  int splits;        // out_mode 2: the K blocks of a tile are cut into this many work items
+  int splits;        // out_mode 2: the K blocks of a tile are cut into this many work items (0: the launch chooses)
   int* status;
   // All-gather mode (ag_world > 1, block-scaled B only): B's rows and the matching scale columns
   // are sharded over the ranks. The epilogue warps of all CTAs first copy the other ranks' e4m3
@@ -716,7 +716,8 @@ static int f8_launch_form(const void* A, const void* B, void* C, Fp8Args& args, 
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_slot);
   const int tiles = ((args.M + F8_BM - 1) / F8_BM) * ((args.N + BN - 1) / BN);
-  args.splits = args.out_mode == 2 ? f8_splits(tiles, args.K / F8_BK, sms) : 1;
+  if (args.out_mode != 2) args.splits = 1;
+  else if (args.splits == 0) args.splits = f8_splits(tiles, args.K / F8_BK, sms);
   const int total = tiles * args.splits;
   const int grid = total < sms ? total : sms;
   if (coop) {
@@ -790,9 +791,10 @@ extern "C" int nplm_fp8_quant_dual(const void* x, int R, int K, int ldx, void* q
 
 // C[M][N] (+)= (A * sa) (B * sb)^T, A e4m3 [M][K], B e4m3 [N][K] (both K-major, K % 128 == 0).
 // sa fp32 [K/128][M]; sb fp32 [K/128][N] (b_block = 0) or [K/128][ceil(N/128)] (b_block = 1).
-// out_mode 0: bf16 C; 1: fp32 C; 2: fp32 C accumulated with atomics.
+// out_mode 0: bf16 C; 1: fp32 C; 2: fp32 C accumulated by TMA reduce-adds, several work items a tile in any order unless
+// whole_tiles is set.
 extern "C" int nplm_gemm_fp8(const void* A, const void* B, void* C, const float* sa, const float* sb,
-                             int M, int N, int K, int ldc, int b_block, int out_mode, int* status,
+                             int M, int N, int K, int ldc, int b_block, int out_mode, int whole_tiles, int* status,
                              cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((K % 128) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
@@ -808,6 +810,7 @@ extern "C" int nplm_gemm_fp8(const void* A, const void* B, void* C, const float*
   args.K = K;
   args.ldc = ldc;
   args.b_block = b_block;
+  args.splits = whole_tiles ? 1 : 0;
   args.out_mode = out_mode;
   args.status = status;
   args.ag_world = 0;
@@ -843,6 +846,7 @@ extern "C" int nplm_gemm_fp8_ag(const void* A, void* const* b_ptrs, void* C, con
   args.K = K;
   args.ldc = ldc;
   args.b_block = 1;
+  args.splits = 0;
   args.out_mode = out_mode;
   args.status = status;
   args.ag_world = world;

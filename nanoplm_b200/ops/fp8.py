@@ -16,6 +16,7 @@ from ctypes import c_int
 
 import torch
 
+from . import kernels as _kernels
 from ._lib import check_rc, count_launch, lib, ptr, status_word, stream_ptr
 
 _BF16 = torch.bfloat16
@@ -97,7 +98,8 @@ def quant_dual(x: torch.Tensor) -> tuple[Quantized, Quantized]:
 
 def gemm_fp8(a: Quantized, b: Quantized, *, out: torch.Tensor | None = None, out_dtype=_BF16,
              accumulate: bool = False) -> torch.Tensor:
-    """C[M,N] (+)= deq(a) deq(b)^T. a: row-scaled [M,K]; b: row- or block-scaled [N,K]."""
+    """C[M,N] (+)= deq(a) deq(b)^T. a: row-scaled [M,K]; b: row- or block-scaled [N,K]. With accumulate several work
+    items may add to a tile, in any order; under `kernels.set_attention_deterministic` one does."""
     if a.block:
         raise ValueError("the A operand must carry 1 x 128 scales")
     M, K = a.q.shape
@@ -113,7 +115,8 @@ def gemm_fp8(a: Quantized, b: Quantized, *, out: torch.Tensor | None = None, out
         raise ValueError("out must be a row-major bf16 or fp32 [M, N] tensor")
     rc = lib("fp8").nplm_gemm_fp8(ptr(a.q), ptr(b.q), ptr(out), ptr(a.scale), ptr(b.scale), c_int(M), c_int(N),
                                   c_int(K), c_int(out.stride(0)), c_int(int(b.block)), c_int(mode),
-                                  ptr(status_word(a.q.device)), stream_ptr())
+                                  c_int(int(_kernels._FA_DETERMINISTIC[0])), ptr(status_word(a.q.device)),
+                                  stream_ptr())
     check_rc(rc, "gemm_fp8")
     count_launch()
     return out

@@ -55,13 +55,13 @@ def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
     if (tiled or narrow) and Kd % 64 == 0:
         if _has_main_grad(w) and (tiled or w.main_grad.data_ptr() % 16 == 0):
             K.gemm(dy2, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=w.main_grad,
-                   splits=K.wgrad_splits(N, Kd, T))
+                   splits=K.weight_grad_splits(N, Kd, T))
             if tiled and _WGRAD_READY[0] is not None:
                 _WGRAD_READY[0](w)
             return None
         acc = torch.zeros((N, Kd), dtype=torch.float32, device=w.device)
         K.gemm(dy2, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=acc,
-               splits=K.wgrad_splits(N, Kd, T))
+               splits=K.weight_grad_splits(N, Kd, T))
         return _param_grad(w, acc)
     g = dy2.float().t() @ x2.float()
     if _has_main_grad(w):

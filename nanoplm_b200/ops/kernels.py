@@ -6,6 +6,7 @@ stream and returns output tensors. ``nanoplm_b200.ops.functional`` builds differ
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_longlong
+from functools import lru_cache
 
 import torch
 
@@ -211,6 +212,15 @@ def wgrad_splits(n_out: int, k_in: int, tokens: int, bn: int = 256, sms: int = 1
         if best_cost is None or cost < 0.98 * best_cost:
             best, best_cost = s, cost
     return best
+
+
+_default_splits = lru_cache(maxsize=1024)(wgrad_splits)
+
+
+def weight_grad_splits(n_out: int, k_in: int, tokens: int) -> int:
+    """Split factor of a weight gradient in a backward pass: `wgrad_splits`, and 1 under
+    `set_attention_deterministic` (several work items add to a tile in any order, one gives the same bits every run)."""
+    return 1 if _FA_DETERMINISTIC[0] else _default_splits(n_out, k_in, tokens)
 
 
 # --------------------------------------------------------------------------- norms
@@ -526,7 +536,9 @@ _FA_DETERMINISTIC = [_os.environ.get("NPLM_FA_DETERMINISTIC", "0") not in ("", "
 
 def set_attention_deterministic(flag: bool) -> None:
     """True: the warp-specialised backward pass forms dQ in a second, query-stationary launch instead
-    of fp32 atomics, so two runs on the same inputs give the same bits (about 1.4x the time)."""
+    of fp32 atomics, so two runs on the same inputs give the same bits (about 1.4x the time). The weight gradients
+    of linear layers (bf16 and e4m3), which by default are summed by several work items in any order, then come
+    from one work item a tile."""
     _FA_DETERMINISTIC[0] = bool(flag)
 
 

@@ -9,7 +9,6 @@ weight gradients."""
 from __future__ import annotations
 
 import ctypes
-from functools import lru_cache
 
 import torch
 import torch.nn.modules.module as _mod
@@ -21,7 +20,6 @@ from ._lib import check_rc, count_launch, lib, raw_stream, status_word
 BF = torch.bfloat16
 _READY = [None]
 _FwdArgs, _BwdArgs = ctypes.c_longlong * 24, ctypes.c_longlong * 37
-_splits = lru_cache(maxsize=1024)(K.wgrad_splits)
 
 
 def _native():
@@ -80,8 +78,9 @@ class _LayerFn(torch.autograd.Function):
         HD = H * 64
         a = _BwdArgs(T, C, I, H, window, norm1, rms, 1, x.data_ptr(), *[p.data_ptr() if p is not None else 0 for p in params],
                      *[g.data_ptr() for g in geo], buf.data_ptr(), dy.data_ptr(), status_word(x.device).data_ptr(),
-                     raw_stream(), dx.data_ptr(), scratch.data_ptr(), *grads, _splits(3 * HD, C, T), _splits(C, HD, T),
-                     _splits(2 * I, C, T), _splits(C, I, T), 3 if K._FA_DETERMINISTIC[0] else -1)
+                     raw_stream(), dx.data_ptr(), scratch.data_ptr(), *grads, K.weight_grad_splits(3 * HD, C, T),
+                     K.weight_grad_splits(C, HD, T), K.weight_grad_splits(2 * I, C, T), K.weight_grad_splits(C, I, T),
+                     3 if K._FA_DETERMINISTIC[0] else -1)
         check_rc(h.nplm_layer_bwd(a, scale), "layer_bwd")
         count_launch(12 + norm1)
         if F_._WGRAD_READY[0] is not None:      # (set after this layer's forward)
