@@ -52,7 +52,9 @@ struct Cut {   // consecutive 256-byte aligned parts of one allocation
   }
 };
 
-// What a forward pass leaves for the backward pass, in one allocation.
+// The tensors of a forward pass, in one allocation. With a backward pass to come everything has a place of its own;
+// without one a tensor takes the place of those that no later kernel reads: o that of h1 (its last reader is the QKV
+// product), and the MLP's h2 and hs those of h1 / o and qkv (last read by the attention and its output product).
 struct Saved {
   void *h1, *qkv, *o, *x1, *h2, *pre, *hs;
   float *mean1, *rstd1, *lse, *mean2, *rstd2;
@@ -60,17 +62,33 @@ struct Saved {
   Saved(void* buf, long long T, long long C, long long I, long long H, bool norm1, bool train) {
     Cut c(buf);
     const size_t t = static_cast<size_t>(T);
+    if (!train) {
+      mean1 = rstd1 = mean2 = rstd2 = nullptr;
+      pre = nullptr;
+      x1 = c.take(t * C * 2);
+      const size_t first = c.at;
+      o = c.take(t * (norm1 && C > H * 64 ? C : H * 64) * 2);
+      h1 = norm1 ? o : nullptr;
+      qkv = c.take(t * 3 * H * 64 * 2);
+      lse = reinterpret_cast<float*>(c.take(t * H * 4));
+      Cut m(buf);
+      m.at = first;
+      h2 = m.take(t * C * 2);
+      hs = m.take(t * I * 2);
+      bytes = c.at > m.at ? c.at : m.at;
+      return;
+    }
     h1 = norm1 ? c.take(t * C * 2) : nullptr;
-    mean1 = norm1 && train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
-    rstd1 = norm1 && train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
+    mean1 = norm1 ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
+    rstd1 = norm1 ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
     qkv = c.take(t * 3 * H * 64 * 2);
     o = c.take(t * H * 64 * 2);
     lse = reinterpret_cast<float*>(c.take(t * H * 4));
     x1 = c.take(t * C * 2);
-    mean2 = train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
-    rstd2 = train ? reinterpret_cast<float*>(c.take(t * 4)) : nullptr;
+    mean2 = reinterpret_cast<float*>(c.take(t * 4));
+    rstd2 = reinterpret_cast<float*>(c.take(t * 4));
     h2 = c.take(t * C * 2);
-    pre = train ? c.take(t * 2 * I * 2) : nullptr;
+    pre = c.take(t * 2 * I * 2);
     hs = c.take(t * I * 2);
     bytes = c.at;
   }
