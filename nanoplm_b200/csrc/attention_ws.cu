@@ -25,6 +25,7 @@
 // Replaces flash_attn_varlen_func as called by the reference
 // (src/nanoplm/pretraining/models/modern_bert/modeling.py:331-366) with window (-1,-1) or (64,64).
 #include "common.cuh"
+#include "entry_points.h"
 
 namespace nplm {
 

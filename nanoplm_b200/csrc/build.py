@@ -110,11 +110,14 @@ def build_host(name: str, force: bool = False) -> Path:
     src = CSRC / name
     out = lib_path(name)
     stamp = out.with_suffix(".sha")
-    digest = hashlib.sha256(src.read_bytes()).hexdigest()
+    h = hashlib.sha256(src.read_bytes())
+    for hdr in sorted(CSRC.glob("*.h")):
+        h.update(hdr.read_bytes())
+    digest = h.hexdigest()
     if not force and out.exists() and stamp.exists() and stamp.read_text() == digest:
         return out
     cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
-    cmd = [cxx, "-O3", "-std=c++17", "-fPIC", "-shared", "-o", "@OUT@", str(src)]
+    cmd = [cxx, "-O3", "-std=c++17", "-fPIC", "-shared", "-I", str(CSRC), "-o", "@OUT@", str(src)]
     return _locked_build(out, digest, cmd, name, False, force)
 
 

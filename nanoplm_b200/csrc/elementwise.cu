@@ -12,6 +12,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "entry_points.h"
 
 namespace nplm {
 

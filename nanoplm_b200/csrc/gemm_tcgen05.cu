@@ -16,31 +16,13 @@
 // Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2.. = epilogue (four, or eight
 // on CTA pairs; a warp reads the TMEM lane quarter warp_idx % 4, two of a quarter split the columns).
 #include "common.cuh"
+#include "entry_points.h"
 
 namespace nplm {
 
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
-
-enum : int {
-  EPI_STORE = 0,       // C(bf16) = acc
-  EPI_ADD = 1,         // C(bf16) = acc + R(bf16)
-  EPI_ATOMIC_F32 = 2,  // C(fp32) += acc   (split-K capable; used for weight gradients)
-  EPI_GELU = 3,        // C(bf16) = gelu(acc) (erf form); also writes the pre-activation to R when R != null
-  EPI_STORE_F32 = 4,   // C(fp32) = acc
-  EPI_SWIGLU = 5,      // B tile = [value rows | gate rows]; C(bf16, N/2 wide) = silu(gate)*value,
-                       // pre-activations (bf16, N wide) written to R
-  EPI_RELU = 7,        // the same with ReLU. A form of its own: chosen at run time inside EPI_GELU it kept that
-                       // epilogue's code and registers (55 424 x 4096 x 1024: 488 -> 350 us)
-  EPI_ROPE = 6,        // C(bf16) = acc with rotary embedding applied to every 64-wide head whose
-                       // first column is < rope_cols (the q and k parts of a fused QKV projection)
-  EPI_STORE_DELTA = 9, // C(bf16) = acc, and delta[col / 64][row] = sum over each 64-column head of
-                       // bf16(acc) * R (the attention backward's rowsum(dO * O), R = O)
-  EPI_SWIGLU_BWD = 8,  // acc = gradient of the SwiGLU output h = silu(gate) * value, N wide;
-                       // R = the pre-activations [value | gate] (bf16, 2N wide); C (bf16, 2N wide) =
-                       // [acc * silu(gate) | acc * value * silu'(gate)], the gradient of R
-};
 
 // PAIR: two CTAs of a cluster (cta_group::2) share one 256 x BN tile; each holds its own 128 rows
 // of A and half of B, which cuts the L2 -> shared-memory traffic per FLOP by a third.

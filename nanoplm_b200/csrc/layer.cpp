@@ -11,33 +11,33 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "entry_points.h"
+
 namespace {
 
-typedef int (*GemmFn)(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int,
-                      int, int, int, const int*, const float*, const float*, int, int*, void*);
-typedef int (*GemmPairFn)(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int,
-                          int, int, const int*, const float*, const float*, int, int*, void*);
-typedef int (*DeltaFn)(const void*, const void*, void*, const void*, float*, int, int, int, int, int, int, int, int, int*,
-                       void*);
-typedef int (*NormFwdFn)(const void*, const int*, const void*, void*, float*, float*, int, int, float, int, void*);
-typedef int (*NormBwdFn)(const void*, const void*, const int*, const void*, const float*, const float*, const void*, void*,
-                         float*, float*, int, int, int, int, void*);
-typedef int (*FaFwdFn)(const void*, void*, float*, const int*, const int*, int, int, int, int, float, int, int*, void*);
-typedef int (*FaBwdFn)(const void*, const void*, const void*, const float*, void*, float*, float*, const int*, const int*,
-                       int, int, int, int, float, const int*, const float*, const float*, int, int, int*, void*);
+using namespace nplm;
 
-struct Entry {
-  GemmFn gemm;
-  GemmPairFn pair;
-  DeltaFn delta;
-  NormFwdFn norm_fwd;
-  NormBwdFn norm_bwd;
-  FaFwdFn fa_fwd;
-  FaBwdFn fa_bwd;
+struct Entry {   // in the order of `_native` in ops/layer.py
+  decltype(&nplm_gemm_bf16) gemm;
+  decltype(&nplm_gemm_bf16_pair) pair;
+  decltype(&nplm_gemm_bf16_delta) delta;
+  decltype(&nplm_norm_fwd) norm_fwd;
+  decltype(&nplm_norm_bwd) norm_bwd;
+  decltype(&nplm_fa_fwd_ws) fa_fwd;
+  decltype(&nplm_fa_bwd_ws_mode) fa_bwd;
 };
 Entry fn;
 
-enum { EPI_STORE = 0, EPI_ADD = 1, EPI_ATOMIC_F32 = 2, EPI_SWIGLU = 5, EPI_ROPE = 6, EPI_SWIGLU_BWD = 8 };
+// Positions in the argument arrays that ops/layer.py fills; BWD_ ones follow those of the forward call.
+enum Arg {
+  A_T, A_C, A_I, A_H, A_WINDOW, A_NORM1, A_RMS, A_TRAIN,
+  A_X, A_W_QKV, A_W_O, A_W_IN, A_W_OUT, A_N1, A_N2,
+  A_SEQ_START, A_SEQ_END, A_POS, A_COS, A_SIN,
+  A_BUF, A_Y, A_STATUS, A_STREAM,
+  BWD_DX, BWD_SCRATCH, BWD_G_QKV, BWD_G_O, BWD_G_IN, BWD_G_OUT, BWD_G_N1, BWD_G_N2,
+  BWD_SPLITS_QKV, BWD_SPLITS_O, BWD_SPLITS_IN, BWD_SPLITS_OUT, BWD_ATTENTION_MODE,
+  BWD_ARGS, FWD_ARGS = BWD_DX
+};
 
 typedef unsigned char u8;
 
@@ -119,7 +119,7 @@ struct Scratch {
 
 struct Call {
   int* status;
-  void* stream;
+  cudaStream_t stream;
   // bf16 output: CTA pairs on 256-wide tiles, as ops.kernels.gemm chooses by default
   int out(const void* A, const void* B, void* Cp, const void* R, int M, int N, int K, int ldb, int ldc, int ldr, int b_mn,
           int epi, const int* pos = nullptr, const float* cosp = nullptr, const float* sinp = nullptr,
@@ -150,14 +150,17 @@ P* ptr(const long long* a, int i) {
 }  // namespace
 
 extern "C" void nplm_layer_init(void* const* f) {
-  fn.gemm = reinterpret_cast<GemmFn>(f[0]);
-  fn.pair = reinterpret_cast<GemmPairFn>(f[1]);
-  fn.delta = reinterpret_cast<DeltaFn>(f[2]);
-  fn.norm_fwd = reinterpret_cast<NormFwdFn>(f[3]);
-  fn.norm_bwd = reinterpret_cast<NormBwdFn>(f[4]);
-  fn.fa_fwd = reinterpret_cast<FaFwdFn>(f[5]);
-  fn.fa_bwd = reinterpret_cast<FaBwdFn>(f[6]);
+  fn.gemm = reinterpret_cast<decltype(fn.gemm)>(f[0]);
+  fn.pair = reinterpret_cast<decltype(fn.pair)>(f[1]);
+  fn.delta = reinterpret_cast<decltype(fn.delta)>(f[2]);
+  fn.norm_fwd = reinterpret_cast<decltype(fn.norm_fwd)>(f[3]);
+  fn.norm_bwd = reinterpret_cast<decltype(fn.norm_bwd)>(f[4]);
+  fn.fa_fwd = reinterpret_cast<decltype(fn.fa_fwd)>(f[5]);
+  fn.fa_bwd = reinterpret_cast<decltype(fn.fa_bwd)>(f[6]);
 }
+
+// Length of the argument array of a forward (0) or backward (1) call.
+extern "C" int nplm_layer_args(int backward) { return backward ? BWD_ARGS : FWD_ARGS; }
 
 // Bytes of the forward pass's buffer (backward = 0) or of the backward pass's scratch (1).
 extern "C" long long nplm_layer_bytes(long long T, long long C, long long I, long long H, int norm1, int train,
@@ -166,21 +169,20 @@ extern "C" long long nplm_layer_bytes(long long T, long long C, long long I, lon
                                          : Saved(nullptr, T, C, I, H, norm1 != 0, train != 0).bytes);
 }
 
-// a: T, C, I, H, window, norm1, rms, train, then addresses: x, w_qkv, w_o, w_in, w_out, n1, n2, seq_start, seq_end,
-// pos, cos, sin, buffer, y, status, stream
+// a: see Arg
 extern "C" int nplm_layer_fwd(const long long* a, double eps1, double eps2, double scale) {
-  const int T = static_cast<int>(a[0]), C = static_cast<int>(a[1]), I = static_cast<int>(a[2]), H = static_cast<int>(a[3]);
-  const int window = static_cast<int>(a[4]), rms = static_cast<int>(a[6]);
-  const bool norm1 = a[5] != 0, train = a[7] != 0;
+  const int T = static_cast<int>(a[A_T]), C = static_cast<int>(a[A_C]), I = static_cast<int>(a[A_I]), H = static_cast<int>(a[A_H]);
+  const int window = static_cast<int>(a[A_WINDOW]), rms = static_cast<int>(a[A_RMS]);
+  const bool norm1 = a[A_NORM1] != 0, train = a[A_TRAIN] != 0;
   const int HD = H * 64;
   if (T <= 0) return 0;
-  const void *x = ptr<void>(a, 8), *wqkv = ptr<void>(a, 9), *wo = ptr<void>(a, 10), *win = ptr<void>(a, 11),
-             *wout = ptr<void>(a, 12), *n1 = ptr<void>(a, 13), *n2 = ptr<void>(a, 14);
-  const int *ss = ptr<int>(a, 15), *se = ptr<int>(a, 16), *pos = ptr<int>(a, 17);
-  const float *cosp = ptr<float>(a, 18), *sinp = ptr<float>(a, 19);
-  const Saved s(ptr<void>(a, 20), T, C, I, H, norm1, train);
-  void* y = ptr<void>(a, 21);
-  const Call k{ptr<int>(a, 22), ptr<void>(a, 23)};
+  const void *x = ptr<void>(a, A_X), *wqkv = ptr<void>(a, A_W_QKV), *wo = ptr<void>(a, A_W_O), *win = ptr<void>(a, A_W_IN),
+             *wout = ptr<void>(a, A_W_OUT), *n1 = ptr<void>(a, A_N1), *n2 = ptr<void>(a, A_N2);
+  const int *ss = ptr<int>(a, A_SEQ_START), *se = ptr<int>(a, A_SEQ_END), *pos = ptr<int>(a, A_POS);
+  const float *cosp = ptr<float>(a, A_COS), *sinp = ptr<float>(a, A_SIN);
+  const Saved s(ptr<void>(a, A_BUF), T, C, I, H, norm1, train);
+  void* y = ptr<void>(a, A_Y);
+  const Call k{ptr<int>(a, A_STATUS), ptr<CUstream_st>(a, A_STREAM)};
   if (norm1)
     TRY(fn.norm_fwd(x, nullptr, n1, s.h1, rms ? nullptr : s.mean1, s.rstd1, T, C, static_cast<float>(eps1), rms, k.stream));
   const void* h1 = norm1 ? s.h1 : x;
@@ -192,40 +194,39 @@ extern "C" int nplm_layer_fwd(const long long* a, double eps1, double eps2, doub
   return k.out(s.hs, wout, y, s.x1, T, C, I, I, C, C, 0, EPI_ADD);
 }
 
-// a: as nplm_layer_fwd with y = the incoming gradient dy, then addresses: dx, scratch, the fp32 gradients of w_qkv, w_o,
-// w_in, w_out, n1, n2 (added to), then the split factors of the four weight gradients and the attention mode
-// (-1 default, 3 reproducible)
+// a: see Arg, with A_Y = the incoming gradient dy. The fp32 gradients are added to; attention mode -1 is the default, 3 the
+// reproducible one.
 extern "C" int nplm_layer_bwd(const long long* a, double scale) {
-  const int T = static_cast<int>(a[0]), C = static_cast<int>(a[1]), I = static_cast<int>(a[2]), H = static_cast<int>(a[3]);
-  const int window = static_cast<int>(a[4]), rms = static_cast<int>(a[6]);
-  const bool norm1 = a[5] != 0;
+  const int T = static_cast<int>(a[A_T]), C = static_cast<int>(a[A_C]), I = static_cast<int>(a[A_I]), H = static_cast<int>(a[A_H]);
+  const int window = static_cast<int>(a[A_WINDOW]), rms = static_cast<int>(a[A_RMS]);
+  const bool norm1 = a[A_NORM1] != 0;
   const int HD = H * 64;
   if (T <= 0) return 0;
-  const void *x = ptr<void>(a, 8), *wqkv = ptr<void>(a, 9), *wo = ptr<void>(a, 10), *win = ptr<void>(a, 11),
-             *wout = ptr<void>(a, 12), *n1 = ptr<void>(a, 13), *n2 = ptr<void>(a, 14);
-  const int *ss = ptr<int>(a, 15), *se = ptr<int>(a, 16), *pos = ptr<int>(a, 17);
-  const float *cosp = ptr<float>(a, 18), *sinp = ptr<float>(a, 19);
-  const Saved s(ptr<void>(a, 20), T, C, I, H, norm1, true);
-  const void* dy = ptr<void>(a, 21);
-  const Call k{ptr<int>(a, 22), ptr<void>(a, 23)};
-  void* dx = ptr<void>(a, 24);
-  const Scratch d(ptr<void>(a, 25), T, C, I, H);
-  float *g_qkv = ptr<float>(a, 26), *g_o = ptr<float>(a, 27), *g_in = ptr<float>(a, 28), *g_out = ptr<float>(a, 29),
-        *g_n1 = ptr<float>(a, 30), *g_n2 = ptr<float>(a, 31);
-  const int mode = static_cast<int>(a[36]);
+  const void *x = ptr<void>(a, A_X), *wqkv = ptr<void>(a, A_W_QKV), *wo = ptr<void>(a, A_W_O), *win = ptr<void>(a, A_W_IN),
+             *wout = ptr<void>(a, A_W_OUT), *n1 = ptr<void>(a, A_N1), *n2 = ptr<void>(a, A_N2);
+  const int *ss = ptr<int>(a, A_SEQ_START), *se = ptr<int>(a, A_SEQ_END), *pos = ptr<int>(a, A_POS);
+  const float *cosp = ptr<float>(a, A_COS), *sinp = ptr<float>(a, A_SIN);
+  const Saved s(ptr<void>(a, A_BUF), T, C, I, H, norm1, true);
+  const void* dy = ptr<void>(a, A_Y);
+  const Call k{ptr<int>(a, A_STATUS), ptr<CUstream_st>(a, A_STREAM)};
+  void* dx = ptr<void>(a, BWD_DX);
+  const Scratch d(ptr<void>(a, BWD_SCRATCH), T, C, I, H);
+  float *g_qkv = ptr<float>(a, BWD_G_QKV), *g_o = ptr<float>(a, BWD_G_O), *g_in = ptr<float>(a, BWD_G_IN), *g_out = ptr<float>(a, BWD_G_OUT),
+        *g_n1 = ptr<float>(a, BWD_G_N1), *g_n2 = ptr<float>(a, BWD_G_N2);
+  const int mode = static_cast<int>(a[BWD_ATTENTION_MODE]);
   // MLP
   TRY(k.out(dy, wout, d.dpre, s.pre, T, I, C, I, 2 * I, 2 * I, 1, EPI_SWIGLU_BWD));
-  TRY(k.wgrad(dy, s.hs, g_out, T, C, I, static_cast<int>(a[35])));
-  TRY(k.wgrad(d.dpre, s.h2, g_in, T, 2 * I, C, static_cast<int>(a[34])));
+  TRY(k.wgrad(dy, s.hs, g_out, T, C, I, static_cast<int>(a[BWD_SPLITS_OUT])));
+  TRY(k.wgrad(d.dpre, s.h2, g_in, T, 2 * I, C, static_cast<int>(a[BWD_SPLITS_IN])));
   TRY(k.out(d.dpre, win, d.dh, nullptr, T, C, 2 * I, C, C, 0, 1, EPI_STORE));
   TRY(fn.norm_bwd(d.dh, s.x1, nullptr, n2, rms ? nullptr : s.mean2, s.rstd2, dy, d.dx1, g_n2, nullptr, T, C, 0, rms,
                   k.stream));
   // attention
   TRY(fn.delta(d.dx1, wo, d.d_o, s.o, d.delta, T, HD, C, C, HD, HD, HD, 1, k.status, k.stream));
-  TRY(k.wgrad(d.dx1, s.o, g_o, T, C, HD, static_cast<int>(a[33])));
+  TRY(k.wgrad(d.dx1, s.o, g_o, T, C, HD, static_cast<int>(a[BWD_SPLITS_O])));
   TRY(fn.fa_bwd(s.qkv, nullptr, d.d_o, s.lse, d.dqkv, mode == 3 ? nullptr : d.dq, d.delta, ss, se, T, H, 64, window,
                 static_cast<float>(scale), pos, cosp, sinp, 0, mode, k.status, k.stream));
-  TRY(k.wgrad(d.dqkv, norm1 ? s.h1 : x, g_qkv, T, 3 * HD, C, static_cast<int>(a[32])));
+  TRY(k.wgrad(d.dqkv, norm1 ? s.h1 : x, g_qkv, T, 3 * HD, C, static_cast<int>(a[BWD_SPLITS_QKV])));
   if (!norm1)   // the layer input enters the projection and the residual: both gradients in one epilogue
     return k.out(d.dqkv, wqkv, dx, d.dx1, T, C, 3 * HD, C, C, C, 1, EPI_ADD);
   TRY(k.out(d.dqkv, wqkv, d.dh, nullptr, T, C, 3 * HD, C, C, 0, 1, EPI_STORE));

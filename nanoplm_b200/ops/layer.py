@@ -25,6 +25,8 @@ _FwdArgs, _BwdArgs = ctypes.c_longlong * 24, ctypes.c_longlong * 37
 def _native():
     if _READY[0] is None:
         h = lib("layer")
+        if (h.nplm_layer_args(0), h.nplm_layer_args(1)) != (_FwdArgs._length_, _BwdArgs._length_):
+            raise RuntimeError("the argument arrays of csrc/layer.cpp have changed")
         fns = [("gemm_tcgen05", "nplm_gemm_bf16"), ("gemm_tcgen05", "nplm_gemm_bf16_pair"),
                ("gemm_tcgen05", "nplm_gemm_bf16_delta"), ("elementwise", "nplm_norm_fwd"),
                ("elementwise", "nplm_norm_bwd"), ("attention_ws", "nplm_fa_fwd_ws"),
