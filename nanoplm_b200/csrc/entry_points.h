@@ -24,6 +24,25 @@ enum : int {
                        // R = the pre-activations [value | gate] (bf16, 2N wide); C (bf16, 2N wide) =
                        // [acc * silu(gate) | acc * value * silu'(gate)], the gradient of R
 };
+
+// Whether a bf16-output GEMM on 256-wide tiles runs on CTA pairs by default (ops/kernels.py has the same rule, and a test
+// compares the two). A pair's tile takes a third less operand traffic per FLOP but costs about 0.6 us more from launch
+// to store and moves 256 rows at a time, so it pays once the tiles fill more than one wave of 148, or several where the
+// contraction is short. Graph-timed single / pair, us:
+//   store, add, GELU, ReLU: 1024 columns of K = 1024, 3 072 rows (96 tiles) 12.4 / 12.8, 4 864 (152) 17.8 / 17.3, 55 424
+//     102 / 91; K = 512, 32 768 x 512 (512 tiles) 25.0 / 25.6, 55 424 x 512 (866) 37.2 / 36.9
+//   SwiGLU: 4096 of 1024, 1 024 rows (128) 12.1 / 13.0, 1 536 (192) 17.8 / 17.3, 55 424 332 / 288; 2048 of 512, 4 864 rows
+//     (304) 15.7 / 15.9, 6 144 (384) 16.4 / 16.3
+//   RoPE (whose pair form has eight epilogue warps, and a stage less): 3072 of 1024, 6 144 rows (576) 31.7 / 32.8, 8 704
+//     (816) 44.7 / 44.3, 55 424 270 / 249; 2304 of 768, 32 768 rows (2 304) 97.1 / 97.7, 55 424 (3 897) 162 / 162; 1536 of
+//     512, 236 rows 9.3 / 12.2, 55 424 82.6 / 88.6
+//   SwiGLU backward (eight epilogue warps): 1 row 12.5 / 11.0, 8 704 x 2048 of 1024 57 / 46, 55 424 292 / 237
+inline bool gemm_pair_pays(long long M, long long N, long long K, int epi) {
+  const long long tiles = (M + 127) / 128 * ((N + 255) / 256);
+  if (epi == EPI_SWIGLU_BWD || epi == EPI_STORE_DELTA) return true;
+  if (epi == EPI_ROPE) return K >= 1024 ? tiles > 740 : K >= 768 && tiles > 2600;
+  return K >= 768 ? tiles > 148 : tiles * K > (epi == EPI_SWIGLU ? 190000 : 400000);
+}
 }  // namespace nplm
 
 extern "C" {

@@ -120,13 +120,14 @@ struct Scratch {
 struct Call {
   int* status;
   cudaStream_t stream;
-  // bf16 output: CTA pairs on 256-wide tiles, as ops.kernels.gemm chooses by default
+  // bf16 output: tiles and CTA pairs as ops.kernels.gemm chooses by default
   int out(const void* A, const void* B, void* Cp, const void* R, int M, int N, int K, int ldb, int ldc, int ldr, int b_mn,
           int epi, const int* pos = nullptr, const float* cosp = nullptr, const float* sinp = nullptr,
           int rope_cols = 0) const {
-    if (N >= 256 || epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD)
+    const bool wide = N >= 256 || epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD;
+    if (wide && gemm_pair_pays(M, N, K, epi))
       return fn.pair(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, 0, pos, cosp, sinp, rope_cols, status, stream);
-    return fn.gemm(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, 128, 0, 0, pos, cosp, sinp, rope_cols, status,
+    return fn.gemm(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, wide ? 256 : 128, 0, 0, pos, cosp, sinp, rope_cols, status,
                    stream);
   }
   // fp32 C[N][K] += dy[T][N]^T x[T][K]
@@ -158,6 +159,8 @@ extern "C" void nplm_layer_init(void* const* f) {
   fn.fa_fwd = reinterpret_cast<decltype(fn.fa_fwd)>(f[5]);
   fn.fa_bwd = reinterpret_cast<decltype(fn.fa_bwd)>(f[6]);
 }
+
+extern "C" int nplm_gemm_pair_pays(long long M, long long N, long long K, int epi) { return gemm_pair_pays(M, N, K, epi); }
 
 // Length of the argument array of a forward (0) or backward (1) call.
 extern "C" int nplm_layer_args(int backward) { return backward ? BWD_ARGS : FWD_ARGS; }

@@ -47,11 +47,21 @@ _GEMM_PAIR_DEFAULT = [{"1": True, "0": False}.get(_os.environ.get("NPLM_GEMM_PAI
 
 
 def set_gemm_pair_default(enabled: bool | None) -> None:
-    """Default of gemm(pair=None): run qualifying GEMMs on CTA pairs (cta_group::2). True / False: all / none;
-    None (the initial value): those with bf16 outputs. Their operand traffic per FLOP is a third lower and
-    their epilogue runs on eight warps (QKV, 55 424 rows: 275 us against 305 us on single CTAs); the fp32
-    weight gradients run at the same rate either way (384 / 377 us for 4096 x 1024) and stay on single CTAs."""
+    """Default of gemm(pair=None): run qualifying GEMMs on CTA pairs (cta_group::2). True / False: all / none; None (the
+    initial value): those with bf16 outputs for which `pair_pays`. The fp32 weight gradients run at the same rate
+    either way (384 / 377 us for 4096 x 1024 over 55 424 tokens) and stay on single CTAs."""
     _GEMM_PAIR_DEFAULT[0] = None if enabled is None else bool(enabled)
+
+
+def pair_pays(M: int, N: int, K: int, epi: int) -> bool:
+    """Whether a bf16-output GEMM on 256-wide tiles runs on CTA pairs by default: the rule of `gemm_pair_pays` in
+    csrc/entry_points.h, which states the measurements on both sides of its lines."""
+    tiles = (M + 127) // 128 * ((N + 255) // 256)
+    if epi in (EPI_SWIGLU_BWD, 9):       # 9: the delta epilogue, which has its own entry point
+        return True
+    if epi == EPI_ROPE:
+        return tiles > 740 if K >= 1024 else K >= 768 and tiles > 2600
+    return tiles > 148 if K >= 768 else tiles * K > (190000 if epi == EPI_SWIGLU else 400000)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
@@ -130,7 +140,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if pair is None:
         pair = _GEMM_PAIR_DEFAULT[0]
         if pair is None:
-            pair = not f32_out
+            pair = not f32_out and bn == 256 and pair_pays(M, N, K, epi)
     aux_p = aux.data_ptr() if aux is not None else None
     rope_p = (r_pos.data_ptr(), r_cos.data_ptr(), r_sin.data_ptr()) if r_pos is not None else (None, None, None)
     if pair and bn == 256 and max_ctas == 0 and not (a_mn and not b_mn):
