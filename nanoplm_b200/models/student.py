@@ -11,6 +11,7 @@ import numpy as np
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from nanoplm_b200.config.schema import StudentConfig
 from nanoplm_b200.data.tokenizer import StudentTokenizer
@@ -100,10 +101,11 @@ class ProtX(EncoderModel):
 
     def _embeds_packed(self, device: torch.device) -> bool:
         """Whether embed_sequences may hand the model flat ids: bf16 on a GPU, and nothing that observes the padded
-        call (a forward of a subclass, hooks on this module)."""
+        call (a forward of a subclass or of this instance, hooks on this module or on all modules)."""
         w = self.final_norm.weight
         return (device.type == "cuda" and w.dtype == torch.bfloat16 and w.shape[0] % 8 == 0
-                and type(self).forward is ProtX.forward and not self._forward_hooks and not self._forward_pre_hooks)
+                and type(self).forward is ProtX.forward and "forward" not in self.__dict__
+                and not self._forward_hooks and not self._forward_pre_hooks and not _has_any_global_hook())
 
     def _embed_packed(self, ids: torch.Tensor, mask: torch.Tensor, device):
         """(hidden states [T, C] of the real tokens, device cu_seqlens, host lengths) of a padded host batch. The
