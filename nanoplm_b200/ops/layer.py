@@ -91,10 +91,14 @@ class _LayerFn(torch.autograd.Function):
         return dx, None, None, None, None, None, None, None, None
 
 
-def _quiet(m) -> bool:
-    """No hooks of any kind on a module whose call would be passed by, and no forward of the instance's own."""
-    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                or "forward" in m.__dict__)
+def _quiet(parts) -> bool:
+    """No hooks of any kind on modules whose calls would be passed by, and no forward of an instance's own."""
+    for m in parts:
+        d = m.__dict__
+        if (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
+                or "forward" in d):
+            return False
+    return True
 
 
 def _ok_weight(w, rows: int, cols: int) -> bool:
@@ -107,23 +111,26 @@ def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
     or None."""
     if F_.functions_observed():     # before anything else: a tracer also sees the sizes that the checks below look at
         return None
-    wqkv, wo, win, wout = attn.Wqkv, attn.Wo, mlp.Wi, mlp.Wo
+    am, mm = attn._modules, mlp._modules
+    wqkv, wo, win, wout = am["Wqkv"], am["Wo"], mm["Wi"], mm["Wo"]
     if not (x.dtype == BF and x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.data_ptr() % 16 == 0
             and x.shape[0] > 0 and attn.head_dim == 64 and mlp.swiglu and not (mlp.p_drop > 0.0 and mlp.training)
             and not F_.fp8_enabled() and K._FA_IMPL[0] == "ws" and K._GEMM_PAIR_DEFAULT[0] is None
             and type(x) is torch.Tensor):
         return None
     parts = (attn, mlp, wqkv, wo, win, wout, norm1, norm2)
-    if (any(l.bias is not None for l in (wqkv, wo, win, wout, norm2)) or not all(map(_quiet, parts))
+    if (any(l.bias is not None for l in (wqkv, wo, win, wout, norm2)) or not _quiet(parts)
             or _mod._has_any_global_hook()):
         return None
-    C, HD, I = x.shape[1], attn.num_heads * 64, wout.weight.shape[1]
     n1 = None
     if type(norm1) is not torch.nn.Identity:
         if norm1.bias is not None or norm1.rms != norm2.rms:
             return None
         n1 = norm1.weight
-    params = (wqkv.weight, wo.weight, win.weight, wout.weight, n1, norm2.weight)
+    params = (*[l._parameters.get("weight") for l in (wqkv, wo, win, wout)], n1, norm2.weight)
+    if any(w is None for w in params[:4]):      # (reparametrised: a weight that is formed on each call)
+        return None
+    C, HD, I = x.shape[1], attn.num_heads * 64, params[3].shape[-1]
     if not (C % 64 == 0 and C <= 4096 and I % 64 == 0 and _ok_weight(params[0], 3 * HD, C) and _ok_weight(params[1], C, HD)
             and _ok_weight(params[2], 2 * I, C) and _ok_weight(params[3], C, I)
             and all(n.dtype == BF and n.is_cuda and n.shape == (C,) and n.data_ptr() % 16 == 0
@@ -132,23 +139,29 @@ def run(attn, mlp, norm1, norm2, x, ctx, window: int, rope: tuple):
     cos, sin = rope
     pos = ctx.position_ids
     # (what is wrong here is for the op-by-op path to refuse)
-    if not (pos.numel() == x.shape[0] and all(t.dtype == torch.int32 and t.is_cuda and t.is_contiguous()
-                                              for t in (pos, ctx.seq_start, ctx.seq_end))
-            and all(t.dtype == torch.float32 and t.is_cuda and t.is_contiguous() and t.shape[-1] == 32
-                    for t in (cos, sin))):
+    i32, f32, ss, se = torch.int32, torch.float32, ctx.seq_start, ctx.seq_end
+    if not (pos.numel() == x.shape[0] and pos.dtype == i32 and ss.dtype == i32 and se.dtype == i32 and pos.is_cuda
+            and ss.is_cuda and se.is_cuda and pos.is_contiguous() and ss.is_contiguous() and se.is_contiguous()
+            and cos.dtype == f32 and sin.dtype == f32 and cos.is_cuda and sin.is_cuda and cos.is_contiguous()
+            and sin.is_contiguous() and cos.shape[-1] == 32 and sin.shape[-1] == 32):
         return None
-    geo = (ctx.seq_start, ctx.seq_end, pos, cos, sin)
+    geo = (ss, se, pos, cos, sin)
     meta = (I, attn.num_heads, window, int(n1 is not None), int(norm2.rms),
             norm1.eps if n1 is not None else 0.0, norm2.eps, attn.scale)
     if torch.is_grad_enabled():
-        if not (x.requires_grad and F_._WGRAD_READY[0] is None
-                and all(p.requires_grad and _main_grad_ok(p) for p in params if p is not None)):
+        if not (x.requires_grad and F_._WGRAD_READY[0] is None and _trained(params)):
             return None
         return _LayerFn.apply(x, *params, geo, meta)
     return _forward(x, params, geo, meta, False)[0]
 
 
-def _main_grad_ok(p) -> bool:
-    g = getattr(p, "main_grad", None)
-    return (g is not None and g.dtype == torch.float32 and g.is_cuda and g.shape == p.shape and g.is_contiguous()
-            and g.data_ptr() % 16 == 0)
+def _trained(params) -> bool:
+    """Every parameter requires a gradient and has a running fp32 one of its shape."""
+    f32 = torch.float32
+    for p in params:
+        if p is not None:
+            g = getattr(p, "main_grad", None)
+            if (g is None or not p.requires_grad or g.dtype != f32 or not g.is_cuda or g.shape != p.shape
+                    or not g.is_contiguous() or g.data_ptr() % 16):
+                return False
+    return True
