@@ -66,3 +66,29 @@ def test_coefficient_gradients_of_the_wrong_size_are_refused(cuda_status):
     alpha, beta, R = _CoefFn.apply(torch.randn(T, 2 * n + n * n, device="cuda").to(BF).requires_grad_(True), *ps, 5, n)
     with pytest.raises(RuntimeError):
         (alpha.sum() + beta.sum() + R.sum()).backward()
+
+
+@pytest.mark.parametrize("n", [2, 4])
+def test_coefficients_do_not_depend_on_how_the_parameters_are_held(n, cuda_status):
+    """bf16 parameters, the same values in fp32, and bf16 with running gradients: the same bits forward and for `pre`; a
+    gradient goes to one place only."""
+    from nanoplm_b200.models.mhc import _CoefFn
+    g = torch.Generator(device="cuda").manual_seed(10 + n)
+    pre = torch.randn(200, 2 * n + n * n, device="cuda", generator=g).to(BF)
+    params = [torch.randn(*s, device="cuda", generator=g).to(BF) for s in ((n,), (n,), (n, n), (3,))]
+    outs = {}
+    for kind in ("bf16", "fp32", "main_grad"):
+        ps = [torch.nn.Parameter(p.float() if kind == "fp32" else p.clone()) for p in params]
+        if kind == "main_grad":
+            for p in ps:
+                p.main_grad = torch.zeros(p.shape, device="cuda")
+        x = pre.clone().requires_grad_(True)
+        alpha, beta, R = _CoefFn.apply(x, *ps, 5, n)
+        (alpha.square().sum() + beta.square().sum() + (R * R).sum()).backward()
+        assert all((p.grad is None) == (kind == "main_grad") for p in ps)
+        if kind == "main_grad":
+            assert all(p.main_grad.abs().sum() > 0 for p in ps)
+        outs[kind] = (alpha, beta, R, x.grad)
+    for kind in ("bf16", "main_grad"):
+        for a, b in zip(outs[kind], outs["fp32"]):
+            assert torch.equal(a, b), kind
