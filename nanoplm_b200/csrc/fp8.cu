@@ -249,11 +249,11 @@ constexpr int F8_REGS_LAUNCH = 168, F8_REGS_LIGHT = 40, F8_REGS_HEAVY = 232;
 static_assert(128 * F8_REGS_LIGHT + 256 * F8_REGS_HEAVY <= F8_THREADS * F8_REGS_LAUNCH,
               "setmaxnreg.inc would wait forever for registers the CTA does not own");
 
-// 256-wide tiles: a K block is 512 cycles of MMAs, and every epilogue warp has those 512 cycles for its 128
-// columns (128 packed multiply-adds or 256, plus the TMEM reads), so the promotion of one block hides behind the
-// products of the next (two TMEM buffers). 128-wide tiles load 4/3 of the bytes per FLOP and were bound by that
-// and by the serial wait -> read -> add -> release chain. They remain for narrow outputs and for weight shards
-// that do not hold whole 256-row tiles.
+// 256-wide tiles: a K block is 512 cycles of MMAs, and reading its partial products out of tensor memory about 1 024 (see
+// the promotion loop), which bounds the kernel: the MMAs of a block hide behind the promotion of the one before (two
+// TMEM buffers). 128-wide tiles load 4/3 of the bytes per FLOP and were bound by that and by the serial
+// wait -> read -> add -> release chain. They remain for narrow outputs and for weight shards that do not hold whole 256-row
+// tiles.
 template <int BN>
 struct F8Cfg {
   static constexpr int ACC = 512 / BN;                             // TMEM partial-product buffers (all of TMEM)

@@ -26,8 +26,6 @@ constexpr int UMMA_K = 16;
 
 // PAIR: two CTAs of a cluster (cta_group::2) share one 256 x BN tile; each holds its own 128 rows
 // of A and half of B, which cuts the L2 -> shared-memory traffic per FLOP by a third.
-// STAGED: the epilogue goes through shared memory (TMA stores); kernels that write straight from
-// registers (fp32 outputs, the direct epilogue) spend that room on one more pipeline stage.
 // Epilogue warps: one per TMEM lane quarter, or two that split the columns. A 128 x 256 tile with K = 1024
 // leaves the epilogue about 8 200 cycles. The forms that read a second operand or tables need more than that on
 // four warps: 55 424 rows, SwiGLU backward 356 -> 277 us, RoPE 322 -> 288, delta 120 -> 107 with eight. The
@@ -37,6 +35,8 @@ template <bool PAIR, bool STAGED, int EPI>
 constexpr int EPI_WARPS_OF =
     (PAIR && STAGED && (EPI == EPI_ROPE || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD)) ? 8 : 4;
 
+// STAGED: the epilogue goes through shared memory (TMA stores and reduce-adds); the direct epilogue, and fp32 outputs of
+// groups whose rows are no multiple of 32, write straight from registers and spend that room on one more pipeline stage.
 template <int BN, bool PAIR = false, bool STAGED = true, int EPI_WARPS_ = 4>
 struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;

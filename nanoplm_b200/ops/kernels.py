@@ -206,12 +206,12 @@ def gemm_ag(a: torch.Tensor, b_full: torch.Tensor, b_ptrs, rank: int, world: int
 def wgrad_splits(n_out: int, k_in: int, tokens: int, bn: int = 256, sms: int = 148) -> int:
     """Split-K factor for a weight-gradient GEMM [n_out, k_in] reduced over `tokens`.
 
-    A work item of kb 64-token blocks costs kb + 25 block times (pipeline fill, atomic epilogue, and what its
-    additions take from the others); the factor with the least waves * cost wins. The 25 fits measurements from both
-    ends: 55 424 tokens, 4096 x 1024 (128 tiles) 377 us unsplit, 405 us in 8; 3072 x 1024 (96 tiles) 400 us unsplit, 331 in
-    3, 342 in 6; 1024 x 1024 (32 tiles) 121 us in 4, 118 in 9. Small outputs are what gains over filling a wave with
-    at most 4 items a tile: 17 000 tokens, 512 x 512 (8 tiles) 33.1 -> 19.4 us.
-    (Taken before the additions went through TMA; with them the same factors are the best or within 4 % of it.)"""
+    A work item of kb 64-token blocks costs kb + 25 block times (pipeline fill, epilogue, and what its additions take from
+    the others); the factor with the least waves * cost wins. Graph-timed us, unsplit / this rule's factor: 55 424 tokens, 3072
+    x 1024 (96 tiles) 286 / 239 in 3, 1024 x 1024 (32 tiles) 279 / 88 in 4, 4096 x 1024 (128 tiles) 324 unsplit, 332
+    in 2; 17 024 tokens, 512 x 512 (8 tiles) 81 / 13.1 in 16, 64 x 768 80 / 11.1 in 16; 1 000 tokens, 1024 x 1024 11.9 / 8.6 in
+    4. Of ten outputs at five token counts (1 000 to 55 424) it picks the best factor of 1 to 16 or one within 2 %, but
+    for 3072 x 1024 at 4 352 tokens (28.2 unsplit, 25.1 in 3)."""
     tiles = ((n_out + 127) // 128) * ((k_in + bn - 1) // bn)
     kb = (tokens + 63) // 64
     best, best_cost = 1, None
