@@ -823,7 +823,13 @@ extern "C" int nplm_gemm_fp8(const void* A, const void* B, void* C, const float*
     args.ag_src[r] = nullptr;
     args.ag_ssrc[r] = nullptr;
   }
-  return N > 128 ? f8_launch<256>(A, B, C, args, false, stream) : f8_launch<128>(A, B, C, args, false, stream);
+  // Few rows: as long as the 128-wide tiles fit one wave of 148 they finish sooner. Graph-timed us, wide / narrow: 256 rows, 2048
+  // columns of 512 6.9 / 5.8; 1 536 rows, 1024 columns of 1024 8.9 / 7.8. Past a wave the wide ones are ahead (2 432 rows
+  // of the latter 9.2; the earlier kernel, all 128-wide, 14.0, and 8.6 - 8.9 below a wave). Both sum a tile's K blocks in the same
+  // order. Accumulated outputs fill the chip by splitting the contraction instead.
+  const long long wide_tiles = (M + 127LL) / 128 * ((N + 255LL) / 256);
+  const bool wide = N > 128 && (out_mode == 2 || 2 * wide_tiles > 148);
+  return wide ? f8_launch<256>(A, B, C, args, false, stream) : f8_launch<128>(A, B, C, args, false, stream);
 }
 
 // All-gather fused into the fp8 GEMM. b_ptrs[r] / sb_ptrs[r]: rank r's full-size e4m3 weight buffer

@@ -58,3 +58,22 @@ def test_quant_dual_equals_the_two_kernels(R, K, padded, cuda_status):
     want_r, want_c = fp8.quant_rows(x), fp8.quant_tile(x, transpose=True, block=False)
     for got, want in ((rows, want_r), (cols, want_c)):
         assert torch.equal(got.q, want.q) and torch.equal(got.scale, want.scale)
+
+
+@pytest.mark.parametrize("N", [136, 256, 264, 392])
+@pytest.mark.parametrize("block", [False, True])
+def test_both_tile_widths_give_the_same_bits(N, block, cuda_status):
+    """300 rows run on 128-wide tiles, 9 601 on 256-wide ones (edges in rows and columns on both)."""
+    from nanoplm_b200.ops import fp8
+    if block and N % 128:
+        pytest.skip("block scales come in whole 128-row blocks")
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(9601, 640, device="cuda", generator=g).to(BF)
+    qb = _quantised(N, 640, 2, block)
+    tall, short = fp8.quant_rows(x), fp8.quant_rows(x[:300].contiguous())
+    for dt in (torch.float32, BF):
+        a, b = fp8.gemm_fp8(tall, qb, out_dtype=dt), fp8.gemm_fp8(short, qb, out_dtype=dt)
+        assert torch.equal(a[:300], b)
+    ref = tall.dequantize().double() @ qb.dequantize().double().t()
+    mag = tall.dequantize().double().abs() @ qb.dequantize().double().abs().t()
+    assert ((fp8.gemm_fp8(tall, qb, out_dtype=torch.float32).double() - ref).abs() <= mag * 2 ** -12).all()
