@@ -53,7 +53,9 @@ def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
     tiled = N % 64 == 0
     narrow = not tiled and N % 8 == 0 and dy2.is_cuda and dy2.dtype == BF and x2.dtype == BF and dy2.data_ptr() % 16 == 0
     if (tiled or narrow) and Kd % 64 == 0:
-        if _has_main_grad(w) and (tiled or w.main_grad.data_ptr() % 16 == 0):
+        # (a narrow gradient goes straight into a running one that the kernel can add to, else through a buffer)
+        if _has_main_grad(w) and (tiled or (w.main_grad.dtype == torch.float32 and w.main_grad.shape == (N, Kd)
+                                            and w.main_grad.is_contiguous() and w.main_grad.data_ptr() % 16 == 0)):
             K.gemm(dy2, x2, a_mn=True, b_mn=True, epi=K.EPI_ATOMIC_F32, out=w.main_grad,
                    splits=K.weight_grad_splits(N, Kd, T))
             if tiled and _WGRAD_READY[0] is not None:

@@ -92,3 +92,20 @@ def test_coefficients_do_not_depend_on_how_the_parameters_are_held(n, cuda_statu
     for kind in ("bf16", "main_grad"):
         for a, b in zip(outs[kind], outs["fp32"]):
             assert torch.equal(a, b), kind
+
+
+@pytest.mark.parametrize("how", ["bf16", "strided", "misaligned"])
+def test_narrow_gradient_into_any_running_gradient(how, cuda_status):
+    """Running gradients that the kernel cannot add to in place take the sum all the same."""
+    from nanoplm_b200.ops.functional import _wgrad
+    g = torch.Generator(device="cuda").manual_seed(4)
+    N, Kd, T = 24, 192, 100
+    dy, x = (torch.randn(T, n, device="cuda", generator=g).to(BF) for n in (N, Kd))
+    w = torch.nn.Parameter(torch.zeros(N, Kd, device="cuda", dtype=BF))
+    w.main_grad = {"bf16": torch.ones(N, Kd, device="cuda", dtype=BF), "strided": torch.ones(Kd, N, device="cuda").t(),
+                   "misaligned": torch.ones(N * Kd + 1, device="cuda")[1:].view(N, Kd)}[how]
+    assert _wgrad(dy, x, w) is None
+    want = 1 + dy.double().t() @ x.double()
+    got = w.main_grad.double().reshape(N, Kd)
+    bound = 2 ** -8 if how == "bf16" else 2 ** -20
+    assert ((got - want).abs() <= want.abs() * bound + (dy.double().abs().t() @ x.double().abs()) * T * 2 ** -24 + 1e-5).all()
