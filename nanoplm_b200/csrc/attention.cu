@@ -38,6 +38,7 @@ __device__ __forceinline__ uint32_t swz(int r, int chunk) {
 // seq_start[t], seq_end[t] from cu_seqlens (n_seq + 1 entries, may contain empty sequences)
 __global__ void seq_bounds_kernel(const int* __restrict__ cu, int n_seq, int* __restrict__ s_start,
                                   int* __restrict__ s_end, int T) {
+  grid_chain();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
     // last i in [0, n_seq) with cu[i] <= t
     int lo = 0, hi = n_seq;
@@ -1157,7 +1158,7 @@ using namespace nplm;
 extern "C" int nplm_seq_bounds(const int* cu_seqlens, int n_seq, int* seq_start, int* seq_end,
                                int T, cudaStream_t st) {
   if (T <= 0 || n_seq <= 0) return 0;
-  seq_bounds_kernel<<<(T + 255) / 256, 256, 0, st>>>(cu_seqlens, n_seq, seq_start, seq_end, T);
+  launch_chained(seq_bounds_kernel, (T + 255) / 256, 256, 0, st, cu_seqlens, n_seq, seq_start, seq_end, T);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -129,6 +129,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   constexpr int NA = C::NA, STAGES = C::STAGES;
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {
+    grid_wait();
     if (threadIdx.x == 0) atomicExch(args.status, ST_BAD_ARG);
     return;
   }
@@ -177,6 +178,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tma_prefetch_desc(&tmKV);
     tma_prefetch_desc(&tmO);
   }
+  grid_wait();
   if (warp == AB_MMA_WARP) {
     __syncwarp();
     tmem_alloc(tmem_slot, 512);
@@ -186,6 +188,7 @@ fa_bias_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_release();
   // columns: S0 [0,64), S1 [64,128), P0 [128,160), P1 [160,192), O0 [256,256+D), O1 [384,384+D)
 
   if (warp == AB_LOADER_WARP) {
@@ -527,7 +530,7 @@ static int ab_launch(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const CUte
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_slot);
   const int n_items = ((a.T + 2 * AB_T - 1) / (2 * AB_T)) * a.H;
-  fa_bias_fwd_kernel<D><<<n_items < sms ? n_items : sms, AB_THREADS, smem, st>>>(tmQ, tmKV, tmO, a);
+  launch_chained(fa_bias_fwd_kernel<D>, n_items < sms ? n_items : sms, AB_THREADS, smem, st, tmQ, tmKV, tmO, a);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -188,6 +188,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                  const FaWsArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1024-byte aligned base
+    grid_wait();
     if (threadIdx.x == 0) atomicExch(args.status, ST_BAD_ARG);
     return;
   }
@@ -236,6 +237,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     fence_proxy_async_smem();
     tma_prefetch_desc(&tmQKV);
   }
+  grid_wait();
   if (warp == WS_MMA_WARP) {
     __syncwarp();
     tmem_alloc(tmem_slot, 512);
@@ -245,6 +247,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_release();
   // columns: S0 [0,128), S1 [128,256), O0 [256,320), O1 [320,384), P0 [384,448), P1 [448,512)
   WS_TRACE_INIT();
 
@@ -769,6 +772,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
                  const FaWsBwdArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {
+    grid_wait();
     if (threadIdx.x == 0) atomicExch(args.status, ST_BAD_ARG);
     return;
   }
@@ -826,6 +830,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     tma_prefetch_desc(&tmQKV);
     tma_prefetch_desc(&tmDO);
   }
+  grid_wait();
   if (warp == Cfg::MMA_WARP) {
     __syncwarp();
     tmem_alloc(tmem_slot, 512);
@@ -835,6 +840,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_release();
   const uint32_t tS = tmem_base;          // S   [q][kv] 128 columns
   const uint32_t tdP = tmem_base + 128;   // dP  [q][kv] 128 columns
   const uint32_t tdQ = tmem_base + 256;   // dQ  [q][d]   64 columns
@@ -1435,6 +1441,7 @@ fa_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
 __global__ void __launch_bounds__(256)
 ws_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                 float* __restrict__ delta, int T, int H) {
+  grid_chain();
   const long long total = static_cast<long long>(T) * H * 8;   // 8 threads per (t, h)
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -1468,6 +1475,7 @@ __global__ void __launch_bounds__(256)
 ws_dq_store_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv, int T, int H,
                    const int* __restrict__ rope_pos, const float* __restrict__ rope_cos,
                    const float* __restrict__ rope_sin) {
+  grid_chain();
   const int HD = H * FA_D;
   const long long total = static_cast<long long>(T) * H * 4;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -1621,9 +1629,9 @@ extern "C" int nplm_fa_fwd_ws(const void* qkv, void* out, float* lse, const int*
     p_smem = (e != nullptr && e[0] == '1') ? 1 : 0;
   }
   if (p_smem)
-    fa_fwd_ws_kernel<false><<<grid, WS_THREADS, WS_FWD_SMEM, st>>>(tm, tmO, a);
+    launch_chained(fa_fwd_ws_kernel<false>, grid, WS_THREADS, WS_FWD_SMEM, st, tm, tmO, a);
   else
-    fa_fwd_ws_kernel<true><<<grid, WS_THREADS, WS_FWD_SMEM, st>>>(tm, tmO, a);
+    launch_chained(fa_fwd_ws_kernel<true>, grid, WS_THREADS, WS_FWD_SMEM, st, tm, tmO, a);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1681,7 +1689,7 @@ static int ws_bwd_impl(const void* qkv, const void* out, const void* dout, const
     const long long total = static_cast<long long>(T) * H * 8;
     long long blocks = (total + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;
-    ws_delta_kernel<<<static_cast<int>(blocks), 256, 0, st>>>(
+    launch_chained(ws_delta_kernel, static_cast<int>(blocks), 256, 0, st,
         reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta, T, H);
   }
   FaWsBwdArgs a;
@@ -1704,21 +1712,21 @@ static int ws_bwd_impl(const void* qkv, const void* out, const void* dout, const
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (grid > n_items) grid = n_items;
   if (mode == 2) {
-    fa_bwd_ws_kernel<2, BWD_KV_DQ><<<grid, WsBwdCfg<2, true>::THREADS, WS_BWD_SMEM, st>>>(tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<2, BWD_KV_DQ>, grid, WsBwdCfg<2, true>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
   } else if (mode == 0) {
-    fa_bwd_ws_kernel<4, BWD_KV><<<grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st>>>(tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_KV>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
   } else if (mode == 3) {
-    fa_bwd_ws_kernel<4, BWD_KV><<<grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st>>>(tmQKV, tmDO, tmDQ, tmOUT, a);
-    fa_bwd_ws_kernel<4, BWD_Q><<<grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st>>>(tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_KV>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_Q>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
     return static_cast<int>(cudaGetLastError());
   } else {
-    fa_bwd_ws_kernel<4, BWD_KV_DQ><<<grid, WsBwdCfg<4, true>::THREADS, WS_BWD_SMEM, st>>>(tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_KV_DQ>, grid, WsBwdCfg<4, true>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
   }
   {
     const long long total = static_cast<long long>(T) * H * 4;
     long long blocks = (total + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;
-    ws_dq_store_kernel<<<static_cast<int>(blocks), 256, 0, st>>>(
+    launch_chained(ws_dq_store_kernel, static_cast<int>(blocks), 256, 0, st,
         dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), T, H, rope_pos, rope_cos, rope_sin);
   }
   return static_cast<int>(cudaGetLastError());

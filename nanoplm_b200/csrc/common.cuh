@@ -63,6 +63,23 @@ __device__ __forceinline__ bool elect_one() {
 // Index of this thread's warp in its block, as a value the compiler knows to be warp-uniform.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
 
+// ---------------------------------------------------------------- chained launches
+// Kernels of a step follow one another in one stream, most of them a few to a few tens of microseconds long. Launched
+// with `launch_chained` a kernel's blocks are placed, and its barriers and descriptors set up, while its predecessor
+// still runs; grid_wait holds them until that one has finished and its writes are visible.
+//   * Every thread calls grid_wait before its first access to global memory (a grid that could finish without it would
+//     break the order for its successors), and before it allocates tensor memory: a block that took
+//     tensor memory while a predecessor still had to allocate would wait for a grid that waits for it.
+//   * grid_release allows the successor to be placed once every block has called it or left. Tensor-memory kernels call it
+//     after their allocation; kernels that wait for other GPUs do not (a waiting successor must not hold the
+//     room that the awaited work may need).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_chain() {   // both, for kernels without tensor memory
+  grid_release();
+  grid_wait();
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -550,6 +567,24 @@ inline CUresult with_context(Call call) {
     if (cudaGetDevice(&d) == cudaSuccess && cudaSetDevice(d) == cudaSuccess) r = call();
   }
   return r;
+}
+
+// kern<<<grid, block, smem, st>>>(args...) for a kernel that calls grid_wait: it may be placed before its predecessor in
+// the stream has finished (see grid_wait).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Args&&>(args)...);
 }
 
 inline int current_device_slot() {

@@ -56,6 +56,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ ids
                 const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int T, int C, float eps,
                 int rms) {
+  grid_chain();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < T;
@@ -125,6 +126,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                 const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                 float* __restrict__ dw, float* __restrict__ dtable, int T, int C, int rms) {
+  grid_chain();
   __shared__ __align__(16) float sm_dw[8][256];  // one 256-channel chunk of every warp's sums
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -251,6 +253,7 @@ norm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                      const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                      float* __restrict__ dw, float* __restrict__ dtable, int T, int C, int V, int rms) {
+  grid_chain();
   extern __shared__ float s_table[];   // [V][C] in embedding mode
   // SUB row groups run side by side in one block (blockDim.x / SUB threads each): they share the
   // table sums, which therefore take shared-memory atomics (two groups may hold the same token)
@@ -365,6 +368,7 @@ __global__ void __launch_bounds__(256)
 rope_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos,
             const float* __restrict__ cos_t, const float* __restrict__ sin_t, int T, int H, int D,
             float sign) {
+  grid_chain();
   const int half = D >> 1;
   const int vec_per_head = half >> 3;  // 8 elements per thread from each half
   const long long total = static_cast<long long>(T) * 2 * H * vec_per_head;
@@ -399,6 +403,7 @@ rope_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos,
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict__ out,
                   long long T, int I) {
+  grid_chain();
   const int vec = I >> 3;
   const long long total = T * vec;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -418,6 +423,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restri
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const __nv_bfloat16* __restrict__ dout,
                   __nv_bfloat16* __restrict__ dpre, long long T, int I) {
+  grid_chain();
   const int vec = I >> 3;
   const long long total = T * vec;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -444,6 +450,7 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const __nv_bfloat16* __
 __global__ void __launch_bounds__(256)
 act_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict__ out,
                long long n8, int act) {
+  grid_chain();
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < n8;
        idx += static_cast<long long>(gridDim.x) * blockDim.x) {
     float p[8], o[8];
@@ -459,6 +466,7 @@ act_fwd_kernel(const __nv_bfloat16* __restrict__ pre, __nv_bfloat16* __restrict_
 __global__ void __launch_bounds__(256)
 act_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const __nv_bfloat16* __restrict__ dout,
                __nv_bfloat16* __restrict__ dpre, long long n8, int act) {
+  grid_chain();
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < n8;
        idx += static_cast<long long>(gridDim.x) * blockDim.x) {
     float p[8], d[8], o[8];
@@ -485,6 +493,7 @@ act_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const __nv_bfloat16* __res
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ idx,
                    __nv_bfloat16* __restrict__ dst, int n, int C) {
+  grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(n) * vec;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -500,6 +509,7 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict_
 __global__ void __launch_bounds__(256)
 scatter_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ idx,
                     __nv_bfloat16* __restrict__ dst, int n, int C) {
+  grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(n) * vec;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -525,6 +535,7 @@ ce_fwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
               const __nv_bfloat16* __restrict__ bias, const int* __restrict__ labels,
               const float* __restrict__ inv_count, float* __restrict__ dlogits,
               float* __restrict__ logits_out, float* __restrict__ loss_sum, int n, int C, int V) {
+  grid_chain();
   extern __shared__ __nv_bfloat16 sW[];  // [V][C]
   for (int i = threadIdx.x * 8; i < V * C; i += blockDim.x * 8)
     *reinterpret_cast<uint4*>(sW + i) = *reinterpret_cast<const uint4*>(W + i);
@@ -600,6 +611,7 @@ ce_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
               const float* __restrict__ dlogits, const float* __restrict__ gscale,
               __nv_bfloat16* __restrict__ dh, float* __restrict__ dW, float* __restrict__ dbias,
               int n, int C, int V) {
+  grid_chain();
   extern __shared__ float sdW[];  // [V][C] fp32, then [32] dbias
   float* sdb = sdW + V * C;
   for (int i = threadIdx.x; i < V * C + 32; i += blockDim.x) sdW[i] = 0.f;
@@ -667,6 +679,7 @@ ce_bwd_tiled_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __
                     const float* __restrict__ dlogits, const float* __restrict__ gscale,
                     __nv_bfloat16* __restrict__ dh, float* __restrict__ dW, float* __restrict__ dbias,
                     int n, int C, int V) {
+  grid_chain();
   extern __shared__ __align__(16) uint8_t ce_smem[];
   __nv_bfloat16* sW = reinterpret_cast<__nv_bfloat16*>(ce_smem);            // [V][C]
   __nv_bfloat16* sH = sW + static_cast<size_t>(V) * C;                       // [32][C]
@@ -742,6 +755,7 @@ ce_bwd_tiled_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __
 // sum of squares of an fp32 buffer, accumulated into out[0]
 __global__ void __launch_bounds__(256)
 sumsq_kernel(const float* __restrict__ x, long long n, float* __restrict__ out) {
+  grid_chain();
   float s = 0.f;
   const long long n4 = n >> 2;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
@@ -772,6 +786,7 @@ adamw_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v
              float* __restrict__ g, __nv_bfloat16* __restrict__ p_bf16,
              const float* __restrict__ hyper, const float* __restrict__ sumsq, long long n,
              int zero_grad) {
+  grid_chain();
   const float lr = hyper[0], b1 = hyper[1], b2 = hyper[2], eps = hyper[3], wd = hyper[4];
   const float bc1 = hyper[5], bc2 = hyper[6], gs = hyper[7], max_norm = hyper[8];
   float scale = gs;
@@ -813,6 +828,7 @@ muon_momentum_kernel(const float* __restrict__ g, float* __restrict__ m,
                      const long long* __restrict__ off, long long numel,
                      __nv_bfloat16* __restrict__ upd, float* __restrict__ usq,
                      const float* __restrict__ sumsq, float gs, float max_norm, float mu, int nesterov) {
+  grid_chain();
   const float scale = clip_scale(sumsq, gs, max_norm);
   const long long base = off[blockIdx.y];
   const float4* g4 = reinterpret_cast<const float4*>(g + base);
@@ -852,6 +868,7 @@ __global__ void __launch_bounds__(256)
 muon_apply_kernel(float* __restrict__ p, __nv_bfloat16* __restrict__ p16,
                   const long long* __restrict__ off, long long numel,
                   const __nv_bfloat16* __restrict__ O, float lr, float wd, int cautious) {
+  grid_chain();
   const long long base = off[blockIdx.y];
   float4* p4 = reinterpret_cast<float4*>(p + base);
   uint2* q4 = p16 ? reinterpret_cast<uint2*>(p16 + base) : nullptr;
@@ -890,6 +907,7 @@ adamw_slots_kernel(float* __restrict__ p, float* __restrict__ m, float* __restri
                    const long long* __restrict__ off, const long long* __restrict__ numel,
                    const int* __restrict__ decay, const float* __restrict__ sumsq, float gs, float max_norm,
                    float lr, float b1, float b2, float eps, float wd, float bc1, float bc2) {
+  grid_chain();
   const float scale = clip_scale(sumsq, gs, max_norm);
   const long long base = off[blockIdx.y], n = numel[blockIdx.y];
   const float decay_mul = decay[blockIdx.y] ? (1.f - lr * wd) : 1.f;
@@ -912,6 +930,7 @@ adamw_slots_kernel(float* __restrict__ p, float* __restrict__ m, float* __restri
 __global__ void __launch_bounds__(256)
 cast_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst,
                         long long n) {
+  grid_chain();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
     dst[i] = __float2bfloat16(src[i]);
@@ -923,6 +942,7 @@ __global__ void __launch_bounds__(256)
 masked_mse_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __restrict__ t,
                   const int* __restrict__ valid, const float* __restrict__ inv_count,
                   __nv_bfloat16* __restrict__ ds, float* __restrict__ loss_sum, int T, int C) {
+  grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(T) * vec;
   const float invc = *inv_count;
@@ -989,7 +1009,7 @@ extern "C" int nplm_norm_fwd(const void* x, const int* ids, const void* w, void*
   if (C % 8) return -3;
   const int blocks = (T + 7) / 8 < 148 * 8 ? (T + 7) / 8 : 148 * 8;
 #define CALL(N_)                                                                               \
-  norm_fwd_kernel<N_><<<blocks, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x), ids,  \
+  launch_chained(norm_fwd_kernel<N_>, blocks, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), ids,  \
                                               reinterpret_cast<const __nv_bfloat16*>(w),       \
                                               reinterpret_cast<__nv_bfloat16*>(y), mean, rstd, \
                                               T, C, eps, rms)
@@ -1021,7 +1041,7 @@ extern "C" int nplm_norm_bwd(const void* dy, const void* x, const int* ids, cons
     if (smem > 48 * 1024)                                                                                 \
       cudaFuncSetAttribute(norm_bwd_rows_kernel<ROWS, SUB_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                            static_cast<int>(smem));                                                       \
-    norm_bwd_rows_kernel<ROWS, SUB_><<<blocks, threads, smem, st>>>(                                      \
+    launch_chained(norm_bwd_rows_kernel<ROWS, SUB_>, blocks, threads, smem, st,                                       \
         reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x), ids,       \
         reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd, reinterpret_cast<const __nv_bfloat16*>(dres), \
         reinterpret_cast<__nv_bfloat16*>(dx), dw, dtable, T, C, V, rms);                                  \
@@ -1035,7 +1055,7 @@ extern "C" int nplm_norm_bwd(const void* dy, const void* x, const int* ids, cons
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 2) blocks = 148 * 2;   // more blocks only add contention on the dw atomics
 #define CALL(N_)                                                                              \
-  norm_bwd_kernel<N_><<<blocks, 256, 0, st>>>(                                                \
+  launch_chained(norm_bwd_kernel<N_>, blocks, 256, 0, st,                                                 \
       reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x),  \
       ids, reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd,                             \
       reinterpret_cast<const __nv_bfloat16*>(dres), reinterpret_cast<__nv_bfloat16*>(dx), dw, \
@@ -1050,7 +1070,7 @@ extern "C" int nplm_rope(void* qkv, const int* pos, const float* cos_t, const fl
   if (T <= 0) return 0;
   if (D % 16) return -3;
   const long long total = static_cast<long long>(T) * 2 * H * (D / 16);
-  rope_kernel<<<grid_for(total, 256), 256, 0, st>>>(reinterpret_cast<__nv_bfloat16*>(qkv), pos,
+  launch_chained(rope_kernel, grid_for(total, 256), 256, 0, st, reinterpret_cast<__nv_bfloat16*>(qkv), pos,
                                                     cos_t, sin_t, T, H, D, backward ? -1.f : 1.f);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1058,7 +1078,7 @@ extern "C" int nplm_rope(void* qkv, const int* pos, const float* cos_t, const fl
 extern "C" int nplm_swiglu_fwd(const void* pre, void* out, long long T, int I, cudaStream_t st) {
   if (T <= 0) return 0;
   if (I % 8) return -3;
-  swiglu_fwd_kernel<<<grid_for(T * (I / 8), 256), 256, 0, st>>>(
+  launch_chained(swiglu_fwd_kernel, grid_for(T * (I / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<__nv_bfloat16*>(out), T, I);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1067,7 +1087,7 @@ extern "C" int nplm_swiglu_bwd(const void* pre, const void* dout, void* dpre, lo
                                cudaStream_t st) {
   if (T <= 0) return 0;
   if (I % 8) return -3;
-  swiglu_bwd_kernel<<<grid_for(T * (I / 8), 256), 256, 0, st>>>(
+  launch_chained(swiglu_bwd_kernel, grid_for(T * (I / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<const __nv_bfloat16*>(dout),
       reinterpret_cast<__nv_bfloat16*>(dpre), T, I);
   return static_cast<int>(cudaGetLastError());
@@ -1076,7 +1096,7 @@ extern "C" int nplm_swiglu_bwd(const void* pre, const void* dout, void* dpre, lo
 extern "C" int nplm_act_fwd(const void* pre, void* out, long long n, int act, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -3;
-  act_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, st>>>(
+  launch_chained(act_fwd_kernel, grid_for(n / 8, 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<__nv_bfloat16*>(out), n / 8, act);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1085,7 +1105,7 @@ extern "C" int nplm_act_bwd(const void* pre, const void* dout, void* dpre, long 
                             cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -3;
-  act_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, st>>>(
+  launch_chained(act_bwd_kernel, grid_for(n / 8, 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<const __nv_bfloat16*>(dout),
       reinterpret_cast<__nv_bfloat16*>(dpre), n / 8, act);
   return static_cast<int>(cudaGetLastError());
@@ -1099,6 +1119,7 @@ namespace nplm {
 __global__ void __launch_bounds__(256)
 transpose_scale_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ scale,
                        __nv_bfloat16* __restrict__ y, int R, int C) {
+  grid_chain();
   __shared__ __nv_bfloat16 tile[64][66];
   const size_t base = static_cast<size_t>(blockIdx.z) * R * C;
   const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
@@ -1131,7 +1152,7 @@ extern "C" int nplm_transpose_scale(const void* x, const void* scale, void* y, i
   if ((R % 64) || (C % 64) || B > 65535 || R / 64 > 65535 || (reinterpret_cast<uintptr_t>(x) & 15) ||
       (reinterpret_cast<uintptr_t>(y) & 15))
     return -3;
-  nplm::transpose_scale_kernel<<<dim3(C / 64, R / 64, B), 256, 0, st>>>(
+  launch_chained(nplm::transpose_scale_kernel, dim3(C / 64, R / 64, B), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(scale),
       reinterpret_cast<__nv_bfloat16*>(y), R, C);
   return static_cast<int>(cudaGetLastError());
@@ -1146,6 +1167,7 @@ namespace nplm {
 __global__ void __launch_bounds__(256)
 segment_mean_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ cu, float* __restrict__ out,
                     int C, int drop_last) {
+  grid_chain();
   __shared__ float part[32][64];
   const int b = blockIdx.x, g = threadIdx.x >> 3, l = threadIdx.x & 7;
   const int c = blockIdx.y * 64 + l * 8;
@@ -1180,7 +1202,7 @@ extern "C" int nplm_segment_mean(const void* x, const int* cu, float* out, int B
                                  cudaStream_t st) {
   if (B <= 0) return 0;
   if ((C % 8) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
-  nplm::segment_mean_kernel<<<dim3(B, (C + 63) / 64), 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x), cu, out,
+  launch_chained(nplm::segment_mean_kernel, dim3(B, (C + 63) / 64), 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), cu, out,
                                                                     C, drop_last);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1189,7 +1211,7 @@ extern "C" int nplm_gather_rows(const void* src, const int* idx, void* dst, int 
                                 cudaStream_t st) {
   if (n <= 0) return 0;
   if (C % 8) return -3;
-  gather_rows_kernel<<<grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st>>>(
+  launch_chained(gather_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(src), idx, reinterpret_cast<__nv_bfloat16*>(dst), n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1198,7 +1220,7 @@ extern "C" int nplm_scatter_rows(const void* src, const int* idx, void* dst, int
                                  cudaStream_t st) {
   if (n <= 0) return 0;
   if (C % 8) return -3;
-  scatter_rows_kernel<<<grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st>>>(
+  launch_chained(scatter_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(src), idx, reinterpret_cast<__nv_bfloat16*>(dst), n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1216,7 +1238,7 @@ extern "C" int nplm_ce_fwd(const void* h, const void* W, const void* bias, const
   do {                                                                                             \
     cudaFuncSetAttribute(ce_fwd_kernel<N_>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
                          static_cast<int>(smem));                                                  \
-    ce_fwd_kernel<N_><<<blocks, CE_WARPS * 32, smem, st>>>(                                        \
+    launch_chained(ce_fwd_kernel<N_>, blocks, CE_WARPS * 32, smem, st,                                         \
         reinterpret_cast<const __nv_bfloat16*>(h), reinterpret_cast<const __nv_bfloat16*>(W),      \
         reinterpret_cast<const __nv_bfloat16*>(bias), labels, inv_count, dlogits, logits, loss_sum, \
         n, C, V);                                                                                  \
@@ -1244,7 +1266,7 @@ extern "C" int nplm_ce_bwd(const void* h, const void* W, const float* dlogits, c
     }
     int tb = (n + CE_TILE_ROWS - 1) / CE_TILE_ROWS;
     if (tb > 148) tb = 148;
-    ce_bwd_tiled_kernel<<<tb, 256, tsm, st>>>(
+    launch_chained(ce_bwd_tiled_kernel, tb, 256, tsm, st,
         reinterpret_cast<const __nv_bfloat16*>(h), reinterpret_cast<const __nv_bfloat16*>(W), dlogits, gscale,
         reinterpret_cast<__nv_bfloat16*>(dh), dW, dbias, n, C, V);
     return static_cast<int>(cudaGetLastError());
@@ -1257,7 +1279,7 @@ extern "C" int nplm_ce_bwd(const void* h, const void* W, const float* dlogits, c
   do {                                                                                        \
     cudaFuncSetAttribute(ce_bwd_kernel<N_>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
                          static_cast<int>(smem));                                             \
-    ce_bwd_kernel<N_><<<blocks, CE_WARPS * 32, smem, st>>>(                                   \
+    launch_chained(ce_bwd_kernel<N_>, blocks, CE_WARPS * 32, smem, st,                                    \
         reinterpret_cast<const __nv_bfloat16*>(h), reinterpret_cast<const __nv_bfloat16*>(W), \
         dlogits, gscale, reinterpret_cast<__nv_bfloat16*>(dh), dW, dbias, n, C, V);           \
   } while (0)
@@ -1269,14 +1291,14 @@ extern "C" int nplm_ce_bwd(const void* h, const void* W, const float* dlogits, c
 extern "C" int nplm_sumsq(const float* x, long long n, float* out, cudaStream_t st) {
   if (n <= 0) return 0;
   if (reinterpret_cast<uintptr_t>(x) & 15) return -3;
-  sumsq_kernel<<<grid_for(n / 4 + 1, 256), 256, 0, st>>>(x, n, out);
+  launch_chained(sumsq_kernel, grid_for(n / 4 + 1, 256), 256, 0, st, x, n, out);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int nplm_adamw(float* p, float* m, float* v, float* g, void* p_bf16, const float* hyper,
                           const float* sumsq, long long n, int zero_grad, cudaStream_t st) {
   if (n <= 0) return 0;
-  adamw_kernel<<<grid_for(n, 256), 256, 0, st>>>(p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16),
+  launch_chained(adamw_kernel, grid_for(n, 256), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16),
                                                  hyper, sumsq, n, zero_grad);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1288,7 +1310,7 @@ extern "C" int nplm_muon_momentum(const float* g, float* m, const long long* off
   if (numel & 3) return -3;
   int bx = grid_for(numel / 4, 256);
   if (bx > 592) bx = 592;
-  muon_momentum_kernel<<<dim3(bx, n_mat), 256, 0, st>>>(g, m, off, numel, reinterpret_cast<__nv_bfloat16*>(upd),
+  launch_chained(muon_momentum_kernel, dim3(bx, n_mat), 256, 0, st, g, m, off, numel, reinterpret_cast<__nv_bfloat16*>(upd),
                                                         usq, sumsq, gs, max_norm, mu, nesterov);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1299,7 +1321,7 @@ extern "C" int nplm_muon_apply(float* p, void* p16, const long long* off, int n_
   if (numel & 3) return -3;
   int bx = grid_for(numel / 4, 256);
   if (bx > 592) bx = 592;
-  muon_apply_kernel<<<dim3(bx, n_mat), 256, 0, st>>>(p, reinterpret_cast<__nv_bfloat16*>(p16), off, numel,
+  launch_chained(muon_apply_kernel, dim3(bx, n_mat), 256, 0, st, p, reinterpret_cast<__nv_bfloat16*>(p16), off, numel,
                                                      reinterpret_cast<const __nv_bfloat16*>(O), lr, wd, cautious);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1311,7 +1333,7 @@ extern "C" int nplm_adamw_slots(float* p, float* m, float* v, const float* g, vo
   if (n_slots <= 0 || max_numel <= 0) return 0;
   int bx = grid_for(max_numel, 256);
   if (bx > 64) bx = 64;
-  adamw_slots_kernel<<<dim3(bx, n_slots), 256, 0, st>>>(p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p16), off,
+  launch_chained(adamw_slots_kernel, dim3(bx, n_slots), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p16), off,
                                                         numel, decay, sumsq, gs, max_norm, lr, b1, b2, eps, wd,
                                                         bc1, bc2);
   return static_cast<int>(cudaGetLastError());
@@ -1319,7 +1341,7 @@ extern "C" int nplm_adamw_slots(float* p, float* m, float* v, const float* g, vo
 
 extern "C" int nplm_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
-  cast_f32_to_bf16_kernel<<<grid_for(n, 256), 256, 0, st>>>(src, reinterpret_cast<__nv_bfloat16*>(dst), n);
+  launch_chained(cast_f32_to_bf16_kernel, grid_for(n, 256), 256, 0, st, src, reinterpret_cast<__nv_bfloat16*>(dst), n);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1328,7 +1350,7 @@ extern "C" int nplm_masked_mse(const void* s, const void* t, const int* valid,
                                cudaStream_t st) {
   if (T <= 0) return 0;
   if (C % 8) return -3;
-  masked_mse_kernel<<<grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st>>>(
+  launch_chained(masked_mse_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(s), reinterpret_cast<const __nv_bfloat16*>(t), valid,
       inv_count, reinterpret_cast<__nv_bfloat16*>(ds), loss_sum, T, C);
   return static_cast<int>(cudaGetLastError());

@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(256)
 dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
               const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
               const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int KS, int flip) {
+  grid_chain();
   const int vec = C >> 3;
   const int r = KS >> 1;
   const long long total = static_cast<long long>(T) * vec;
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(256)
 dwconv_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
                    const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip) {
+  grid_chain();
   constexpr int R = KS / 2;
   const int vec = C >> 3;
   const int n_tb = (T + DW_TT - 1) / DW_TT;
@@ -159,6 +161,7 @@ dwconv_bwd_w_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
                     const int* __restrict__ s_start, const int* __restrict__ s_end,
                     float* __restrict__ dw, float* __restrict__ dbias, int T, int C, int KS,
                     int tokens_per_block) {
+  grid_chain();
   __shared__ float red[8][32][MAX_KS + 1];
   const int cl = threadIdx.x & 31;       // channel lane
   const int tl = threadIdx.x >> 5;       // token lane
@@ -205,6 +208,7 @@ dwconv_bwd_w_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
                          const int* __restrict__ s_start, const int* __restrict__ s_end,
                          float* __restrict__ dw, float* __restrict__ dbias, int T, int C,
                          int tokens_per_block) {
+  grid_chain();
   constexpr int R = KS / 2;
   __shared__ float red[8][32][KS + 1];
   const int cl = threadIdx.x & 31;       // channel lane
@@ -260,6 +264,7 @@ constexpr int MAX_STREAMS = 8;
 __global__ void __launch_bounds__(256)
 mhc_read_kernel(const __nv_bfloat16* __restrict__ X, const float* __restrict__ alpha,
                 __nv_bfloat16* __restrict__ h, int T, int n, int C) {
+  grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(T) * vec;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -285,6 +290,7 @@ __global__ void __launch_bounds__(256)
 mhc_write_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ y,
                  const float* __restrict__ R, const float* __restrict__ beta,
                  __nv_bfloat16* __restrict__ Xn, int T, int C) {
+  grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(T) * vec;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -353,6 +359,7 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
                const __nv_bfloat16* __restrict__ dXn, const __nv_bfloat16* __restrict__ dh,
                __nv_bfloat16* __restrict__ dX, __nv_bfloat16* __restrict__ dy, float* __restrict__ dR,
                float* __restrict__ dalpha, float* __restrict__ dbeta, int T, int C) {
+  grid_chain();
   static_assert(N * N + 2 * N <= 32, "too many streams for the warp-transpose reduction");
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
@@ -440,6 +447,7 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
 // z[t][:] = (1/n) sum_i X[t][i][:]   (what the coefficient network of a site sees)
 __global__ void __launch_bounds__(256)
 mhc_mean_kernel(const __nv_bfloat16* __restrict__ X, __nv_bfloat16* __restrict__ z, int T, int n, int C) {
+  grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(T) * vec;
   const float inv = 1.f / static_cast<float>(n);
@@ -467,6 +475,7 @@ __global__ void __launch_bounds__(256)
 mhc_dx_combine_kernel(const __nv_bfloat16* __restrict__ g, const float* __restrict__ alpha,
                       const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ dz,
                       __nv_bfloat16* __restrict__ dX, int T, int n, int C) {
+  grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(T) * vec;
   const float inv = 1.f / static_cast<float>(n);
@@ -511,7 +520,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
   if ((KS == 3 || KS == 5 || KS == 7 || KS == 9) && aligned) {   // the tile kernel loads 16-byte words of w
     const int grid = grid_for(static_cast<long long>((T + DW_TT - 1) / DW_TT) * (C / 8), 256);
 #define NPLM_DWCONV(KS_)                                                                                   \
-  dwconv_tile_kernel<KS_><<<grid, 256, 0, st>>>(                                                           \
+  launch_chained(dwconv_tile_kernel<KS_>, grid, 256, 0, st,                                                            \
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),                \
       reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip)
     switch (KS) {
@@ -523,7 +532,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
 #undef NPLM_DWCONV
     return static_cast<int>(cudaGetLastError());
   }
-  dwconv_kernel<<<grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st>>>(
+  launch_chained(dwconv_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
       reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C,
       KS, flip);
@@ -538,7 +547,7 @@ extern "C" int nplm_dwconv_bwd_w(const void* x, const void* dy, const int* s_sta
   dim3 grid((T + tokens_per_block - 1) / tokens_per_block, (C + 31) / 32);
   if (KS == 3 || KS == 5 || KS == 7 || KS == 9) {
 #define NPLM_DWCONV_W(KS_)                                                                              \
-  dwconv_bwd_w_tile_kernel<KS_><<<grid, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x),          \
+  launch_chained(dwconv_bwd_w_tile_kernel<KS_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),          \
                                                       reinterpret_cast<const __nv_bfloat16*>(dy), s_start, \
                                                       s_end, dw, dbias, T, C, tokens_per_block)
     switch (KS) {
@@ -550,7 +559,7 @@ extern "C" int nplm_dwconv_bwd_w(const void* x, const void* dy, const int* s_sta
 #undef NPLM_DWCONV_W
     return static_cast<int>(cudaGetLastError());
   }
-  dwconv_bwd_w_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x),
+  launch_chained(dwconv_bwd_w_kernel, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),
                                             reinterpret_cast<const __nv_bfloat16*>(dy), s_start, s_end, dw,
                                             dbias, T, C, KS, tokens_per_block);
   return static_cast<int>(cudaGetLastError());
@@ -559,7 +568,7 @@ extern "C" int nplm_dwconv_bwd_w(const void* x, const void* dy, const int* s_sta
 extern "C" int nplm_mhc_read(const void* X, const float* alpha, void* h, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS) return -3;
-  mhc_read_kernel<<<grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st>>>(
+  launch_chained(mhc_read_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(X), alpha, reinterpret_cast<__nv_bfloat16*>(h), T, n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -567,7 +576,7 @@ extern "C" int nplm_mhc_read(const void* X, const float* alpha, void* h, int T, 
 extern "C" int nplm_mhc_mean(const void* X, void* z, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS) return -3;
-  mhc_mean_kernel<<<grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st>>>(
+  launch_chained(mhc_mean_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<__nv_bfloat16*>(z), T, n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -576,7 +585,7 @@ extern "C" int nplm_mhc_dx_combine(const void* g, const float* alpha, const void
                                    int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS || (dh != nullptr && alpha == nullptr)) return -3;
-  mhc_dx_combine_kernel<<<grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st>>>(
+  launch_chained(mhc_dx_combine_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(g), alpha, reinterpret_cast<const __nv_bfloat16*>(dh),
       reinterpret_cast<const __nv_bfloat16*>(dz), reinterpret_cast<__nv_bfloat16*>(dX), T, n, C);
   return static_cast<int>(cudaGetLastError());
@@ -588,7 +597,7 @@ extern "C" int nplm_mhc_write(const void* X, const void* y, const float* R, cons
   if ((C % 8) || n < 1 || n > 4) return -3;
   const int grid = grid_for(static_cast<long long>(T) * (C / 8), 256);
 #define NPLM_MHC_WRITE(N_)                                                                              \
-  mhc_write_kernel<N_><<<grid, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(X),                  \
+  launch_chained(mhc_write_kernel<N_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(X),                  \
                                              reinterpret_cast<const __nv_bfloat16*>(y), R, beta,         \
                                              reinterpret_cast<__nv_bfloat16*>(Xn), T, C)
   switch (n) {
@@ -609,7 +618,7 @@ extern "C" int nplm_mhc_bwd(const void* X, const void* y, const float* R, const 
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
 #define NPLM_MHC_BWD(N_)                                                                                  \
-  mhc_bwd_kernel<N_><<<blocks, 256, 0, st>>>(                                                              \
+  launch_chained(mhc_bwd_kernel<N_>, blocks, 256, 0, st,                                                               \
       reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, alpha, beta, \
       reinterpret_cast<const __nv_bfloat16*>(dXn), reinterpret_cast<const __nv_bfloat16*>(dh),              \
       reinterpret_cast<__nv_bfloat16*>(dX), reinterpret_cast<__nv_bfloat16*>(dy), dR, dalpha, dbeta, T, C)
@@ -770,6 +779,7 @@ __global__ void __launch_bounds__(128)
 mhc_coef_fwd_kernel(const __nv_bfloat16* __restrict__ pre, const P* __restrict__ pa, const P* __restrict__ pb,
                     const P* __restrict__ pr, const P* __restrict__ ps, int iters, int T, float* __restrict__ alpha_out, float* __restrict__ beta_out,
                     float* __restrict__ R_out) {
+  grid_chain();
   constexpr int M = 2 * N + N * N;
   const MhcStatic<N, P> st(pa, pb, pr, ps);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
@@ -795,6 +805,7 @@ mhc_coef_bwd_kernel(const __nv_bfloat16* __restrict__ pre, const P* __restrict__
                     const float* __restrict__ dR, __nv_bfloat16* __restrict__ dpre,
                     float* __restrict__ da, float* __restrict__ db, float* __restrict__ dr,
                     float* __restrict__ ds) {
+  grid_chain();
   constexpr int M = 2 * N + N * N;
   static_assert(M + 3 <= 32, "parameter gradients are reduced with one value per lane");
   const MhcStatic<N, P> st(pa, pb, pr, ps);
@@ -883,7 +894,7 @@ namespace nplm {
 template <int N, typename P>
 static void mhc_coef_fwd_launch(const __nv_bfloat16* pre, const void* a, const void* b, const void* r, const void* s,
                                 int iters, int T, float* alpha, float* beta, float* R, int blocks, cudaStream_t st) {
-  mhc_coef_fwd_kernel<N, P><<<blocks, 128, 0, st>>>(pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
+  launch_chained(mhc_coef_fwd_kernel<N, P>, blocks, 128, 0, st, pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
                                                     reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters,
                                                     T, alpha, beta, R);
 }
@@ -892,7 +903,7 @@ static void mhc_coef_bwd_launch(const __nv_bfloat16* pre, const void* a, const v
                                 int iters, int T, const float* dalpha, const float* dbeta, const float* dR,
                                 __nv_bfloat16* dpre, float* da, float* db, float* dr, float* ds, int blocks,
                                 cudaStream_t st) {
-  mhc_coef_bwd_kernel<N, P><<<blocks, 128, 0, st>>>(pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
+  launch_chained(mhc_coef_bwd_kernel<N, P>, blocks, 128, 0, st, pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
                                                     reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters,
                                                     T, dalpha, dbeta, dR, dpre, da, db, dr, ds);
 }

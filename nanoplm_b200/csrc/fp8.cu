@@ -35,6 +35,7 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
 __global__ void __launch_bounds__(256)
 quant_rows_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, uint8_t* __restrict__ q,
                   float* __restrict__ scale) {
+  grid_chain();
   const int KB = K / 128;
   const long long groups = static_cast<long long>(R) * KB;
   const int sub = threadIdx.x & 15;
@@ -81,6 +82,7 @@ template <bool TRANSPOSE, bool BLOCK>
 __global__ void __launch_bounds__(256)
 quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, uint8_t* __restrict__ q,
                   float* __restrict__ scale) {
+  grid_chain();
   __shared__ __nv_bfloat16 tile[128][130];
   __shared__ float s_red[128];
   const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
@@ -175,6 +177,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, ui
 __global__ void __launch_bounds__(256)
 quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, uint8_t* __restrict__ qr,
                   float* __restrict__ sr, uint8_t* __restrict__ qt, float* __restrict__ st) {
+  grid_chain();
   __shared__ __align__(16) uint8_t tile[128 * 128];
   __shared__ float cmax[8][128];
   const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
@@ -307,6 +310,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   constexpr int STAGES = C8::STAGES, ACC = C8::ACC, HC = C8::HC;
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1024-byte aligned base
+    grid_wait();
     if (threadIdx.x == 0) atomicExch(args.status, ST_BAD_ARG);
     return;
   }
@@ -360,6 +364,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     tma_prefetch_desc(&tmB);
     tma_prefetch_desc(&tmC);
   }
+  grid_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, ACC * BN);
     tmem_relinquish();
@@ -368,6 +373,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (args.ag_world <= 1) grid_release();
 
   if (warp < 4) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(F8_REGS_LIGHT));
@@ -725,7 +731,7 @@ static int f8_launch_form(const void* A, const void* B, void* C, Fp8Args& args, 
     return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(gemm_fp8_kernel<BN, B_BLOCK>), dim3(grid),
                                                         dim3(F8_THREADS), params, F8Cfg<BN>::SMEM, stream));
   }
-  gemm_fp8_kernel<BN, B_BLOCK><<<grid, F8_THREADS, F8Cfg<BN>::SMEM, stream>>>(tmA, tmB, tmC, args);
+  launch_chained(gemm_fp8_kernel<BN, B_BLOCK>, grid, F8_THREADS, F8Cfg<BN>::SMEM, stream, tmA, tmB, tmC, args);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -752,7 +758,7 @@ extern "C" int nplm_fp8_quant_rows(const void* x, int R, int K, int ldx, void* q
   if (R <= 0 || K <= 0) return 0;
   if ((K % 128) || (ldx % 8)) return -3;
   const long long threads = static_cast<long long>(R) * (K / 128) * 16;
-  quant_rows_kernel<<<f8_grid(threads, 256), 256, 0, stream>>>(
+  launch_chained(quant_rows_kernel, f8_grid(threads, 256), 256, 0, stream,
       reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx, reinterpret_cast<uint8_t*>(q), scale);
   return static_cast<int>(cudaGetLastError());
 }
@@ -769,11 +775,11 @@ extern "C" int nplm_fp8_quant_tile(const void* x, int R, int K, int ldx, int tra
   const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x);
   uint8_t* qp = reinterpret_cast<uint8_t*>(q);
   if (!transpose)
-    quant_tile_kernel<false, true><<<grid, 256, 0, stream>>>(xp, R, K, ldx, qp, scale);
+    launch_chained(quant_tile_kernel<false, true>, grid, 256, 0, stream, xp, R, K, ldx, qp, scale);
   else if (block)
-    quant_tile_kernel<true, true><<<grid, 256, 0, stream>>>(xp, R, K, ldx, qp, scale);
+    launch_chained(quant_tile_kernel<true, true>, grid, 256, 0, stream, xp, R, K, ldx, qp, scale);
   else
-    quant_tile_kernel<true, false><<<grid, 256, 0, stream>>>(xp, R, K, ldx, qp, scale);
+    launch_chained(quant_tile_kernel<true, false>, grid, 256, 0, stream, xp, R, K, ldx, qp, scale);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -783,7 +789,7 @@ extern "C" int nplm_fp8_quant_dual(const void* x, int R, int K, int ldx, void* q
   if (R <= 0 || K <= 0) return 0;
   if ((K % 128) || (R % 128) || (ldx % 4) || (reinterpret_cast<uintptr_t>(x) & 7)) return -3;
   if (R / 128 > 65535) return -3;
-  quant_dual_kernel<<<dim3(K / 128, R / 128), 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx,
+  launch_chained(quant_dual_kernel, dim3(K / 128, R / 128), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx,
                                                                 reinterpret_cast<uint8_t*>(qr), sr,
                                                                 reinterpret_cast<uint8_t*>(qt), st);
   return static_cast<int>(cudaGetLastError());

@@ -275,6 +275,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tma_prefetch_desc(&tmR);
     }
   }
+  grid_wait();
   if (warp == 1) {
     if constexpr (PAIR) {
       tmem_alloc_pair(tmem_slot, 2 * BN);
@@ -289,6 +290,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if constexpr (PAIR) cluster_sync_all();   // the peer's barriers are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (args.row_arrive == nullptr && args.ag_world <= 1) grid_release();
   // hands accumulator `a` back to the MMA thread (of rank 0)
   auto release_acc = [&](int a) {
     if constexpr (PAIR) {
@@ -1042,7 +1044,7 @@ static int launch_impl(const GemmMaps& maps, const GemmArgs& args, int max_ctas,
     return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(grid),
                                                         dim3(S::THREADS), params, S::TOTAL, stream));
   }
-  kern<<<grid, S::THREADS, S::TOTAL, stream>>>(tmA, tmB, maps.C, maps.R, args);
+  launch_chained(kern, grid, S::THREADS, S::TOTAL, stream, tmA, tmB, maps.C, maps.R, args);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1073,13 +1075,15 @@ static int launch_pair_impl(const GemmMaps& maps, const GemmArgs& args, cudaStre
   cfg.blockDim = dim3(S::THREADS);
   cfg.dynamicSmemBytes = S::TOTAL;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (see grid_wait)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, maps.A, maps.B, maps.C, maps.R, args));
 }
 

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256)
 router_topk_kernel(const __nv_bfloat16* __restrict__ logits, int T, int E, int k,
                    float* __restrict__ probs, float* __restrict__ gates, int* __restrict__ experts,
                    float* __restrict__ probsum, int* __restrict__ counts) {
+  grid_chain();
   __shared__ float s_sum[MOE_MAX_E];
   __shared__ int s_cnt[MOE_MAX_E];
   for (int i = threadIdx.x; i < E; i += blockDim.x) {
@@ -126,6 +127,7 @@ router_bwd_kernel(const float* __restrict__ probs, const float* __restrict__ gat
                   const int* __restrict__ experts, const float* __restrict__ d_gates,
                   const float* __restrict__ aux_grad_per_expert,  // [E], already scaled, or null
                   int T, int E, int k, __nv_bfloat16* __restrict__ dlogits) {
+  grid_chain();
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   constexpr int PER = MOE_MAX_E / 32;
@@ -474,7 +476,7 @@ extern "C" int nplm_router_topk(const void* logits, int T, int E, int k, float* 
                                 int* experts, float* probsum, int* counts, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (E < 1 || E > MOE_MAX_E || k < 1 || k > MOE_MAX_K || k > E) return -3;
-  router_topk_kernel<<<grid_for(T, 8), 256, 0, stream>>>(
+  launch_chained(router_topk_kernel, grid_for(T, 8), 256, 0, stream,
       reinterpret_cast<const __nv_bfloat16*>(logits), T, E, k, probs, gates, experts, probsum, counts);
   return static_cast<int>(cudaGetLastError());
 }
@@ -484,7 +486,7 @@ extern "C" int nplm_router_bwd(const float* probs, const float* gates, const int
                                void* dlogits, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (E < 1 || E > MOE_MAX_E || k < 1 || k > MOE_MAX_K) return -3;
-  router_bwd_kernel<<<grid_for(T, 8), 256, 0, stream>>>(probs, gates, experts, d_gates, aux_grad, T, E,
+  launch_chained(router_bwd_kernel, grid_for(T, 8), 256, 0, stream, probs, gates, experts, d_gates, aux_grad, T, E,
                                                         k, reinterpret_cast<__nv_bfloat16*>(dlogits));
   return static_cast<int>(cudaGetLastError());
 }
