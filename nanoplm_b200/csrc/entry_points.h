@@ -45,6 +45,25 @@ inline bool gemm_pair_pays(long long M, long long N, long long K, int epi) {
 }
 }  // namespace nplm
 
+// Tile width (columns) of a bf16-output GEMM by default (ops/kernels.py has the same rule, and a test compares the two): the
+// narrowest tiles that one wave of 148 CTAs covers. Below a wave a GEMM takes as long as one tile, i.e. launch, first
+// loads, K / 64 steps and the epilogue of a tile's columns one 64-column chunk after the other; a narrow tile has fewer of
+// those and loads less a step, and the idle multiprocessors take the other columns. Past a wave the wide tiles'
+// lower operand traffic wins. Graph-timed us, 64 / 128 / 256 columns:
+//   add, 512 columns of K = 512: 236 rows 5.1 / 5.8 / 8.1, 2 050 (136 tiles of 64) 5.4 / 6.1 / 8.5, 4 600 (144 of 128) 7.8 /
+//     6.5 / 8.6, 8 160 (128 of 256) 12.0 / 8.9 / 9.1; of K = 1024: 236 rows 6.8 / 7.5 / 10.3
+//   RoPE, 1536 of 512: 236 rows 6.6 / 7.0 / 8.5, 1 000 (96 of 128) 9.1 / 7.2 / 8.7, 2 050 (102 of 256) 11.8 / 10.2 / 9.0
+//   SwiGLU (a tile's columns are value and gate, so 128 at least), 2048 of 512: 236 rows - / 6.0 / 7.7, 1 000 (128 of 128)
+//     - / 6.8 / 8.1, 2 050 (136 of 256) - / 9.1 / 8.8
+//   GELU, 512 of 512: 236 rows 7.5 / 8.9 / 12.5; data gradient, 512 of 2048: 236 rows 9.7 / 10.1 / 13.0
+inline int gemm_tile_width(long long M, long long N, int epi) {
+  if (epi == EPI_SWIGLU_BWD || epi == EPI_STORE_DELTA || epi == EPI_ATOMIC_F32 || epi == EPI_STORE_F32)
+    return N >= 256 || epi == EPI_SWIGLU_BWD || epi == EPI_STORE_DELTA ? 256 : 128;
+  const long long rows = (M + 127) / 128;
+  if (epi != EPI_SWIGLU && rows * ((N + 63) / 64) <= 148) return 64;
+  return (N < 256 && epi != EPI_SWIGLU) || rows * ((N + 127) / 128) <= 148 ? 128 : 256;
+}
+
 extern "C" {
 int nplm_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
                    int ldr, int a_mn, int b_mn, int epi, int splits, int bn, int max_ctas, int direct_epilogue,

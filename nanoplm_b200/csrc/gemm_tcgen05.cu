@@ -36,19 +36,20 @@ constexpr int EPI_WARPS_OF =
     (PAIR && STAGED && (EPI == EPI_ROPE || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD)) ? 8 : 4;
 
 // STAGED: the epilogue goes through shared memory (TMA stores and reduce-adds); the direct epilogue, and fp32 outputs of
-// groups whose rows are no multiple of 32, write straight from registers and spend that room on one more pipeline stage.
+// groups whose rows are no multiple of 32, write straight from registers and spend that room on pipeline stages.
 template <int BN, bool PAIR = false, bool STAGED = true, int EPI_WARPS_ = 4>
 struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = PAIR ? (STAGED ? (EPI_WARPS_ == 8 ? 5 : 6) : 7) : ((BN == 256) ? 4 : (STAGED ? 6 : 7));
   static constexpr int BAR_BYTES = 512;
   static constexpr int EPI_WARPS = EPI_WARPS_;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   // epilogue staging: 2 buffers x (32 rows x 128 B) per warp, written swizzled, read by TMA stores
   static constexpr int EPI_BYTES = STAGED ? EPI_WARPS * 2 * 4096 : 0;
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + BAR_BYTES + 1024;  // + alignment slack
+  static constexpr int FIXED = EPI_BYTES + BAR_BYTES + 1024;                     // + alignment slack
+  static constexpr int STAGES = (227 * 1024 - FIXED) / STAGE_BYTES;              // what a CTA's 227 KB hold: 3 to 9
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + FIXED;
 };
 
 struct GemmArgs {
@@ -1158,7 +1159,7 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   if (epi == EPI_SWIGLU && (b_mn || (N % 2) || ((N / 2) % 8))) return -4;
   if ((epi == EPI_ATOMIC_F32 || epi == EPI_STORE_F32) ? (N % 4 || ldc % 4) : (N % 8 || ldc % 8))
     return -5;
-  if (bn != 128 && bn != 256) return -6;
+  if (bn != 64 && bn != 128 && bn != 256) return -6;
   if (epi == EPI_ROPE && (a_mn || b_mn || direct_epilogue || rope_pos == nullptr || rope_cos == nullptr ||
                           rope_sin == nullptr || (rope_cols % 64) || (N % 64)))
     return -7;
@@ -1394,6 +1395,24 @@ extern "C" int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const
 extern "C" int nplm_gemm_bf16_grouped_gated(const void* A, const void* B, void* C, const void* R, int M,
                                             int N, int K, int lda, int ldb, int ldc, int ldr, int b_mn,
                                             int epi, int bn, int groups, const int* tile_group,
+  if (bn == 64) {   // bf16 outputs of plain GEMMs with few rows (gemm_tile_width)
+    if (a_mn || grp.mode != 0 || grp.ag_world > 1) return -6;
+    if (!b_mn) {
+      switch (epi) {
+        case EPI_STORE: return launch<64, false, false, EPI_STORE>(maps, args, max_ctas, stream);
+        case EPI_ADD: return launch<64, false, false, EPI_ADD>(maps, args, max_ctas, stream);
+        case EPI_GELU: return launch<64, false, false, EPI_GELU>(maps, args, max_ctas, stream);
+        case EPI_RELU: return launch<64, false, false, EPI_RELU>(maps, args, max_ctas, stream);
+        case EPI_ROPE: return launch<64, false, false, EPI_ROPE>(maps, args, max_ctas, stream);
+        default: return -6;
+      }
+    }
+    switch (epi) {
+      case EPI_STORE: return launch<64, false, true, EPI_STORE>(maps, args, max_ctas, stream);
+      case EPI_ADD: return launch<64, false, true, EPI_ADD>(maps, args, max_ctas, stream);
+      default: return -6;
+    }
+  }
                                             int b_group_rows, const unsigned* row_arrive,
                                             const int* row_expect, int* status, cudaStream_t stream) {
   if ((row_arrive == nullptr) != (row_expect == nullptr)) return -3;

@@ -124,10 +124,10 @@ struct Call {
   int out(const void* A, const void* B, void* Cp, const void* R, int M, int N, int K, int ldb, int ldc, int ldr, int b_mn,
           int epi, const int* pos = nullptr, const float* cosp = nullptr, const float* sinp = nullptr,
           int rope_cols = 0) const {
-    const bool wide = N >= 256 || epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD;
-    if (wide && gemm_pair_pays(M, N, K, epi))
+    const int bn = gemm_tile_width(M, N, epi);
+    if (bn == 256 && gemm_pair_pays(M, N, K, epi))
       return fn.pair(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, 0, pos, cosp, sinp, rope_cols, status, stream);
-    return fn.gemm(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, wide ? 256 : 128, 0, 0, pos, cosp, sinp, rope_cols, status,
+    return fn.gemm(A, B, Cp, R, M, N, K, K, ldb, ldc, ldr, 0, b_mn, epi, 1, bn, 0, 0, pos, cosp, sinp, rope_cols, status,
                    stream);
   }
   // fp32 C[N][K] += dy[T][N]^T x[T][K]
@@ -160,6 +160,7 @@ extern "C" void nplm_layer_init(void* const* f) {
   fn.fa_bwd = reinterpret_cast<decltype(fn.fa_bwd)>(f[6]);
 }
 
+extern "C" int nplm_gemm_tile_width(long long M, long long N, int epi) { return gemm_tile_width(M, N, epi); }
 extern "C" int nplm_gemm_pair_pays(long long M, long long N, long long K, int epi) { return gemm_pair_pays(M, N, K, epi); }
 
 // Length of the argument array of a forward (0) or backward (1) call.

@@ -64,6 +64,17 @@ def pair_pays(M: int, N: int, K: int, epi: int) -> bool:
     return tiles > 148 if K >= 768 else tiles * K > (190000 if epi == EPI_SWIGLU else 400000)
 
 
+def tile_width(M: int, N: int, epi: int) -> int:
+    """Default tile width of a GEMM: the rule of `gemm_tile_width` in csrc/entry_points.h, which states the measurements on
+    both sides of its lines."""
+    if epi in (EPI_SWIGLU_BWD, 9, EPI_ATOMIC_F32, EPI_STORE_F32):
+        return 256 if N >= 256 or epi in (EPI_SWIGLU_BWD, 9) else 128
+    rows = (M + 127) // 128
+    if epi != EPI_SWIGLU and rows * ((N + 63) // 64) <= 148:
+        return 64
+    return 128 if (N < 256 and epi != EPI_SWIGLU) or rows * ((N + 127) // 128) <= 148 else 256
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          epi: int = EPI_STORE, out: torch.Tensor | None = None, aux: torch.Tensor | None = None,
          splits: int = 1, bn: int | None = None, max_ctas: int = 0,
@@ -126,7 +137,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     elif epi == EPI_SWIGLU_BWD:
         raise ValueError("EPI_SWIGLU_BWD needs the pre-activations passed as aux")
     if bn is None:
-        bn = 256 if (N >= 256 or epi in (EPI_SWIGLU, EPI_SWIGLU_BWD)) else 128
+        if pair is None and _GEMM_PAIR_DEFAULT[0] is None and max_ctas == 0 and not direct_epilogue and not a_mn:
+            bn = tile_width(M, N, epi)
+        else:
+            bn = 256 if (N >= 256 or epi in (EPI_SWIGLU, EPI_SWIGLU_BWD)) else 128
     r_pos = r_cos = r_sin = None
     r_cols = 0
     if epi == EPI_ROPE:
