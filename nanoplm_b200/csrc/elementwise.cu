@@ -238,125 +238,119 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   }
 }
 
-// Norm backward with a thread block per group of ROWS rows (C/8 threads, each owning 8 channels
-// of every row of the group). All loads of a group are issued before the first reduction, so a
-// block keeps ROWS * 3 * C * 2 bytes in flight; the row reductions of the whole group share one
-// __syncthreads. Registers per thread stay low enough for several blocks per SM.
-//   ids == nullptr : dx[row] = [dres[row] +] norm-backward(dy[row]),  dw += sum dy * xhat
-//   ids != nullptr : embedding mode. x rows are table[ids[row]]; the row gradients are summed per
-//                    vocabulary entry in shared memory (each thread owns its channels, so no
-//                    atomics inside the block) and flushed to dtable with one atomic per element.
-template <int ROWS, int SUB>
+// ------------------------------------------------------------------ embedding + norm backward
+// Rows with the same token have the same x, mean and rstd, and the norm's backward pass is linear in dy: the gradient of a
+// table row is the norm backward of S[v] = sum of dy over the rows of token v. So a first kernel reads dy once and only adds
+// (bound by that read: 2 C bytes a token), a second one applies the norm's backward pass to the V sums. One norm backward
+// per token row, its two reductions behind block barriers and the sums in shared-memory atomics of one block a
+// multiprocessor, took 396 us for 55 424 x 1024 and 32 us for 2 600 x 256, mostly the flush of 148 whole tables.
+//
+// A warp walks rows of a 128-channel slice, a lane owns four channels and adds them into the warp's own table in shared
+// memory [V][128] (nobody else's, so plain adds); the block's tables meet at the end and leave as 16-byte reductions.
+// sums: fp32 [V][C], then int [V] = 1 + a row that holds the token (0: none), all zero before the launch.
+constexpr int EMB_SLICE = 128, EMB_ROWS = 16;
+
 __global__ void __launch_bounds__(512)
-norm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                     const int* __restrict__ ids, const __nv_bfloat16* __restrict__ w,
-                     const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
-                     const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                     float* __restrict__ dw, float* __restrict__ dtable, int T, int C, int V, int rms) {
+embed_grad_sums_kernel(const __nv_bfloat16* __restrict__ dy, const int* __restrict__ ids,
+                       float* __restrict__ sums, int T, int C, int V) {
   grid_chain();
-  extern __shared__ float s_table[];   // [V][C] in embedding mode
-  // SUB row groups run side by side in one block (blockDim.x / SUB threads each): they share the
-  // table sums, which therefore take shared-memory atomics (two groups may hold the same token)
-  __shared__ float red[2][SUB][ROWS][8][2];
-  const int cthreads = blockDim.x / SUB;
-  const int sub = threadIdx.x / cthreads, tid = threadIdx.x % cthreads;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = cthreads >> 5;
-  const int i = tid * 8;
-  const bool on = i < C;
-  if (ids != nullptr) {
-    for (int k = threadIdx.x; k < V * C; k += blockDim.x) s_table[k] = 0.f;
-    __syncthreads();
-  }
-  float wv[8], acc[8];
+  extern __shared__ __align__(16) float emb_tables[];   // [warps][V][128]
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int table = V * EMB_SLICE;
+  for (int i = threadIdx.x * 4; i < warps * table; i += blockDim.x * 4)
+    *reinterpret_cast<float4*>(emb_tables + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  const int c = blockIdx.x * EMB_SLICE + lane * 4;
+  const bool on = c < C;
+  float* mine = emb_tables + warp * table + lane * 4;
+  int* some_row = reinterpret_cast<int*>(sums + static_cast<size_t>(V) * C);
+  const int step = gridDim.y * warps;
+  for (int row0 = blockIdx.y * warps + warp; row0 < T; row0 += step * EMB_ROWS) {
+    uint2 d[EMB_ROWS];
+    int id[EMB_ROWS];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    wv[e] = 1.f;
-    acc[e] = 0.f;
-  }
-  if (on && w) load8(w + i, wv);
-  int buf = 0;
-  // every thread of the block runs the same number of iterations (the barrier below is block-wide)
-  for (int base = blockIdx.x * ROWS * SUB; base < T; base += gridDim.x * ROWS * SUB, buf ^= 1) {
-    const int row0 = base + sub * ROWS;
-    float xh[ROWS][8], g[ROWS][8];
-    float rstd[ROWS];
-    int id[ROWS];
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const int row = row0 + r;
-      float sg = 0.f, sgx = 0.f;
-      rstd[r] = 0.f;
-      id[r] = 0;
+    for (int k = 0; k < EMB_ROWS; ++k) {
+      const int row = row0 + k * step;
+      d[k] = make_uint2(0u, 0u);
+      id[k] = -1;
       if (row < T) {
-        const float mean = rms ? 0.f : mean_in[row];
-        rstd[r] = rstd_in[row];
-        if (ids != nullptr) id[r] = ids[row];
-        if (on) {
-          float xv[8], dv[8];
-          const __nv_bfloat16* src = ids ? x + static_cast<size_t>(id[r]) * C : x + static_cast<size_t>(row) * C;
-          load8(src + i, xv);
-          load8(dy + static_cast<size_t>(row) * C + i, dv);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            xh[r][e] = (xv[e] - mean) * rstd[r];
-            g[r][e] = dv[e] * wv[e];
-            sg += g[r][e];
-            sgx += g[r][e] * xh[r][e];
-            acc[e] += dv[e] * xh[r][e];
-          }
-        }
-      }
-      sg = warp_sum(sg);
-      sgx = warp_sum(sgx);
-      if (lane == 0) {
-        red[buf][sub][r][warp][0] = sg;
-        red[buf][sub][r][warp][1] = sgx;
+        id[k] = __ldg(ids + row);
+        if (on) d[k] = __ldg(reinterpret_cast<const uint2*>(dy + static_cast<size_t>(row) * C + c));
       }
     }
-    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const int row = row0 + r;
-      if (row < T && on) {
-        float tg = 0.f, tgx = 0.f;
-        for (int k = 0; k < nwarps; ++k) {
-          tg += red[buf][sub][r][k][0];
-          tgx += red[buf][sub][r][k][1];
-        }
-        tg = rms ? 0.f : tg / C;
-        tgx /= C;
-        float o[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = rstd[r] * (g[r][e] - tg - xh[r][e] * tgx);
-        if (ids != nullptr) {
-          float* dst = s_table + static_cast<size_t>(id[r]) * C + i;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (SUB > 1) atomicAdd(&dst[e], o[e]);
-            else dst[e] += o[e];
-          }
-        } else {
-          if (dres) {
-            float rr[8];
-            load8(dres + static_cast<size_t>(row) * C + i, rr);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] += rr[e];
-          }
-          store8(dx + static_cast<size_t>(row) * C + i, o);
-        }
+    for (int k = 0; k < EMB_ROWS; ++k) {
+      if (id[k] >= 0) {
+        float4* t = reinterpret_cast<float4*>(mine + id[k] * EMB_SLICE);
+        const float2 a = unpack_bf16x2(d[k].x), b = unpack_bf16x2(d[k].y);
+        float4 v = *t;
+        v.x += a.x;
+        v.y += a.y;
+        v.z += b.x;
+        v.w += b.y;
+        *t = v;
+        if (blockIdx.x == 0 && lane == 0) some_row[id[k]] = 1 + row0 + k * step;   // (any of them: see above)
       }
     }
   }
-  if (dw && on) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) atomicAdd(&dw[i + e], acc[e]);
-  }
-  if (ids != nullptr) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < V * C; k += blockDim.x) {
-      const float v = s_table[k];
-      if (v != 0.f) atomicAdd(&dtable[k], v);
+  __syncthreads();
+  for (int i = threadIdx.x; i < V * (EMB_SLICE / 4); i += blockDim.x) {
+    const int v = i / (EMB_SLICE / 4), ch = blockIdx.x * EMB_SLICE + (i % (EMB_SLICE / 4)) * 4;
+    if (ch >= C) continue;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int w = 0; w < warps; ++w) {
+      const float4 t = *reinterpret_cast<const float4*>(emb_tables + w * table + i * 4);
+      s.x += t.x;
+      s.y += t.y;
+      s.z += t.z;
+      s.w += t.w;
     }
+    if (s.x != 0.f || s.y != 0.f || s.z != 0.f || s.w != 0.f)
+      atomicAdd(reinterpret_cast<float4*>(sums + static_cast<size_t>(v) * C + ch), s);
+  }
+}
+
+// One block a token: dtable[v] += norm backward of S[v], dw += S[v] * xhat[v].
+__global__ void __launch_bounds__(256)
+embed_grad_finish_kernel(const float* __restrict__ sums, const __nv_bfloat16* __restrict__ table,
+                         const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
+                         const float* __restrict__ rstd_in, float* __restrict__ dtable, float* __restrict__ dw, int C,
+                         int V, int rms) {
+  grid_chain();
+  __shared__ float red[8][2];
+  const int v = blockIdx.x;
+  const int row = reinterpret_cast<const int*>(sums + static_cast<size_t>(V) * C)[v] - 1;
+  if (row < 0) return;   // the token does not occur (the whole block leaves)
+  const float mean = rms ? 0.f : mean_in[row], rstd = rstd_in[row];
+  const float* S = sums + static_cast<size_t>(v) * C;
+  const __nv_bfloat16* x = table + static_cast<size_t>(v) * C;
+  float sg = 0.f, sgx = 0.f;
+  for (int c = threadIdx.x; c < C; c += 256) {
+    const float xh = (__bfloat162float(x[c]) - mean) * rstd;
+    const float g = S[c] * (w ? __bfloat162float(w[c]) : 1.f);
+    sg += g;
+    sgx += g * xh;
+  }
+  sg = warp_sum(sg);
+  sgx = warp_sum(sgx);
+  if ((threadIdx.x & 31) == 0) {
+    red[threadIdx.x >> 5][0] = sg;
+    red[threadIdx.x >> 5][1] = sgx;
+  }
+  __syncthreads();
+  sg = sgx = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    sg += red[k][0];
+    sgx += red[k][1];
+  }
+  sg = rms ? 0.f : sg / C;
+  sgx /= C;
+  for (int c = threadIdx.x; c < C; c += 256) {
+    const float xh = (__bfloat162float(x[c]) - mean) * rstd;
+    const float g = S[c] * (w ? __bfloat162float(w[c]) : 1.f);
+    dtable[static_cast<size_t>(v) * C + c] += rstd * (g - sg - xh * sgx);
+    if (dw) atomicAdd(&dw[c], S[c] * xh);
   }
 }
 
@@ -604,151 +598,85 @@ ce_fwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
 
 // Backward: dh[row] = g * sum_v dl[row][v] W[v];  dW[v] += g * sum_rows dl[row][v] h[row];
 // dbias[v] += g * sum_rows dl[row][v].  g = *gscale (upstream gradient of the loss).
-// dW is accumulated per block in shared memory ([V][C] fp32) and flushed with atomics.
-template <int CHUNKS>
-__global__ void __launch_bounds__(CE_WARPS * 32)
+// Bound by its 2 x 32 fp32 multiply-adds an element of h. A thread owns two channels: W and the sums dW of all 32 entries
+// of the vocabulary stay in registers (128 of them, three blocks a multiprocessor), the dlogits of 16 rows are read as
+// broadcasts from shared memory, doubled for the packed multiply-adds. A block takes 256 channels of `rows` rows, so that
+// 1 300 rows already fill the chip (a block a 32-row tile left most of it idle: 89 us; 8 300 rows x 1024 224 us).
+constexpr int CE_ROWS = 16;
+
+__global__ void __launch_bounds__(128, 3)
 ce_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ W,
               const float* __restrict__ dlogits, const float* __restrict__ gscale,
               __nv_bfloat16* __restrict__ dh, float* __restrict__ dW, float* __restrict__ dbias,
-              int n, int C, int V) {
+              int n, int C, int V, int rows) {
   grid_chain();
-  extern __shared__ float sdW[];  // [V][C] fp32, then [32] dbias
-  float* sdb = sdW + V * C;
-  for (int i = threadIdx.x; i < V * C + 32; i += blockDim.x) sdW[i] = 0.f;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const float g = *gscale;
-  for (int row = blockIdx.x * CE_WARPS + (threadIdx.x >> 5); row < n; row += gridDim.x * CE_WARPS) {
-    const float dl = dlogits[static_cast<size_t>(row) * 32 + lane] * g;
-    if (__ballot_sync(0xffffffffu, dl != 0.f) == 0u) {
-      // ignored row: zero gradient
-#pragma unroll
-      for (int c = 0; c < CHUNKS; ++c) {
-        const int i = c * 256 + lane * 8;
-        if (i < C) *reinterpret_cast<uint4*>(dh + static_cast<size_t>(row) * C + i) = make_uint4(0, 0, 0, 0);
-      }
-      continue;
-    }
-    if (lane < V) atomicAdd(&sdb[lane], dl);
-    // broadcast every dlogit to every lane first: the shuffles need the whole warp, the channel
-    // loop below does not run on lanes whose channels lie beyond C
-    float dv[32];
-#pragma unroll
-    for (int v = 0; v < 32; ++v) dv[v] = __shfl_sync(0xffffffffu, dl, v);
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-      const int i = c * 256 + lane * 8;
-      if (i < C) {
-        float hv[8], o[8];
-        load8(h + static_cast<size_t>(row) * C + i, hv);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = 0.f;
-#pragma unroll
-        for (int v = 0; v < 32; ++v) {
-          if (v < V) {
-            const float d = dv[v];
-            float wv[8];
-            load8(W + static_cast<size_t>(v) * C + i, wv);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              o[e] += d * wv[e];
-              atomicAdd(&sdW[v * C + i + e], d * hv[e]);
-            }
-          }
-        }
-        store8(dh + static_cast<size_t>(row) * C + i, o);
-      }
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < V * C; i += blockDim.x) {
-    const float v = sdW[i];
-    if (v != 0.f) atomicAdd(&dW[i], v);
-  }
-  if (dbias && threadIdx.x < V) atomicAdd(&dbias[threadIdx.x], sdb[threadIdx.x]);
-}
-
-// Same backward for C <= 1024 (C % 4 == 0) as a tiled product: a block stages 32 rows of h (bf16)
-// and their dlogits in shared memory next to W; thread t owns channels 4t .. 4t+3 and keeps
-// dW[v][4t..4t+3] for all v in registers (4 V accumulators), so a row costs 8 V FMAs per thread and
-// no atomics; the block's dW is flushed once at the end.
-constexpr int CE_TILE_ROWS = 32;
-
-__global__ void __launch_bounds__(256)
-ce_bwd_tiled_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ W,
-                    const float* __restrict__ dlogits, const float* __restrict__ gscale,
-                    __nv_bfloat16* __restrict__ dh, float* __restrict__ dW, float* __restrict__ dbias,
-                    int n, int C, int V) {
-  grid_chain();
-  extern __shared__ __align__(16) uint8_t ce_smem[];
-  __nv_bfloat16* sW = reinterpret_cast<__nv_bfloat16*>(ce_smem);            // [V][C]
-  __nv_bfloat16* sH = sW + static_cast<size_t>(V) * C;                       // [32][C]
-  float* sD = reinterpret_cast<float*>(sH + static_cast<size_t>(CE_TILE_ROWS) * C);  // [32][32]
-  const int t = threadIdx.x;
-  for (int i = t * 8; i < V * C; i += 256 * 8)
-    *reinterpret_cast<uint4*>(sW + i) = *reinterpret_cast<const uint4*>(W + i);
-  const float g = *gscale;
-  const int ch = t * 4;
+  __shared__ __align__(16) float2 sd[CE_ROWS][32];
+  const int tid = threadIdx.x;
+  const int ch = blockIdx.x * 256 + tid * 2;
   const bool own = ch < C;
-  float acc[32][4];
+  const int r1 = min(n, (static_cast<int>(blockIdx.y) + 1) * rows);
+  const float g = *gscale;
+  float2 w[32], acc[32];
 #pragma unroll
-  for (int v = 0; v < 32; ++v)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[v][e] = 0.f;
+  for (int v = 0; v < 32; ++v) {
+    w[v] = own && v < V ? unpack_bf16x2(__ldg(reinterpret_cast<const uint32_t*>(W + static_cast<size_t>(v) * C + ch)))
+                        : make_float2(0.f, 0.f);
+    acc[v] = make_float2(0.f, 0.f);
+  }
   float db = 0.f;
-  const int tiles = (n + CE_TILE_ROWS - 1) / CE_TILE_ROWS;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int r0 = tile * CE_TILE_ROWS;
-    __syncthreads();   // previous tile fully consumed (and sW written, first time round)
-    for (int i = t * 8; i < CE_TILE_ROWS * C; i += 256 * 8) {
-      const int r = i / C;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (r0 + r < n) val = *reinterpret_cast<const uint4*>(h + static_cast<size_t>(r0) * C + i);
-      *reinterpret_cast<uint4*>(sH + i) = val;
-    }
-    for (int i = t; i < CE_TILE_ROWS * 32; i += 256) {
-      const int r = i >> 5;
-      sD[i] = (r0 + r < n) ? dlogits[static_cast<size_t>(r0) * 32 + i] * g : 0.f;
+  for (int base = blockIdx.y * rows; base < r1; base += CE_ROWS) {
+    __syncthreads();   // the previous rows are consumed
+#pragma unroll
+    for (int i = tid; i < CE_ROWS * 32; i += 128) {
+      const int r = base + (i >> 5);
+      const float d = r < r1 ? dlogits[static_cast<size_t>(r) * 32 + (i & 31)] * g : 0.f;
+      sd[i >> 5][i & 31] = make_float2(d, d);
     }
     __syncthreads();
-    if (t < V) {
-#pragma unroll 8
-      for (int r = 0; r < CE_TILE_ROWS; ++r) db += sD[r * 32 + t];
-    }
-    if (own) {
-      const int rows = min(CE_TILE_ROWS, n - r0);
-      for (int r = 0; r < rows; ++r) {
-        const uint2 hp = *reinterpret_cast<const uint2*>(sH + static_cast<size_t>(r) * C + ch);
-        const float2 h01 = unpack_bf16x2(hp.x), h23 = unpack_bf16x2(hp.y);
-        float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+    if (blockIdx.x == 0 && tid < 32) {
 #pragma unroll
-        for (int v = 0; v < 32; ++v) {
-          if (v < V) {
-            const float d = sD[r * 32 + v];
-            const uint2 wp = *reinterpret_cast<const uint2*>(sW + static_cast<size_t>(v) * C + ch);
-            const float2 w01 = unpack_bf16x2(wp.x), w23 = unpack_bf16x2(wp.y);
-            o0 += d * w01.x; o1 += d * w01.y; o2 += d * w23.x; o3 += d * w23.y;
-            acc[v][0] += d * h01.x; acc[v][1] += d * h01.y; acc[v][2] += d * h23.x; acc[v][3] += d * h23.y;
-          }
+      for (int r = 0; r < CE_ROWS; ++r) db += sd[r][tid].x;
+    }
+#pragma unroll 1
+    for (int r = 0; r < CE_ROWS && base + r < r1; r += 4) {
+      float2 hv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        hv[q] = own && base + r + q < r1
+                    ? unpack_bf16x2(__ldg(reinterpret_cast<const uint32_t*>(h + static_cast<size_t>(base + r + q) * C + ch)))
+                    : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float2 o0 = make_float2(0.f, 0.f), o1 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int v = 0; v < 32; v += 2) {
+          const float4 d = *reinterpret_cast<const float4*>(&sd[r + q][v]);
+          const float2 d0 = make_float2(d.x, d.y), d1 = make_float2(d.z, d.w);
+          o0 = fma2(d0, w[v], o0);
+          o1 = fma2(d1, w[v + 1], o1);
+          acc[v] = fma2(d0, hv[q], acc[v]);
+          acc[v + 1] = fma2(d1, hv[q], acc[v + 1]);
         }
-        uint2 op;
-        op.x = pack_bf16x2(o0, o1);
-        op.y = pack_bf16x2(o2, o3);
-        *reinterpret_cast<uint2*>(dh + static_cast<size_t>(r0 + r) * C + ch) = op;
+        o0 = add2(o0, o1);
+        if (own && base + r + q < r1)
+          *reinterpret_cast<uint32_t*>(dh + static_cast<size_t>(base + r + q) * C + ch) = pack_bf16x2(o0.x, o0.y);
       }
     }
   }
   if (own) {
 #pragma unroll
-    for (int v = 0; v < 32; ++v) {
-      if (v < V) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (acc[v][e] != 0.f) atomicAdd(&dW[static_cast<size_t>(v) * C + ch + e], acc[v][e]);
+    for (int v = 0; v < 32; ++v)
+      if (v < V && (acc[v].x != 0.f || acc[v].y != 0.f)) {
+        float* dst = dW + static_cast<size_t>(v) * C + ch;
+        if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+          atomicAdd(reinterpret_cast<float2*>(dst), acc[v]);
+        } else {
+          atomicAdd(dst, acc[v].x);
+          atomicAdd(dst + 1, acc[v].y);
+        }
       }
-    }
   }
-  if (dbias && t < V && db != 0.f) atomicAdd(&dbias[t], db);
+  if (dbias && blockIdx.x == 0 && tid < V && db != 0.f) atomicAdd(&dbias[tid], db);
 }
 
 // ------------------------------------------------------------------ optimizer
@@ -1023,35 +951,6 @@ extern "C" int nplm_norm_bwd(const void* dy, const void* x, const int* ids, cons
                              float* dw, float* dtable, int T, int C, int V, int rms, cudaStream_t st) {
   if (T <= 0) return 0;
   if (C % 8) return -3;
-  if (C >= 256 && C <= 2048 && ids != nullptr && dtable != nullptr && V > 0) {
-    // embedding gradient: row-group kernel, per-vocabulary-entry sums in shared memory
-    // (C/8 threads, rounded up to whole warps)
-    // the table sums fill the SM's shared memory (one block per SM), so the block itself keeps
-    // ROWS * SUB rows in flight: 4 groups of C/8 threads up to C = 1024, 2 beyond (512 threads)
-    constexpr int ROWS = 4;
-    const int sub = C <= 1024 ? 4 : 2;
-    const int threads = ((C / 8) + 31) / 32 * 32 * sub;
-    const size_t smem = static_cast<size_t>(V) * C * sizeof(float);
-    if (smem <= 200 * 1024) {
-      const int groups = (T + ROWS * sub - 1) / (ROWS * sub);
-      int blocks = 148;
-      if (blocks > groups) blocks = groups;
-#define CALL_ROWS(SUB_)                                                                                   \
-  do {                                                                                                    \
-    if (smem > 48 * 1024)                                                                                 \
-      cudaFuncSetAttribute(norm_bwd_rows_kernel<ROWS, SUB_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                           static_cast<int>(smem));                                                       \
-    launch_chained(norm_bwd_rows_kernel<ROWS, SUB_>, blocks, threads, smem, st,                                       \
-        reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x), ids,       \
-        reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd, reinterpret_cast<const __nv_bfloat16*>(dres), \
-        reinterpret_cast<__nv_bfloat16*>(dx), dw, dtable, T, C, V, rms);                                  \
-  } while (0)
-      if (sub == 4) CALL_ROWS(4);
-      else CALL_ROWS(2);
-#undef CALL_ROWS
-      return static_cast<int>(cudaGetLastError());
-    }
-  }
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 2) blocks = 148 * 2;   // more blocks only add contention on the dw atomics
 #define CALL(N_)                                                                              \
@@ -1062,6 +961,39 @@ extern "C" int nplm_norm_bwd(const void* dy, const void* x, const int* ids, cons
       dtable, T, C, rms)
   NPLM_CHUNK_DISPATCH(C, CALL);
 #undef CALL
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Embedding + norm backward (x = table[ids]): dtable (fp32 [V][C]) and dw (fp32 [C], may be null) are added to. scratch: fp32
+// [V * (C + 1)], cleared here. A block keeps one table of 512 V bytes a warp in shared memory, so up to V = 200 at least
+// two warps fit; larger vocabularies return -3 (nplm_norm_bwd with ids takes them).
+extern "C" int nplm_embed_bwd(const void* dy, const void* table, const int* ids, const void* w, const float* mean,
+                              const float* rstd, float* dw, float* dtable, float* scratch, int T, int C, int V, int rms,
+                              cudaStream_t st) {
+  if (T <= 0) return 0;
+  if ((C % 8) || V < 1 || V > 200 || (reinterpret_cast<uintptr_t>(dy) & 7) || (reinterpret_cast<uintptr_t>(scratch) & 15))
+    return -3;
+  const int table_bytes = V * EMB_SLICE * 4;
+  int warps = 200 * 1024 / table_bytes;
+  if (warps > 12) warps = 12;
+  const int slices = (C + EMB_SLICE - 1) / EMB_SLICE;
+  // one block a multiprocessor; with few tokens fewer blocks, so that a warp has at least one full set of loads
+  int by = 148 / slices;
+  if (by < 1) by = 1;
+  const int full = (T + warps * EMB_ROWS - 1) / (warps * EMB_ROWS);
+  if (by > full) by = full;
+  NPLM_CUDA_CHECK(cudaMemsetAsync(scratch, 0, static_cast<size_t>(V) * (C + 1) * sizeof(float), st));
+  static bool configured_on[nplm::MAX_DEVICES];
+  const int dev_slot = nplm::current_device_slot();
+  if (dev_slot < 0) return -4;
+  if (!configured_on[dev_slot]) {
+    NPLM_CUDA_CHECK(cudaFuncSetAttribute(embed_grad_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    configured_on[dev_slot] = true;
+  }
+  launch_chained(embed_grad_sums_kernel, dim3(slices, by), 32 * warps, static_cast<size_t>(warps) * table_bytes, st,
+                 reinterpret_cast<const __nv_bfloat16*>(dy), ids, scratch, T, C, V);
+  launch_chained(embed_grad_finish_kernel, V, 256, 0, st, scratch, reinterpret_cast<const __nv_bfloat16*>(table),
+                 reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd, dtable, dw, C, V, rms);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1253,38 +1185,17 @@ extern "C" int nplm_ce_bwd(const void* h, const void* W, const float* dlogits, c
                            cudaStream_t st) {
   if (n <= 0) return 0;
   if (V > 32 || V < 1 || (C % 8)) return -3;
-  if (C <= 1024) {
-    const size_t tsm = (static_cast<size_t>(V) * C + static_cast<size_t>(CE_TILE_ROWS) * C) * 2 +
-                       CE_TILE_ROWS * 32 * 4;
-    static bool configured_on[nplm::MAX_DEVICES];
-    const int dev_slot = nplm::current_device_slot();
-    if (dev_slot < 0) return -4;
-    bool& configured = configured_on[dev_slot];
-    if (!configured) {
-      cudaFuncSetAttribute(ce_bwd_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      configured = true;
-    }
-    int tb = (n + CE_TILE_ROWS - 1) / CE_TILE_ROWS;
-    if (tb > 148) tb = 148;
-    launch_chained(ce_bwd_tiled_kernel, tb, 256, tsm, st,
-        reinterpret_cast<const __nv_bfloat16*>(h), reinterpret_cast<const __nv_bfloat16*>(W), dlogits, gscale,
-        reinterpret_cast<__nv_bfloat16*>(dh), dW, dbias, n, C, V);
-    return static_cast<int>(cudaGetLastError());
-  }
-  const size_t smem = (static_cast<size_t>(V) * C + 32) * 4;
-  if (smem > 220 * 1024) return -4;
-  int blocks = (n + CE_WARPS - 1) / CE_WARPS;
-  if (blocks > 148) blocks = 148;
-#define CALL(N_)                                                                              \
-  do {                                                                                        \
-    cudaFuncSetAttribute(ce_bwd_kernel<N_>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                         static_cast<int>(smem));                                             \
-    launch_chained(ce_bwd_kernel<N_>, blocks, CE_WARPS * 32, smem, st,                                    \
-        reinterpret_cast<const __nv_bfloat16*>(h), reinterpret_cast<const __nv_bfloat16*>(W), \
-        dlogits, gscale, reinterpret_cast<__nv_bfloat16*>(dh), dW, dbias, n, C, V);           \
-  } while (0)
-  NPLM_CHUNK_DISPATCH(C, CALL);
-#undef CALL
+  if ((reinterpret_cast<uintptr_t>(h) & 3) || (reinterpret_cast<uintptr_t>(W) & 3) ||
+      (reinterpret_cast<uintptr_t>(dh) & 3))
+    return -3;
+  // three blocks a multiprocessor, at least 16 rows each
+  const int slices = (C + 255) / 256;
+  int by = (148 * 3 + slices - 1) / slices;
+  int rows = ((n + by - 1) / by + CE_ROWS - 1) / CE_ROWS * CE_ROWS;
+  by = (n + rows - 1) / rows;
+  launch_chained(ce_bwd_kernel, dim3(slices, by), 128, 0, st, reinterpret_cast<const __nv_bfloat16*>(h),
+                 reinterpret_cast<const __nv_bfloat16*>(W), dlogits, gscale, reinterpret_cast<__nv_bfloat16*>(dh), dW,
+                 dbias, n, C, V, rows);
   return static_cast<int>(cudaGetLastError());
 }
 

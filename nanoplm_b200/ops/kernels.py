@@ -308,6 +308,14 @@ def rope_(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: torch.Te
 
 
 def swiglu_fwd(pre: torch.Tensor) -> torch.Tensor:
+    if ids is not None and dtable is not None and V <= 200:
+        scratch = torch.empty(V * (C + 1), dtype=torch.float32, device=dy.device)
+        rc = typed("elementwise", "nplm_embed_bwd", "ppppppppp" + "iiiip")(
+            dy2.data_ptr(), x.data_ptr(), ids.data_ptr(), _dp(w), _dp(mean), rstd.data_ptr(), _dp(dw), dtable.data_ptr(),
+            scratch.data_ptr(), T, C, V, rms, raw_stream())
+        check_rc(rc, "embed_bwd")
+        count_launch(2)
+        return None
     T, two_i = pre.shape
     out = torch.empty((T, two_i // 2), dtype=_BF16, device=pre.device)
     rc = lib("elementwise").nplm_swiglu_fwd(ptr(pre), ptr(out), c_longlong(T), c_int(two_i // 2),
