@@ -20,6 +20,7 @@ enum : int {
                        // first column is < rope_cols (the q and k parts of a fused QKV projection)
   EPI_STORE_DELTA = 9, // C(bf16) = acc, and delta[col / 64][row] = sum over each 64-column head of
                        // bf16(acc) * R (the attention backward's rowsum(dO * O), R = O)
+  EPI_AXPBY = 10,      // C(bf16) = alpha * acc + beta * R(bf16, may be null); stacks of equal problems only
   EPI_SWIGLU_BWD = 8,  // acc = gradient of the SwiGLU output h = silu(gate) * value, N wide;
                        // R = the pre-activations [value | gate] (bf16, 2N wide); C (bf16, 2N wide) =
                        // [acc * silu(gate) | acc * value * silu'(gate)], the gradient of R

@@ -33,7 +33,7 @@ constexpr int UMMA_K = 16;
 // 264 -> 275).
 template <bool PAIR, bool STAGED, int EPI>
 constexpr int EPI_WARPS_OF =
-    (PAIR && STAGED && (EPI == EPI_ROPE || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD)) ? 8 : 4;
+    (PAIR && STAGED && (EPI == EPI_ROPE || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD || EPI == EPI_AXPBY)) ? 8 : 4;
 
 // STAGED: the epilogue goes through shared memory (TMA stores and reduce-adds); the direct epilogue, and fp32 outputs of
 // groups whose rows are no multiple of 32, write straight from registers and spend that room on pipeline stages.
@@ -73,8 +73,13 @@ struct GemmArgs {
   //   group_mode 2: weight gradients. A and B are MN-major over a common row axis; group g
   //                 contracts rows [group_off[g], group_off[g+1]) (multiples of 128) and adds the
   //                 M x N result into C + g * c_group_stride.
+  //   group_mode 3: a stack of equal problems (CTA pairs): rows of A / C in groups of group_rows (a multiple of 256). sym: the
+  //                 products are symmetric (N = group_rows); 256 x 256 tiles right of the diagonal are not visited, their
+  //                 values are stored by the tile across it.
   int group_mode;
   int groups;
+  int group_rows, sym;
+  float alpha, beta;   // EPI_AXPBY
   const int* tile_group;
   // group_mode 1, optional: rows of A arrive from other GPUs. The producer loads the rows of tile t only
   // after row_arrive[t] (bumped once per landed row, system scope) has reached row_expect[t].
@@ -196,14 +201,34 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const long long sk_hi = sk_units * (work_first + 1) / work_stride;
   const int w_begin = stream_k ? 0 : work_first;
   const int w_step = stream_k ? 1 : work_stride;
+  // group_mode 3: tiles of one problem of the stack
+  const int stack_m = args.group_rows / MT;
+  const int stack_tiles = args.sym ? stack_m * (stack_m + 1) / 2 : stack_m * num_n;
   const int total_work = stream_k ? static_cast<int>((sk_hi + num_kb - 1) / num_kb - sk_lo / num_kb)
-                                  : (args.group_mode == 2 ? args.groups : splits) * num_m * num_n;
+                         : EPI == EPI_AXPBY ? args.groups * stack_tiles
+                                            : (args.group_mode == 2 ? args.groups : splits) * num_m * num_n;
 
   // work item -> tile coordinates and contraction range; false = nothing to do for this item
   auto decode = [&](int w, WorkItem& it) -> bool {
     it.b_row = 0;
     it.c_off = 0;
     it.c_row = 0;
+    if constexpr (EPI == EPI_AXPBY) {
+      const int g = w / stack_tiles;
+      int tile = w % stack_tiles, i;
+      if (args.sym) {
+        for (i = 0; tile > i; ++i) tile -= i + 1;   // row i of the lower triangle has i + 1 tiles
+      } else {
+        i = tile / num_n;
+        tile -= i * num_n;
+      }
+      it.m0 = g * args.group_rows + i * MT + static_cast<int>(rank) * BM;
+      it.n0 = tile * TILE_N;
+      it.kb0 = 0;
+      it.kb1 = num_kb;
+      it.b_row = g * args.b_group_rows;
+      return true;
+    }
     if (args.group_mode == 2) {
       const int per = num_m * num_n;
       const int g = w / per, tile = w % per;
@@ -379,12 +404,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               tma_load_2d_pair(sb, &tmB, &full_bar[stage], k0,
                                (rank == 0 ? 0 : args.swiglu_half) + n0);
             } else if constexpr (!B_MN) {
-              tma_load_2d_pair(sb, &tmB, &full_bar[stage], k0, n0 + static_cast<int>(rank) * (BN / 2));
+              tma_load_2d_pair(sb, &tmB, &full_bar[stage], k0, brow + n0 + static_cast<int>(rank) * (BN / 2));
             } else {
 #pragma unroll
               for (int g = 0; g < BN / 128; ++g)
                 tma_load_2d_pair(sb + g * (BK * 128), &tmB, &full_bar[stage],
-                                 n0 + (static_cast<int>(rank) * (BN / 128) + g) * 64, k0);
+                                 n0 + (static_cast<int>(rank) * (BN / 128) + g) * 64, brow + k0);
             }
           } else {
           mbar_arrive_expect_tx(&full_bar[stage], S::STAGE_BYTES);
@@ -532,10 +557,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       WorkItem it;
       if (!decode(w, it)) continue;
       const int m0 = it.m0, n0 = it.n0;
-      if constexpr (TMA_EPI && (EPI == EPI_ADD || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD)) {
+      if constexpr (TMA_EPI && (EPI == EPI_ADD || EPI == EPI_STORE_DELTA || EPI == EPI_SWIGLU_BWD || EPI == EPI_AXPBY)) {
         // the second operand does not depend on the product: its first tiles travel while the MMAs run
         const int y0 = m0 + quarter * 32, x0 = n0 + c0 * 64;
-        if (y0 < M && x0 < N) {
+        if (y0 < M && x0 < N && (EPI != EPI_AXPBY || args.R != nullptr)) {
           operand_load(0, x0, y0);
           if constexpr (EPI == EPI_SWIGLU_BWD) operand_load(1, N + x0, y0);
           else if (NCHW > 1 && x0 + 64 < N) operand_load(1, x0 + 64, y0);
@@ -782,6 +807,47 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
                 stage_store_inplace(rb, &tmC, packed, x, y0, lane);
                 if (c + 2 < c1 && chunk_in(c + 2)) operand_load(buf, x + 128, y0);
+              }
+            } else if constexpr (EPI == EPI_AXPBY) {
+              if (active) {
+                const int buf = (c - c0) & 1;
+                uint8_t* rb = stage + buf * 4096;
+                if (args.R != nullptr) {
+                  if (!operand_wait(buf)) {
+                    if (lane == 0) atomicExch(args.status, ST_TIMEOUT_MISC);
+                  }
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) {
+                    const uint4 rv = *reinterpret_cast<const uint4*>(rb + lane * 128 + ((j ^ (lane & 7)) << 4));
+                    const uint32_t* rr = reinterpret_cast<const uint32_t*>(&rv);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                      const float2 t = unpack_bf16x2(rr[e]);
+                      packed[j * 4 + e] = pack_bf16x2(args.alpha * f[j * 8 + 2 * e] + args.beta * t.x,
+                                                      args.alpha * f[j * 8 + 2 * e + 1] + args.beta * t.y);
+                    }
+                  }
+                } else {
+#pragma unroll
+                  for (int e = 0; e < 32; ++e) packed[e] = pack_bf16x2(args.alpha * f[2 * e], args.alpha * f[2 * e + 1]);
+                  if (elect_one()) tma_store_wait_read<1>();   // the store that read this buffer two chunks ago
+                }
+                stage_store_inplace(rb, &tmC, packed, x, y0, lane);
+                if (args.R != nullptr && c + 2 < c1 && chunk_in(c + 2)) operand_load(buf, x + 128, y0);
+                const int m_tile = m0 - static_cast<int>(rank) * BM;
+                if (args.sym && it.b_row + n0 < m_tile) {
+                  // the tile across the diagonal: column x + e of this row is row x + e there. Lanes 2i and 2i + 1 exchange
+                  // halves, so that a lane stores two rows' values of one column (two columns, 64 bytes each, a store)
+                  __nv_bfloat16* Ct = reinterpret_cast<__nv_bfloat16*>(args.C) +
+                                      static_cast<size_t>(it.b_row + x + (lane & 1)) * args.ldc + (y0 - it.b_row) + (lane & ~1);
+#pragma unroll
+                  for (int e = 0; e < 32; ++e) {
+                    const uint32_t other = __shfl_xor_sync(0xffffffffu, packed[e], 1);
+                    const uint32_t v = (lane & 1) ? __byte_perm(other, packed[e], 0x7632)
+                                                  : __byte_perm(packed[e], other, 0x5410);
+                    *reinterpret_cast<uint32_t*>(Ct + static_cast<size_t>(2 * e) * args.ldc) = v;
+                  }
+                }
               }
             } else if constexpr (EPI == EPI_GELU || EPI == EPI_RELU) {
               if (active) {
@@ -1066,8 +1132,11 @@ static int launch_pair_impl(const GemmMaps& maps, const GemmArgs& args, cudaStre
   const int n_extent = (EPI == EPI_SWIGLU) ? args.swiglu_half : args.N;
   const int num_m = (args.M + 2 * BM - 1) / (2 * BM);
   const int num_n = (n_extent + TILE_N - 1) / TILE_N;
-  const long long total = static_cast<long long>(num_m) * num_n *
-                          (args.splits == 0 ? (args.K + BK - 1) / BK : args.splits);
+  const int stack_m = args.group_rows / (2 * BM);
+  const long long total = EPI == EPI_AXPBY
+                              ? static_cast<long long>(args.groups) * stack_m * (args.sym ? stack_m + 1 : 2 * num_n) / 2
+                              : static_cast<long long>(num_m) * num_n *
+                                    (args.splits == 0 ? (args.K + BK - 1) / BK : args.splits);
   int pairs = num_sms() / 2;
   if (pairs > total) pairs = static_cast<int>(total);
   if (pairs <= 0) return 0;
@@ -1090,7 +1159,7 @@ static int launch_pair_impl(const GemmMaps& maps, const GemmArgs& args, cudaStre
 
 template <bool A_MN, bool B_MN, int EPI>
 static int launch_pair(const GemmMaps& maps, const GemmArgs& args, cudaStream_t stream) {
-  if constexpr (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD || EPI == EPI_STORE_DELTA) {
+  if constexpr (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD || EPI == EPI_STORE_DELTA || EPI == EPI_AXPBY) {
     return launch_pair_impl<A_MN, B_MN, EPI, true>(maps, args, stream);
   } else {
     if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_GELU || EPI == EPI_RELU || EPI == EPI_SWIGLU ||
@@ -1138,6 +1207,9 @@ struct GroupSpec {
   void* const* ag_ptrs = nullptr;  // every rank's full B buffer (this rank's one is B itself)
   unsigned* ag_flags = nullptr;
   float* delta = nullptr;          // EPI_STORE_DELTA side output
+  // mode 3 (EPI_AXPBY): a stack of `groups` problems of group_rows rows
+  int group_rows = 0, sym = 0;
+  float alpha = 1.f, beta = 0.f;
 };
 
 static int gemm_entry(const void* A, const void* B, void* C, const void* R, int M, int N,
@@ -1170,16 +1242,22 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   if (epi == EPI_SWIGLU_BWD && (a_mn || direct_epilogue || R == nullptr || (N % 64) || (ldr % 8) || (ldc % 8) ||
                                 (reinterpret_cast<uintptr_t>(R) & 15) || grp.mode != 0 || grp.ag_world > 1))
     return -7;
+  if ((epi == EPI_AXPBY) != (grp.mode == 3)) return -9;
+  if (grp.mode == 3 && (a_mn || direct_epilogue || !grp.pair || bn != 256 || max_ctas != 0 || grp.groups < 1 ||
+                        grp.group_rows < 1 || (grp.group_rows % 256) || (K % BK) || (N % 64) || (ldc % 8) || (ldr % 8) ||
+                        (reinterpret_cast<uintptr_t>(R) & 15) || (grp.sym && (N != grp.group_rows || grp.b_group_rows != grp.group_rows)) || grp.ag_world > 1))
+    return -9;
   const int num_kb = (K + BK - 1) / BK;
   if (splits < 0) splits = 1;
   if (splits > num_kb) splits = num_kb;
   if (epi != EPI_ATOMIC_F32 || grp.mode != 0) splits = 1;   // splits == 0 (stream-K) adds atomically too
   if (splits == 0 && grp.ag_world > 1) splits = 1;
   // outer (row) extent of the B tensor map: all groups' operands stacked
-  const uint64_t b_rows_kmajor = grp.mode == 1 ? static_cast<uint64_t>(grp.b_group_rows) * grp.groups : N;
-  const uint64_t b_rows_mnmajor = grp.mode == 1 ? static_cast<uint64_t>(grp.b_group_rows) * grp.groups : K;
+  const bool stacked = grp.mode == 1 || grp.mode == 3;
+  const uint64_t b_rows_kmajor = stacked ? static_cast<uint64_t>(grp.b_group_rows) * grp.groups : N;
+  const uint64_t b_rows_mnmajor = stacked ? static_cast<uint64_t>(grp.b_group_rows) * grp.groups : K;
 
-  const bool pair = grp.pair && bn == 256 && grp.mode == 0 && grp.ag_world <= 1 && max_ctas == 0 &&
+  const bool pair = grp.pair && bn == 256 && (grp.mode == 0 || grp.mode == 3) && grp.ag_world <= 1 && max_ctas == 0 &&
                     !(a_mn && !b_mn);
   GemmMaps maps;
   CUtensorMap& tmA = maps.A;
@@ -1204,7 +1282,7 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   const bool f32_tma = f32_out && (grp.mode != 2 || (M % 32 == 0 && grp.c_group_stride == static_cast<long long>(M) * ldc));
   maps.tma_epi = !direct_epilogue &&
                  (f32_tma || epi == EPI_STORE || epi == EPI_ADD || epi == EPI_GELU || epi == EPI_RELU || epi == EPI_SWIGLU ||
-                  epi == EPI_ROPE || epi == EPI_SWIGLU_BWD || epi == EPI_STORE_DELTA) &&
+                  epi == EPI_ROPE || epi == EPI_SWIGLU_BWD || epi == EPI_STORE_DELTA || epi == EPI_AXPBY) &&
                  !(epi == EPI_ADD && (R == nullptr || (reinterpret_cast<uintptr_t>(R) & 15) || (ldr % 8)));
   maps.C = tmA;
   maps.R = tmA;
@@ -1240,6 +1318,10 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   args.rope_cols = rope_cols;
   args.group_mode = grp.mode;
   args.groups = grp.groups;
+  args.group_rows = grp.group_rows;
+  args.sym = grp.sym;
+  args.alpha = grp.alpha;
+  args.beta = grp.beta;
   args.tile_group = grp.tile_group;
   args.row_arrive = grp.row_arrive;
   args.row_expect = grp.row_expect;
@@ -1301,6 +1383,9 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
     if (epi == EPI_STORE_DELTA)
       return b_mn ? launch_pair<false, true, EPI_STORE_DELTA>(maps, args, stream)
                   : launch_pair<false, false, EPI_STORE_DELTA>(maps, args, stream);
+    if (epi == EPI_AXPBY)
+      return b_mn ? launch_pair<false, true, EPI_AXPBY>(maps, args, stream)
+                  : launch_pair<false, false, EPI_AXPBY>(maps, args, stream);
     if (epi == EPI_SWIGLU_BWD)
       return b_mn ? launch_pair<false, true, EPI_SWIGLU_BWD>(maps, args, stream)
                   : launch_pair<false, false, EPI_SWIGLU_BWD>(maps, args, stream);
@@ -1309,6 +1394,24 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
     else { NPLM_DISPATCH_PAIR(true, true) }
 #undef NPLM_DISPATCH_PAIR
     return -8;
+  }
+  if (bn == 64) {   // bf16 outputs of plain GEMMs with few rows (gemm_tile_width)
+    if (a_mn || grp.mode != 0 || grp.ag_world > 1) return -6;
+    if (!b_mn) {
+      switch (epi) {
+        case EPI_STORE: return launch<64, false, false, EPI_STORE>(maps, args, max_ctas, stream);
+        case EPI_ADD: return launch<64, false, false, EPI_ADD>(maps, args, max_ctas, stream);
+        case EPI_GELU: return launch<64, false, false, EPI_GELU>(maps, args, max_ctas, stream);
+        case EPI_RELU: return launch<64, false, false, EPI_RELU>(maps, args, max_ctas, stream);
+        case EPI_ROPE: return launch<64, false, false, EPI_ROPE>(maps, args, max_ctas, stream);
+        default: return -6;
+      }
+    }
+    switch (epi) {
+      case EPI_STORE: return launch<64, false, true, EPI_STORE>(maps, args, max_ctas, stream);
+      case EPI_ADD: return launch<64, false, true, EPI_ADD>(maps, args, max_ctas, stream);
+      default: return -6;
+    }
   }
   if (epi == EPI_GELU) {
     if (a_mn || b_mn) return -7;
@@ -1383,6 +1486,31 @@ extern "C" int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const
                     nullptr, nullptr, 0, status, stream, g);
 }
 
+// A stack of `groups` equal products on CTA pairs: C_g = alpha A_g B_g^T + beta R_g (b_mn = 0, B_g [N][K]) or alpha A_g B_g + beta
+// R_g (b_mn = 1, B_g [K][N]), all bf16 with fp32 accumulation and one rounding; A_g, C_g and R_g (may be null) are rows [g *
+// rows, (g + 1) * rows) of their matrices. rows a multiple of 256, K and N of 64. sym: every C_g is symmetric and square
+// (the caller's promise: A = B, or commuting symmetric operands), so only the tiles on and below the diagonal
+// are computed: 160 tiles of 256 x 256 for 16 matrices of 1024 x 1024 instead of 256. The symmetric products (K 1024 to
+// 4096) of a Newton-Schulz step over 64 matrices take 39.6 us a launch on average, 51 as full products on single CTAs;
+// the others 65, with the sum that they end in, 78 without. Bound by the tensor pipe and by the waves of 74 pairs (2.2 of
+// them round up to 3).
+extern "C" int nplm_gemm_bf16_stack(const void* A, const void* B, void* C, const void* R, int groups, int rows, int N, int K,
+                                    int lda, int ldb, int ldc, int ldr, int b_mn, float alpha, float beta, int sym,
+                                    int* status, cudaStream_t stream) {
+  if (groups < 1 || rows < 1) return -9;
+  GroupSpec g;
+  g.mode = 3;
+  g.pair = true;
+  g.groups = groups;
+  g.group_rows = rows;
+  g.b_group_rows = b_mn ? K : N;
+  g.sym = sym;
+  g.alpha = alpha;
+  g.beta = beta;
+  return gemm_entry(A, B, C, R, groups * rows, N, K, lda, ldb, ldc, ldr, 0, b_mn, EPI_AXPBY, 1, 256, 0, 0, nullptr,
+                    nullptr, nullptr, 0, status, stream, g);
+}
+
 // Grouped GEMM over row groups (mixture-of-experts forward and data gradient).
 //   A [M][K] (rows of all groups, every group padded to whole 128-row tiles), C [M][N] likewise;
 //   B holds `groups` operands stacked along its row axis, b_group_rows apart (N rows per group
@@ -1395,24 +1523,6 @@ extern "C" int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const
 extern "C" int nplm_gemm_bf16_grouped_gated(const void* A, const void* B, void* C, const void* R, int M,
                                             int N, int K, int lda, int ldb, int ldc, int ldr, int b_mn,
                                             int epi, int bn, int groups, const int* tile_group,
-  if (bn == 64) {   // bf16 outputs of plain GEMMs with few rows (gemm_tile_width)
-    if (a_mn || grp.mode != 0 || grp.ag_world > 1) return -6;
-    if (!b_mn) {
-      switch (epi) {
-        case EPI_STORE: return launch<64, false, false, EPI_STORE>(maps, args, max_ctas, stream);
-        case EPI_ADD: return launch<64, false, false, EPI_ADD>(maps, args, max_ctas, stream);
-        case EPI_GELU: return launch<64, false, false, EPI_GELU>(maps, args, max_ctas, stream);
-        case EPI_RELU: return launch<64, false, false, EPI_RELU>(maps, args, max_ctas, stream);
-        case EPI_ROPE: return launch<64, false, false, EPI_ROPE>(maps, args, max_ctas, stream);
-        default: return -6;
-      }
-    }
-    switch (epi) {
-      case EPI_STORE: return launch<64, false, true, EPI_STORE>(maps, args, max_ctas, stream);
-      case EPI_ADD: return launch<64, false, true, EPI_ADD>(maps, args, max_ctas, stream);
-      default: return -6;
-    }
-  }
                                             int b_group_rows, const unsigned* row_arrive,
                                             const int* row_expect, int* status, cudaStream_t stream) {
   if ((row_arrive == nullptr) != (row_expect == nullptr)) return -3;

@@ -217,6 +217,29 @@ def gemm_ag(a: torch.Tensor, b_full: torch.Tensor, b_ptrs, rank: int, world: int
     return out
 
 
+def gemm_stack(a: torch.Tensor, b: torch.Tensor, *, b_mn: bool = False, alpha: float = 1.0, r: torch.Tensor | None = None,
+               beta: float = 0.0, symmetric: bool = False) -> torch.Tensor:
+    """alpha a_i op(b_i) + beta r_i for stacks a [B, m, k], b [B, n, k] (or [B, k, n] with b_mn), r [B, m, n], all bf16
+    and contiguous, with one rounding; m a multiple of 256, k and n of 64. symmetric: the results are symmetric (and
+    square), and only the tiles on and below the diagonal are computed."""
+    B, m, k = a.shape
+    n = b.shape[2] if b_mn else b.shape[1]
+    if tuple(b.shape) != ((B, k, n) if b_mn else (B, n, k)) or (r is not None and tuple(r.shape) != (B, m, n)):
+        raise ValueError(f"shapes do not match: {tuple(a.shape)}, {tuple(b.shape)}, {None if r is None else tuple(r.shape)}")
+    for t, name in ((a, "a"), (b, "b"), (r, "r")):
+        if t is not None:
+            _chk(t, _BF16, name)
+            if not t.is_contiguous():
+                raise ValueError(f"{name} must be contiguous")
+    out = torch.empty((B, m, n), dtype=_BF16, device=a.device)
+    rc = typed("gemm_tcgen05", "nplm_gemm_bf16_stack", "pppp" + "i" * 9 + "ffipp")(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), _dp(r), B, m, n, k, k, b.shape[2], n, n, b_mn, alpha, beta, symmetric,
+        status_word(a.device).data_ptr(), raw_stream())
+    check_rc(rc, "gemm_bf16_stack")
+    count_launch()
+    return out
+
+
 def wgrad_splits(n_out: int, k_in: int, tokens: int, bn: int = 256, sms: int = 148) -> int:
     """Split-K factor for a weight-gradient GEMM [n_out, k_in] reduced over `tokens`.
 
@@ -285,6 +308,14 @@ def norm_bwd(dy, x, w, mean, rstd, *, rms=False, dres=None, dw=None, ids=None, d
         dy2 = dy2.contiguous()
     dx = None if ids is not None else torch.empty((T, C), dtype=_BF16, device=dy.device)
     V = x.shape[0] if ids is not None else 0
+    if ids is not None and dtable is not None and V <= 200:
+        scratch = torch.empty(V * (C + 1), dtype=torch.float32, device=dy.device)
+        rc = typed("elementwise", "nplm_embed_bwd", "ppppppppp" + "iiiip")(
+            dy2.data_ptr(), x.data_ptr(), ids.data_ptr(), _dp(w), _dp(mean), rstd.data_ptr(), _dp(dw), dtable.data_ptr(),
+            scratch.data_ptr(), T, C, V, rms, raw_stream())
+        check_rc(rc, "embed_bwd")
+        count_launch(2)
+        return None
     rc = typed("elementwise", "nplm_norm_bwd", "pppppppppp" + "iiiip")(
         dy2.data_ptr(), x.data_ptr(), _dp(ids), _dp(w), _dp(mean), _dp(rstd), _dp(dres), _dp(dx), _dp(dw),
         _dp(dtable), T, C, V, rms, raw_stream())
@@ -308,14 +339,6 @@ def rope_(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: torch.Te
 
 
 def swiglu_fwd(pre: torch.Tensor) -> torch.Tensor:
-    if ids is not None and dtable is not None and V <= 200:
-        scratch = torch.empty(V * (C + 1), dtype=torch.float32, device=dy.device)
-        rc = typed("elementwise", "nplm_embed_bwd", "ppppppppp" + "iiiip")(
-            dy2.data_ptr(), x.data_ptr(), ids.data_ptr(), _dp(w), _dp(mean), rstd.data_ptr(), _dp(dw), dtable.data_ptr(),
-            scratch.data_ptr(), T, C, V, rms, raw_stream())
-        check_rc(rc, "embed_bwd")
-        count_launch(2)
-        return None
     T, two_i = pre.shape
     out = torch.empty((T, two_i // 2), dtype=_BF16, device=pre.device)
     rc = lib("elementwise").nplm_swiglu_fwd(ptr(pre), ptr(out), c_longlong(T), c_int(two_i // 2),

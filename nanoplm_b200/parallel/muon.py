@@ -72,6 +72,11 @@ def _grouped_ok(X: torch.Tensor) -> bool:
     return X.is_cuda and X.dtype == torch.bfloat16 and X.shape[1] % 128 == 0 and X.shape[2] % 64 == 0
 
 
+def _stack_ok(X: torch.Tensor) -> bool:
+    """Stack [B, m, n] for `kernels.gemm_stack`: whole 256-row tiles (CTA pairs)."""
+    return _grouped_ok(X) and X.shape[1] % 256 == 0 and X.is_contiguous() and X.data_ptr() % 16 == 0
+
+
 def _bmm_nt(a: torch.Tensor, b: torch.Tensor, grouped: bool) -> torch.Tensor:
     """a[i] @ b[i]^T for stacks a [B, m, k], b [B, n, k]."""
     if grouped:
@@ -96,7 +101,10 @@ def orthogonalize_batched(G: torch.Tensor, coeffs=NS_QUINTIC, eps: float = 1e-7,
     X <- aX + (bA + cA^2)X, A = X X^T (bf16 on CUDA, fp32 elsewhere). `sumsq` [B]: squared
     Frobenius norms of the matrices when the caller already has them.
 
-    On the grouped-GEMM path the polynomial is applied through the products only:
+    Stacks of whole 256-row tiles: an iteration is three launches, A = X X^T, B = c A A^T + b A and X = B X + a X, the
+    sums in the products' epilogues (fp32, one rounding each). A and B are symmetric, so of their 256 x 256 tiles only those
+    on and below the diagonal are computed (10 of 16 at 1024 rows).
+    Other stacks that fit the grouped GEMM apply the polynomial through the products only:
     bA + cA^2 = (cA + bI) A and aX + BX = (B + aI) X, so an iteration is three GEMM launches plus
     three small operations on the [B, m, m] Gram stack and never touches X elementwise."""
     dt = torch.bfloat16 if G.is_cuda else torch.float32
@@ -119,6 +127,13 @@ def orthogonalize_batched(G: torch.Tensor, coeffs=NS_QUINTIC, eps: float = 1e-7,
     if grouped:
         if not scaled:
             X = X.mul_(inv) if (X.data_ptr() != G.data_ptr() or sumsq is not None) else X * inv
+        if _stack_ok(X):
+            from nanoplm_b200.ops import kernels as K
+            for a, b, c in coeffs:
+                A = K.gemm_stack(X, X, symmetric=True)
+                A = K.gemm_stack(A, A, alpha=c, r=A, beta=b, symmetric=True)
+                X = K.gemm_stack(A, X, b_mn=True, r=X, beta=a)
+            coeffs = ()
         for a, b, c in coeffs:
             A = _bmm_nt(X, X, grouped)                          # X X^T, symmetric [B, m, m]
             Ac = A * c
