@@ -44,7 +44,6 @@ inline bool gemm_pair_pays(long long M, long long N, long long K, int epi) {
   if (epi == EPI_ROPE) return K >= 1024 ? tiles > 740 : K >= 768 && tiles > 2600;
   return K >= 768 ? tiles > 148 : tiles * K > (epi == EPI_SWIGLU ? 190000 : 400000);
 }
-}  // namespace nplm
 
 // Tile width (columns) of a bf16-output GEMM by default (ops/kernels.py has the same rule, and a test compares the two): the
 // narrowest tiles that one wave of 148 CTAs covers. Below a wave a GEMM takes as long as one tile, i.e. launch, first
@@ -64,6 +63,7 @@ inline int gemm_tile_width(long long M, long long N, int epi) {
   if (epi != EPI_SWIGLU && rows * ((N + 63) / 64) <= 148) return 64;
   return (N < 256 && epi != EPI_SWIGLU) || rows * ((N + 127) / 128) <= 148 ? 128 : 256;
 }
+}  // namespace nplm
 
 extern "C" {
 int nplm_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,

@@ -168,27 +168,27 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, ui
 }
 
 // ------------------------------------------------------------------ both forms of an operand in one pass
-// x bf16 [R][K] (R, K multiples of 128) -> what quant_rows_kernel and quant_tile_kernel<true, false> give, bit for
-// bit: qr [R][K] with scales sr[(k/128) * R + r], qt [K][R] with scales st[(r/128) * K + k]. Bound by memory: 2
-// bytes read and 2 written an element, against 6 for the two kernels. A warp holds 16 rows x 128 columns of
-// the tile in registers (a lane four columns, so a row is one 256-byte request): row maxima by warp reduction, column
-// maxima through shared memory; the transposed bytes cross the block in shared memory (16-byte chunks swizzled so that
-// neither side conflicts) and leave as whole 128-byte lines.
-__global__ void __launch_bounds__(256)
-quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, uint8_t* __restrict__ qr,
-                  float* __restrict__ sr, uint8_t* __restrict__ qt, float* __restrict__ st) {
-  grid_chain();
-  __shared__ __align__(16) uint8_t tile[128 * 128];
-  __shared__ float cmax[8][128];
-  const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
+// A 128 x 128 tile of a bf16 operand [R][K] (R, K multiples of 128) -> what quant_rows_kernel and
+// quant_tile_kernel<true, false> give, bit for bit: qr [R][K] with scales sr[(k/128) * R + r], qt [K][R] with scales
+// st[(r/128) * K + k]. A warp holds eight rows x 128 columns of the tile in registers (a lane four columns, so a row is one
+// 256-byte request): row maxima by warp reduction, column maxima through shared memory; the transposed bytes cross the
+// block in shared memory (16-byte chunks swizzled against bank conflicts) and leave as whole 128-byte lines. Two blocks of
+// 512 threads a multiprocessor: 55 424 x 1024 in 43 us (5.2 TB/s), SwiGLU form below 125, against 50 and 145 with 16 rows a
+// warp in two blocks of 256 (44 and 148 in three).
+constexpr int DUAL_ROWS = 8, DUAL_THREADS = 32 * 128 / DUAL_ROWS;
+
+struct DualSmem {
+  alignas(16) uint8_t tile[128 * 128];
+  float cmax[128 / DUAL_ROWS][128];
+};
+
+__device__ __forceinline__ void quant_dual_tile(const uint2 (&v)[DUAL_ROWS], DualSmem& sm, int r0, int k0, int R, int K,
+                                                uint8_t* __restrict__ qr, float* __restrict__ sr,
+                                                uint8_t* __restrict__ qt, float* __restrict__ st) {
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  uint2 v[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i)
-    v[i] = __ldg(reinterpret_cast<const uint2*>(x + static_cast<size_t>(r0 + w * 16 + i) * ldx + k0 + 4 * l));
   float cm[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < DUAL_ROWS; ++i) {
     const float2 a = unpack_bf16x2(v[i].x), b = unpack_bf16x2(v[i].y);
     const float m[4] = {fabsf(a.x), fabsf(a.y), fabsf(b.x), fabsf(b.y)};
     float rm = 0.f;
@@ -201,28 +201,28 @@ quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, ui
     rm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rm)));
     const float s = fmaxf(rm, 1e-12f) / E4M3_MAX;
     const float inv = 1.f / s;
-    *reinterpret_cast<uint32_t*>(qr + static_cast<size_t>(r0 + w * 16 + i) * K + k0 + 4 * l) =
+    *reinterpret_cast<uint32_t*>(qr + static_cast<size_t>(r0 + w * DUAL_ROWS + i) * K + k0 + 4 * l) =
         pack_e4m3x4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
-    if (l == i) sr[static_cast<size_t>(blockIdx.x) * R + r0 + w * 16 + i] = s;
+    if (l == i) sr[static_cast<size_t>(k0 >> 7) * R + r0 + w * DUAL_ROWS + i] = s;
   }
-  *reinterpret_cast<float4*>(&cmax[w][4 * l]) = make_float4(cm[0], cm[1], cm[2], cm[3]);
+  *reinterpret_cast<float4*>(&sm.cmax[w][4 * l]) = make_float4(cm[0], cm[1], cm[2], cm[3]);
   __syncthreads();
   if (threadIdx.x < 128) {
-    float m = cmax[0][threadIdx.x];
+    float m = sm.cmax[0][threadIdx.x];
 #pragma unroll
-    for (int j = 1; j < 8; ++j) m = fmaxf(m, cmax[j][threadIdx.x]);
+    for (int j = 1; j < 128 / DUAL_ROWS; ++j) m = fmaxf(m, sm.cmax[j][threadIdx.x]);
     const float s = fmaxf(m, 1e-12f) / E4M3_MAX;
-    cmax[0][threadIdx.x] = s;
-    st[static_cast<size_t>(blockIdx.y) * K + k0 + threadIdx.x] = s;
+    sm.cmax[0][threadIdx.x] = s;
+    st[static_cast<size_t>(r0 >> 7) * K + k0 + threadIdx.x] = s;
   }
   __syncthreads();
-  const float4 s4 = *reinterpret_cast<const float4*>(&cmax[0][4 * l]);
+  const float4 s4 = *reinterpret_cast<const float4*>(&sm.cmax[0][4 * l]);
   const float ss[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    uint32_t pk[4];
+    uint32_t pk[DUAL_ROWS / 4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < DUAL_ROWS / 4; ++q) {
       float f[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -231,15 +231,112 @@ quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, ui
       }
       pk[q] = pack_e4m3x4(f[0], f[1], f[2], f[3]);
     }
-    *reinterpret_cast<uint4*>(tile + (4 * l + j) * 128 + ((w ^ (l & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    uint8_t* row = sm.tile + (4 * l + j) * 128;
+    *reinterpret_cast<uint2*>(row + (((w >> 1) ^ (l & 7)) << 4) + ((w & 1) << 3)) = make_uint2(pk[0], pk[1]);
   }
   __syncthreads();
 #pragma unroll
-  for (int i = threadIdx.x; i < 128 * 8; i += 256) {
+  for (int i = threadIdx.x; i < 128 * 8; i += DUAL_THREADS) {
     const int col = i >> 3, c = i & 7;
     *reinterpret_cast<uint4*>(qt + static_cast<size_t>(k0 + col) * R + r0 + c * 16) =
-        *reinterpret_cast<const uint4*>(tile + col * 128 + ((c ^ ((col >> 2) & 7)) << 4));
+        *reinterpret_cast<const uint4*>(sm.tile + col * 128 + ((c ^ ((col >> 2) & 7)) << 4));
   }
+}
+
+// Bound by memory: 2 bytes read and 2 written an element, against 6 for the two kernels.
+__global__ void __launch_bounds__(DUAL_THREADS, 2)
+quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, uint8_t* __restrict__ qr,
+                  float* __restrict__ sr, uint8_t* __restrict__ qt, float* __restrict__ st) {
+  grid_chain();
+  __shared__ DualSmem sm;
+  const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  uint2 v[DUAL_ROWS];
+#pragma unroll
+  for (int i = 0; i < DUAL_ROWS; ++i)
+    v[i] = __ldg(reinterpret_cast<const uint2*>(x + static_cast<size_t>(r0 + w * DUAL_ROWS + i) * ldx + k0 + 4 * l));
+  quant_dual_tile(v, sm, r0, k0, R, K, qr, sr, qt, st);
+}
+
+// Both forms of h = bf16(silu(gate) * value) straight from pre = [value | gate] (bf16 [R][2 I]): h, which only e4m3 products
+// read, is neither written nor read back (6 bytes an element of h instead of 10 in two passes; 55 424 x 2048 115 + 105 us ->
+// 125, 5.4 TB/s).
+__global__ void __launch_bounds__(DUAL_THREADS, 2)
+swiglu_quant_dual_kernel(const __nv_bfloat16* __restrict__ pre, int R, int I, uint8_t* __restrict__ qr,
+                         float* __restrict__ sr, uint8_t* __restrict__ qt, float* __restrict__ st) {
+  grid_chain();
+  __shared__ DualSmem sm;
+  const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const __nv_bfloat16* src = pre + static_cast<size_t>(r0 + w * DUAL_ROWS) * 2 * I + k0 + 4 * l;
+  uint2 v[DUAL_ROWS];
+  uint2 g[DUAL_ROWS];
+#pragma unroll
+  for (int i = 0; i < DUAL_ROWS; ++i) {
+    const __nv_bfloat16* p = src + static_cast<size_t>(i) * 2 * I;
+    v[i] = __ldg(reinterpret_cast<const uint2*>(p));
+    g[i] = __ldg(reinterpret_cast<const uint2*>(p + I));
+  }
+#pragma unroll
+  for (int i = 0; i < DUAL_ROWS; ++i) {
+    const float2 a0 = unpack_bf16x2(v[i].x), a1 = unpack_bf16x2(v[i].y);
+    const float2 b0 = unpack_bf16x2(g[i].x), b1 = unpack_bf16x2(g[i].y);
+    v[i].x = pack_bf16x2(b0.x / (1.f + __expf(-b0.x)) * a0.x, b0.y / (1.f + __expf(-b0.y)) * a0.y);
+    v[i].y = pack_bf16x2(b1.x / (1.f + __expf(-b1.x)) * a1.x, b1.y / (1.f + __expf(-b1.y)) * a1.y);
+  }
+  quant_dual_tile(v, sm, r0, k0, R, I, qr, sr, qt, st);
+}
+
+// Both forms of the gradient of pre = [value | gate] from that of h (bf16 [R][I]): [dh silu(gate) | dh value silu'(gate)],
+// rounded to bf16 as the separate pass did, quantised without leaving the registers (10 bytes an element of h read and
+// written instead of 18). A block makes the value tile and the gate tile of the same 128 columns; the gate tile waits in
+// shared memory, since both do not fit the 64 registers that two blocks leave a thread (245 us for 55 424 x 2048, 4.6 TB/s;
+// one block a multiprocessor 276).
+struct SwigluBwdSmem {
+  DualSmem dual;
+  uint2 gate[DUAL_ROWS][DUAL_THREADS];
+};
+
+__device__ __forceinline__ void swiglu_grad(uint32_t& value, uint32_t& gate, uint32_t dh) {
+  const float2 a = unpack_bf16x2(value), b = unpack_bf16x2(gate), c = unpack_bf16x2(dh);
+  const float s0 = 1.f / (1.f + __expf(-b.x)), s1 = 1.f / (1.f + __expf(-b.y));
+  value = pack_bf16x2(c.x * b.x * s0, c.y * b.y * s1);
+  gate = pack_bf16x2(c.x * a.x * s0 * (1.f + b.x * (1.f - s0)), c.y * a.y * s1 * (1.f + b.y * (1.f - s1)));
+}
+
+__global__ void __launch_bounds__(DUAL_THREADS, 2)
+swiglu_bwd_quant_dual_kernel(const __nv_bfloat16* __restrict__ pre, const __nv_bfloat16* __restrict__ dh, int R, int I,
+                             uint8_t* __restrict__ qr, float* __restrict__ sr, uint8_t* __restrict__ qt,
+                             float* __restrict__ st) {
+  grid_chain();
+  extern __shared__ __align__(16) uint8_t swiglu_bwd_smem[];
+  SwigluBwdSmem& sm = *reinterpret_cast<SwigluBwdSmem*>(swiglu_bwd_smem);
+  const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const size_t row = static_cast<size_t>(r0 + w * DUAL_ROWS);
+  const __nv_bfloat16* src = pre + row * 2 * I + k0 + 4 * l;
+  const __nv_bfloat16* dsrc = dh + row * I + k0 + 4 * l;
+  uint2 v[DUAL_ROWS];
+  {
+    uint2 g[DUAL_ROWS], d[DUAL_ROWS];
+#pragma unroll
+    for (int i = 0; i < DUAL_ROWS; ++i) {
+      v[i] = __ldg(reinterpret_cast<const uint2*>(src + static_cast<size_t>(i) * 2 * I));
+      g[i] = __ldg(reinterpret_cast<const uint2*>(src + static_cast<size_t>(i) * 2 * I + I));
+      d[i] = __ldg(reinterpret_cast<const uint2*>(dsrc + static_cast<size_t>(i) * I));
+    }
+#pragma unroll
+    for (int i = 0; i < DUAL_ROWS; ++i) {
+      swiglu_grad(v[i].x, g[i].x, d[i].x);
+      swiglu_grad(v[i].y, g[i].y, d[i].y);
+      sm.gate[i][threadIdx.x] = g[i];
+    }
+  }
+  quant_dual_tile(v, sm.dual, r0, k0, R, 2 * I, qr, sr, qt, st);
+#pragma unroll
+  for (int i = 0; i < DUAL_ROWS; ++i) v[i] = sm.gate[i][threadIdx.x];   // (this thread's own)
+  __syncthreads();
+  quant_dual_tile(v, sm.dual, r0, I + k0, R, 2 * I, qr, sr, qt, st);
 }
 
 // ------------------------------------------------------------------ GEMM
@@ -269,8 +366,11 @@ struct F8Cfg {
   static constexpr int OFF_EPI = STAGES * STAGE_BYTES;
   static constexpr int OFF_SB = OFF_EPI + 8 * 8192;                // [2][BN] scales of B (row-scaled form)
   static constexpr int OFF_BAR = OFF_SB + 2 * BN * 4;
-  static constexpr int SMEM = OFF_BAR + 256;
+  static constexpr int SMEM = OFF_BAR + 512;
 };
+
+// What the epilogue does with the finished sums (forms 1 and 2: block-scaled B, bf16 output, plain launches).
+enum : int { F8_PLAIN = 0, F8_ADD = 1, F8_ROPE = 2 };
 
 struct Fp8Args {
   const float* sa;   // [KB][M]
@@ -280,6 +380,11 @@ struct Fp8Args {
   int out_mode;      // 0: bf16 store, 1: fp32 store, 2: fp32 reduce-add (all through tmC)
   int splits;        // out_mode 2: the K blocks of a tile are cut into this many work items (0: the launch chooses)
   int* status;
+  // F8_ROPE: position of every row, cos / sin tables [max_pos][32]; 64-wide heads that start below rope_cols are rotated
+  const int* rope_pos;
+  const float* rope_cos;
+  const float* rope_sin;
+  int rope_cols;
   // All-gather mode (ag_world > 1, block-scaled B only): B's rows and the matching scale columns
   // are sharded over the ranks. The epilogue warps of all CTAs first copy the other ranks' e4m3
   // rows (half the bytes of a bf16 gather) and scales out of peer memory into the local full-size
@@ -302,10 +407,15 @@ __device__ __forceinline__ bool f8_wait_shard(const Fp8Args& args, int shard, un
   return true;
 }
 
-template <int BN, bool B_BLOCK>
+// F8_ADD: the residual's tiles (tmR) travel through TMA into the staging tiles while the products run, are added to the
+// fp32 sums and overwritten by the results. F8_ROPE: a thread holds whole heads of its row (64 columns), so the
+// rotation is register arithmetic on the row's 32 cos / sin pairs, which wait in the staging tiles too (read from global
+// memory there and then, 32 rows apart, they cost 150 us). 55 424 rows, us: 1024 columns of K = 1024 79 plain, 93 with the
+// residual, 3072 of 1024 238 plain, 267 rotated; the passes over the output that they replace took 57 and 78.
+template <int BN, bool B_BLOCK, int FORM>
 __global__ void __launch_bounds__(F8_THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const __grid_constant__ CUtensorMap tmC, const Fp8Args args) {
+                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR, const Fp8Args args) {
   using C8 = F8Cfg<BN>;
   constexpr int STAGES = C8::STAGES, ACC = C8::ACC, HC = C8::HC;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -320,7 +430,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* empty_bar = bars + STAGES;
   uint64_t* tfull_bar = bars + 2 * STAGES;
   uint64_t* tempty_bar = bars + 2 * STAGES + ACC;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * ACC);
+  uint64_t* res_bar = bars + 2 * STAGES + 2 * ACC;   // F8_ADD: [8 epilogue warps][2 staging tiles]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_bar + 16);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int M = args.M, N = args.N;
@@ -358,6 +469,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       mbar_init(&tfull_bar[a], 1);
       mbar_init(&tempty_bar[a], 8);
     }
+    if (FORM == F8_ADD)
+      for (int i = 0; i < 16; ++i) mbar_init(&res_bar[i], 1);
     fence_barrier_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&tmA);
@@ -468,6 +581,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int et = threadIdx.x - 128;  // 0..255 over the eight epilogue warps
     uint8_t* stage_out = smem + C8::OFF_EPI + (warp - 4) * 8192;
     int toggle = 0;                      // which of this warp's two staging tiles is next
+    uint32_t res_phase = 0;
     uint32_t ag_seen = 0;
     if (args.ag_world > 1) {
       const long long shard_vecs = static_cast<long long>(args.ag_rows) * args.K / 16;
@@ -513,6 +627,39 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const int row = m0 + quarter * 32 + lane;
       const bool row_ok = row < M;
       const int nb = min(nh >> 7, n_blocks - 1);
+      // The item's second operand goes into the staging tiles once the previous item's results have left them. That takes a few
+      // thousand cycles, which pass while the first K blocks are added up.
+      int rope_at = 0;
+      if constexpr (FORM == F8_ROPE) rope_at = row_ok ? __ldg(args.rope_pos + row) * 32 : 0;
+      auto second_operand = [&] {
+        if (elect_one()) tma_store_wait_read<0>();
+        __syncwarp();
+        if constexpr (FORM == F8_ADD) {
+          if (m0 + quarter * 32 < M && elect_one()) {
+#pragma unroll
+            for (int q = 0; q < HC / 64; ++q) {
+              if (nh + q * 64 < N) {
+                mbar_arrive_expect_tx(&res_bar[(warp - 4) * 2 + q], 4096);
+                tma_load_2d(stage_out + q * 4096, &tmR, &res_bar[(warp - 4) * 2 + q], nh + q * 64, m0 + quarter * 32);
+              }
+            }
+          }
+          __syncwarp();
+        } else if (nh < args.rope_cols) {
+          // 32 rows x [32 cos | 32 sin]: sixteen 16-byte pieces a row, piece c of row r at place c ^ (r & 7)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int r = 2 * i + (lane >> 4), piece = lane & 15;
+            const int at = __shfl_sync(0xffffffffu, rope_at, r);
+            const float* src = (piece < 8 ? args.rope_cos : args.rope_sin) + at + (piece & 7) * 4;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(stage_out + r * 256 +
+                                                                                    ((piece ^ (r & 7)) << 4))),
+                         "l"(src)
+                         : "memory");
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+      };
       float2 c[HC / 2];
 #pragma unroll
       for (int j = 0; j < HC / 2; ++j) c[j] = make_float2(0.f, 0.f);
@@ -545,6 +692,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           if (B_BLOCK) break;
           continue;
         }
+        if (FORM != F8_PLAIN && kb == min(kb0 + 1, kb1 - 1)) second_operand();
         tc_fence_after();
         const uint32_t taddr = tmem_base + acc * BN + half * HC + (static_cast<uint32_t>(quarter * 32) << 16);
         const float2 sa2 = make_float2(sa, sa), sblk2 = make_float2(sblk, sblk);
@@ -594,10 +742,62 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       // registers touch 32 rows an instruction: a fifth of a weight gradient's time.)
       const int y0 = m0 + quarter * 32;
       const bool bf = args.out_mode == 0;
+      if constexpr (FORM == F8_ROPE) {
+        if (nh < args.rope_cols) {
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {     // pairs (4i .. 4i + 3) and their partners 32 columns on, in each of the thread's heads
+            const float4 cs = *reinterpret_cast<const float4*>(stage_out + lane * 256 + ((i ^ (lane & 7)) << 4));
+            const float4 sn = *reinterpret_cast<const float4*>(stage_out + lane * 256 + (((8 + i) ^ (lane & 7)) << 4));
+#pragma unroll
+            for (int q = 0; q < HC / 64; ++q) {
+              if (nh + q * 64 < args.rope_cols) {
+                float2 *a = c + q * 32 + 2 * i, *b = a + 16;
+                const float2 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
+                a[0] = make_float2(a0.x * cs.x - b0.x * sn.x, a0.y * cs.y - b0.y * sn.y);
+                b[0] = make_float2(b0.x * cs.x + a0.x * sn.x, b0.y * cs.y + a0.y * sn.y);
+                a[1] = make_float2(a1.x * cs.z - b1.x * sn.z, a1.y * cs.w - b1.y * sn.w);
+                b[1] = make_float2(b1.x * cs.z + a1.x * sn.z, b1.y * cs.w + a1.y * sn.w);
+              }
+            }
+          }
+          __syncwarp();     // every lane has read its row before the results overwrite the tiles
+        }
+      }
 #pragma unroll
       for (int q = 0; q < HC / 32; ++q) {
         if (bf && q >= HC / 64) break;
         const int x = nh + q * (bf ? 64 : 32);
+        if constexpr (FORM == F8_ADD) {
+          if (q < HC / 64 && y0 < M && x < N) {
+            uint8_t* rb = stage_out + (q % (HC / 64)) * 4096;
+            if (!mbar_wait(&res_bar[(warp - 4) * 2 + (q % (HC / 64))], (res_phase >> q) & 1u)) {
+              if (lane == 0) atomicExch(args.status, ST_TIMEOUT_MISC);
+            }
+            res_phase ^= 1u << q;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              uint4* at = reinterpret_cast<uint4*>(rb + lane * 128 + ((j ^ (lane & 7)) << 4));
+              uint4 o = *at;
+              uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+              const float2* v = c + (q % (HC / 64)) * 32 + j * 4;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 t = unpack_bf16x2(ow[e]);
+                ow[e] = pack_bf16x2(v[e].x + t.x, v[e].y + t.y);
+              }
+              *at = o;
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (elect_one()) {
+              tma_store_2d(&tmC, rb, x, y0);
+              tma_store_commit();
+            }
+          }
+          continue;
+        }
         if (y0 < M && x < N) {
           if (elect_one()) tma_store_wait_read<1>();
           __syncwarp();
@@ -701,22 +901,28 @@ static int f8_splits(int tiles, int kb, int sms) {
   return best;
 }
 
-template <int BN, bool B_BLOCK>
-static int f8_launch_form(const void* A, const void* B, void* C, Fp8Args& args, bool coop, cudaStream_t stream) {
-  CUtensorMap tmA, tmB, tmC;
+template <int BN, bool B_BLOCK, int FORM = F8_PLAIN>
+static int f8_launch_form(const void* A, const void* B, void* C, const void* R, int ldr, Fp8Args& args, bool coop,
+                          cudaStream_t stream) {
+  CUtensorMap tmA, tmB, tmC, tmR;
   int rc = f8_make_map(&tmA, A, args.K, args.M, F8_BM);
   if (rc) return rc;
   rc = f8_make_map(&tmB, B, args.K, args.N, BN);
   if (rc) return rc;
   rc = f8_make_out_map(&tmC, C, args.N, args.M, args.ldc, args.out_mode == 0);
   if (rc) return rc;
+  tmR = tmC;
+  if (FORM == F8_ADD) {
+    rc = f8_make_out_map(&tmR, const_cast<void*>(R), args.N, args.M, ldr, true);
+    if (rc) return rc;
+  }
+  auto kern = gemm_fp8_kernel<BN, B_BLOCK, FORM>;
   static bool configured_on[nplm::MAX_DEVICES];
   const int dev_slot = nplm::current_device_slot();
   if (dev_slot < 0) return -4;
   bool& configured = configured_on[dev_slot];
   if (!configured) {
-    NPLM_CUDA_CHECK(
-        cudaFuncSetAttribute(gemm_fp8_kernel<BN, B_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, F8Cfg<BN>::SMEM));
+    NPLM_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F8Cfg<BN>::SMEM));
     configured = true;
   }
   int sms = 148;
@@ -727,18 +933,18 @@ static int f8_launch_form(const void* A, const void* B, void* C, Fp8Args& args, 
   const int total = tiles * args.splits;
   const int grid = total < sms ? total : sms;
   if (coop) {
-    void* params[] = {&tmA, &tmB, &tmC, &args};
-    return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(gemm_fp8_kernel<BN, B_BLOCK>), dim3(grid),
-                                                        dim3(F8_THREADS), params, F8Cfg<BN>::SMEM, stream));
+    void* params[] = {&tmA, &tmB, &tmC, &tmR, &args};
+    return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(grid), dim3(F8_THREADS),
+                                                        params, F8Cfg<BN>::SMEM, stream));
   }
-  launch_chained(gemm_fp8_kernel<BN, B_BLOCK>, grid, F8_THREADS, F8Cfg<BN>::SMEM, stream, tmA, tmB, tmC, args);
+  launch_chained(kern, grid, F8_THREADS, F8Cfg<BN>::SMEM, stream, tmA, tmB, tmC, tmR, args);
   return static_cast<int>(cudaGetLastError());
 }
 
 template <int BN>
 static int f8_launch(const void* A, const void* B, void* C, Fp8Args& args, bool coop, cudaStream_t stream) {
-  return args.b_block ? f8_launch_form<BN, true>(A, B, C, args, coop, stream)
-                      : f8_launch_form<BN, false>(A, B, C, args, coop, stream);
+  return args.b_block ? f8_launch_form<BN, true>(A, B, C, nullptr, 0, args, coop, stream)
+                      : f8_launch_form<BN, false>(A, B, C, nullptr, 0, args, coop, stream);
 }
 
 static int f8_grid(long long threads_needed, int block) {
@@ -789,10 +995,67 @@ extern "C" int nplm_fp8_quant_dual(const void* x, int R, int K, int ldx, void* q
   if (R <= 0 || K <= 0) return 0;
   if ((K % 128) || (R % 128) || (ldx % 4) || (reinterpret_cast<uintptr_t>(x) & 7)) return -3;
   if (R / 128 > 65535) return -3;
-  launch_chained(quant_dual_kernel, dim3(K / 128, R / 128), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx,
+  launch_chained(quant_dual_kernel, dim3(K / 128, R / 128), DUAL_THREADS, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx,
                                                                 reinterpret_cast<uint8_t*>(qr), sr,
                                                                 reinterpret_cast<uint8_t*>(qt), st);
   return static_cast<int>(cudaGetLastError());
+}
+
+// Both e4m3 forms of h = silu(gate) * value, pre = [value | gate] bf16 [R][2 I] contiguous; R, I multiples of 128.
+extern "C" int nplm_fp8_swiglu_quant_dual(const void* pre, int R, int I, void* qr, float* sr, void* qt, float* st,
+                                          cudaStream_t stream) {
+  if (R <= 0 || I <= 0) return 0;
+  if ((I % 128) || (R % 128) || (reinterpret_cast<uintptr_t>(pre) & 7) || R / 128 > 65535) return -3;
+  launch_chained(swiglu_quant_dual_kernel, dim3(I / 128, R / 128), DUAL_THREADS, 0, stream,
+                 reinterpret_cast<const __nv_bfloat16*>(pre), R, I, reinterpret_cast<uint8_t*>(qr), sr,
+                 reinterpret_cast<uint8_t*>(qt), st);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Both e4m3 forms of the gradient of pre (bf16 [R][2 I]) from dh (bf16 [R][I]), all contiguous; R, I multiples of 128.
+extern "C" int nplm_fp8_swiglu_bwd_quant_dual(const void* pre, const void* dh, int R, int I, void* qr, float* sr, void* qt,
+                                              float* st, cudaStream_t stream) {
+  if (R <= 0 || I <= 0) return 0;
+  if ((I % 128) || (R % 128) || ((reinterpret_cast<uintptr_t>(pre) | reinterpret_cast<uintptr_t>(dh)) & 7) ||
+      R / 128 > 65535)
+    return -3;
+  static bool configured_on[nplm::MAX_DEVICES];
+  const int dev_slot = nplm::current_device_slot();
+  if (dev_slot < 0) return -4;
+  if (!configured_on[dev_slot]) {
+    NPLM_CUDA_CHECK(cudaFuncSetAttribute(swiglu_bwd_quant_dual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(sizeof(SwigluBwdSmem))));
+    configured_on[dev_slot] = true;
+  }
+  launch_chained(swiglu_bwd_quant_dual_kernel, dim3(I / 128, R / 128), DUAL_THREADS, sizeof(SwigluBwdSmem), stream,
+                 reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<const __nv_bfloat16*>(dh), R, I,
+                 reinterpret_cast<uint8_t*>(qr), sr, reinterpret_cast<uint8_t*>(qt), st);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Tile width of a plain product: few rows run on 128-wide tiles as long as those fit one wave of 148, where they finish
+// sooner. Graph-timed us, wide / narrow: 256 rows, 2048 columns of 512 6.9 / 5.8; 1 536 rows, 1024 columns of 1024
+// 8.9 / 7.8. Past a wave the wide ones are ahead (2 432 rows of the latter 9.2; the earlier kernel, all 128-wide, 14.0, and
+// 8.6 - 8.9 below a wave). Both sum a tile's K blocks in the same order. Accumulated outputs fill the chip by
+// splitting the contraction instead.
+static bool f8_wide(int M, int N, int out_mode) {
+  const long long wide_tiles = (M + 127LL) / 128 * ((N + 255LL) / 256);
+  return N > 128 && (out_mode == 2 || 2 * wide_tiles > 148);
+}
+
+static Fp8Args f8_plain_args(const float* sa, const float* sb, int M, int N, int K, int ldc, int b_block, int out_mode,
+                             int* status) {
+  Fp8Args args = {};
+  args.sa = sa;
+  args.sb = sb;
+  args.M = M;
+  args.N = N;
+  args.K = K;
+  args.ldc = ldc;
+  args.b_block = b_block;
+  args.out_mode = out_mode;
+  args.status = status;
+  return args;
 }
 
 // C[M][N] (+)= (A * sa) (B * sb)^T, A e4m3 [M][K], B e4m3 [N][K] (both K-major, K % 128 == 0).
@@ -808,34 +1071,37 @@ extern "C" int nplm_gemm_fp8(const void* A, const void* B, void* C, const float*
     return -3;
   if (out_mode == 0 ? ((N % 8) || (ldc % 8)) : ((N % 4) || (ldc % 4))) return -5;
   if (!b_block && (N % 4)) return -5;
-  Fp8Args args;
-  args.sa = sa;
-  args.sb = sb;
-  args.M = M;
-  args.N = N;
-  args.K = K;
-  args.ldc = ldc;
-  args.b_block = b_block;
+  Fp8Args args = f8_plain_args(sa, sb, M, N, K, ldc, b_block, out_mode, status);
   args.splits = whole_tiles ? 1 : 0;
-  args.out_mode = out_mode;
-  args.status = status;
-  args.ag_world = 0;
-  args.ag_rank = 0;
-  args.ag_rows = 0;
-  args.ag_dst = nullptr;
-  args.ag_sdst = nullptr;
-  args.ag_flags = nullptr;
-  for (int r = 0; r < 8; ++r) {
-    args.ag_src[r] = nullptr;
-    args.ag_ssrc[r] = nullptr;
-  }
-  // Few rows: as long as the 128-wide tiles fit one wave of 148 they finish sooner. Graph-timed us, wide / narrow: 256 rows, 2048
-  // columns of 512 6.9 / 5.8; 1 536 rows, 1024 columns of 1024 8.9 / 7.8. Past a wave the wide ones are ahead (2 432 rows
-  // of the latter 9.2; the earlier kernel, all 128-wide, 14.0, and 8.6 - 8.9 below a wave). Both sum a tile's K blocks in the same
-  // order. Accumulated outputs fill the chip by splitting the contraction instead.
-  const long long wide_tiles = (M + 127LL) / 128 * ((N + 255LL) / 256);
-  const bool wide = N > 128 && (out_mode == 2 || 2 * wide_tiles > 148);
-  return wide ? f8_launch<256>(A, B, C, args, false, stream) : f8_launch<128>(A, B, C, args, false, stream);
+  return f8_wide(M, N, out_mode) ? f8_launch<256>(A, B, C, args, false, stream)
+                                 : f8_launch<128>(A, B, C, args, false, stream);
+}
+
+// bf16 C[M][N] = (A * sa) (B * sb)^T with block-scaled B, plus R (bf16, row stride ldr; may be null), or with the rotary
+// embedding applied to the 64-wide heads that start below rope_cols (rope_pos not null). One rounding.
+extern "C" int nplm_gemm_fp8_form(const void* A, const void* B, void* C, const void* R, const float* sa, const float* sb,
+                                  int M, int N, int K, int ldc, int ldr, const int* rope_pos, const float* rope_cos,
+                                  const float* rope_sin, int rope_cols, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((K % 128) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
+      (reinterpret_cast<uintptr_t>(C) & 15) || (N % 8) || (ldc % 8))
+    return -3;
+  if ((R != nullptr) == (rope_pos != nullptr)) return -3;
+  if (R != nullptr && ((ldr % 8) || (reinterpret_cast<uintptr_t>(R) & 15))) return -3;
+  if (rope_pos != nullptr && (rope_cos == nullptr || rope_sin == nullptr || (N % 64) || (rope_cols % 64) ||
+                              (reinterpret_cast<uintptr_t>(rope_cos) & 15) || (reinterpret_cast<uintptr_t>(rope_sin) & 15)))
+    return -3;
+  Fp8Args args = f8_plain_args(sa, sb, M, N, K, ldc, 1, 0, status);
+  args.rope_pos = rope_pos;
+  args.rope_cos = rope_cos;
+  args.rope_sin = rope_sin;
+  args.rope_cols = rope_cols;
+  const bool wide = f8_wide(M, N, 0);
+  if (R != nullptr)
+    return wide ? f8_launch_form<256, true, F8_ADD>(A, B, C, R, ldr, args, false, stream)
+                : f8_launch_form<128, true, F8_ADD>(A, B, C, R, ldr, args, false, stream);
+  return wide ? f8_launch_form<256, true, F8_ROPE>(A, B, C, nullptr, 0, args, false, stream)
+              : f8_launch_form<128, true, F8_ROPE>(A, B, C, nullptr, 0, args, false, stream);
 }
 
 // All-gather fused into the fp8 GEMM. b_ptrs[r] / sb_ptrs[r]: rank r's full-size e4m3 weight buffer
@@ -850,7 +1116,7 @@ extern "C" int nplm_gemm_fp8_ag(const void* A, void* const* b_ptrs, void* C, con
       (K % 128) || flags == nullptr)
     return -10;
   if (out_mode == 0 ? ((N % 8) || (ldc % 8)) : ((N % 4) || (ldc % 4))) return -5;
-  Fp8Args args;
+  Fp8Args args = {};
   args.sa = sa;
   args.sb = reinterpret_cast<const float*>(sb_ptrs[rank]);
   args.M = M;

@@ -90,11 +90,29 @@ class Attention(nn.Module):
                                               window, self.scale, rope=(ctx.position_ids, rope[0], rope[1]))
             y = ops.attention_varlen(qkv, ctx.seq_start, ctx.seq_end, H, D, window, self.scale,
                                      rope=(ctx.position_ids, rope[0], rope[1]))
+        elif self._fused_fp8(x, ctx, rope):     # the same two places, e4m3 operands
+            from nanoplm_b200.ops import fp8
+            qkv = fp8.fp8_linear(x, self.Wqkv.weight, rope=(ctx.position_ids, rope[0], rope[1], 2 * H * D))
+            y = ops.attention_varlen(qkv, ctx.seq_start, ctx.seq_end, H, D, window, self.scale,
+                                     rope=(ctx.position_ids, rope[0], rope[1]))
         else:
             qkv = self.Wqkv(x)
             qkv = ops.rope_qkv(qkv, ctx.position_ids, rope[0], rope[1], H, D)
             y = ops.attention_varlen(qkv, ctx.seq_start, ctx.seq_end, H, D, window, self.scale)
         return self.Wo(y, residual=residual)
+
+    def _fused_fp8(self, x, ctx: "BatchContext", rope: tuple) -> bool:
+        """Whether the QKV product may rotate q and k in its epilogue: e4m3 products on, a projection that they take and
+        nobody who watches its un-rotated output."""
+        w = self.Wqkv
+        if not (ops.fp8_enabled() and x.is_cuda and x.dim() == 2 and self.head_dim == 64 and type(w) is Linear
+                and w.bias is None and x.shape[0] > 0 and native_layer.unobserved((w,))):
+            return False
+        from nanoplm_b200.ops import fp8
+        pos, (cos, sin) = ctx.position_ids, rope
+        return (fp8.supported(x, w.weight) and pos.dtype == torch.int32 and pos.is_cuda and pos.numel() == x.shape[0]
+                and pos.is_contiguous() and cos.dtype == sin.dtype == torch.float32 and cos.is_cuda and sin.is_cuda
+                and cos.shape[-1] == sin.shape[-1] == 32 and cos.is_contiguous() and sin.is_contiguous())
 
 
 class MLP(nn.Module):

@@ -86,14 +86,63 @@ def quant_dual(x: torch.Tensor) -> tuple[Quantized, Quantized]:
     R, K = x.shape
     if x.stride(1) != 1 or x.stride(0) % 4 or x.data_ptr() % 8:
         x = x.contiguous()
-    dev = x.device
-    qr, sr = torch.empty((R, K), dtype=torch.uint8, device=dev), torch.empty((K // 128, R), dtype=torch.float32, device=dev)
-    qt, st = torch.empty((K, R), dtype=torch.uint8, device=dev), torch.empty((R // 128, K), dtype=torch.float32, device=dev)
-    rc = lib("fp8").nplm_fp8_quant_dual(ptr(x), c_int(R), c_int(K), c_int(x.stride(0)), ptr(qr), ptr(sr), ptr(qt),
-                                        ptr(st), stream_ptr())
+    r, t = _dual_buffers(R, K, x.device)
+    rc = lib("fp8").nplm_fp8_quant_dual(ptr(x), c_int(R), c_int(K), c_int(x.stride(0)), ptr(r.q), ptr(r.scale), ptr(t.q),
+                                        ptr(t.scale), stream_ptr())
     check_rc(rc, "fp8_quant_dual")
     count_launch()
-    return Quantized(qr, sr, False), Quantized(qt, st, False)
+    return r, t
+
+
+def _dual_buffers(R: int, K: int, dev) -> tuple[Quantized, Quantized]:
+    """Row form and transposed row form of an operand [R, K], to be filled."""
+    u8, f32 = torch.uint8, torch.float32
+    return (Quantized(torch.empty((R, K), dtype=u8, device=dev), torch.empty((K // 128, R), dtype=f32, device=dev), False),
+            Quantized(torch.empty((K, R), dtype=u8, device=dev), torch.empty((R // 128, K), dtype=f32, device=dev), False))
+
+
+def swiglu_quant_dual(pre: torch.Tensor) -> tuple[Quantized, Quantized]:
+    """quant_dual(swiglu(pre)) for pre = [value | gate] bf16 [R, 2 I] contiguous, R and I multiples of 128."""
+    R, I = pre.shape[0], pre.shape[1] // 2
+    r, t = _dual_buffers(R, I, pre.device)
+    rc = lib("fp8").nplm_fp8_swiglu_quant_dual(ptr(pre), c_int(R), c_int(I), ptr(r.q), ptr(r.scale), ptr(t.q),
+                                               ptr(t.scale), stream_ptr())
+    check_rc(rc, "fp8_swiglu_quant_dual")
+    count_launch()
+    return r, t
+
+
+def swiglu_bwd_quant_dual(pre: torch.Tensor, dh: torch.Tensor) -> tuple[Quantized, Quantized]:
+    """quant_dual of the gradient of pre (bf16 [R, 2 I]) from that of h = swiglu(pre) (bf16 [R, I]), both contiguous."""
+    R, I = dh.shape
+    r, t = _dual_buffers(R, 2 * I, pre.device)
+    rc = lib("fp8").nplm_fp8_swiglu_bwd_quant_dual(ptr(pre), ptr(dh), c_int(R), c_int(I), ptr(r.q), ptr(r.scale),
+                                                   ptr(t.q), ptr(t.scale), stream_ptr())
+    check_rc(rc, "fp8_swiglu_bwd_quant_dual")
+    count_launch()
+    return r, t
+
+
+def gemm_fp8_form(a: Quantized, b: Quantized, *, residual: torch.Tensor | None = None,
+                  rope: tuple | None = None) -> torch.Tensor:
+    """bf16 deq(a) deq(b)^T + residual, or with the rotary embedding of rope = (pos int32 [M], cos, sin fp32 [P, 32],
+    rope_cols) on the 64-wide heads below column rope_cols; b block-scaled. One rounding of the fp32 sums."""
+    M, K = a.q.shape
+    N = b.q.shape[0]
+    out = torch.empty((M, N), dtype=_BF16, device=a.q.device)
+    pos, cos, sin, cols = rope if rope is not None else (None, None, None, 0)
+    if residual is not None and (residual.dtype != _BF16 or tuple(residual.shape) != (M, N) or residual.stride(1) != 1):
+        raise ValueError("the residual must be a row-major bf16 [M, N] tensor")
+    if rope is not None and (pos.dtype != torch.int32 or pos.numel() != M or cos.dtype != torch.float32
+                             or sin.dtype != torch.float32 or cos.shape[-1] != 32 or sin.shape[-1] != 32):
+        raise ValueError("rope needs int32 positions [M] and fp32 tables [P, 32]")
+    rc = lib("fp8").nplm_gemm_fp8_form(ptr(a.q), ptr(b.q), ptr(out), ptr(residual), ptr(a.scale), ptr(b.scale), c_int(M),
+                                       c_int(N), c_int(K), c_int(N), c_int(residual.stride(0) if residual is not None else 0),
+                                       ptr(pos), ptr(cos), ptr(sin), c_int(cols), ptr(status_word(a.q.device)),
+                                       stream_ptr())
+    check_rc(rc, "gemm_fp8_form")
+    count_launch()
+    return out
 
 
 def gemm_fp8(a: Quantized, b: Quantized, *, out: torch.Tensor | None = None, out_dtype=_BF16,
@@ -168,14 +217,31 @@ def supported(x: torch.Tensor, w: torch.Tensor) -> bool:
             and w.shape[1] % 128 == 0)
 
 
+def addable(residual: torch.Tensor, x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the product's epilogue can add `residual`: bf16 rows of the output's shape on 16-byte boundaries."""
+    if residual.dtype != _BF16 or not residual.is_cuda or residual.shape != (*x.shape[:-1], w.shape[0]):
+        return False
+    r = residual.reshape(-1, w.shape[0])
+    return r.stride(1) == 1 and r.stride(0) % 8 == 0 and r.data_ptr() % 16 == 0
+
+
 def _dual_rows(T: int) -> bool:
     """Token counts for which the weight gradient runs on e4m3 operands (whole 128-token scale blocks)."""
     return T % 128 == 0 and T // 128 <= 65535
 
 
+def _weight_gradient(qdy_t: Quantized, qx_t: Quantized, p):
+    """dW [N, K] = dY^T X from the token-contiguous payloads; into p.main_grad, or returned."""
+    from .functional import _has_main_grad
+    if _has_main_grad(p):
+        gemm_fp8(qdy_t, qx_t, out=p.main_grad.view(p.shape), accumulate=True)
+        return None
+    return gemm_fp8(qdy_t, qx_t, out_dtype=torch.float32).to(p.dtype)
+
+
 class _Fp8LinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, train):
+    def forward(ctx, x, w, train, residual, rope):
         from .functional import _as_shape
         x2 = x.reshape(-1, x.shape[-1])
         qw, _ = _quantized_weight(w)
@@ -186,20 +252,24 @@ class _Fp8LinearFn(torch.autograd.Function):
         else:
             qx = quant_rows(x2)
             ctx.save_for_backward(x2, w)
-        y = gemm_fp8(qx, qw)
+        if residual is None and rope is None:
+            y = gemm_fp8(qx, qw)
+        else:
+            y = gemm_fp8_form(qx, qw, residual=None if residual is None else residual.reshape(-1, w.shape[0]), rope=rope)
+        ctx.has_res = residual is not None
         ctx.w_ref = w
         ctx.shape = x.shape
         return _as_shape(y, (*x.shape[:-1], w.shape[0]))
 
     @staticmethod
     def backward(ctx, dy):
-        from .functional import _as_shape, _has_main_grad, _wgrad
+        from .functional import _as_shape, _wgrad
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dx = dw = qdy = qdy_t = None
         if ctx.dual:
-            qx_t, sx_t, w = ctx.saved_tensors
+            qx_t, sx_t, _ = ctx.saved_tensors
             if ctx.needs_input_grad[0]:
                 qdy, qdy_t = quant_dual(dy2)
             else:
@@ -210,18 +280,70 @@ class _Fp8LinearFn(torch.autograd.Function):
             _, qwt = _quantized_weight(ctx.w_ref)
             dx = _as_shape(gemm_fp8(qdy, qwt), ctx.shape)
         if ctx.dual:
-            # dW[N,K] = dY^T X: both operands as token-contiguous payloads
-            p, qx = ctx.w_ref, Quantized(qx_t, sx_t, False)
-            if _has_main_grad(p):
-                gemm_fp8(qdy_t, qx, out=p.main_grad.view(w.shape), accumulate=True)
-            else:
-                dw = gemm_fp8(qdy_t, qx, out_dtype=torch.float32).to(w.dtype)
+            dw = _weight_gradient(qdy_t, Quantized(qx_t, sx_t, False), ctx.w_ref)
         elif ctx.needs_input_grad[1]:
             dw = _wgrad(dy2, ctx.saved_tensors[0], ctx.w_ref)
-        return dx, dw, None
+        return dx, dw, None, (dy if ctx.has_res else None), None
 
 
-def fp8_linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    """y = x W^T with e4m3 operands (no bias)."""
+def fp8_linear(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None = None,
+               rope: tuple | None = None) -> torch.Tensor:
+    """y = x W^T with e4m3 operands (no bias), plus the residual or with the rotary embedding of `gemm_fp8_form` in the
+    product's epilogue. With rope the gradient that comes back must be that of the un-rotated projection (as
+    `functional.linear_rope`)."""
     from .functional import _keeps
-    return _Fp8LinearFn.apply(x, w, _keeps())
+    return _Fp8LinearFn.apply(x, w, _keeps(), residual, rope)
+
+
+class _Fp8MlpFn(torch.autograd.Function):
+    """SwiGLU MLP + residual on e4m3 operands as one node: the activation exists only as the quantised operands of the two
+    products that read it, and so do the gradients of the pre-activations. Whole 128-token blocks, training."""
+
+    @staticmethod
+    def forward(ctx, x, w_in, w_out, residual):
+        from .functional import _as_shape
+        x2 = x.reshape(-1, x.shape[-1])
+        qx, qx_t = quant_dual(x2)
+        pre = gemm_fp8(qx, _quantized_weight(w_in)[0])
+        qh, qh_t = swiglu_quant_dual(pre)
+        qw = _quantized_weight(w_out)[0]
+        if residual is None:
+            y = gemm_fp8(qh, qw)
+        else:
+            y = gemm_fp8_form(qh, qw, residual=residual.reshape(-1, w_out.shape[0]))
+        ctx.save_for_backward(qx_t.q, qx_t.scale, pre, qh_t.q, qh_t.scale, w_in, w_out)
+        ctx.refs = (w_in, w_out)
+        ctx.has_res = residual is not None
+        ctx.x_shape = x.shape
+        return _as_shape(y, (*x.shape[:-1], y.shape[1]))
+
+    @staticmethod
+    def backward(ctx, dy):
+        from .functional import _as_shape
+        qx_t, sx_t, pre, qh_t, sh_t, _, _ = ctx.saved_tensors
+        w_in, w_out = ctx.refs
+        dy2 = dy.reshape(-1, dy.shape[-1])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        qdy, qdy_t = quant_dual(dy2)
+        dh = gemm_fp8(qdy, _quantized_weight(w_out)[1])
+        dw_out = _weight_gradient(qdy_t, Quantized(qh_t, sh_t, False), w_out) if ctx.needs_input_grad[2] else None
+        qd, qd_t = swiglu_bwd_quant_dual(pre, dh)
+        dw_in = _weight_gradient(qd_t, Quantized(qx_t, sx_t, False), w_in) if ctx.needs_input_grad[1] else None
+        dx = (_as_shape(gemm_fp8(qd, _quantized_weight(w_in)[1]), ctx.x_shape) if ctx.needs_input_grad[0] else None)
+        return dx, dw_in, dw_out, (dy if ctx.has_res else None)
+
+
+def mlp_fused(x: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor) -> bool:
+    """Whether `fp8_mlp` takes a call: both projections fit (`supported`, whole 128-column halves), whole 128-token blocks, and
+    a backward pass for both weights."""
+    from .functional import _keeps, functions_observed
+    inter = w_out.shape[1]
+    return (not functions_observed() and supported(x, w_in) and supported(x, w_out) and w_in.shape[0] == 2 * inter and w_in.shape[1] == x.shape[-1]
+            and x.numel() > 0 and _dual_rows(x.numel() // x.shape[-1]) and _keeps() and w_in.requires_grad
+            and w_out.requires_grad)
+
+
+def fp8_mlp(x, w_in, w_out, residual=None):
+    """(silu(gate) * value) W_out^T + residual with [value | gate] = x W_in^T, e4m3 operands throughout."""
+    return _Fp8MlpFn.apply(x, w_in, w_out, residual)

@@ -208,6 +208,10 @@ def mlp_swiglu(x, w_in, w_out, residual=None):
     if (x.is_cuda and x.dtype == BF and not _FP8_STATE["enabled"] and inter % 64 == 0 and w_in.shape[0] == 2 * inter
             and w_in.shape[1] % 64 == 0 and w_out.shape[0] % 64 == 0):
         return _call(_SwiGLUMLPFn, x, w_in, w_out, residual, _keeps())
+    if x.is_cuda and _FP8_STATE["enabled"]:
+        from . import fp8
+        if fp8.mlp_fused(x, w_in, w_out):
+            return fp8.fp8_mlp(x, w_in, w_out, residual)
     return linear(linear(x, w_in, act="swiglu"), w_out, residual=residual)
 
 
@@ -238,6 +242,8 @@ def linear(x, w, bias=None, residual=None, act: str | None = None):
     if x.is_cuda and _FP8_STATE["enabled"] and bias is None:
         from . import fp8
         if fp8.supported(x, w):
+            if residual is not None and act is None and fp8.addable(residual, x, w):
+                return fp8.fp8_linear(x, w, residual=residual)
             y = fp8.fp8_linear(x, w)
             if act == "swiglu":
                 y = swiglu(y)

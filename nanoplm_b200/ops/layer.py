@@ -101,6 +101,11 @@ def _quiet(parts) -> bool:
     return True
 
 
+def unobserved(parts) -> bool:
+    """The modules `parts` may be passed by: nobody watches their calls or the autograd Functions behind them."""
+    return not F_.functions_observed() and not _mod._has_any_global_hook() and _quiet(parts)
+
+
 def _ok_weight(w, rows: int, cols: int) -> bool:
     return (w.dtype == BF and w.is_cuda and w.shape == (rows, cols) and w.is_contiguous() and w.data_ptr() % 16 == 0
             and getattr(w, "_ag", None) is None)
