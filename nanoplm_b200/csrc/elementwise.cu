@@ -523,6 +523,26 @@ scatter_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict
 // inv_count is read from device memory (1 / number of valid labels).
 constexpr int CE_WARPS = 8;
 
+// inv[0] = 1 / max(number of labels >= 0, 1), loss[0] = 0: one small launch for what were six (comparison, sum, clamp,
+// conversion, division, zeros).
+__global__ void __launch_bounds__(1024)
+ce_count_kernel(const int* __restrict__ labels, int n, float* __restrict__ inv, float* __restrict__ loss) {
+  grid_chain();
+  __shared__ int part[32];
+  int valid = 0;
+  for (int i = threadIdx.x; i < n; i += 1024) valid += labels[i] >= 0;
+  valid = __reduce_add_sync(0xffffffffu, valid);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = valid;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int total = __reduce_add_sync(0xffffffffu, part[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      inv[0] = __fdiv_rn(1.f, static_cast<float>(max(total, 1)));
+      loss[0] = 0.f;
+    }
+  }
+}
+
 template <int CHUNKS>
 __global__ void __launch_bounds__(CE_WARPS * 32)
 ce_fwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ W,
@@ -1154,6 +1174,12 @@ extern "C" int nplm_scatter_rows(const void* src, const int* idx, void* dst, int
   if (C % 8) return -3;
   launch_chained(scatter_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(src), idx, reinterpret_cast<__nv_bfloat16*>(dst), n, C);
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int nplm_ce_count(const int* labels, int n, float* inv, float* loss, cudaStream_t st) {
+  if (n < 0) return -3;
+  launch_chained(ce_count_kernel, 1, 1024, 0, st, labels, n, inv, loss);
   return static_cast<int>(cudaGetLastError());
 }
 

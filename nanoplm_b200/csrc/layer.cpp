@@ -1,5 +1,5 @@
-// Host-side launch sequences of one plain encoder layer (pre-norm, rotary attention, SwiGLU MLP, no biases): all
-// kernels of a layer's forward pass from one call, and all of its backward pass from another.
+// Host-side launch sequences of plain encoder layers (pre-norm, rotary attention, SwiGLU MLP, no biases): all
+// kernels of a forward pass from one call, and all of its backward pass from another, for one layer or a run of layers.
 //
 // The kernels and their order are those of the op-by-op path (nanoplm_b200/models/encoder.py: EncoderLayer); what
 // this saves is the interpreter between them: a launch from Python costs 15 - 20 us (wrapper, checks, allocation, autograd
@@ -235,4 +235,16 @@ extern "C" int nplm_layer_bwd(const long long* a, double scale) {
     return k.out(d.dqkv, wqkv, dx, d.dx1, T, C, 3 * HD, C, C, C, 1, EPI_ADD);
   TRY(k.out(d.dqkv, wqkv, d.dh, nullptr, T, C, 3 * HD, C, C, 0, 1, EPI_STORE));
   return fn.norm_bwd(d.dh, x, nullptr, n1, rms ? nullptr : s.mean1, s.rstd1, d.dx1, dx, g_n1, nullptr, T, C, 0, rms, k.stream);
+}
+
+// `layers` consecutive layers: their argument arrays and (eps1, eps2, scale) triples one after the other. Backward calls go from
+// the last array to the first.
+extern "C" int nplm_layers_fwd(const long long* a, const double* d, int layers) {
+  for (int l = 0; l < layers; ++l) TRY(nplm_layer_fwd(a + l * FWD_ARGS, d[3 * l], d[3 * l + 1], d[3 * l + 2]));
+  return 0;
+}
+
+extern "C" int nplm_layers_bwd(const long long* a, const double* d, int layers) {
+  for (int l = layers - 1; l >= 0; --l) TRY(nplm_layer_bwd(a + l * BWD_ARGS, d[3 * l + 2]));
+  return 0;
 }

@@ -222,6 +222,11 @@ class EncoderLayer(nn.Module):
         return x, aux
 
 
+def _stackable(layer) -> bool:
+    """A layer whose own call may be passed by: one of this class, nobody's hooks or forward on it."""
+    return (type(layer) is EncoderLayer and layer.mhc_attn is None and native_layer.unwatched(layer) and layer._plain())
+
+
 class EncoderModel(nn.Module):
     """Embeddings + layers + final norm; forward takes flat ids and a BatchContext."""
 
@@ -252,7 +257,14 @@ class EncoderModel(nn.Module):
         if n > 1:
             x = x.unsqueeze(1).expand(-1, n, -1).contiguous()
         aux_total = None
-        for layer in self.layers:
+        layers = list(self.layers)
+        if n <= 1 and x.is_cuda:    # several layers to a native call, as far as they are plain
+            types = [layer.attention_type for layer in layers]
+            x, done = native_layer.run_stack(layers, _stackable, x, ctx,
+                                             [-1 if t == "full_attention" else cfg.sliding_window for t in types],
+                                             [rope[t] for t in types])
+            layers = layers[done:]
+        for layer in layers:
             lt = layer.attention_type
             window = -1 if lt == "full_attention" else cfg.sliding_window
             x, aux = layer(x, ctx, window, rope[lt])

@@ -107,18 +107,16 @@ class ProtX(EncoderModel):
                 and type(self).forward is ProtX.forward and "forward" not in self.__dict__
                 and not self._forward_hooks and not self._forward_pre_hooks and not _has_any_global_hook())
 
-    def _embed_packed(self, ids: torch.Tensor, mask: torch.Tensor, device):
-        """(hidden states [T, C] of the real tokens, device cu_seqlens, host lengths) of a padded host batch. The
-        padding is dropped on the host, where the lengths are known: ids, positions and offsets go over in one
-        copy from pinned memory and nothing waits for the device."""
-        lens = mask.sum(dim=1).numpy()
-        T, B = int(lens.sum()), len(lens)
+    def _embed_packed(self, ids: np.ndarray, lens: np.ndarray, device):
+        """(hidden states [T, C] of the real tokens, device cu_seqlens, host lengths) of a packed host batch: ids, positions
+        and offsets go over in one copy from pinned memory and nothing waits for the device."""
+        T, B = len(ids), len(lens)
         Tp = (T + 3) // 4 * 4                                  # every part starts on 16 bytes
         host = torch.empty(2 * Tp + B + 1, dtype=torch.int32, pin_memory=True)
         buf = host.numpy()
         cu = np.zeros(B + 1, np.int32)
         np.cumsum(lens, out=cu[1:])
-        buf[:T] = ids.numpy()[mask.numpy().astype(bool)]
+        buf[:T] = ids
         buf[Tp:Tp + T] = np.arange(T, dtype=np.int32) - np.repeat(cu[:-1], lens)
         buf[2 * Tp:] = cu
         dev = host.to(device, non_blocking=True)
@@ -131,8 +129,13 @@ class ProtX(EncoderModel):
                         device: Optional[torch.device] = None) -> list[torch.Tensor]:
         """Mean-pooled (EOS excluded) or per-token embeddings for raw sequences."""
         device = device or next(self.parameters()).device
-        # (walking all modules to set a flag that is set already costs more than several layers' launches)
-        was_training = any(m.training for m in self.modules())
+        # (walking all modules to set a flag that is set already costs more than several layers' launches, and so does
+        # looking at it through `modules()`, which remembers whom it has met)
+        was_training, walk = False, [self]
+        while walk and not was_training:
+            m = walk.pop()
+            was_training = m.training
+            walk += [c for c in m._modules.values() if c is not None]
         restore = self.training
         if was_training:
             self.eval()
@@ -143,20 +146,27 @@ class ProtX(EncoderModel):
             """One copy to the host for all results that wait on the device; every sequence gets its own tensor."""
             nonlocal rows
             if waiting:
-                host = torch.cat([t for t, _ in waiting]).cpu()
+                host = (waiting[0][0] if len(waiting) == 1 else torch.cat([t for t, _ in waiting])).cpu()
                 lens = [n for _, ns in waiting for n in ns]
                 for part in host.split(lens):
                     out.append(part.float() if per_token else part[0].clone())
                 waiting.clear()
                 rows = 0
 
+        direct = packed and type(self.tokenizer) is StudentTokenizer and self.tokenizer.packs()
         for i in range(0, len(sequences), batch_size):
-            enc = self.tokenizer(sequences[i:i + batch_size], padding=True, return_tensors="pt")
-            ids, mask = enc["input_ids"], enc["attention_mask"]
-            # the real tokens first, at least one, then padding
-            if (packed and not ids.is_cuda and bool(mask[:, 0].all())
-                    and bool((mask[:, :-1] >= mask[:, 1:]).all())):
-                h, cu, lens = self._embed_packed(ids, mask, device)
+            batch, flat = sequences[i:i + batch_size], None
+            if direct and type(batch) is list and all(type(t) is str for t in batch):
+                flat = self.tokenizer.pack(batch)
+            else:
+                enc = self.tokenizer(batch, padding=True, return_tensors="pt")
+                ids, mask = enc["input_ids"], enc["attention_mask"]
+                # the real tokens first, at least one, then padding
+                if (packed and not ids.is_cuda and bool(mask[:, 0].all())
+                        and bool((mask[:, :-1] >= mask[:, 1:]).all())):
+                    flat = ids.numpy()[mask.numpy().astype(bool)], mask.sum(dim=1).numpy()
+            if flat is not None:
+                h, cu, lens = self._embed_packed(*flat, device)
                 if per_token:       # the residues' rows, without the trailing </s> of every sequence
                     keep = torch.cat([torch.arange(e - n, e - 1) for n, e in zip(lens, np.cumsum(lens).tolist())])
                     h = h[keep.to(device)]

@@ -580,9 +580,8 @@ def gather_rows(x, idx):
 class _CEFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, W, bias, labels, want_logits):
-        n_valid = (labels >= 0).sum().clamp(min=1).float()
-        inv = (1.0 / n_valid).reshape(1)
-        loss, dlogits, logits = K.ce_fwd(h, W, bias, labels, inv, want_logits)
+        inv, loss = K.ce_count(labels)
+        loss, dlogits, logits = K.ce_fwd(h, W, bias, labels, inv, want_logits, loss)
         ctx.save_for_backward(h, W, dlogits)
         ctx.bias_ref = bias
         ctx.w_ref = W

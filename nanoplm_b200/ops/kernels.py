@@ -414,15 +414,28 @@ def segment_mean(x: torch.Tensor, cu: torch.Tensor, drop_last: int = 0) -> torch
 
 
 # --------------------------------------------------------------------------- cross entropy
-def ce_fwd(h, W, bias, labels, inv_count, want_logits=False):
+def ce_count(labels):
+    """(1 / number of labels >= 0, at least one; 0), fp32 [1] each: what `ce_fwd` takes as inv_count and loss."""
+    _chk(labels, torch.int32, "labels")
+    both = torch.empty(8, dtype=torch.float32, device=labels.device)
+    inv, loss = both[:1], both[4:5]
+    rc = typed("elementwise", "nplm_ce_count", "pippp")(labels.data_ptr(), labels.numel(), inv.data_ptr(), loss.data_ptr(),
+                                                        raw_stream())
+    check_rc(rc, "ce_count")
+    count_launch()
+    return inv, loss
+
+
+def ce_fwd(h, W, bias, labels, inv_count, want_logits=False, loss=None):
     n, C = h.shape
     V = W.shape[0]
     dlogits = torch.empty((n, 32), dtype=torch.float32, device=h.device)
     logits = torch.empty((n, V), dtype=torch.float32, device=h.device) if want_logits else None
-    loss = torch.zeros(1, dtype=torch.float32, device=h.device)
-    rc = lib("elementwise").nplm_ce_fwd(ptr(h), ptr(W), ptr(bias), ptr(labels), ptr(inv_count),
-                                        ptr(dlogits), ptr(logits), ptr(loss), c_int(n), c_int(C),
-                                        c_int(V), stream_ptr())
+    if loss is None:
+        loss = torch.zeros(1, dtype=torch.float32, device=h.device)
+    rc = typed("elementwise", "nplm_ce_fwd", "ppppppppiiip")(
+        h.data_ptr(), W.data_ptr(), _dp(bias), labels.data_ptr(), inv_count.data_ptr(), dlogits.data_ptr(), _dp(logits),
+        loss.data_ptr(), n, C, V, raw_stream())
     check_rc(rc, "ce_fwd")
     count_launch()
     return loss, dlogits, logits
@@ -432,8 +445,9 @@ def ce_bwd(h, W, dlogits, gscale, dW, dbias):
     n, C = h.shape
     V = W.shape[0]
     dh = torch.empty_like(h)
-    rc = lib("elementwise").nplm_ce_bwd(ptr(h), ptr(W), ptr(dlogits), ptr(gscale), ptr(dh), ptr(dW),
-                                        ptr(dbias), c_int(n), c_int(C), c_int(V), stream_ptr())
+    rc = typed("elementwise", "nplm_ce_bwd", "pppppppiiip")(
+        h.data_ptr(), W.data_ptr(), dlogits.data_ptr(), gscale.data_ptr(), dh.data_ptr(), dW.data_ptr(), _dp(dbias), n, C, V,
+        raw_stream())
     check_rc(rc, "ce_bwd")
     count_launch()
     return dh

@@ -58,3 +58,11 @@ def test_decoder_backward(n, C, V, offset, cuda_status):
     # each sum is added to the 1 that is there: 2^-24 of it on top of the sums' own rounding
     assert (dW.double() - 1 - d.t() @ h.double()).abs().max() < 1e-5
     assert (db.double() - 1 - d.sum(0)).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("n", [0, 1, 31, 1024, 1025, 70001])
+def test_label_count(n, cuda_status):
+    from nanoplm_b200.ops import kernels as k
+    labels = torch.randint(-2, 3, (n,), device="cuda", dtype=torch.int32)
+    inv, loss = k.ce_count(labels)
+    assert inv.item() == (1.0 / (labels >= 0).sum().clamp(min=1).float()).item() and loss.item() == 0
