@@ -1159,6 +1159,120 @@ extern "C" int nplm_segment_mean(const void* x, const int* cu, float* out, int B
   return static_cast<int>(cudaGetLastError());
 }
 
+// ------------------------------------------------------------------ padded batches
+// What a padded [B][S] batch needs before its first layer: the kept positions, their ids, the position of each inside its
+// sequence and the sequences' offsets. Three launches and one wait for the token count; composed of tensor operations it was
+// fifteen launches with the GPU idle between them (0.25 ms before the first layer of 9 x 1001 positions). A mask
+// may have holes: a token's position is its rank among the kept ones of its row, as the composition had it.
+namespace nplm {
+template <typename M>
+__global__ void __launch_bounds__(256)
+unpad_count_kernel(const M* __restrict__ mask, int S, int* __restrict__ counts) {
+  grid_chain();
+  __shared__ int part[8];
+  const M* row = mask + static_cast<size_t>(blockIdx.x) * S;
+  int n = 0;
+  for (int s = threadIdx.x; s < S; s += 256) n += row[s] != 0;
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = n;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+    for (int i = 0; i < 8; ++i) total += part[i];
+    counts[blockIdx.x] = total;
+  }
+}
+
+// cu[0 .. B] = running sums of counts[0 .. B - 1], one block
+__global__ void __launch_bounds__(1024)
+running_sum_kernel(const int* __restrict__ counts, int B, int* __restrict__ cu) {
+  grid_chain();
+  __shared__ int warp_sum_[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int before = 0;
+  if (threadIdx.x == 0) cu[0] = 0;
+  for (int b0 = 0; b0 < B; b0 += 1024) {
+    const int b = b0 + threadIdx.x;
+    int v = b < B ? counts[b] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) warp_sum_[warp] = v;
+    __syncthreads();
+    int add = before;
+    for (int i = 0; i < warp; ++i) add += warp_sum_[i];
+    if (b < B) cu[b + 1] = v + add;
+    for (int i = 0; i < 32; ++i) before += warp_sum_[i];
+    __syncthreads();
+  }
+}
+
+template <typename M, typename I>
+__global__ void __launch_bounds__(256)
+unpad_fill_kernel(const M* __restrict__ mask, const I* __restrict__ ids, const int* __restrict__ cu, int S,
+                  long long* __restrict__ index, I* __restrict__ flat, int* __restrict__ pos) {
+  grid_chain();
+  __shared__ int part[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t row = static_cast<size_t>(blockIdx.x) * S;
+  const int first = cu[blockIdx.x];
+  int before = 0;
+  for (int s0 = 0; s0 < S; s0 += 256) {
+    const int s = s0 + threadIdx.x;
+    const bool keep = s < S && mask[row + s] != 0;
+    const unsigned votes = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) part[warp] = __popc(votes);
+    __syncthreads();
+    int rank = before + __popc(votes & ((1u << lane) - 1u));
+    for (int i = 0; i < 8; ++i) {
+      if (i < warp) rank += part[i];
+      before += part[i];
+    }
+    if (keep) {
+      index[first + rank] = static_cast<long long>(row + s);
+      flat[first + rank] = ids[row + s];
+      pos[first + rank] = rank;
+    }
+    __syncthreads();
+  }
+}
+
+template <typename M>
+static int unpad_fill(const void* mask, const void* ids, int id_bytes, const int* cu, int B, int S, long long* index,
+                      void* flat, int* pos, cudaStream_t st) {
+  if (id_bytes == 8)
+    launch_chained(unpad_fill_kernel<M, long long>, B, 256, 0, st, static_cast<const M*>(mask),
+                   static_cast<const long long*>(ids), cu, S, index, static_cast<long long*>(flat), pos);
+  else
+    launch_chained(unpad_fill_kernel<M, int>, B, 256, 0, st, static_cast<const M*>(mask), static_cast<const int*>(ids), cu,
+                   S, index, static_cast<int*>(flat), pos);
+  return static_cast<int>(cudaGetLastError());
+}
+}  // namespace nplm
+
+// mask [B][S] (mask_bytes 1, 4 or 8: bool / integers, kept where not zero); counts: int [B] scratch, cu: int [B + 1].
+extern "C" int nplm_unpad_count(const void* mask, int mask_bytes, int B, int S, int* counts, int* cu, cudaStream_t st) {
+  if (B <= 0 || S <= 0) return -3;
+  if (mask_bytes == 1) launch_chained(unpad_count_kernel<signed char>, B, 256, 0, st, static_cast<const signed char*>(mask), S, counts);
+  else if (mask_bytes == 4) launch_chained(unpad_count_kernel<int>, B, 256, 0, st, static_cast<const int*>(mask), S, counts);
+  else if (mask_bytes == 8) launch_chained(unpad_count_kernel<long long>, B, 256, 0, st, static_cast<const long long*>(mask), S, counts);
+  else return -3;
+  launch_chained(running_sum_kernel, 1, 1024, 0, st, counts, B, cu);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// ids [B][S] (id_bytes 4 or 8) -> flat ids, int64 indices into B * S and int positions of the kept tokens.
+extern "C" int nplm_unpad_fill(const void* mask, int mask_bytes, const void* ids, int id_bytes, const int* cu, int B, int S,
+                               long long* index, void* flat, int* pos, cudaStream_t st) {
+  if (B <= 0 || S <= 0 || (id_bytes != 4 && id_bytes != 8)) return -3;
+  if (mask_bytes == 1) return nplm::unpad_fill<signed char>(mask, ids, id_bytes, cu, B, S, index, flat, pos, st);
+  if (mask_bytes == 4) return nplm::unpad_fill<int>(mask, ids, id_bytes, cu, B, S, index, flat, pos, st);
+  if (mask_bytes == 8) return nplm::unpad_fill<long long>(mask, ids, id_bytes, cu, B, S, index, flat, pos, st);
+  return -3;
+}
+
 extern "C" int nplm_gather_rows(const void* src, const int* idx, void* dst, int n, int C,
                                 cudaStream_t st) {
   if (n <= 0) return 0;

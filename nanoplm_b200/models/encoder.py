@@ -370,6 +370,10 @@ class ProtEncoderMLM(nn.Module):
         B, S = input_ids.shape
         if attention_mask is None:
             attention_mask = torch.ones_like(input_ids)
+        if cu_seqlens is None and ops.unpad_takes(input_ids, attention_mask):
+            flat_ids, indices, position_ids, cu_seqlens = ops.unpad(input_ids, attention_mask)
+            flat_labels = labels.reshape(-1)[indices] if labels is not None else None
+            return flat_ids, flat_labels, cu_seqlens, position_ids, (indices, B, S)
         keep = attention_mask.reshape(-1).bool()
         indices = torch.nonzero(keep, as_tuple=False).flatten()
         flat_ids = input_ids.reshape(-1)[indices]

@@ -17,6 +17,7 @@ from nanoplm_b200.config.schema import StudentConfig
 from nanoplm_b200.data.tokenizer import StudentTokenizer
 from nanoplm_b200.models.encoder import (BatchContext, EncoderModel, Linear, Norm,
                                          position_ids_from_cu_seqlens)
+from nanoplm_b200.ops import functional as ops
 from nanoplm_b200.ops import kernels as K
 
 
@@ -55,11 +56,14 @@ class ProtX(EncoderModel):
             B, S = input_ids.shape
             if attention_mask is None:
                 attention_mask = torch.ones_like(input_ids)
-            keep = attention_mask.reshape(-1).bool()
-            indices = torch.nonzero(keep, as_tuple=False).flatten()
-            ids = input_ids.reshape(-1)[indices]
-            lens = attention_mask.sum(dim=-1, dtype=torch.int32)
-            cu_seqlens = F.pad(torch.cumsum(lens, 0, dtype=torch.int32), (1, 0))
+            if position_ids is None and ops.unpad_takes(input_ids, attention_mask):
+                ids, indices, position_ids, cu_seqlens = ops.unpad(input_ids, attention_mask)
+            else:
+                keep = attention_mask.reshape(-1).bool()
+                indices = torch.nonzero(keep, as_tuple=False).flatten()
+                ids = input_ids.reshape(-1)[indices]
+                lens = attention_mask.sum(dim=-1, dtype=torch.int32)
+                cu_seqlens = F.pad(torch.cumsum(lens, 0, dtype=torch.int32), (1, 0))
             pad_info = (indices, B, S)
         else:
             ids = input_ids

@@ -518,6 +518,9 @@ def attention_out_proj(qkv, w_out, residual, seq_start, seq_end, H: int, D: int,
                   residual=residual)
 
 
+unpad_takes, unpad = K.unpad_takes, K.unpad
+
+
 def seq_bounds(cu_seqlens: torch.Tensor, T: int):
     """Per-token [start, end) of the sequence each flat token belongs to."""
     if cu_seqlens.is_cuda:

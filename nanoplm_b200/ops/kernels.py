@@ -33,6 +33,10 @@ def _dp(t: torch.Tensor | None):
     return None if t is None else t.data_ptr()
 
 
+def _is_tracing() -> bool:
+    return torch._C._is_tracing()
+
+
 def _rowmajor(t: torch.Tensor, name: str) -> int:
     """Returns the row stride of a 2-D tensor whose last dim is contiguous."""
     if t.dim() != 2 or t.stride(1) != 1:
@@ -396,6 +400,38 @@ def scatter_rows_(dst: torch.Tensor, idx: torch.Tensor, src: torch.Tensor) -> to
     check_rc(rc, "scatter_rows")
     count_launch()
     return dst
+
+
+_UNPAD_MASKS = {torch.bool: 1, torch.uint8: 1, torch.int8: 1, torch.int32: 4, torch.int64: 8}
+
+
+def unpad_takes(ids: torch.Tensor, mask: torch.Tensor) -> bool:
+    """Whether `unpad` takes a padded batch: [B, S] integers on one GPU, contiguous, not empty."""
+    return (ids.is_cuda and mask.is_cuda and ids.device == mask.device and ids.dim() == 2 and ids.shape == mask.shape
+            and ids.numel() > 0 and ids.dtype in (torch.int32, torch.int64) and mask.dtype in _UNPAD_MASKS
+            and ids.is_contiguous() and mask.is_contiguous() and not _is_tracing())
+
+
+def unpad(ids: torch.Tensor, mask: torch.Tensor):
+    """(flat ids, indices int64 into the B * S positions, positions int32, cu_seqlens int32 [B + 1]) of the tokens that the
+    mask keeps. Waits for the device once, for their number."""
+    B, S = ids.shape
+    mb = _UNPAD_MASKS[mask.dtype]
+    work = torch.empty(2 * B + 1, dtype=torch.int32, device=ids.device)
+    cu, counts = work[:B + 1], work[B + 1:]
+    rc = typed("elementwise", "nplm_unpad_count", "piiippp")(mask.data_ptr(), mb, B, S, counts.data_ptr(), cu.data_ptr(),
+                                                             raw_stream())
+    check_rc(rc, "unpad_count")
+    T = int(cu[-1])
+    flat = torch.empty(T, dtype=ids.dtype, device=ids.device)
+    index = torch.empty(T, dtype=torch.int64, device=ids.device)
+    pos = torch.empty(T, dtype=torch.int32, device=ids.device)
+    rc = typed("elementwise", "nplm_unpad_fill", "pipipiipppp")(
+        mask.data_ptr(), mb, ids.data_ptr(), ids.element_size(), cu.data_ptr(), B, S, index.data_ptr(), flat.data_ptr(),
+        pos.data_ptr(), raw_stream())
+    check_rc(rc, "unpad_fill")
+    count_launch(3)
+    return flat, index, pos, cu
 
 
 def segment_mean(x: torch.Tensor, cu: torch.Tensor, drop_last: int = 0) -> torch.Tensor:
