@@ -1689,7 +1689,7 @@ static int ws_bwd_impl(const void* qkv, const void* out, const void* dout, const
     const long long total = static_cast<long long>(T) * H * 8;
     long long blocks = (total + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;
-    launch_chained(ws_delta_kernel, static_cast<int>(blocks), 256, 0, st,
+    launch_when(static_cast<long long>(T) * HD <= CHAIN_ELEMENTS, ws_delta_kernel, static_cast<int>(blocks), 256, 0, st,
         reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta, T, H);
   }
   FaWsBwdArgs a;
@@ -1726,7 +1726,7 @@ static int ws_bwd_impl(const void* qkv, const void* out, const void* dout, const
     const long long total = static_cast<long long>(T) * H * 4;
     long long blocks = (total + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;
-    launch_chained(ws_dq_store_kernel, static_cast<int>(blocks), 256, 0, st,
+    launch_when(static_cast<long long>(T) * HD <= CHAIN_ELEMENTS, ws_dq_store_kernel, static_cast<int>(blocks), 256, 0, st,
         dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), T, H, rope_pos, rope_cos, rope_sin);
   }
   return static_cast<int>(cudaGetLastError());

@@ -569,11 +569,17 @@ inline CUresult with_context(Call call) {
   return r;
 }
 
-// kern<<<grid, block, smem, st>>>(args...) for a kernel that calls grid_wait: it may be placed before its predecessor in
-// the stream has finished (see grid_wait).
+// Elements up to which a kernel whose blocks walk fixed shares of its data is chained. Blocks that are placed while the
+// predecessor's leave crowd onto the multiprocessors that are free first, and a crowded one finishes its shares late; past
+// some 10 us that costs more than the gap that the chain closes. The norms of a layer, chained / not, us a training step of the
+// default encoder: 2 600 - 8 704 rows of 1024 13 340 / 13 420, 55 424 rows 68 900 / 67 200.
+constexpr long long CHAIN_ELEMENTS = 16LL << 20;
+
+// kern<<<grid, block, smem, st>>>(args...) for a kernel that calls grid_wait: where `chained`, it may be placed before its
+// predecessor in the stream has finished (see grid_wait).
 template <typename... Params, typename... Args>
-inline cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                  Args&&... args) {
+inline cudaError_t launch_when(bool chained, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -583,8 +589,14 @@ inline cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, dim3 block
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<Args&&>(args)...);
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  Args&&... args) {
+  return launch_when(true, kern, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
 
 inline int current_device_slot() {

@@ -957,7 +957,7 @@ extern "C" int nplm_norm_fwd(const void* x, const int* ids, const void* w, void*
   if (C % 8) return -3;
   const int blocks = (T + 7) / 8 < 148 * 8 ? (T + 7) / 8 : 148 * 8;
 #define CALL(N_)                                                                               \
-  launch_chained(norm_fwd_kernel<N_>, blocks, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), ids,  \
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, norm_fwd_kernel<N_>, blocks, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), ids,  \
                                               reinterpret_cast<const __nv_bfloat16*>(w),       \
                                               reinterpret_cast<__nv_bfloat16*>(y), mean, rstd, \
                                               T, C, eps, rms)
@@ -974,7 +974,7 @@ extern "C" int nplm_norm_bwd(const void* dy, const void* x, const int* ids, cons
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 2) blocks = 148 * 2;   // more blocks only add contention on the dw atomics
 #define CALL(N_)                                                                              \
-  launch_chained(norm_bwd_kernel<N_>, blocks, 256, 0, st,                                                 \
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, norm_bwd_kernel<N_>, blocks, 256, 0, st,                                                 \
       reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x),  \
       ids, reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd,                             \
       reinterpret_cast<const __nv_bfloat16*>(dres), reinterpret_cast<__nv_bfloat16*>(dx), dw, \
@@ -1010,7 +1010,7 @@ extern "C" int nplm_embed_bwd(const void* dy, const void* table, const int* ids,
     NPLM_CUDA_CHECK(cudaFuncSetAttribute(embed_grad_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     configured_on[dev_slot] = true;
   }
-  launch_chained(embed_grad_sums_kernel, dim3(slices, by), 32 * warps, static_cast<size_t>(warps) * table_bytes, st,
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, embed_grad_sums_kernel, dim3(slices, by), 32 * warps, static_cast<size_t>(warps) * table_bytes, st,
                  reinterpret_cast<const __nv_bfloat16*>(dy), ids, scratch, T, C, V);
   launch_chained(embed_grad_finish_kernel, V, 256, 0, st, scratch, reinterpret_cast<const __nv_bfloat16*>(table),
                  reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd, dtable, dw, C, V, rms);
@@ -1022,7 +1022,7 @@ extern "C" int nplm_rope(void* qkv, const int* pos, const float* cos_t, const fl
   if (T <= 0) return 0;
   if (D % 16) return -3;
   const long long total = static_cast<long long>(T) * 2 * H * (D / 16);
-  launch_chained(rope_kernel, grid_for(total, 256), 256, 0, st, reinterpret_cast<__nv_bfloat16*>(qkv), pos,
+  launch_when(static_cast<long long>(T) * 2 * H * D <= CHAIN_ELEMENTS, rope_kernel, grid_for(total, 256), 256, 0, st, reinterpret_cast<__nv_bfloat16*>(qkv), pos,
                                                     cos_t, sin_t, T, H, D, backward ? -1.f : 1.f);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1030,7 +1030,7 @@ extern "C" int nplm_rope(void* qkv, const int* pos, const float* cos_t, const fl
 extern "C" int nplm_swiglu_fwd(const void* pre, void* out, long long T, int I, cudaStream_t st) {
   if (T <= 0) return 0;
   if (I % 8) return -3;
-  launch_chained(swiglu_fwd_kernel, grid_for(T * (I / 8), 256), 256, 0, st,
+  launch_when(T * I <= CHAIN_ELEMENTS, swiglu_fwd_kernel, grid_for(T * (I / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<__nv_bfloat16*>(out), T, I);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1039,7 +1039,7 @@ extern "C" int nplm_swiglu_bwd(const void* pre, const void* dout, void* dpre, lo
                                cudaStream_t st) {
   if (T <= 0) return 0;
   if (I % 8) return -3;
-  launch_chained(swiglu_bwd_kernel, grid_for(T * (I / 8), 256), 256, 0, st,
+  launch_when(T * I <= CHAIN_ELEMENTS, swiglu_bwd_kernel, grid_for(T * (I / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<const __nv_bfloat16*>(dout),
       reinterpret_cast<__nv_bfloat16*>(dpre), T, I);
   return static_cast<int>(cudaGetLastError());
@@ -1048,7 +1048,7 @@ extern "C" int nplm_swiglu_bwd(const void* pre, const void* dout, void* dpre, lo
 extern "C" int nplm_act_fwd(const void* pre, void* out, long long n, int act, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -3;
-  launch_chained(act_fwd_kernel, grid_for(n / 8, 256), 256, 0, st,
+  launch_when(n <= CHAIN_ELEMENTS, act_fwd_kernel, grid_for(n / 8, 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<__nv_bfloat16*>(out), n / 8, act);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1057,7 +1057,7 @@ extern "C" int nplm_act_bwd(const void* pre, const void* dout, void* dpre, long 
                             cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -3;
-  launch_chained(act_bwd_kernel, grid_for(n / 8, 256), 256, 0, st,
+  launch_when(n <= CHAIN_ELEMENTS, act_bwd_kernel, grid_for(n / 8, 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(pre), reinterpret_cast<const __nv_bfloat16*>(dout),
       reinterpret_cast<__nv_bfloat16*>(dpre), n / 8, act);
   return static_cast<int>(cudaGetLastError());
@@ -1277,7 +1277,7 @@ extern "C" int nplm_gather_rows(const void* src, const int* idx, void* dst, int 
                                 cudaStream_t st) {
   if (n <= 0) return 0;
   if (C % 8) return -3;
-  launch_chained(gather_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(n) * C <= CHAIN_ELEMENTS, gather_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(src), idx, reinterpret_cast<__nv_bfloat16*>(dst), n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1286,7 +1286,7 @@ extern "C" int nplm_scatter_rows(const void* src, const int* idx, void* dst, int
                                  cudaStream_t st) {
   if (n <= 0) return 0;
   if (C % 8) return -3;
-  launch_chained(scatter_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(n) * C <= CHAIN_ELEMENTS, scatter_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(src), idx, reinterpret_cast<__nv_bfloat16*>(dst), n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1342,14 +1342,14 @@ extern "C" int nplm_ce_bwd(const void* h, const void* W, const float* dlogits, c
 extern "C" int nplm_sumsq(const float* x, long long n, float* out, cudaStream_t st) {
   if (n <= 0) return 0;
   if (reinterpret_cast<uintptr_t>(x) & 15) return -3;
-  launch_chained(sumsq_kernel, grid_for(n / 4 + 1, 256), 256, 0, st, x, n, out);
+  launch_when(n <= CHAIN_ELEMENTS, sumsq_kernel, grid_for(n / 4 + 1, 256), 256, 0, st, x, n, out);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int nplm_adamw(float* p, float* m, float* v, float* g, void* p_bf16, const float* hyper,
                           const float* sumsq, long long n, int zero_grad, cudaStream_t st) {
   if (n <= 0) return 0;
-  launch_chained(adamw_kernel, grid_for(n, 256), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16),
+  launch_when(n <= CHAIN_ELEMENTS, adamw_kernel, grid_for(n, 256), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16),
                                                  hyper, sumsq, n, zero_grad);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1361,7 +1361,7 @@ extern "C" int nplm_muon_momentum(const float* g, float* m, const long long* off
   if (numel & 3) return -3;
   int bx = grid_for(numel / 4, 256);
   if (bx > 592) bx = 592;
-  launch_chained(muon_momentum_kernel, dim3(bx, n_mat), 256, 0, st, g, m, off, numel, reinterpret_cast<__nv_bfloat16*>(upd),
+  launch_when(n_mat * numel <= CHAIN_ELEMENTS, muon_momentum_kernel, dim3(bx, n_mat), 256, 0, st, g, m, off, numel, reinterpret_cast<__nv_bfloat16*>(upd),
                                                         usq, sumsq, gs, max_norm, mu, nesterov);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1372,7 +1372,7 @@ extern "C" int nplm_muon_apply(float* p, void* p16, const long long* off, int n_
   if (numel & 3) return -3;
   int bx = grid_for(numel / 4, 256);
   if (bx > 592) bx = 592;
-  launch_chained(muon_apply_kernel, dim3(bx, n_mat), 256, 0, st, p, reinterpret_cast<__nv_bfloat16*>(p16), off, numel,
+  launch_when(n_mat * numel <= CHAIN_ELEMENTS, muon_apply_kernel, dim3(bx, n_mat), 256, 0, st, p, reinterpret_cast<__nv_bfloat16*>(p16), off, numel,
                                                      reinterpret_cast<const __nv_bfloat16*>(O), lr, wd, cautious);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1384,7 +1384,7 @@ extern "C" int nplm_adamw_slots(float* p, float* m, float* v, const float* g, vo
   if (n_slots <= 0 || max_numel <= 0) return 0;
   int bx = grid_for(max_numel, 256);
   if (bx > 64) bx = 64;
-  launch_chained(adamw_slots_kernel, dim3(bx, n_slots), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p16), off,
+  launch_when(n_slots * max_numel <= CHAIN_ELEMENTS, adamw_slots_kernel, dim3(bx, n_slots), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p16), off,
                                                         numel, decay, sumsq, gs, max_norm, lr, b1, b2, eps, wd,
                                                         bc1, bc2);
   return static_cast<int>(cudaGetLastError());
@@ -1392,7 +1392,7 @@ extern "C" int nplm_adamw_slots(float* p, float* m, float* v, const float* g, vo
 
 extern "C" int nplm_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
-  launch_chained(cast_f32_to_bf16_kernel, grid_for(n, 256), 256, 0, st, src, reinterpret_cast<__nv_bfloat16*>(dst), n);
+  launch_when(n <= CHAIN_ELEMENTS, cast_f32_to_bf16_kernel, grid_for(n, 256), 256, 0, st, src, reinterpret_cast<__nv_bfloat16*>(dst), n);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1401,7 +1401,7 @@ extern "C" int nplm_masked_mse(const void* s, const void* t, const int* valid,
                                cudaStream_t st) {
   if (T <= 0) return 0;
   if (C % 8) return -3;
-  launch_chained(masked_mse_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, masked_mse_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(s), reinterpret_cast<const __nv_bfloat16*>(t), valid,
       inv_count, reinterpret_cast<__nv_bfloat16*>(ds), loss_sum, T, C);
   return static_cast<int>(cudaGetLastError());

@@ -532,7 +532,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
 #undef NPLM_DWCONV
     return static_cast<int>(cudaGetLastError());
   }
-  launch_chained(dwconv_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, dwconv_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
       reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C,
       KS, flip);
@@ -568,7 +568,7 @@ extern "C" int nplm_dwconv_bwd_w(const void* x, const void* dy, const int* s_sta
 extern "C" int nplm_mhc_read(const void* X, const float* alpha, void* h, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS) return -3;
-  launch_chained(mhc_read_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_read_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(X), alpha, reinterpret_cast<__nv_bfloat16*>(h), T, n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -576,7 +576,7 @@ extern "C" int nplm_mhc_read(const void* X, const float* alpha, void* h, int T, 
 extern "C" int nplm_mhc_mean(const void* X, void* z, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS) return -3;
-  launch_chained(mhc_mean_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_mean_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<__nv_bfloat16*>(z), T, n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -585,7 +585,7 @@ extern "C" int nplm_mhc_dx_combine(const void* g, const float* alpha, const void
                                    int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS || (dh != nullptr && alpha == nullptr)) return -3;
-  launch_chained(mhc_dx_combine_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_dx_combine_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(g), alpha, reinterpret_cast<const __nv_bfloat16*>(dh),
       reinterpret_cast<const __nv_bfloat16*>(dz), reinterpret_cast<__nv_bfloat16*>(dX), T, n, C);
   return static_cast<int>(cudaGetLastError());
@@ -597,7 +597,7 @@ extern "C" int nplm_mhc_write(const void* X, const void* y, const float* R, cons
   if ((C % 8) || n < 1 || n > 4) return -3;
   const int grid = grid_for(static_cast<long long>(T) * (C / 8), 256);
 #define NPLM_MHC_WRITE(N_)                                                                              \
-  launch_chained(mhc_write_kernel<N_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(X),                  \
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_write_kernel<N_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(X),                  \
                                              reinterpret_cast<const __nv_bfloat16*>(y), R, beta,         \
                                              reinterpret_cast<__nv_bfloat16*>(Xn), T, C)
   switch (n) {
@@ -618,7 +618,7 @@ extern "C" int nplm_mhc_bwd(const void* X, const void* y, const float* R, const 
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
 #define NPLM_MHC_BWD(N_)                                                                                  \
-  launch_chained(mhc_bwd_kernel<N_>, blocks, 256, 0, st,                                                               \
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_bwd_kernel<N_>, blocks, 256, 0, st,                                                               \
       reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, alpha, beta, \
       reinterpret_cast<const __nv_bfloat16*>(dXn), reinterpret_cast<const __nv_bfloat16*>(dh),              \
       reinterpret_cast<__nv_bfloat16*>(dX), reinterpret_cast<__nv_bfloat16*>(dy), dR, dalpha, dbeta, T, C)
