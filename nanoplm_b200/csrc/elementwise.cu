@@ -888,7 +888,7 @@ cast_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict
 // (src/nanoplm/distillation/trainer.py:30-40). ds = 2 (s-t) * inv_count for valid rows, else 0.
 __global__ void __launch_bounds__(256)
 masked_mse_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __restrict__ t,
-                  const int* __restrict__ valid, const float* __restrict__ inv_count,
+                  const int* __restrict__ valid, const long long* __restrict__ rows, const float* __restrict__ inv_count,
                   __nv_bfloat16* __restrict__ ds, float* __restrict__ loss_sum, int T, int C) {
   grid_chain();
   const int vec = C >> 3;
@@ -903,7 +903,7 @@ masked_mse_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __re
     if (valid == nullptr || valid[r]) {
       float a[8], b[8];
       load8(s + static_cast<size_t>(r) * C + c, a);
-      load8(t + static_cast<size_t>(r) * C + c, b);
+      load8(t + static_cast<size_t>(rows == nullptr ? r : rows[r]) * C + c, b);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float d = a[e] - b[e];
@@ -1396,13 +1396,14 @@ extern "C" int nplm_cast_f32_bf16(const float* src, void* dst, long long n, cuda
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int nplm_masked_mse(const void* s, const void* t, const int* valid,
+// rows (may be null): row r of s is compared with row rows[r] of t
+extern "C" int nplm_masked_mse(const void* s, const void* t, const int* valid, const long long* rows,
                                const float* inv_count, void* ds, float* loss_sum, int T, int C,
                                cudaStream_t st) {
   if (T <= 0) return 0;
   if (C % 8) return -3;
   launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, masked_mse_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(s), reinterpret_cast<const __nv_bfloat16*>(t), valid,
-      inv_count, reinterpret_cast<__nv_bfloat16*>(ds), loss_sum, T, C);
+      rows, inv_count, reinterpret_cast<__nv_bfloat16*>(ds), loss_sum, T, C);
   return static_cast<int>(cudaGetLastError());
 }

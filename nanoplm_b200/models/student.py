@@ -18,6 +18,7 @@ from nanoplm_b200.data.tokenizer import StudentTokenizer
 from nanoplm_b200.models.encoder import (BatchContext, EncoderModel, Linear, Norm,
                                          position_ids_from_cu_seqlens)
 from nanoplm_b200.ops import functional as ops
+from nanoplm_b200.ops import functional as ops
 from nanoplm_b200.ops import kernels as K
 
 
@@ -51,6 +52,16 @@ class ProtX(EncoderModel):
                 position_ids=None):
         """Padded (B, S) or flat ids. Returns {"last_hidden_state"} in the input's layout; with
         training_mode the projected + normed states (teacher width)."""
+        x, pad_info = self._states(input_ids, attention_mask, training_mode, cu_seqlens, position_ids)
+        if pad_info is not None:
+            indices, B, S = pad_info
+            full = torch.zeros((B * S, x.shape[-1]), dtype=x.dtype, device=x.device)
+            full = full.index_copy(0, indices, x)
+            x = full.view(B, S, -1)
+        return {"last_hidden_state": x}
+
+    def _states(self, input_ids, attention_mask, training_mode, cu_seqlens=None, position_ids=None):
+        """(states of the real tokens [T, width], (their indices, B, S) of a padded batch or None)."""
         pad_info = None
         if input_ids.dim() == 2:
             B, S = input_ids.shape
@@ -74,12 +85,18 @@ class ProtX(EncoderModel):
         x, _ = EncoderModel.forward(self, ids, ctx)
         if training_mode and self.proj is not None:
             x = self.proj_norm(self.proj(x))
-        if pad_info is not None:
-            indices, B, S = pad_info
-            full = torch.zeros((B * S, x.shape[-1]), dtype=x.dtype, device=x.device)
-            full = full.index_copy(0, indices, x)
-            x = full.view(B, S, -1)
-        return {"last_hidden_state": x}
+        return x, pad_info
+
+    def packed_states(self, input_ids, attention_mask):
+        """(states in the training mode [T, width], int64 indices of their rows among the B * S positions) of a padded batch
+        on a GPU, for callers that need no padded output; None where somebody observes calls of this module."""
+        if not (type(self).forward is ProtX.forward and "forward" not in self.__dict__ and not self._forward_hooks
+                and not self._forward_pre_hooks and not self._backward_hooks and not self._backward_pre_hooks
+                and not _has_any_global_hook() and self.final_norm.weight.dtype == torch.bfloat16
+                and input_ids.dim() == 2 and ops.unpad_takes(input_ids, attention_mask)):
+            return None
+        x, (indices, _, _) = self._states(input_ids, attention_mask, True)
+        return x, indices
 
     # ---- utilities of the reference student (model.py:111-497) ---------------------------------
     def num_parameters(self) -> int:

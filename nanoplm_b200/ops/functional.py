@@ -626,7 +626,12 @@ def mlm_cross_entropy(h, W, bias, labels, want_logits: bool = False):
 
 class _MSEFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, s, t, valid):
+    def forward(ctx, s, t, valid, rows=None):
+        if rows is not None:
+            inv = torch.full((1,), 1.0 / max(1, s.shape[0]), dtype=torch.float32, device=s.device)
+            loss, ds = K.masked_mse(s, t, None, inv, want_grad=True, rows=rows)
+            ctx.save_for_backward(ds)
+            return loss.squeeze(0)
         v32 = None if valid is None else valid.to(torch.int32).contiguous()
         n = (v32.sum() if v32 is not None else torch.tensor(s.shape[0], device=s.device)).clamp(min=1).float()
         inv = (1.0 / n).reshape(1)
@@ -637,7 +642,13 @@ class _MSEFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         (ds,) = ctx.saved_tensors
-        return ds * dloss.to(ds.dtype), None, None
+        return ds * dloss.to(ds.dtype), None, None, None
+
+
+def masked_mse_rows(student, teacher, rows):
+    """masked_mse of packed rows: student [T, C] bf16 on a GPU against rows `rows` (int64 [T]) of teacher [N, C]; the mean is
+    over all T. Neither a padded copy of the student's states nor of its gradient is made."""
+    return _MSEFn.apply(student.contiguous(), teacher.to(BF).contiguous(), None, rows)
 
 
 def masked_mse(student, teacher, valid=None):

@@ -562,11 +562,12 @@ def cast_f32_bf16_(src: torch.Tensor, dst: torch.Tensor) -> None:
     count_launch()
 
 
-def masked_mse(s, t, valid, inv_count, want_grad=True):
+def masked_mse(s, t, valid, inv_count, want_grad=True, rows=None):
+    """rows (int64 [T], contiguous): row r of s is compared with row rows[r] of t."""
     T, C = s.shape
     ds = torch.empty_like(s) if want_grad else None
     loss = torch.zeros(1, dtype=torch.float32, device=s.device)
-    rc = lib("elementwise").nplm_masked_mse(ptr(s), ptr(t), ptr(valid), ptr(inv_count), ptr(ds),
+    rc = lib("elementwise").nplm_masked_mse(ptr(s), ptr(t), ptr(valid), ptr(rows), ptr(inv_count), ptr(ds),
                                             ptr(loss), c_int(T), c_int(C), stream_ptr())
     check_rc(rc, "masked_mse")
     count_launch()

@@ -69,6 +69,13 @@ def distillation_loss(student: ProtX, batch: dict, teacher=None) -> torch.Tensor
         with torch.no_grad():
             target = teacher(batch["teacher_input_ids"], batch["teacher_attention_mask"],
                              lengths=batch.get("teacher_lengths"))
+    packed = None
+    if isinstance(student, ProtX) and torch.is_tensor(mask) and target.is_cuda and target.shape[:2] == ids.shape:
+        width = student.config.hidden_size if student.proj is None else student.proj.out_features
+        if target.dim() == 3 and target.shape[2] == width and width % 8 == 0:
+            packed = student.packed_states(ids, mask)
+    if packed is not None:      # only the real tokens' states and gradients exist
+        return ops.masked_mse_rows(packed[0], target.reshape(-1, target.shape[2]), packed[1])
     out = student(ids, mask, training_mode=True)["last_hidden_state"]
     B, S, D = out.shape
     return ops.masked_mse(out.reshape(B * S, D), target.reshape(B * S, D).to(out.dtype), mask.reshape(-1))
