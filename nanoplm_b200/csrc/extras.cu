@@ -80,77 +80,96 @@ dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   }
 }
 
-// Same convolution with the kernel size known at compile time: a thread owns 8 channels of
-// DW_TT consecutive tokens, keeps its 8 x KS weights in registers and walks the DW_TT + KS - 1 input
-// rows once (the general kernel above re-reads KS rows and 8 x KS scalar weights per output row).
-constexpr int DW_TT = 8;
+// Kernel size known at compile time: a warp owns 128 channels (a lane four: one 256-byte request a row) of a run of
+// consecutive tokens and slides over them, the KS rows around a token and the weights in registers, four rows loaded
+// ahead (eight: 17.5 us, fewer warps fit). Every row is read once but for KS - 1 at the ends of a run; tokens whose whole window lies inside their sequence (all
+// but KS - 1 of it) take no masks. 17 024 x 768, 7 taps: 24.8 -> 16.4 us; 55 424 x 1024 110 -> 83 (2.7 TB/s: bound by the latency of the
+// rows, 16 warps a multiprocessor). The form before, eight
+// channels x eight tokens a thread, read 14 rows for eight and ran one block of 243 registers a multiprocessor.
+constexpr int DW_CH = 4, DW_AHEAD = 4;
+
+__device__ __forceinline__ void ld4(const __nv_bfloat16* p, float2 (&f)[2]) {
+  const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+  f[0] = unpack_bf16x2(u.x);
+  f[1] = unpack_bf16x2(u.y);
+}
+
+// rows[j] = x[t - R + j] of this lane's channels for j in [from, KS - 1 + DW_AHEAD), zero outside the tensor
+template <int KS, int FROM>
+__device__ __forceinline__ void dw_load(const __nv_bfloat16* __restrict__ x, int t, int T, int C, int c,
+                                        float2 (&rows)[KS - 1 + DW_AHEAD][2]) {
+#pragma unroll
+  for (int j = FROM; j < KS - 1 + DW_AHEAD; ++j) {
+    const int src = t - KS / 2 + j;
+    if (src >= 0 && src < T) ld4(x + static_cast<size_t>(src) * C + c, rows[j]);
+    else rows[j][0] = rows[j][1] = make_float2(0.f, 0.f);
+  }
+}
 
 template <int KS>
-__global__ void __launch_bounds__(256)
-dwconv_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                   const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
-                   const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip) {
+__global__ void __launch_bounds__(256, 2)
+dwconv_run_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                  const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
+                  const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip, int run) {
   grid_chain();
   constexpr int R = KS / 2;
-  const int vec = C >> 3;
-  const int n_tb = (T + DW_TT - 1) / DW_TT;
-  const long long total = static_cast<long long>(n_tb) * vec;
-  for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int t0 = static_cast<int>(idx / vec) * DW_TT;
-    const int c = static_cast<int>(idx % vec) * 8;
-    // all loads of the thread are issued before the first use: DW_TT + KS - 1 input rows (16 bytes
-    // each, zero outside the tensor) and the 8 x KS weights, which are contiguous in w[C][KS]
-    uint4 xr[DW_TT + KS - 1];
+  const int lane = threadIdx.x & 31;
+  const int c = (blockIdx.y * 32 + lane) * DW_CH;
+  const bool on = c < C;
+  const int cc = on ? c : 0;          // (every lane takes part in the shuffles below)
+  const int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * run, t1 = min(T, t0 + run);
+  if (t0 >= t1) return;
+  float2 wt[KS][2], b4[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-    for (int j = 0; j < DW_TT + KS - 1; ++j) {
-      const int src = t0 - R + j;
-      xr[j] = (src >= 0 && src < T) ? __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(src) * C + c))
-                                    : make_uint4(0u, 0u, 0u, 0u);
+  for (int k = 0; k < KS; ++k) {
+    const __nv_bfloat16* p = w + static_cast<size_t>(cc) * KS + (flip ? KS - 1 - k : k);
+    wt[k][0] = make_float2(__bfloat162float(p[0]), __bfloat162float(p[KS]));
+    wt[k][1] = make_float2(__bfloat162float(p[2 * KS]), __bfloat162float(p[3 * KS]));
+  }
+  if (bias != nullptr && !flip) {
+    b4[0] = make_float2(__bfloat162float(bias[cc]), __bfloat162float(bias[cc + 1]));
+    b4[1] = make_float2(__bfloat162float(bias[cc + 2]), __bfloat162float(bias[cc + 3]));
+  }
+  float2 rows[KS - 1 + DW_AHEAD][2];
+  dw_load<KS, 0>(x, t0, T, C, cc, rows);
+  for (int t = t0; t < t1; t += DW_AHEAD) {
+    int lo = 0, hi = 0;
+    if (lane < DW_AHEAD && t + lane < t1) {
+      lo = s_start[t + lane];
+      hi = s_end[t + lane];
     }
-    uint4 wr[KS];      // 8 channels x KS taps = 8 * KS bf16 = KS 16-byte words (c is a multiple of 8)
 #pragma unroll
-    for (int q = 0; q < KS; ++q) wr[q] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(c) * KS) + q);
-    float wt[KS][8];   // wt[k][e]: weight of tap k (already flipped for the input gradient)
-    {
-      const __nv_bfloat16* wl = reinterpret_cast<const __nv_bfloat16*>(wr);
+    for (int i = 0; i < DW_AHEAD; ++i) {
+      const int a = __shfl_sync(0xffffffffu, lo, i), b = __shfl_sync(0xffffffffu, hi, i);
+      if (t + i < t1) {
+        float2 acc[2] = {b4[0], b4[1]};
+        if (t + i - R >= a && t + i + R < b) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
+          for (int k = 0; k < KS; ++k)
 #pragma unroll
-        for (int k = 0; k < KS; ++k) wt[k][e] = __bfloat162float(wl[e * KS + (flip ? KS - 1 - k : k)]);
-    }
-    float acc[DW_TT][8];
-    int lo[DW_TT], hi[DW_TT];
-    float b8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (bias != nullptr && !flip) ld8(bias + c, b8);
+            for (int e = 0; e < 2; ++e) acc[e] = fma2(rows[i + k][e], wt[k][e], acc[e]);
+        } else {
 #pragma unroll
-    for (int i = 0; i < DW_TT; ++i) {
-      const int t = t0 + i;
-      lo[i] = t < T ? s_start[t] : 0;
-      hi[i] = t < T ? s_end[t] : 0;
+          for (int k = 0; k < KS; ++k) {
+            const int src = t + i + k - R;
+            if (src >= a && src < b) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[i][e] = b8[e];
-    }
-    // output t0 + i takes input row src with tap k = src - (t0 + i) + R (after the flip both
-    // directions read "tap k at offset k - R"); rows outside [lo, hi) belong to another sequence
-#pragma unroll
-    for (int j = 0; j < DW_TT + KS - 1; ++j) {
-      const int src = t0 - R + j;
-      float xv[8];
-      unpack8x(xr[j], xv);
-#pragma unroll
-      for (int i = 0; i < DW_TT; ++i) {
-        const int k = j - i;   // = src - (t0 + i) + R
-        if (k >= 0 && k < KS) {
-          const float m = (src >= lo[i] && src < hi[i]) ? 1.f : 0.f;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[i][e] += m * xv[e] * wt[k][e];
+              for (int e = 0; e < 2; ++e) acc[e] = fma2(rows[i + k][e], wt[k][e], acc[e]);
+            }
+          }
         }
+        if (on)
+          *reinterpret_cast<uint2*>(y + static_cast<size_t>(t + i) * C + c) =
+              make_uint2(pack_bf16x2(acc[0].x, acc[0].y), pack_bf16x2(acc[1].x, acc[1].y));
       }
     }
+    if (t + DW_AHEAD < t1) {
 #pragma unroll
-    for (int i = 0; i < DW_TT; ++i)
-      if (t0 + i < T) st8(y + static_cast<size_t>(t0 + i) * C + c, acc[i]);
+      for (int j = 0; j < KS - 1; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) rows[j][e] = rows[j + DW_AHEAD][e];
+      dw_load<KS, KS - 1>(x, t + DW_AHEAD, T, C, cc, rows);
+    }
   }
 }
 
@@ -199,62 +218,93 @@ dwconv_bwd_w_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
   }
 }
 
-// Weight gradient with the kernel size known at compile time: same block shape, but a token lane
-// walks one contiguous run of the slab and keeps the KS input values around the current token in
-// registers, so a token costs one x and one dy load instead of KS + 1.
+// Weight gradient with the kernel size known at compile time: warps slide over runs of tokens as above, with the 4 x (KS +
+// 1) sums of a lane's channels in registers; the eight warps of a block meet in shared memory. 17 024 x 768, 7 taps: 51 ->
+// 18.6 us, 55 424 x 1024 220 -> 91; with one channel a lane a warp's requests were 64 bytes and its loads waited for one another.
 template <int KS>
-__global__ void __launch_bounds__(256)
-dwconv_bwd_w_tile_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                         const int* __restrict__ s_start, const int* __restrict__ s_end,
-                         float* __restrict__ dw, float* __restrict__ dbias, int T, int C,
-                         int tokens_per_block) {
+__global__ void __launch_bounds__(256, 2)
+dwconv_bwd_w_run_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+                        const int* __restrict__ s_start, const int* __restrict__ s_end,
+                        float* __restrict__ dw, float* __restrict__ dbias, int T, int C, int run) {
   grid_chain();
   constexpr int R = KS / 2;
-  __shared__ float red[8][32][KS + 1];
-  const int cl = threadIdx.x & 31;       // channel lane
-  const int tl = threadIdx.x >> 5;       // token lane
-  const int c = blockIdx.y * 32 + cl;
-  float acc[KS + 1];
+  __shared__ float4 red[8][KS + 1][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = (blockIdx.y * 32 + lane) * DW_CH;
+  const int cc = c < C ? c : 0;
+  const int t0 = (blockIdx.x * 8 + warp) * run, t1 = min(T, t0 + run);
+  float2 acc[KS + 1][2];
 #pragma unroll
-  for (int k = 0; k <= KS; ++k) acc[k] = 0.f;
-  const int run = (tokens_per_block + 7) / 8;
-  const int ts = blockIdx.x * tokens_per_block + tl * run;
-  const int te = min(min(T, ts + run), (static_cast<int>(blockIdx.x) + 1) * tokens_per_block);
-  if (c < C && ts < te) {
-    float win[KS];   // x[t - R .. t + R] of channel c
+  for (int k = 0; k <= KS; ++k) acc[k][0] = acc[k][1] = make_float2(0.f, 0.f);
+  if (t0 < t1) {
+    float2 rows[KS - 1 + DW_AHEAD][2];
+    dw_load<KS, 0>(x, t0, T, C, cc, rows);
+    for (int t = t0; t < t1; t += DW_AHEAD) {
+      uint2 g[DW_AHEAD];
 #pragma unroll
-    for (int k = 0; k < KS; ++k) {
-      const int src = ts - R + k;
-      win[k] = (src >= 0 && src < T) ? __bfloat162float(x[static_cast<size_t>(src) * C + c]) : 0.f;
-    }
-    for (int t = ts; t < te; ++t) {
-      const float g = __bfloat162float(dy[static_cast<size_t>(t) * C + c]);
-      const int a = s_start[t], b = s_end[t];
-      const int nsrc = t + 1 + R;
-      const float nx = nsrc < T ? __bfloat162float(x[static_cast<size_t>(nsrc) * C + c]) : 0.f;
-      acc[KS] += g;
-#pragma unroll
-      for (int k = 0; k < KS; ++k) {
-        const int src = t + k - R;
-        if (src >= a && src < b) acc[k] += g * win[k];
+      for (int i = 0; i < DW_AHEAD; ++i)
+        g[i] = t + i < t1 ? __ldg(reinterpret_cast<const uint2*>(dy + static_cast<size_t>(t + i) * C + cc))
+                          : make_uint2(0u, 0u);
+      int lo = 0, hi = 0;
+      if (lane < DW_AHEAD && t + lane < t1) {
+        lo = s_start[t + lane];
+        hi = s_end[t + lane];
       }
 #pragma unroll
-      for (int k = 0; k + 1 < KS; ++k) win[k] = win[k + 1];
-      win[KS - 1] = nx;
+      for (int i = 0; i < DW_AHEAD; ++i) {
+        const int a = __shfl_sync(0xffffffffu, lo, i), b = __shfl_sync(0xffffffffu, hi, i);
+        const float2 gv[2] = {unpack_bf16x2(g[i].x), unpack_bf16x2(g[i].y)};
+        if (t + i < t1) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) acc[KS][e] = add2(acc[KS][e], gv[e]);
+          if (t + i - R >= a && t + i + R < b) {
+#pragma unroll
+            for (int k = 0; k < KS; ++k)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) acc[k][e] = fma2(gv[e], rows[i + k][e], acc[k][e]);
+          } else {
+#pragma unroll
+            for (int k = 0; k < KS; ++k) {
+              const int src = t + i + k - R;
+              if (src >= a && src < b) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) acc[k][e] = fma2(gv[e], rows[i + k][e], acc[k][e]);
+              }
+            }
+          }
+        }
+      }
+      if (t + DW_AHEAD < t1) {
+#pragma unroll
+        for (int j = 0; j < KS - 1; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) rows[j][e] = rows[j + DW_AHEAD][e];
+        dw_load<KS, KS - 1>(x, t + DW_AHEAD, T, C, cc, rows);
+      }
     }
   }
 #pragma unroll
-  for (int k = 0; k <= KS; ++k) red[tl][cl][k] = acc[k];
+  for (int k = 0; k <= KS; ++k) red[warp][k][lane] = make_float4(acc[k][0].x, acc[k][0].y, acc[k][1].x, acc[k][1].y);
   __syncthreads();
-  if (tl == 0 && c < C) {
+  for (int i = threadIdx.x; i < (KS + 1) * 32 * DW_CH; i += 256) {
+    const int k = i / (32 * DW_CH), ch = blockIdx.y * 32 * DW_CH + i % (32 * DW_CH);
+    if (ch >= C) continue;
+    const float* p = reinterpret_cast<const float*>(&red[0][k][0]) + i % (32 * DW_CH);
+    float sum = 0.f;
 #pragma unroll
-    for (int k = 0; k <= KS; ++k) {
-      float sum = 0.f;
-      for (int j = 0; j < 8; ++j) sum += red[j][cl][k];
-      if (k < KS) atomicAdd(&dw[c * KS + k], sum);
-      else if (dbias != nullptr) atomicAdd(&dbias[c], sum);
-    }
+    for (int j = 0; j < 8; ++j) sum += p[j * (KS + 1) * 32 * DW_CH];
+    if (k < KS) atomicAdd(&dw[ch * KS + k], sum);
+    else if (dbias != nullptr) atomicAdd(&dbias[ch], sum);
   }
+}
+
+// Tokens a warp walks: as many as leave the two blocks of eight warps that a multiprocessor holds (more blocks wait for a
+// second round: 17 024 x 768 22 us with three), in whole batches of rows loaded ahead, 16 at least (a run reads KS - 1 rows more than it has) and 256 at most.
+static int dw_run(int T, int C) {
+  const long long groups = (C + 127) / 128;
+  long long run = (T * groups + 148 * 2 * 8 - 1) / (148 * 2 * 8);
+  run = (run + DW_AHEAD - 1) / DW_AHEAD * DW_AHEAD;
+  return static_cast<int>(run < 16 ? 16 : (run > 256 ? 256 : run));
 }
 
 // ---------------------------------------------------------------------------- mHC
@@ -352,7 +402,9 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {
 //   dy[t][:]     = sum_i beta[t][i] dXn[t][i][:]
 //   dR[t][i][j]  = <dXn[t][i], X[t][j]>,  dbeta[t][i] = <dXn[t][i], y[t]>,  dalpha[t][j] = <dh[t], X[t][j]>
 // All loads of a 256-channel slice are issued before the first use and kept packed in registers.
-template <int N>
+// WRITE / READ: which parts there are. As run-time flags the read part alone (what a training step asks for beside the
+// write part) carried the write part's N x N sums along, on zeros: 17 024 x 4 x 768 53 -> 27 us, the write part alone 70 -> 61.
+template <int N, bool WRITE, bool READ>
 __global__ void __launch_bounds__(256, 2)
 mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ y,
                const float* __restrict__ R, const float* __restrict__ alpha, const float* __restrict__ beta,
@@ -363,7 +415,7 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
   static_assert(N * N + 2 * N <= 32, "too many streams for the warp-transpose reduction");
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
-  const bool has_w = dXn != nullptr, has_r = dh != nullptr;
+  constexpr bool has_w = WRITE, has_r = READ;
   for (int t = blockIdx.x * warps + (threadIdx.x >> 5); t < T; t += gridDim.x * warps) {
     // sums[i * N + j] = dR[i][j], sums[N*N + i] = dbeta[i], sums[N*N + N + j] = dalpha[j]
     float sums[32];
@@ -401,10 +453,12 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
       for (int j = 0; j < N; ++j) {
         float xv[8];
         unpack8x(xr[j], xv);
+        if constexpr (has_r) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sums[N * N + N + j] += hv[e] * xv[e];
+          for (int e = 0; e < 8; ++e) sums[N * N + N + j] += hv[e] * xv[e];
+        }
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
+        for (int i = 0; i < (has_w ? N : 0); ++i) {
           float gv[8];
           unpack8x(gr[i], gv);
 #pragma unroll
@@ -412,7 +466,7 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
         }
       }
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
+      for (int i = 0; i < (has_w ? N : 0); ++i) {
         float gv[8];
         unpack8x(gr[i], gv);
 #pragma unroll
@@ -426,7 +480,6 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
           for (int e = 0; e < 8; ++e) o[j][e] += rc[i][j] * gv[e];
       }
       if (has_w) st8(dy + static_cast<size_t>(t) * C + c, dyv);
-#pragma unroll
       if (dX != nullptr) {
 #pragma unroll
         for (int j = 0; j < N; ++j) st8(dX + (static_cast<size_t>(t) * N + j) * C + c, o[j]);
@@ -516,13 +569,14 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
                            const int* s_end, void* y, int T, int C, int KS, int flip, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || KS < 1 || KS > MAX_KS || !(KS & 1)) return -3;
-  const bool aligned = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
-  if ((KS == 3 || KS == 5 || KS == 7 || KS == 9) && aligned) {   // the tile kernel loads 16-byte words of w
-    const int grid = grid_for(static_cast<long long>((T + DW_TT - 1) / DW_TT) * (C / 8), 256);
+  if ((KS == 3 || KS == 5 || KS == 7 || KS == 9) &&
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 7) == 0) {
+    const int run = dw_run(T, C);
+    const dim3 grid((T + 8 * run - 1) / (8 * run), (C + 127) / 128);
 #define NPLM_DWCONV(KS_)                                                                                   \
-  launch_chained(dwconv_tile_kernel<KS_>, grid, 256, 0, st,                                                            \
-      reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),                \
-      reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip)
+  launch_chained(dwconv_run_kernel<KS_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),      \
+                 reinterpret_cast<const __nv_bfloat16*>(w), reinterpret_cast<const __nv_bfloat16*>(bias),   \
+                 s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip, run)
     switch (KS) {
       case 3: NPLM_DWCONV(3); break;
       case 5: NPLM_DWCONV(5); break;
@@ -543,13 +597,13 @@ extern "C" int nplm_dwconv_bwd_w(const void* x, const void* dy, const int* s_sta
                                  float* dw, float* dbias, int T, int C, int KS, cudaStream_t st) {
   if (T <= 0) return 0;
   if (KS < 1 || KS > MAX_KS || !(KS & 1)) return -3;
-  const int tokens_per_block = 512;
-  dim3 grid((T + tokens_per_block - 1) / tokens_per_block, (C + 31) / 32);
-  if (KS == 3 || KS == 5 || KS == 7 || KS == 9) {
-#define NPLM_DWCONV_W(KS_)                                                                              \
-  launch_chained(dwconv_bwd_w_tile_kernel<KS_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),          \
-                                                      reinterpret_cast<const __nv_bfloat16*>(dy), s_start, \
-                                                      s_end, dw, dbias, T, C, tokens_per_block)
+  if ((KS == 3 || KS == 5 || KS == 7 || KS == 9) && C % DW_CH == 0 &&
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 7) == 0) {
+    const int run = dw_run(T, C);
+    const dim3 grid((T + 8 * run - 1) / (8 * run), (C + 127) / 128);
+#define NPLM_DWCONV_W(KS_)                                                                                   \
+  launch_chained(dwconv_bwd_w_run_kernel<KS_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),  \
+                 reinterpret_cast<const __nv_bfloat16*>(dy), s_start, s_end, dw, dbias, T, C, run)
     switch (KS) {
       case 3: NPLM_DWCONV_W(3); break;
       case 5: NPLM_DWCONV_W(5); break;
@@ -559,6 +613,8 @@ extern "C" int nplm_dwconv_bwd_w(const void* x, const void* dy, const int* s_sta
 #undef NPLM_DWCONV_W
     return static_cast<int>(cudaGetLastError());
   }
+  const int tokens_per_block = 512;
+  const dim3 grid((T + tokens_per_block - 1) / tokens_per_block, (C + 31) / 32);
   launch_chained(dwconv_bwd_w_kernel, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),
                                             reinterpret_cast<const __nv_bfloat16*>(dy), s_start, s_end, dw,
                                             dbias, T, C, KS, tokens_per_block);
@@ -615,10 +671,12 @@ extern "C" int nplm_mhc_bwd(const void* X, const void* y, const float* R, const 
                             float* dR, float* dalpha, float* dbeta, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > 4) return -3;
+  if (dXn == nullptr && dh == nullptr) return 0;
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
 #define NPLM_MHC_BWD(N_)                                                                                  \
-  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_bwd_kernel<N_>, blocks, 256, 0, st,                                                               \
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, dXn != nullptr ? (dh != nullptr ? mhc_bwd_kernel<N_, true, true> : mhc_bwd_kernel<N_, true, false>) \
+                                : mhc_bwd_kernel<N_, false, true>, blocks, 256, 0, st,                                \
       reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, alpha, beta, \
       reinterpret_cast<const __nv_bfloat16*>(dXn), reinterpret_cast<const __nv_bfloat16*>(dh),              \
       reinterpret_cast<__nv_bfloat16*>(dX), reinterpret_cast<__nv_bfloat16*>(dy), dR, dalpha, dbeta, T, C)
