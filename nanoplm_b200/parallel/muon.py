@@ -313,7 +313,10 @@ class MuonEngine(ShardedEngine):
         n = len(st.slots)
         dt = torch.bfloat16 if self.on_cuda else torch.float32
         peer = self.fused is not None
-        if peer:
+        alone = not peer and not self.distributed      # this rank's run is the whole stack: its result is the answer
+        if alone:
+            O = None
+        elif peer:
             index = self.stacks.index(st)
             O = self.fused.stack_buffers[index].tensor.view((n,) + st.shape)
         elif not st.even and self.distributed:
@@ -345,6 +348,8 @@ class MuonEngine(ShardedEngine):
                 mine = mine / (v.sqrt()[:, :, None] + self.muon_eps)
                 scale = 0.2 * math.sqrt(mine[0].numel()) / (mine.flatten(1).norm(dim=1) + self.muon_eps)
                 mine = mine * scale[:, None, None]                                        # rms_norm scaling
+            if alone:
+                return mine.to(dt)
             O[st.lo:st.hi] = mine.to(dt)
         if peer:
             self.fused.push_run(index, st.lo, st.hi - st.lo, st.slots[0].numel)   # visible after the next barrier
