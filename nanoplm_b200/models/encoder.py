@@ -140,12 +140,13 @@ class MLP(nn.Module):
 
 
 class BatchContext:
-    """Per-batch device metadata shared by all layers."""
+    """Per-batch device metadata shared by all layers. bounds: (first key, one past the last key) of every token, int32 [T]
+    each, where the caller has them; else the sequence of `cu_seqlens` that the token lies in."""
 
-    def __init__(self, cu_seqlens: torch.Tensor, position_ids: torch.Tensor, T: int):
+    def __init__(self, cu_seqlens: torch.Tensor, position_ids: torch.Tensor, T: int, bounds: Optional[tuple] = None):
         self.cu_seqlens = cu_seqlens
         self.position_ids = position_ids.to(torch.int32)
-        self.seq_start, self.seq_end = ops.seq_bounds(cu_seqlens, T)
+        self.seq_start, self.seq_end = ops.seq_bounds(cu_seqlens, T) if bounds is None else bounds
         self.T = T
 
 

@@ -22,6 +22,11 @@ from nanoplm_b200.ops import functional as ops
 from nanoplm_b200.ops import kernels as K
 
 
+# Tokens up to which embed_sequences joins batches: their activations (5 to 10 KB a token at 512 to 1024 channels) stay within
+# 350 MB, and longer runs gain nothing more (GEMMs of 32 768 rows fill 256 tiles of 128 rows a column of tiles).
+_EMBED_TOKENS = 32768
+
+
 class ProtX(EncoderModel):
     def __init__(self, cfg: StudentConfig, tokenizer: Optional[StudentTokenizer] = None):
         self.tokenizer = tokenizer or StudentTokenizer()
@@ -128,22 +133,49 @@ class ProtX(EncoderModel):
                 and type(self).forward is ProtX.forward and "forward" not in self.__dict__
                 and not self._forward_hooks and not self._forward_pre_hooks and not _has_any_global_hook())
 
-    def _embed_packed(self, ids: np.ndarray, lens: np.ndarray, device):
-        """(hidden states [T, C] of the real tokens, device cu_seqlens, host lengths) of a packed host batch: ids, positions
-        and offsets go over in one copy from pinned memory and nothing waits for the device."""
+    def _pack_batches(self, batches: list[list[str]]) -> tuple[np.ndarray, np.ndarray, list[bool]]:
+        """(ids, lengths, which of the sequences are real) of several batches one after the other. Every batch starts on a
+        multiple of 256 tokens, behind padding: the attention's tiles then cut a batch where they cut it alone, and the
+        padding has no keys, as rows past the end have none, so that a batch's results have the bits they have alone."""
+        if len(batches) == 1:
+            return *self.tokenizer.pack(batches[0]), [True] * len(batches[0])
+        ids, lens, real = [], [], []
+        for i, b in enumerate(batches):
+            tokens, n = self.tokenizer.pack(b)
+            ids.append(tokens)
+            lens.append(n)
+            real += [True] * len(n)
+            pad = -len(tokens) % 256 if i + 1 < len(batches) else 0
+            if pad:
+                ids.append(np.full(pad, self.tokenizer.pad_token_id, np.int32))
+                lens.append(np.array([pad], np.int32))
+                real.append(False)
+        return np.concatenate(ids), np.concatenate(lens), real
+
+    def _embed_packed(self, ids: np.ndarray, lens: np.ndarray, device, real: list[bool]):
+        """(hidden states [T, C] of the tokens, device cu_seqlens) of a packed host batch: ids, positions, the tokens' key
+        ranges and offsets go over in one copy from pinned memory and nothing waits for the device."""
         T, B = len(ids), len(lens)
         Tp = (T + 3) // 4 * 4                                  # every part starts on 16 bytes
-        host = torch.empty(2 * Tp + B + 1, dtype=torch.int32, pin_memory=True)
+        host = torch.empty(4 * Tp + B + 1, dtype=torch.int32, pin_memory=True)
         buf = host.numpy()
         cu = np.zeros(B + 1, np.int32)
         np.cumsum(lens, out=cu[1:])
+        at = np.arange(T, dtype=np.int32)
+        start, end = np.repeat(cu[:-1], lens), np.repeat(cu[1:], lens)
+        if not all(real):
+            pad = ~np.repeat(np.array(real), lens)
+            start[pad] = end[pad] = at[pad]
         buf[:T] = ids
-        buf[Tp:Tp + T] = np.arange(T, dtype=np.int32) - np.repeat(cu[:-1], lens)
-        buf[2 * Tp:] = cu
+        buf[Tp:Tp + T] = at - start
+        buf[2 * Tp:2 * Tp + T] = start
+        buf[3 * Tp:3 * Tp + T] = end
+        buf[4 * Tp:] = cu
         dev = host.to(device, non_blocking=True)
-        cu_dev = dev[2 * Tp:]
-        h = self(dev[:T], cu_seqlens=cu_dev, position_ids=dev[Tp:Tp + T])["last_hidden_state"]
-        return h, cu_dev, lens.tolist()
+        cu_dev = dev[4 * Tp:]
+        ctx = BatchContext(cu_dev, dev[Tp:Tp + T], T, bounds=(dev[2 * Tp:2 * Tp + T], dev[3 * Tp:3 * Tp + T]))
+        h, _ = EncoderModel.forward(self, dev[:T], ctx)
+        return h, cu_dev
 
     @torch.no_grad()
     def embed_sequences(self, sequences: list[str], batch_size: int = 16, per_token: bool = False,
@@ -152,10 +184,11 @@ class ProtX(EncoderModel):
         device = device or next(self.parameters()).device
         # (walking all modules to set a flag that is set already costs more than several layers' launches, and so does
         # looking at it through `modules()`, which remembers whom it has met)
-        was_training, walk = False, [self]
-        while walk and not was_training:
+        was_training, watched, walk = False, False, [self]
+        while walk:
             m = walk.pop()
-            was_training = m.training
+            was_training |= m.training
+            watched |= bool(m._forward_hooks) or bool(m._forward_pre_hooks) or "forward" in m.__dict__
             walk += [c for c in m._modules.values() if c is not None]
         restore = self.training
         if was_training:
@@ -169,16 +202,34 @@ class ProtX(EncoderModel):
             if waiting:
                 host = (waiting[0][0] if len(waiting) == 1 else torch.cat([t for t, _ in waiting])).cpu()
                 lens = [n for _, ns in waiting for n in ns]
-                for part in host.split(lens):
-                    out.append(part.float() if per_token else part[0].clone())
+                for n, part in zip(lens, host.split([abs(n) for n in lens])):
+                    if n >= 0:                                  # (negative: the mean of a stretch of padding)
+                        out.append(part.float() if per_token else part[0].clone())
                 waiting.clear()
                 rows = 0
 
         direct = packed and type(self.tokenizer) is StudentTokenizer and self.tokenizer.packs()
-        for i in range(0, len(sequences), batch_size):
-            batch, flat = sequences[i:i + batch_size], None
-            if direct and type(batch) is list and all(type(t) is str for t in batch):
-                flat = self.tokenizer.pack(batch)
+        plain = lambda b: type(b) is list and all(type(t) is str for t in b)
+        i, end = 0, len(sequences) if range(0, 1, batch_size) else 0       # (a step of 0 is an error, a negative one no steps)
+        while i < end:
+            batch, flat, real = sequences[i:i + batch_size], None, None
+            i += batch_size
+            if direct and plain(batch):
+                # Packed rows neither know their batch nor pad it: further batches join while they fit, unless a hook on some
+                # part may count them, and a layer's launches fill the chip. 91 proteins of 46 000 tokens at 512 channels took 36
+                # layers of 8 000 rows, one to two waves of tiles a GEMM.
+                joined = [batch]
+                tokens = sum(map(len, batch)) + len(batch)
+                while not watched and i < end:
+                    more = sequences[i:i + batch_size]
+                    if not plain(more):
+                        break
+                    tokens += 255 + sum(map(len, more)) + len(more)
+                    if tokens > _EMBED_TOKENS:
+                        break
+                    joined.append(more)
+                    i += batch_size
+                *flat, real = self._pack_batches(joined)
             else:
                 enc = self.tokenizer(batch, padding=True, return_tensors="pt")
                 ids, mask = enc["input_ids"], enc["attention_mask"]
@@ -187,14 +238,18 @@ class ProtX(EncoderModel):
                         and bool((mask[:, :-1] >= mask[:, 1:]).all())):
                     flat = ids.numpy()[mask.numpy().astype(bool)], mask.sum(dim=1).numpy()
             if flat is not None:
-                h, cu, lens = self._embed_packed(*flat, device)
+                ids, lens = flat
+                real = real or [True] * len(lens)
+                h, cu = self._embed_packed(ids, lens, device, real)
                 if per_token:       # the residues' rows, without the trailing </s> of every sequence
-                    keep = torch.cat([torch.arange(e - n, e - 1) for n, e in zip(lens, np.cumsum(lens).tolist())])
+                    ends = np.cumsum(lens).tolist()
+                    lens = lens.tolist()
+                    keep = torch.cat([torch.arange(e - n, e - 1) for n, e, r in zip(lens, ends, real) if r])
                     h = h[keep.to(device)]
-                    waiting.append((h, [n - 1 for n in lens]))
+                    waiting.append((h, [n - 1 for n, r in zip(lens, real) if r]))
                 else:
                     h = K.segment_mean(h, cu, drop_last=1)
-                    waiting.append((h, [1] * len(lens)))
+                    waiting.append((h, [1 if r else -1 for r in real]))
                 rows += h.shape[0]
                 if rows >= 65536:   # bounds what waits on the device
                     collect()
