@@ -258,6 +258,63 @@ quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, ui
   quant_dual_tile(v, sm, r0, k0, R, K, qr, sr, qt, st);
 }
 
+// Both forms of the gradient of an un-rotated QKV projection from that of the rotated one (x, bf16 [R][K]): 64-wide heads
+// that start below rope_cols are rotated back (in fp32, rounded to bf16, as the separate pass does it in place) on the
+// way. A lane's partner channels, 32 on, are eight lanes away. A warp copies the cos and sin lines of its eight rows to
+// shared memory while its loads of x are in flight (cos lies where the transposed bytes go later). 55 424 x 3072: 165 us in
+// place of 78 + 123; 187 with the lines read row by row behind the row's position, 210 with several tiles a block that
+// share the lines (112 bytes of spills).
+__global__ void __launch_bounds__(DUAL_THREADS, 2)
+rope_quant_dual_kernel(const __nv_bfloat16* __restrict__ x, int R, int K, int ldx, const int* __restrict__ pos,
+                       const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rope_cols,
+                       uint8_t* __restrict__ qr, float* __restrict__ sr, uint8_t* __restrict__ qt, float* __restrict__ st) {
+  grid_chain();
+  __shared__ DualSmem sm;
+  __shared__ alignas(16) float sin_rows[128 * 32];
+  float* cos_rows = reinterpret_cast<float*>(sm.tile);
+  const int r0 = blockIdx.y * 128, k0 = blockIdx.x * 128;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int row_pos = __ldg(pos + r0 + w * DUAL_ROWS + (l & (DUAL_ROWS - 1)));
+  uint2 v[DUAL_ROWS];
+#pragma unroll
+  for (int i = 0; i < DUAL_ROWS; ++i)
+    v[i] = __ldg(reinterpret_cast<const uint2*>(x + static_cast<size_t>(r0 + w * DUAL_ROWS + i) * ldx + k0 + 4 * l));
+  if (k0 < rope_cols) {
+#pragma unroll
+    for (int j = 0; j < DUAL_ROWS; j += 4) {   // four rows at a time, a 16-byte chunk a lane
+      const int i = j + (l >> 3);
+      const size_t from = static_cast<size_t>(__shfl_sync(0xffffffffu, row_pos, i)) * 32 + (l & 7) * 4;
+      const int to = (w * DUAL_ROWS + i) * 32 + (l & 7) * 4;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(cos_rows + to)), "l"(cos_t + from) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(sin_rows + to)), "l"(sin_t + from) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();     // (the other lanes' chunks)
+    const bool rotate = k0 + (l >> 4) * 64 < rope_cols;
+    const bool second = (l & 8) != 0;           // this lane holds the second halves of the pairs
+#pragma unroll
+    for (int i = 0; i < DUAL_ROWS; ++i) {
+      const uint2 o = make_uint2(__shfl_xor_sync(0xffffffffu, v[i].x, 8), __shfl_xor_sync(0xffffffffu, v[i].y, 8));
+      if (rotate) {
+        const int at = (w * DUAL_ROWS + i) * 32 + (l & 7) * 4;
+        const float4 c = *reinterpret_cast<const float4*>(cos_rows + at);
+        float4 s = *reinterpret_cast<const float4*>(sin_rows + at);
+        s = make_float4(-s.x, -s.y, -s.z, -s.w);
+        const float2 m0 = unpack_bf16x2(v[i].x), m1 = unpack_bf16x2(v[i].y), p0 = unpack_bf16x2(o.x), p1 = unpack_bf16x2(o.y);
+        if (second) {
+          v[i].x = pack_bf16x2(m0.x * c.x + p0.x * s.x, m0.y * c.y + p0.y * s.y);
+          v[i].y = pack_bf16x2(m1.x * c.z + p1.x * s.z, m1.y * c.w + p1.y * s.w);
+        } else {
+          v[i].x = pack_bf16x2(m0.x * c.x - p0.x * s.x, m0.y * c.y - p0.y * s.y);
+          v[i].y = pack_bf16x2(m1.x * c.z - p1.x * s.z, m1.y * c.w - p1.y * s.w);
+        }
+      }
+    }
+  }
+  quant_dual_tile(v, sm, r0, k0, R, K, qr, sr, qt, st);
+}
+
 // Both forms of h = bf16(silu(gate) * value) straight from pre = [value | gate] (bf16 [R][2 I]): h, which only e4m3 products
 // read, is neither written nor read back (6 bytes an element of h instead of 10 in two passes; 55 424 x 2048 115 + 105 us ->
 // 125, 5.4 TB/s).
@@ -369,6 +426,8 @@ struct F8Cfg {
   static constexpr int SMEM = OFF_BAR + 512;
 };
 
+__device__ __forceinline__ float2 bf16_rounded(float2 v) { return unpack_bf16x2(pack_bf16x2(v.x, v.y)); }
+
 // What the epilogue does with the finished sums (forms 1 and 2: block-scaled B, bf16 output, plain launches).
 enum : int { F8_PLAIN = 0, F8_ADD = 1, F8_ROPE = 2 };
 
@@ -407,11 +466,13 @@ __device__ __forceinline__ bool f8_wait_shard(const Fp8Args& args, int shard, un
   return true;
 }
 
+// The forms start from the product rounded to bf16, which is what the passes that they replace read: e4m3 training
+// amplifies a last bit of one activation to per cents of a small batch's gradients, so the forms keep every bit.
 // F8_ADD: the residual's tiles (tmR) travel through TMA into the staging tiles while the products run, are added to the
-// fp32 sums and overwritten by the results. F8_ROPE: a thread holds whole heads of its row (64 columns), so the
+// product and overwritten by the results. F8_ROPE: a thread holds whole heads of its row (64 columns), so the
 // rotation is register arithmetic on the row's 32 cos / sin pairs, which wait in the staging tiles too (read from global
-// memory there and then, 32 rows apart, they cost 150 us). 55 424 rows, us: 1024 columns of K = 1024 79 plain, 93 with the
-// residual, 3072 of 1024 238 plain, 267 rotated; the passes over the output that they replace took 57 and 78.
+// memory there and then, 32 rows apart, they cost 150 us). 55 424 rows, us: 1024 columns of K = 1024 79 plain, 95 with the
+// residual, 3072 of 1024 225 plain, 266 rotated; the passes over the output that they replace took 57 and 78.
 template <int BN, bool B_BLOCK, int FORM>
 __global__ void __launch_bounds__(F8_THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -754,11 +815,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             for (int q = 0; q < HC / 64; ++q) {
               if (nh + q * 64 < args.rope_cols) {
                 float2 *a = c + q * 32 + 2 * i, *b = a + 16;
-                const float2 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
-                a[0] = make_float2(a0.x * cs.x - b0.x * sn.x, a0.y * cs.y - b0.y * sn.y);
-                b[0] = make_float2(b0.x * cs.x + a0.x * sn.x, b0.y * cs.y + a0.y * sn.y);
-                a[1] = make_float2(a1.x * cs.z - b1.x * sn.z, a1.y * cs.w - b1.y * sn.w);
-                b[1] = make_float2(b1.x * cs.z + a1.x * sn.z, b1.y * cs.w + a1.y * sn.w);
+                const float2 a0 = bf16_rounded(a[0]), a1 = bf16_rounded(a[1]);
+                const float2 b0 = bf16_rounded(b[0]), b1 = bf16_rounded(b[1]);
+                a[0] = make_float2(fmaf(a0.x, cs.x, -__fmul_rn(b0.x, sn.x)), fmaf(a0.y, cs.y, -__fmul_rn(b0.y, sn.y)));
+                b[0] = make_float2(fmaf(b0.x, cs.x, __fmul_rn(a0.x, sn.x)), fmaf(b0.y, cs.y, __fmul_rn(a0.y, sn.y)));
+                a[1] = make_float2(fmaf(a1.x, cs.z, -__fmul_rn(b1.x, sn.z)), fmaf(a1.y, cs.w, -__fmul_rn(b1.y, sn.w)));
+                b[1] = make_float2(fmaf(b1.x, cs.z, __fmul_rn(a1.x, sn.z)), fmaf(b1.y, cs.w, __fmul_rn(a1.y, sn.w)));
               }
             }
           }
@@ -785,7 +847,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const float2 t = unpack_bf16x2(ow[e]);
-                ow[e] = pack_bf16x2(v[e].x + t.x, v[e].y + t.y);
+                const float2 p = bf16_rounded(v[e]);
+                ow[e] = pack_bf16x2(p.x + t.x, p.y + t.y);
               }
               *at = o;
             }
@@ -1001,6 +1064,21 @@ extern "C" int nplm_fp8_quant_dual(const void* x, int R, int K, int ldx, void* q
   return static_cast<int>(cudaGetLastError());
 }
 
+// Row and transposed row form of x bf16 [R][K] with the rotary embedding of its 64-wide heads below column rope_cols
+// undone; R and K multiples of 128, rope_cols of 64, cos / sin fp32 [max_pos][32].
+extern "C" int nplm_fp8_rope_quant_dual(const void* x, int R, int K, int ldx, const int* pos, const float* cos_t,
+                                        const float* sin_t, int rope_cols, void* qr, float* sr, void* qt, float* st,
+                                        cudaStream_t stream) {
+  if (R <= 0 || K <= 0) return 0;
+  if ((K % 128) || (R % 128) || (ldx % 4) || (reinterpret_cast<uintptr_t>(x) & 7) || R / 128 > 65535 || (rope_cols % 64) ||
+      ((reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15))
+    return -3;
+  launch_chained(rope_quant_dual_kernel, dim3(K / 128, R / 128), DUAL_THREADS, 0, stream,
+                 reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx, pos, cos_t, sin_t, rope_cols,
+                 reinterpret_cast<uint8_t*>(qr), sr, reinterpret_cast<uint8_t*>(qt), st);
+  return static_cast<int>(cudaGetLastError());
+}
+
 // Both e4m3 forms of h = silu(gate) * value, pre = [value | gate] bf16 [R][2 I] contiguous; R, I multiples of 128.
 extern "C" int nplm_fp8_swiglu_quant_dual(const void* pre, int R, int I, void* qr, float* sr, void* qt, float* st,
                                           cudaStream_t stream) {
@@ -1078,7 +1156,8 @@ extern "C" int nplm_gemm_fp8(const void* A, const void* B, void* C, const float*
 }
 
 // bf16 C[M][N] = (A * sa) (B * sb)^T with block-scaled B, plus R (bf16, row stride ldr; may be null), or with the rotary
-// embedding applied to the 64-wide heads that start below rope_cols (rope_pos not null). One rounding.
+// embedding applied to the 64-wide heads that start below rope_cols (rope_pos not null). Either starts from the product
+// rounded to bf16.
 extern "C" int nplm_gemm_fp8_form(const void* A, const void* B, void* C, const void* R, const float* sa, const float* sb,
                                   int M, int N, int K, int ldc, int ldr, const int* rope_pos, const float* rope_cos,
                                   const float* rope_sin, int rope_cols, int* status, cudaStream_t stream) {

@@ -90,11 +90,10 @@ class Attention(nn.Module):
                                               window, self.scale, rope=(ctx.position_ids, rope[0], rope[1]))
             y = ops.attention_varlen(qkv, ctx.seq_start, ctx.seq_end, H, D, window, self.scale,
                                      rope=(ctx.position_ids, rope[0], rope[1]))
-        elif self._fused_fp8(x, ctx, rope):     # the same two places, e4m3 operands
+        elif self._fused_fp8(x, ctx, rope):     # e4m3: in the product's epilogue and in the quantisation of its gradient
             from nanoplm_b200.ops import fp8
             qkv = fp8.fp8_linear(x, self.Wqkv.weight, rope=(ctx.position_ids, rope[0], rope[1], 2 * H * D))
-            y = ops.attention_varlen(qkv, ctx.seq_start, ctx.seq_end, H, D, window, self.scale,
-                                     rope=(ctx.position_ids, rope[0], rope[1]))
+            y = ops.attention_varlen(qkv, ctx.seq_start, ctx.seq_end, H, D, window, self.scale)
         else:
             qkv = self.Wqkv(x)
             qkv = ops.rope_qkv(qkv, ctx.position_ids, rope[0], rope[1], H, D)

@@ -101,6 +101,21 @@ def _dual_buffers(R: int, K: int, dev) -> tuple[Quantized, Quantized]:
             Quantized(torch.empty((K, R), dtype=u8, device=dev), torch.empty((R // 128, K), dtype=f32, device=dev), False))
 
 
+def rope_quant_dual(x: torch.Tensor, rope: tuple) -> tuple[Quantized, Quantized]:
+    """quant_dual of x bf16 [R, K] with the rotary embedding rope = (pos int32 [R], cos, sin fp32 [P, 32], rope_cols) undone
+    on the 64-wide heads below column rope_cols: the gradient of an un-rotated projection from that of the rotated one."""
+    pos, cos, sin, cols = rope
+    R, K = x.shape
+    if x.stride(1) != 1 or x.stride(0) % 4 or x.data_ptr() % 8:
+        x = x.contiguous()
+    r, t = _dual_buffers(R, K, x.device)
+    rc = lib("fp8").nplm_fp8_rope_quant_dual(ptr(x), c_int(R), c_int(K), c_int(x.stride(0)), ptr(pos), ptr(cos), ptr(sin),
+                                             c_int(cols), ptr(r.q), ptr(r.scale), ptr(t.q), ptr(t.scale), stream_ptr())
+    check_rc(rc, "fp8_rope_quant_dual")
+    count_launch()
+    return r, t
+
+
 def swiglu_quant_dual(pre: torch.Tensor) -> tuple[Quantized, Quantized]:
     """quant_dual(swiglu(pre)) for pre = [value | gate] bf16 [R, 2 I] contiguous, R and I multiples of 128."""
     R, I = pre.shape[0], pre.shape[1] // 2
@@ -126,7 +141,8 @@ def swiglu_bwd_quant_dual(pre: torch.Tensor, dh: torch.Tensor) -> tuple[Quantize
 def gemm_fp8_form(a: Quantized, b: Quantized, *, residual: torch.Tensor | None = None,
                   rope: tuple | None = None) -> torch.Tensor:
     """bf16 deq(a) deq(b)^T + residual, or with the rotary embedding of rope = (pos int32 [M], cos, sin fp32 [P, 32],
-    rope_cols) on the 64-wide heads below column rope_cols; b block-scaled. One rounding of the fp32 sums."""
+    rope_cols) on the 64-wide heads below column rope_cols; b block-scaled. The bits of the product in bf16 followed by the
+    separate pass."""
     M, K = a.q.shape
     N = b.q.shape[0]
     out = torch.empty((M, N), dtype=_BF16, device=a.q.device)
@@ -258,6 +274,7 @@ class _Fp8LinearFn(torch.autograd.Function):
             y = gemm_fp8_form(qx, qw, residual=None if residual is None else residual.reshape(-1, w.shape[0]), rope=rope)
         ctx.has_res = residual is not None
         ctx.w_ref = w
+        ctx.rope = rope
         ctx.shape = x.shape
         return _as_shape(y, (*x.shape[:-1], w.shape[0]))
 
@@ -268,10 +285,13 @@ class _Fp8LinearFn(torch.autograd.Function):
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dx = dw = qdy = qdy_t = None
+        if ctx.rope is not None and not (ctx.dual and ctx.needs_input_grad[0]):
+            pos, cos, sin, cols = ctx.rope
+            dy2 = _kernels.rope_(dy2.clone(), pos, cos, sin, cols // 128, 64, backward=True)   # (q and k: two thirds)
         if ctx.dual:
             qx_t, sx_t, _ = ctx.saved_tensors
             if ctx.needs_input_grad[0]:
-                qdy, qdy_t = quant_dual(dy2)
+                qdy, qdy_t = quant_dual(dy2) if ctx.rope is None else rope_quant_dual(dy2, ctx.rope)
             else:
                 qdy_t = quant_tile(dy2, transpose=True, block=False)
         elif ctx.needs_input_grad[0]:
@@ -288,9 +308,9 @@ class _Fp8LinearFn(torch.autograd.Function):
 
 def fp8_linear(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None = None,
                rope: tuple | None = None) -> torch.Tensor:
-    """y = x W^T with e4m3 operands (no bias), plus the residual or with the rotary embedding of `gemm_fp8_form` in the
-    product's epilogue. With rope the gradient that comes back must be that of the un-rotated projection (as
-    `functional.linear_rope`)."""
+    """y = x W^T with e4m3 operands (no bias), plus the residual or with the rotary embedding of `gemm_fp8_form` (q and k of a
+    packed QKV projection: two thirds of its columns) in the product's epilogue and its inverse in the quantisation of the
+    incoming gradient."""
     from .functional import _keeps
     return _Fp8LinearFn.apply(x, w, _keeps(), residual, rope)
 

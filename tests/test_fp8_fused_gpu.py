@@ -16,27 +16,59 @@ def _operands(M, N, K):
 
 
 # both tile widths (the wide one from 74 wide tiles), ragged last rows, half a wide tile of columns
-@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (130, 384, 256), (1000, 1024, 128), (9601, 384, 256), (5000, 640, 1024)])
+@pytest.mark.parametrize("M,N,K", [(1, 384, 128), (130, 384, 256), (1000, 768, 128), (9601, 384, 256), (5000, 768, 1024)])
 def test_residual_and_rotary_epilogues(M, N, K, cuda_status):
+    """Bit for bit the product followed by the separate pass."""
     from nanoplm_b200.ops import fp8
     from nanoplm_b200.ops import functional as F_
     from nanoplm_b200.ops import kernels as k
     torch.manual_seed(M)
     a, b = _operands(M, N, K)
-    exact = fp8.gemm_fp8(a, b, out_dtype=torch.float32)          # the sums that the epilogues start from
-    wide = _randn(M, N + 64)
-    res = wide[:, :N]                                            # (a row stride of its own)
-    assert torch.equal(fp8.gemm_fp8_form(a, b, residual=res), (exact + res.float()).to(BF))
-    cos, sin = F_.rope_tables(300, 64, 10000.0, torch.device("cuda"))
-    pos = torch.randint(0, 300, (M,), device="cuda", dtype=torch.int32)
-    cols = N // 128 * 64
-    y = fp8.gemm_fp8_form(a, b, rope=(pos, cos, sin, cols))
-    assert torch.equal(y[:, cols:], exact[:, cols:].to(BF))
-    h = exact[:, :cols].double().view(M, -1, 2, 32)
-    c, s = cos[pos.long()].double()[:, None], sin[pos.long()].double()[:, None]
-    ref = torch.stack((h[:, :, 0] * c - h[:, :, 1] * s, h[:, :, 1] * c + h[:, :, 0] * s), 2)
-    bound = ref.abs() * 2 ** -8 + h.abs().sum(2, keepdim=True) * 2 ** -22    # one bf16 rounding, three fp32 ones
-    assert ((y[:, :cols].double().view(ref.shape) - ref).abs() <= bound).all()
+    product = fp8.gemm_fp8(a, b)
+    res = _randn(M, N + 64)[:, :N]                               # (a row stride of its own)
+    assert torch.equal(fp8.gemm_fp8_form(a, b, residual=res), product + res)
+    rope = _rope(M)
+    want = k.rope_(product.clone(), *rope, N // 192, 64)
+    assert torch.equal(fp8.gemm_fp8_form(a, b, rope=(*rope, N // 3 * 2)), want)
+
+
+def _rope(M):
+    from nanoplm_b200.ops import functional as F_
+    return (torch.randint(0, 300, (M,), device="cuda", dtype=torch.int32),
+            *F_.rope_tables(300, 64, 10000.0, torch.device("cuda")))
+
+
+@pytest.mark.parametrize("R,N", [(128, 384), (1152, 768), (256, 3072)])
+def test_rotary_gradient_with_quantisation(R, N, cuda_status):
+    from nanoplm_b200.ops import fp8
+    from nanoplm_b200.ops import kernels as k
+    torch.manual_seed(R)
+    d, rope = _randn(R, N), _rope(R)
+    want = fp8.quant_dual(k.rope_(d.clone(), *rope, N // 192, 64, backward=True))
+    for got, ref in zip(fp8.rope_quant_dual(d, (*rope, N // 3 * 2)), want):
+        assert torch.equal(got.q, ref.q) and torch.equal(got.scale, ref.scale)
+
+
+@pytest.mark.parametrize("T", [256, 200])        # whole 128-token blocks, and not
+@pytest.mark.parametrize("train_input", [True, False])
+def test_rotary_projection_is_the_two_nodes(T, train_input, cuda_status):
+    from nanoplm_b200.ops import fp8
+    from nanoplm_b200.ops import functional as F_
+    torch.manual_seed(T)
+    x0, w0, dy, rope = _randn(T, 128), _randn(384, 128, scale=0.1), _randn(T, 384), _rope(T)
+
+    def run(fused):
+        fp8.invalidate_weight_cache()
+        x, w = x0.clone().requires_grad_(train_input), w0.clone().requires_grad_(True)
+        w.main_grad = torch.zeros(w.shape, device="cuda")
+        y = fp8.fp8_linear(x, w, rope=(*rope, 256)) if fused else F_.rope_qkv(fp8.fp8_linear(x, w), *rope, 2, 64)
+        y.backward(dy)
+        return y.detach(), x.grad, w.main_grad
+
+    y, dx, dw = run(True)
+    y_ref, dx_ref, dw_ref = run(False)
+    assert torch.equal(y, y_ref) and (dx is None or torch.equal(dx, dx_ref))
+    assert (dw - dw_ref).norm() <= 1e-5 * dw_ref.norm()          # fp32 sums of the work items in any order
 
 
 @pytest.mark.parametrize("R,I", [(128, 128), (384, 256), (1152, 2048)])
@@ -48,10 +80,7 @@ def test_swiglu_with_quantisation(R, I, cuda_status):
     pre[:, I // 2] = 0
     for got, want in zip((*fp8.swiglu_quant_dual(pre), *fp8.swiglu_bwd_quant_dual(pre, dh)),
                          (*fp8.quant_dual(k.swiglu_fwd(pre)), *fp8.quant_dual(k.swiglu_bwd(pre, dh)))):
-        # the scales are the maxima of the same bf16 values; those may differ in the last bit where the compiler contracts
-        # the two kernels' arithmetic differently
-        assert torch.allclose(got.scale, want.scale, rtol=2 ** -7, atol=0)
-        assert ((got.dequantize() - want.dequantize()).norm() <= 2 ** -9 * want.dequantize().norm())
+        assert torch.equal(got.q, want.q) and torch.equal(got.scale, want.scale)
 
 
 def test_mlp_node_is_the_composition(cuda_status):
@@ -77,8 +106,10 @@ def test_mlp_node_is_the_composition(cuda_status):
 
     F_.set_fp8(True)
     try:
-        for a, b in zip(run(True), run(False)):
-            assert (a.float() - b.float()).norm() <= 2 ** -7 * b.float().norm()      # bf16 roundings of y, dx
+        (y, dx, dr, dwi, dwo), ref = run(True), run(False)
+        assert torch.equal(y, ref[0]) and torch.equal(dx, ref[1]) and torch.equal(dr, ref[2])
+        for a, b in ((dwi, ref[3]), (dwo, ref[4])):
+            assert (a - b).norm() <= 1e-5 * b.norm()             # fp32 sums of the work items in any order
     finally:
         F_.set_fp8(False)
         fp8.invalidate_weight_cache()
