@@ -1240,7 +1240,7 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
                                  grp.ag_world > 1 || bn != 256))
     return -7;
   if (epi == EPI_SWIGLU_BWD && (a_mn || direct_epilogue || R == nullptr || (N % 64) || (ldr % 8) || (ldc % 8) ||
-                                (reinterpret_cast<uintptr_t>(R) & 15) || grp.mode != 0 || grp.ag_world > 1))
+                                (reinterpret_cast<uintptr_t>(R) & 15) || grp.mode > 1 || grp.ag_world > 1))
     return -7;
   if ((epi == EPI_AXPBY) != (grp.mode == 3)) return -9;
   if (grp.mode == 3 && (a_mn || direct_epilogue || !grp.pair || bn != 256 || max_ctas != 0 || grp.groups < 1 ||

@@ -61,7 +61,7 @@ def router_bwd(probs, gates, experts, d_gates, aux_grad):
 def gemm_grouped(a, b, tile_group, *, b_mn=False, epi=K.EPI_STORE, aux=None, bn=None, out=None,
                  arrive=None, expect=None):
     """Row-grouped GEMM. a [P,K] bf16 (P multiple of 128), b [G, N, K] (b_mn False) or [G, K, N]
-    (b_mn True), tile_group int32 [P/128]. Returns [P, N] (N/2 wide for EPI_SWIGLU).
+    (b_mn True), tile_group int32 [P/128]. Returns [P, N] (N/2 wide for EPI_SWIGLU, 2 N for EPI_SWIGLU_BWD).
     arrive / expect (int32 [P/128] each, both or neither): the rows of `a` are being stored by other GPUs;
     a tile is loaded once its arrival counter has reached its expected row count."""
     P, Kd = a.shape
@@ -76,14 +76,16 @@ def gemm_grouped(a, b, tile_group, *, b_mn=False, epi=K.EPI_STORE, aux=None, bn=
             raise ValueError("inner dims differ")
     if P % 128 or tile_group.numel() < P // 128:
         raise ValueError("grouped GEMM rows must be whole 128-row tiles described by tile_group")
-    out_cols = N // 2 if epi == K.EPI_SWIGLU else N
+    out_cols = N // 2 if epi == K.EPI_SWIGLU else (2 * N if epi == K.EPI_SWIGLU_BWD else N)
+    if epi == K.EPI_SWIGLU_BWD and (aux is None or tuple(aux.shape) != (P, 2 * N) or aux.dtype != _BF16):
+        raise ValueError("EPI_SWIGLU_BWD needs the pre-activations [P, 2 N] as aux")
     if out is None:
         out = torch.empty((P, out_cols), dtype=_BF16, device=a.device)
     elif tuple(out.shape) != (P, out_cols) or out.dtype != _BF16:
         raise ValueError("out has the wrong shape or dtype")
     b2 = b.reshape(-1, b.shape[2])
     if bn is None:
-        bn = 256 if (N >= 256 or epi == K.EPI_SWIGLU) else 128
+        bn = 256 if (N >= 256 or epi in (K.EPI_SWIGLU, K.EPI_SWIGLU_BWD)) else 128
     ldr = aux.stride(0) if aux is not None else 0
     if (arrive is None) != (expect is None):
         raise ValueError("arrive and expect go together")
@@ -386,6 +388,8 @@ class _ExpertsFn(torch.autograd.Function):
             ys_ptrs = _ptr_array([ys.data_ptr()])
         n = plan.T * c.k
         dy = dy.contiguous()
+        # The SwiGLU backward rides in the data gradient's epilogue, as without experts; 8 experts, 53 400 rows in all, 1024
+        # columns of K = 1024: 154 us, the plain data gradient and a pass over it 183.
         # gradient of combine: d_gates = <dy, ys row> (pulled), d_ys = gate * dy (pushed to the owner)
         dys, dys_ptrs = c.buffer("dys", plan.cap, dev)
         _zero_pad(plan, dys)
@@ -402,14 +406,14 @@ class _ExpertsFn(torch.autograd.Function):
             # no barrier: the down-projection's data gradient starts tile by tile as the d_ys rows land,
             # and the data gradient of the dispatched rows goes to a buffer of its own (peers may still
             # be reading ys)
-            d_h = gemm_grouped(dys, Wo, plan.tile_group, b_mn=True, arrive=arrive_b.tensor, expect=plan.tile_rows)
+            d_pre = gemm_grouped(dys, Wo, plan.tile_group, b_mn=True, epi=K.EPI_SWIGLU_BWD, aux=pre,
+                                 arrive=arrive_b.tensor, expect=plan.tile_rows)
             dxs, dx_ptrs = c.buffer("dxs", plan.cap, dev)
         else:
             c.barrier(dev)                                # d_ys complete, nobody reads ys any more
-            d_h = gemm_grouped(dys, Wo, plan.tile_group, b_mn=True)
+            d_pre = gemm_grouped(dys, Wo, plan.tile_group, b_mn=True, epi=K.EPI_SWIGLU_BWD, aux=pre)
             # the data gradient of the dispatched rows lands in the buffer that held ys
             dxs, dx_ptrs = (ys, ys_ptrs) if ep else (None, None)
-        d_pre = K.swiglu_bwd(pre, d_h)
         dxs = gemm_grouped(d_pre, Wi, plan.tile_group, b_mn=True, out=dxs)
         if not ep:
             dx_ptrs = _ptr_array([dxs.data_ptr()])
