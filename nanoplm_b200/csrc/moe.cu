@@ -375,11 +375,12 @@ moe_push_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restric
   }
 }
 
-// One warp per token: out[t] = sum_s (gates ? gates[t,s] : 1) * src_owner[pos_of[t,s]]
+// One warp per token: out[t] = sum_s (gates ? gates[t,s] : 1) * src_owner[pos_of[t,s]], plus residual[t] when given: added to
+// the sum rounded to bf16, as a pass of its own adds it (whose 6 bytes an element become 2 here).
 __global__ void __launch_bounds__(256)
 moe_pull_rows_kernel(MoePeers src, const int* __restrict__ experts, const int* __restrict__ pos_of,
-                     const float* __restrict__ gates, int T, int k, int C, int experts_per_rank,
-                     int capacity_rows, __nv_bfloat16* __restrict__ out) {
+                     const float* __restrict__ gates, const __nv_bfloat16* __restrict__ residual, int T, int k, int C,
+                     int experts_per_rank, int capacity_rows, __nv_bfloat16* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < T; t += gridDim.x * wpb) {
@@ -407,6 +408,15 @@ moe_pull_rows_kernel(MoePeers src, const int* __restrict__ experts, const int* _
       uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
       for (int q = 0; q < 4; ++q) ow[q] = pack_bf16x2(acc[2 * q], acc[2 * q + 1]);
+      if (residual != nullptr) {
+        const uint4 r = reinterpret_cast<const uint4*>(residual + static_cast<size_t>(t) * C)[c];
+        const uint32_t* rw = reinterpret_cast<const uint32_t*>(&r);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 a = unpack_bf16x2(ow[q]), b = unpack_bf16x2(rw[q]);
+          ow[q] = pack_bf16x2(a.x + b.x, a.y + b.y);
+        }
+      }
       reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * C)[c] = o;
     }
   }
@@ -542,13 +552,14 @@ extern "C" int nplm_moe_push_rows(const void* src, const int* experts, const int
 }
 
 extern "C" int nplm_moe_pull_rows(void* const* src, const int* experts, const int* pos_of,
-                                  const float* gates, int T, int k, int C, int experts_per_rank,
+                                  const float* gates, const void* residual, int T, int k, int C, int experts_per_rank,
                                   int capacity_rows, void* out, int world, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if ((C % 8) || world < 1 || world > MOE_MAX_PEERS) return -3;
+  if ((C % 8) || world < 1 || world > MOE_MAX_PEERS || (reinterpret_cast<uintptr_t>(residual) & 15)) return -3;
   MoePeers s;
   for (int p = 0; p < MOE_MAX_PEERS; ++p) s.p[p] = p < world ? src[p] : nullptr;
-  moe_pull_rows_kernel<<<grid_for(T, 8), 256, 0, stream>>>(s, experts, pos_of, gates, T, k, C,
+  moe_pull_rows_kernel<<<grid_for(T, 8), 256, 0, stream>>>(s, experts, pos_of, gates,
+                                                           reinterpret_cast<const __nv_bfloat16*>(residual), T, k, C,
                                                            experts_per_rank, capacity_rows,
                                                            reinterpret_cast<__nv_bfloat16*>(out));
   return static_cast<int>(cudaGetLastError());

@@ -111,15 +111,16 @@ class MoEMLP(nn.Module):
         parallelism, where the buffers are sized for the batch)."""
         return 0 if self._comm is None else self._comm.dropped_rows()
 
-    def forward(self, x: torch.Tensor):
+    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None):
+        """(y, balance loss); y includes the residual when it is given."""
         T, C = x.shape
         if self._use_device_path(x):
             from nanoplm_b200.ops import moe as M
             if self._comm is None:
                 self._comm = M.MoEComm(self.hidden, self.num_experts, self.top_k, group=self.ep_group,
                                        capacity_factor=self.capacity_factor)
-            logits = ops.linear(x, self.router.weight)
-            return M.moe_mlp(x, logits, self.experts_Wi, self.experts_Wo, self.top_k, self._comm)
+            logits, x = M.router_logits(x, self.router.weight)
+            return M.moe_mlp(x, logits, self.experts_Wi, self.experts_Wo, self.top_k, self._comm, residual)
         logits = F.linear(x, self.router.weight)
         gates, experts, aux = route_topk(logits, self.top_k)
         flat_e = experts.reshape(-1)
@@ -135,4 +136,4 @@ class MoEMLP(nn.Module):
         w = gates.reshape(-1)[order].to(y_rows.dtype)
         y = torch.zeros((T, C), dtype=y_rows.dtype, device=x.device)
         y.index_add_(0, token_of.long(), y_rows * w[:, None])
-        return y, aux
+        return y if residual is None else residual + y, aux
