@@ -335,11 +335,13 @@ mhc_read_kernel(const __nv_bfloat16* __restrict__ X, const float* __restrict__ a
 
 // Xn[t][i][:] = sum_j R[t][i][j] X[t][j][:] + beta[t][i] y[t][:]
 // N = number of streams (compile-time, so every per-stream array stays in registers).
-template <int N>
+// MEAN: also z[t][:] = (1/N) sum_i Xn[t][i][:] of the rounded streams, which mhc_mean_kernel would read them back for
+// (17 024 x 4 x 768: 50 us, 71 in two passes).
+template <int N, bool MEAN>
 __global__ void __launch_bounds__(256)
 mhc_write_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ y,
                  const float* __restrict__ R, const float* __restrict__ beta,
-                 __nv_bfloat16* __restrict__ Xn, int T, int C) {
+                 __nv_bfloat16* __restrict__ Xn, __nv_bfloat16* __restrict__ z, int T, int C) {
   grid_chain();
   const int vec = C >> 3;
   const long long total = static_cast<long long>(T) * vec;
@@ -373,6 +375,16 @@ mhc_write_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __res
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) st8(Xn + (static_cast<size_t>(t) * N + i) * C + c, acc[i]);
+    if constexpr (MEAN) {
+      float m[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) m[e] += __bfloat162float(__float2bfloat16_rn(acc[i][e]));
+#pragma unroll
+      for (int e = 0; e < 8; ++e) m[e] *= 1.f / static_cast<float>(N);
+      st8(z + static_cast<size_t>(t) * C + c, m);
+    }
   }
 }
 
@@ -402,16 +414,20 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {
 //   dy[t][:]     = sum_i beta[t][i] dXn[t][i][:]
 //   dR[t][i][j]  = <dXn[t][i], X[t][j]>,  dbeta[t][i] = <dXn[t][i], y[t]>,  dalpha[t][j] = <dh[t], X[t][j]>
 // All loads of a 256-channel slice are issued before the first use and kept packed in registers.
+// JOIN (with WRITE alone): the written streams are the ones of the next site, whose gradient mhc_dx_combine_kernel forms from
+// dXn (here the next site's own write), its alpha and dh and the gradient dz of its stream mean; formed here, with the same
+// bits, it is neither written nor read back (17 024 x 4 x 768: 77 us, 112 in two passes).
 // WRITE / READ: which parts there are. As run-time flags the read part alone (what a training step asks for beside the
 // write part) carried the write part's N x N sums along, on zeros: 17 024 x 4 x 768 53 -> 27 us, the write part alone 70 -> 61.
-template <int N, bool WRITE, bool READ>
+template <int N, bool WRITE, bool READ, bool JOIN = false>
 __global__ void __launch_bounds__(256, 2)
 mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ y,
                const float* __restrict__ R, const float* __restrict__ alpha, const float* __restrict__ beta,
                const __nv_bfloat16* __restrict__ dXn, const __nv_bfloat16* __restrict__ dh,
-               __nv_bfloat16* __restrict__ dX, __nv_bfloat16* __restrict__ dy, float* __restrict__ dR,
-               float* __restrict__ dalpha, float* __restrict__ dbeta, int T, int C) {
+               const __nv_bfloat16* __restrict__ dz, __nv_bfloat16* __restrict__ dX, __nv_bfloat16* __restrict__ dy,
+               float* __restrict__ dR, float* __restrict__ dalpha, float* __restrict__ dbeta, int T, int C) {
   grid_chain();
+  static_assert(!JOIN || (WRITE && !READ), "the joined form is the write part's");
   static_assert(N * N + 2 * N <= 32, "too many streams for the warp-transpose reduction");
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
@@ -425,7 +441,7 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       bt[i] = has_w ? beta[t * N + i] : 0.f;
-      al[i] = has_r ? alpha[t * N + i] : 0.f;
+      al[i] = has_r || JOIN ? alpha[t * N + i] : 0.f;
 #pragma unroll
       for (int j = 0; j < N; ++j) rc[i][j] = has_w ? R[(t * N + i) * N + j] : 0.f;
     }
@@ -439,8 +455,24 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
                       : make_uint4(0u, 0u, 0u, 0u);
       }
       if (has_w) yr = __ldg(reinterpret_cast<const uint4*>(y + static_cast<size_t>(t) * C + c));
-      if (has_r) hr = __ldg(reinterpret_cast<const uint4*>(dh + static_cast<size_t>(t) * C + c));
+      if (has_r || JOIN) hr = __ldg(reinterpret_cast<const uint4*>(dh + static_cast<size_t>(t) * C + c));
       float yv[8], hv[8];
+      if constexpr (JOIN) {
+        float zv[8];
+        unpack8x(__ldg(reinterpret_cast<const uint4*>(dz + static_cast<size_t>(t) * C + c)), zv);
+        unpack8x(hr, hv);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) zv[e] *= 1.f / static_cast<float>(N);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          float gv[8];
+          unpack8x(gr[i], gv);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) gv[e] += fmaf(al[i], hv[e], zv[e]);
+          gr[i] = make_uint4(pack_bf16x2(gv[0], gv[1]), pack_bf16x2(gv[2], gv[3]), pack_bf16x2(gv[4], gv[5]),
+                             pack_bf16x2(gv[6], gv[7]));
+        }
+      }
       unpack8x(yr, yv);
       unpack8x(hr, hv);
       float dyv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -448,7 +480,7 @@ mhc_bwd_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restr
 #pragma unroll
       for (int j = 0; j < N; ++j)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[j][e] = al[j] * hv[e];
+        for (int e = 0; e < 8; ++e) o[j][e] = has_r ? al[j] * hv[e] : 0.f;
 #pragma unroll
       for (int j = 0; j < N; ++j) {
         float xv[8];
@@ -647,15 +679,16 @@ extern "C" int nplm_mhc_dx_combine(const void* g, const float* alpha, const void
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int nplm_mhc_write(const void* X, const void* y, const float* R, const float* beta, void* Xn,
+// z (bf16 [T][C], may be null): the stream mean of what is written.
+extern "C" int nplm_mhc_write(const void* X, const void* y, const float* R, const float* beta, void* Xn, void* z,
                               int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > 4) return -3;
   const int grid = grid_for(static_cast<long long>(T) * (C / 8), 256);
 #define NPLM_MHC_WRITE(N_)                                                                              \
-  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_write_kernel<N_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(X),                  \
-                                             reinterpret_cast<const __nv_bfloat16*>(y), R, beta,         \
-                                             reinterpret_cast<__nv_bfloat16*>(Xn), T, C)
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, z != nullptr ? mhc_write_kernel<N_, true> : mhc_write_kernel<N_, false>, grid, 256, 0, st, \
+              reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, beta,   \
+              reinterpret_cast<__nv_bfloat16*>(Xn), reinterpret_cast<__nv_bfloat16*>(z), T, C)
   switch (n) {
     case 1: NPLM_MHC_WRITE(1); break;
     case 2: NPLM_MHC_WRITE(2); break;
@@ -666,20 +699,28 @@ extern "C" int nplm_mhc_write(const void* X, const void* y, const float* R, cons
   return static_cast<int>(cudaGetLastError());
 }
 
+// With dz (and dXn, alpha, dh) the joined form: dXn, alpha, dh and dz are the parts of the next site's gradient.
 extern "C" int nplm_mhc_bwd(const void* X, const void* y, const float* R, const float* alpha,
-                            const float* beta, const void* dXn, const void* dh, void* dX, void* dy,
+                            const float* beta, const void* dXn, const void* dh, const void* dz, void* dX, void* dy,
                             float* dR, float* dalpha, float* dbeta, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > 4) return -3;
+  if (dz != nullptr && (dXn == nullptr || dh == nullptr || alpha == nullptr)) return -3;
   if (dXn == nullptr && dh == nullptr) return 0;
   int blocks = (T + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
-#define NPLM_MHC_BWD(N_)                                                                                  \
-  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, dXn != nullptr ? (dh != nullptr ? mhc_bwd_kernel<N_, true, true> : mhc_bwd_kernel<N_, true, false>) \
-                                : mhc_bwd_kernel<N_, false, true>, blocks, 256, 0, st,                                \
-      reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, alpha, beta, \
-      reinterpret_cast<const __nv_bfloat16*>(dXn), reinterpret_cast<const __nv_bfloat16*>(dh),              \
-      reinterpret_cast<__nv_bfloat16*>(dX), reinterpret_cast<__nv_bfloat16*>(dy), dR, dalpha, dbeta, T, C)
+  const auto go = [&](auto kern) {
+    launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, kern, blocks, 256, 0, st,
+                reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, alpha, beta,
+                reinterpret_cast<const __nv_bfloat16*>(dXn), reinterpret_cast<const __nv_bfloat16*>(dh),
+                reinterpret_cast<const __nv_bfloat16*>(dz), reinterpret_cast<__nv_bfloat16*>(dX),
+                reinterpret_cast<__nv_bfloat16*>(dy), dR, dalpha, dbeta, T, C);
+  };
+#define NPLM_MHC_BWD(N_)                                         \
+  dz != nullptr    ? go(mhc_bwd_kernel<N_, true, false, true>)   \
+  : dXn == nullptr ? go(mhc_bwd_kernel<N_, false, true>)         \
+  : dh != nullptr  ? go(mhc_bwd_kernel<N_, true, true>)          \
+                   : go(mhc_bwd_kernel<N_, true, false>)
   switch (n) {
     case 1: NPLM_MHC_BWD(1); break;
     case 2: NPLM_MHC_BWD(2); break;

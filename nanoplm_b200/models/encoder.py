@@ -219,16 +219,22 @@ class EncoderLayer(nn.Module):
                 h, skip = self.mlp_norm.with_residual(x)
                 x = self.mlp(h, residual=skip)
             return x, aux
-        # hyper-connections: x is (T, n, C)
-        h, state = self.mhc_attn.read(x)
-        x = self.mhc_attn.write(x, self._attn_branch(h, ctx, window, rope, residual=None), state)
-        h, state = self.mhc_mlp.read(x)
+        return self._streams(x, ctx, window, rope)[:2]
+
+    def _streams(self, x, ctx, window, rope, entry=None, nxt=None):
+        """The layer on hyper-connection streams x (T, n, C): (x, aux, entry'). entry: what reading x at this layer's first
+        site gave, when that is done already; nxt: the site to read next, whose entry' is then given."""
+        aux = None
+        h, state = self.mhc_attn.read(x) if entry is None else entry
+        x, h, state = self.mhc_attn.write_read(x, self._attn_branch(h, ctx, window, rope, residual=None), state, self.mhc_mlp)
         if self.is_moe:
             y, aux = self.mlp(self.mlp_norm(h))
         else:
             y = self.mlp(self.mlp_norm(h))
-        x = self.mhc_mlp.write(x, y, state)
-        return x, aux
+        if nxt is None:
+            return self.mhc_mlp.write(x, y, state), aux, None
+        x, h, state = self.mhc_mlp.write_read(x, y, state, nxt)
+        return x, aux, (h, state)
 
 
 def _stackable(layer) -> bool:
@@ -273,10 +279,17 @@ class EncoderModel(nn.Module):
                                              [-1 if t == "full_attention" else cfg.sliding_window for t in types],
                                              [rope[t] for t in types])
             layers = layers[done:]
-        for layer in layers:
+        # on streams, a layer's last write and the next one's first read are one where nobody watches the layers' calls
+        own = [n > 1 and x.is_cuda and type(layer) is EncoderLayer and native_layer.unobserved((layer,)) for layer in layers]
+        entry = None
+        for i, layer in enumerate(layers):
             lt = layer.attention_type
             window = -1 if lt == "full_attention" else cfg.sliding_window
-            x, aux = layer(x, ctx, window, rope[lt])
+            if own[i]:
+                nxt = layers[i + 1].mhc_attn if i + 1 < len(layers) and own[i + 1] else None
+                x, aux, entry = layer._streams(x, ctx, window, rope[lt], entry, nxt)
+            else:
+                x, aux = layer(x, ctx, window, rope[lt])
             if aux is not None:
                 aux_total = aux if aux_total is None else aux_total + aux
         if n > 1:

@@ -97,6 +97,33 @@ class _MeanFn(torch.autograd.Function):
         return K.mhc_dx_combine(g, alpha, dh, dz, ctx.shape), None
 
 
+class _WriteMeanFn(torch.autograd.Function):
+    """_WriteFn of one site and _MeanFn of the next, which reads what the first one wrote: the stream mean comes out of
+    the write, and the gradient that _MeanFn forms is formed where the write's backward reads it."""
+
+    @staticmethod
+    def forward(ctx, X, y, R, beta, site):
+        X, y = X.contiguous(), y.contiguous()
+        R, beta = R.float().contiguous(), beta.float().contiguous()
+        ctx.save_for_backward(X, y, R, beta)
+        ctx.site = site
+        return K.mhc_write(X, y, R, beta, mean=True)
+
+    @staticmethod
+    def backward(ctx, g, dz):
+        X, y, R, beta = ctx.saved_tensors
+        site = ctx.site
+        alpha, dh = site.alpha, site.dh
+        site.alpha = site.dh = None
+        g, dz = (t.contiguous() if t is not None else None for t in (g, dz))
+        if g is None or dh is None or dz is None:       # a part that nobody asked for
+            if g is None and dh is None and dz is None:
+                return None, None, None, None, None
+            g, alpha, dh, dz = K.mhc_dx_combine(g, alpha, dh, dz, tuple(X.shape)), None, None, None
+        dX, dy, dR, _, dbeta = K.mhc_bwd(X, y, R, alpha, beta, g, dh, dz=dz)
+        return dX, dy, dR, dbeta, None
+
+
 class _ReadThreadFn(torch.autograd.Function):
     """h = sum_i alpha_i X1_i, and X1 handed on as X2 for the write. Backward: d alpha only; the
     gradient arriving for X2 goes back unchanged and _MeanFn adds the read's share to it."""
@@ -210,11 +237,25 @@ class HyperConnection(nn.Module):
         if self._threaded(X):
             site = _SiteGrad()
             z, X1 = _MeanFn.apply(X.contiguous(), site)
-            alpha, beta, R = self.coefficients(X1, z)
-            h, X2 = _ReadThreadFn.apply(X1, alpha, site)
-            return h, (beta, R, X2)
+            return self._read_threaded(X1, z, site)
         alpha, beta, R = self.coefficients(X)
         return mhc_read(X, alpha), (beta, R, None)
+
+    def _read_threaded(self, X1, z, site):
+        alpha, beta, R = self.coefficients(X1, z)
+        h, X2 = _ReadThreadFn.apply(X1, alpha, site)
+        return h, (beta, R, X2)
+
+    def write_read(self, X, y, state, nxt):
+        """X' = self.write(X, y, state) and (h, state') = nxt.read(X') of the next site: (X', h, state')."""
+        beta, R, threaded = state
+        if (threaded is not None and nxt._threaded(threaded) and type(self).write is HyperConnection.write
+                and type(nxt).read is HyperConnection.read and not ({"write", "read"} & (vars(self).keys() | vars(nxt).keys()))):
+            site = _SiteGrad()
+            Xn, z = _WriteMeanFn.apply(threaded, y, R, beta, site)
+            return Xn, *nxt._read_threaded(Xn, z, site)
+        X = self.write(X, y, state)
+        return X, *nxt.read(X)
 
     def write(self, X, y, state):
         beta, R, threaded = state

@@ -739,14 +739,16 @@ def mhc_read(X, alpha):
     return h
 
 
-def mhc_write(X, y, R, beta):
+def mhc_write(X, y, R, beta, mean: bool = False):
+    """With mean also the mean over the written streams [T, C]."""
     T, n, C = X.shape
     Xn = torch.empty_like(X)
-    rc = lib("extras").nplm_mhc_write(ptr(X), ptr(y), ptr(R), ptr(beta), ptr(Xn), c_int(T), c_int(n), c_int(C),
+    z = torch.empty((T, C), dtype=_BF16, device=X.device) if mean else None
+    rc = lib("extras").nplm_mhc_write(ptr(X), ptr(y), ptr(R), ptr(beta), ptr(Xn), ptr(z), c_int(T), c_int(n), c_int(C),
                                       stream_ptr())
     check_rc(rc, "mhc_write")
     count_launch()
-    return Xn
+    return (Xn, z) if mean else Xn
 
 
 def mhc_mean(X):
@@ -772,17 +774,18 @@ def mhc_dx_combine(g, alpha, dh, dz, shape):
     return dX
 
 
-def mhc_bwd(X, y, R, alpha, beta, dXn, dh, want_dx: bool = True):
+def mhc_bwd(X, y, R, alpha, beta, dXn, dh, want_dx: bool = True, dz=None):
     """Backward of write (dXn given) and / or read (dh given). Returns (dX, dy, dR, dalpha, dbeta);
-    want_dx=False skips the dX output (only the coefficient gradients are computed)."""
+    want_dx=False skips the dX output (only the coefficient gradients are computed). With dz the backward of write alone,
+    of the gradient mhc_dx_combine(dXn, alpha, dh, dz)."""
     T, n, C = X.shape
     dev = X.device
     dX = torch.empty_like(X) if want_dx else None
     dy = torch.empty((T, C), dtype=_BF16, device=dev) if dXn is not None else None
     dR = torch.empty((T, n, n), dtype=torch.float32, device=dev) if dXn is not None else None
     dbeta = torch.empty((T, n), dtype=torch.float32, device=dev) if dXn is not None else None
-    dalpha = torch.empty((T, n), dtype=torch.float32, device=dev) if dh is not None else None
-    rc = lib("extras").nplm_mhc_bwd(ptr(X), ptr(y), ptr(R), ptr(alpha), ptr(beta), ptr(dXn), ptr(dh), ptr(dX),
+    dalpha = torch.empty((T, n), dtype=torch.float32, device=dev) if dh is not None and dz is None else None
+    rc = lib("extras").nplm_mhc_bwd(ptr(X), ptr(y), ptr(R), ptr(alpha), ptr(beta), ptr(dXn), ptr(dh), ptr(dz), ptr(dX),
                                     ptr(dy), ptr(dR), ptr(dalpha), ptr(dbeta), c_int(T), c_int(n), c_int(C),
                                     stream_ptr())
     check_rc(rc, "mhc_bwd")
