@@ -48,10 +48,11 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
 constexpr int MAX_KS = 9;
 
 // flip = 0: forward (tap k reads t + k - r);  flip = 1: input gradient (tap k reads t - (k - r))
+// skip: y = x + the convolution rounded to bf16 (forward of the residual block, and its input gradient with x the output's)
 __global__ void __launch_bounds__(256)
 dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
               const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
-              const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int KS, int flip) {
+              const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int KS, int flip, int skip) {
   grid_chain();
   const int vec = C >> 3;
   const int r = KS >> 1;
@@ -75,6 +76,12 @@ dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       ld8(x + static_cast<size_t>(src) * C + c, xv);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] += xv[e] * __bfloat162float(w[(c + e) * KS + k]);
+    }
+    if (skip) {
+      float xv[8];
+      ld8(x + static_cast<size_t>(t) * C + c, xv);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = xv[e] + __bfloat162float(__float2bfloat16_rn(acc[e]));
     }
     st8(y + static_cast<size_t>(t) * C + c, acc);
   }
@@ -110,7 +117,7 @@ template <int KS>
 __global__ void __launch_bounds__(256, 2)
 dwconv_run_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                   const __nv_bfloat16* __restrict__ bias, const int* __restrict__ s_start,
-                  const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip, int run) {
+                  const int* __restrict__ s_end, __nv_bfloat16* __restrict__ y, int T, int C, int flip, int skip, int run) {
   grid_chain();
   constexpr int R = KS / 2;
   const int lane = threadIdx.x & 31;
@@ -158,9 +165,12 @@ dwconv_run_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
             }
           }
         }
-        if (on)
-          *reinterpret_cast<uint2*>(y + static_cast<size_t>(t + i) * C + c) =
-              make_uint2(pack_bf16x2(acc[0].x, acc[0].y), pack_bf16x2(acc[1].x, acc[1].y));
+        uint2 out = make_uint2(pack_bf16x2(acc[0].x, acc[0].y), pack_bf16x2(acc[1].x, acc[1].y));
+        if (skip) {     // (the row itself is the middle tap's)
+          const float2 o0 = add2(unpack_bf16x2(out.x), rows[i + R][0]), o1 = add2(unpack_bf16x2(out.y), rows[i + R][1]);
+          out = make_uint2(pack_bf16x2(o0.x, o0.y), pack_bf16x2(o1.x, o1.y));
+        }
+        if (on) *reinterpret_cast<uint2*>(y + static_cast<size_t>(t + i) * C + c) = out;
       }
     }
     if (t + DW_AHEAD < t1) {
@@ -598,7 +608,7 @@ static int grid_for(long long work, int threads) {
 using namespace nplm;
 
 extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const int* s_start,
-                           const int* s_end, void* y, int T, int C, int KS, int flip, cudaStream_t st) {
+                           const int* s_end, void* y, int T, int C, int KS, int flip, int skip, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || KS < 1 || KS > MAX_KS || !(KS & 1)) return -3;
   if ((KS == 3 || KS == 5 || KS == 7 || KS == 9) &&
@@ -608,7 +618,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
 #define NPLM_DWCONV(KS_)                                                                                   \
   launch_chained(dwconv_run_kernel<KS_>, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),      \
                  reinterpret_cast<const __nv_bfloat16*>(w), reinterpret_cast<const __nv_bfloat16*>(bias),   \
-                 s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip, run)
+                 s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C, flip, skip, run)
     switch (KS) {
       case 3: NPLM_DWCONV(3); break;
       case 5: NPLM_DWCONV(5); break;
@@ -621,7 +631,7 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
   launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, dwconv_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
       reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C,
-      KS, flip);
+      KS, flip, skip);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -31,18 +31,19 @@ def dwconv_reference(x, w, bias, seq_start, seq_end):
 
 class _DWConvFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, bias, ss, se):
+    def forward(ctx, x, w, bias, ss, se, skip):
         x = x.contiguous()
         ctx.save_for_backward(x, w, ss, se)
         ctx.bias_ref = bias
         ctx.w_ref = w
-        return K.dwconv(x, w.contiguous(), bias, ss, se)
+        ctx.skip = skip
+        return K.dwconv(x, w.contiguous(), bias, ss, se, skip=skip)
 
     @staticmethod
     def backward(ctx, dy):
         x, w, ss, se = ctx.saved_tensors
         dy = dy.contiguous()
-        dx = K.dwconv(dy, w.contiguous(), None, ss, se, flip=True)
+        dx = K.dwconv(dy, w.contiguous(), None, ss, se, flip=True, skip=ctx.skip)
         bias = ctx.bias_ref
         dw = w.main_grad if _has_main_grad(w) else torch.zeros(w.shape, dtype=torch.float32, device=w.device)
         db = None
@@ -51,13 +52,15 @@ class _DWConvFn(torch.autograd.Function):
         K.dwconv_bwd_w(x, dy, ss, se, dw, db)
         gw = None if _has_main_grad(w) else dw.to(w.dtype)
         gb = None if (bias is None or _has_main_grad(bias)) else db.to(bias.dtype)
-        return dx, gw, gb, None, None
+        return dx, gw, gb, None, None, None
 
 
-def dwconv_varlen(x, w, bias, seq_start, seq_end):
+def dwconv_varlen(x, w, bias, seq_start, seq_end, skip: bool = False):
+    """The convolution of x; with skip x plus it, in the same pass."""
     if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and w.shape[1] <= 9:
-        return _DWConvFn.apply(x, w, bias, seq_start, seq_end)
-    return dwconv_reference(x, w, bias, seq_start, seq_end)
+        return _DWConvFn.apply(x, w, bias, seq_start, seq_end, skip)
+    y = dwconv_reference(x, w, bias, seq_start, seq_end)
+    return x + y if skip else y
 
 
 class VarlenDepthwiseConv(nn.Module):
@@ -69,5 +72,5 @@ class VarlenDepthwiseConv(nn.Module):
         self.weight = nn.Parameter(w)
         self.bias = nn.Parameter(torch.zeros(channels)) if bias else None
 
-    def forward(self, x, ctx):
-        return dwconv_varlen(x, self.weight, self.bias, ctx.seq_start, ctx.seq_end)
+    def forward(self, x, ctx, skip: bool = False):
+        return dwconv_varlen(x, self.weight, self.bias, ctx.seq_start, ctx.seq_end, skip)

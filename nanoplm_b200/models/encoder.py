@@ -178,7 +178,11 @@ class EncoderLayer(nn.Module):
         if not normed:
             h = self.attn_norm(h)
         if self.conv is not None:
-            h = h + self.conv(h, ctx)
+            from .conv import VarlenDepthwiseConv
+            if h.is_cuda and type(self.conv) is VarlenDepthwiseConv and native_layer.unobserved((self.conv,)):
+                h = self.conv(h, ctx, skip=True)
+            else:
+                h = h + self.conv(h, ctx)
         return self.attn(h, ctx, window, rope, residual=residual)
 
     def _plain(self) -> bool:

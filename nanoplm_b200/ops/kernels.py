@@ -710,12 +710,13 @@ def check_status() -> None:
 
 
 # --------------------------------------------------------------------------- conv / mHC
-def dwconv(x, w, bias, seq_start, seq_end, flip=False):
+def dwconv(x, w, bias, seq_start, seq_end, flip=False, skip=False):
+    """With skip x plus the convolution, both bf16."""
     T, C = x.shape
     KS = w.shape[1]
     y = torch.empty_like(x)
     rc = lib("extras").nplm_dwconv(ptr(x), ptr(w), ptr(bias), ptr(seq_start), ptr(seq_end), ptr(y), c_int(T),
-                                   c_int(C), c_int(KS), c_int(int(flip)), stream_ptr())
+                                   c_int(C), c_int(KS), c_int(int(flip)), c_int(int(skip)), stream_ptr())
     check_rc(rc, "dwconv")
     count_launch()
     return y
