@@ -1635,7 +1635,7 @@ extern "C" int nplm_fa_fwd_ws(const void* qkv, void* out, float* lse, const int*
   return static_cast<int>(cudaGetLastError());
 }
 
-// Backward. dq_acc: caller-provided fp32 scratch [T][H*D], cleared here. delta: fp32 scratch [H][T],
+// Backward. dq_acc: caller-provided fp32 scratch [T][H*D], cleared here unless the caller has (zeroed). delta: fp32 scratch [H][T],
 // computed here from out and dout unless out is null (then it must hold rowsum(dO * O) already).
 // rope_* (may be null): q / k were rotated before the forward pass; dQ and dK are returned as
 // gradients of the un-rotated projections.
@@ -1647,7 +1647,7 @@ static int ws_bwd_impl(const void* qkv, const void* out, const void* dout, const
                        void* dqkv, float* dq_acc, float* delta, const int* seq_start,
                        const int* seq_end, int T, int H, int D, int window, float scale,
                        const int* rope_pos, const float* rope_cos, const float* rope_sin,
-                       int max_ctas, int mode, int* status, cudaStream_t st) {
+                       int max_ctas, int mode, bool zeroed, int* status, cudaStream_t st) {
   if (T <= 0) return 0;
   if (D != FA_D || H <= 0) return -3;
   if ((reinterpret_cast<uintptr_t>(qkv) & 15) || (reinterpret_cast<uintptr_t>(dout) & 15)) return -3;
@@ -1683,7 +1683,7 @@ static int ws_bwd_impl(const void* qkv, const void* out, const void* dout, const
   rc = ws_configure(&sms);
   if (rc) return rc;
   const int HD = H * D;
-  if (mode != 3)
+  if (mode != 3 && !zeroed)
     NPLM_CUDA_CHECK(cudaMemsetAsync(dq_acc, 0, static_cast<size_t>(T) * HD * sizeof(float), st));
   if (out != nullptr) {
     const long long total = static_cast<long long>(T) * H * 8;
@@ -1738,7 +1738,7 @@ extern "C" int nplm_fa_bwd_ws(const void* qkv, const void* out, const void* dout
                               const int* rope_pos, const float* rope_cos, const float* rope_sin,
                               int max_ctas, int* status, cudaStream_t st) {
   return ws_bwd_impl(qkv, out, dout, lse, dqkv, dq_acc, delta, seq_start, seq_end, T, H, D, window, scale,
-                     rope_pos, rope_cos, rope_sin, max_ctas, -1, status, st);
+                     rope_pos, rope_cos, rope_sin, max_ctas, -1, false, status, st);
 }
 
 // Same with the mode given by the caller (see ws_bwd_impl).
@@ -1748,7 +1748,17 @@ extern "C" int nplm_fa_bwd_ws_mode(const void* qkv, const void* out, const void*
                                    const int* rope_pos, const float* rope_cos, const float* rope_sin,
                                    int max_ctas, int mode, int* status, cudaStream_t st) {
   return ws_bwd_impl(qkv, out, dout, lse, dqkv, dq_acc, delta, seq_start, seq_end, T, H, D, window, scale,
-                     rope_pos, rope_cos, rope_sin, max_ctas, mode, status, st);
+                     rope_pos, rope_cos, rope_sin, max_ctas, mode, false, status, st);
+}
+
+// The same with dq_acc zero already.
+extern "C" int nplm_fa_bwd_ws_zeroed(const void* qkv, const void* out, const void* dout, const float* lse,
+                                     void* dqkv, float* dq_acc, float* delta, const int* seq_start,
+                                     const int* seq_end, int T, int H, int D, int window, float scale,
+                                     const int* rope_pos, const float* rope_cos, const float* rope_sin,
+                                     int max_ctas, int mode, int* status, cudaStream_t st) {
+  return ws_bwd_impl(qkv, out, dout, lse, dqkv, dq_acc, delta, seq_start, seq_end, T, H, D, window, scale,
+                     rope_pos, rope_cos, rope_sin, max_ctas, mode, true, status, st);
 }
 
 #ifdef NPLM_WS_TRACE

@@ -74,16 +74,17 @@ int nplm_gemm_bf16_pair(const void* A, const void* B, void* C, const void* R, in
                         int ldc, int ldr, int a_mn, int b_mn, int epi, int splits, int direct_epilogue,
                         const int* rope_pos, const float* rope_cos, const float* rope_sin, int rope_cols, int* status,
                         cudaStream_t stream);
-int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const void* R, float* delta, int M, int N, int K, int lda,
-                         int ldb, int ldc, int ldr, int b_mn, int* status, cudaStream_t stream);
+// clear (fp32 [M][N], may be null) is set to zero.
+int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const void* R, float* delta, float* clear, int M, int N, int K,
+                         int lda, int ldb, int ldc, int ldr, int b_mn, int* status, cudaStream_t stream);
 int nplm_norm_fwd(const void* x, const int* ids, const void* w, void* y, float* mean, float* rstd, int T, int C, float eps,
                   int rms, cudaStream_t st);
 int nplm_norm_bwd(const void* dy, const void* x, const int* ids, const void* w, const float* mean, const float* rstd,
                   const void* dres, void* dx, float* dw, float* dtable, int T, int C, int V, int rms, cudaStream_t st);
 int nplm_fa_fwd_ws(const void* qkv, void* out, float* lse, const int* seq_start, const int* seq_end, int T, int H, int D,
                    int window, float scale, int max_ctas, int* status, cudaStream_t st);
-int nplm_fa_bwd_ws_mode(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc,
-                        float* delta, const int* seq_start, const int* seq_end, int T, int H, int D, int window,
-                        float scale, const int* rope_pos, const float* rope_cos, const float* rope_sin, int max_ctas,
-                        int mode, int* status, cudaStream_t st);
+int nplm_fa_bwd_ws_zeroed(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc,
+                          float* delta, const int* seq_start, const int* seq_end, int T, int H, int D, int window,
+                          float scale, const int* rope_pos, const float* rope_cos, const float* rope_sin, int max_ctas,
+                          int mode, int* status, cudaStream_t st);
 }

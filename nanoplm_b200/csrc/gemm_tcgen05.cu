@@ -59,6 +59,7 @@ struct GemmArgs {
   int ldc, ldr;
   int splits;
   float* delta;     // EPI_STORE_DELTA: fp32 [N / 64][M]
+  float* clear;     // EPI_STORE_DELTA: fp32 [M][N] set to zero on the way, may be null
   int swiglu_half;  // EPI_SWIGLU: row offset of the gate half inside B (= N/2)
   int* status;
   // EPI_ROPE: position of every output row, cos / sin tables [max_pos][32] (head_dim 64)
@@ -564,6 +565,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           operand_load(0, x0, y0);
           if constexpr (EPI == EPI_SWIGLU_BWD) operand_load(1, N + x0, y0);
           else if (NCHW > 1 && x0 + 64 < N) operand_load(1, x0 + 64, y0);
+        }
+        if constexpr (EPI == EPI_STORE_DELTA) {
+          // The attention backward's sums of dQ start from zero: this tile's part of them, written while the MMAs run, half a
+          // warp to a row's 256 bytes. Product with this / product and a memset, us: 55 424 x 1024 of K = 1024 129 / 131 (there
+          // memory is busy either way), 8 704 27.6 / 33.2, 4 300 17.2 / 21.0, 600 x 256 of 256 10.9 / 16.5.
+          if (args.clear != nullptr) {
+            for (int x = x0; x < min(N, n0 + c1 * 64); x += 64)
+#pragma unroll 4
+              for (int r = y0 + (lane >> 4); r < min(M, y0 + 32); r += 2)
+                *reinterpret_cast<float4*>(args.clear + static_cast<size_t>(r) * N + x + (lane & 15) * 4) =
+                    make_float4(0.f, 0.f, 0.f, 0.f);
+          }
         }
       }
       if (!mbar_wait(&tfull_bar[acc], acc_phase)) {
@@ -1207,6 +1220,7 @@ struct GroupSpec {
   void* const* ag_ptrs = nullptr;  // every rank's full B buffer (this rank's one is B itself)
   unsigned* ag_flags = nullptr;
   float* delta = nullptr;          // EPI_STORE_DELTA side output
+  float* clear = nullptr;          // and what it sets to zero
   // mode 3 (EPI_AXPBY): a stack of `groups` problems of group_rows rows
   int group_rows = 0, sym = 0;
   float alpha = 1.f, beta = 0.f;
@@ -1310,6 +1324,7 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   args.ldr = ldr;
   args.splits = splits;
   args.delta = grp.delta;
+  args.clear = grp.clear;
   args.swiglu_half = N / 2;
   args.status = status;
   args.rope_pos = rope_pos;
@@ -1476,12 +1491,14 @@ extern "C" int nplm_gemm_bf16_pair(const void* A, const void* B, void* C, const 
 // C = A B^T (b_mn = 0) or A B (b_mn = 1) in bf16, plus delta[h][row] = sum_{64 columns of head h}
 // C[row] * R[row] (fp32 [N / 64][M]): the data gradient of the attention output projection and the
 // rowsum(dO * O) term of the attention backward in one pass (R = the attention output O).
-extern "C" int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const void* R, float* delta, int M,
+extern "C" int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const void* R, float* delta, float* clear, int M,
                                     int N, int K, int lda, int ldb, int ldc, int ldr, int b_mn, int* status,
                                     cudaStream_t stream) {
+  if (reinterpret_cast<uintptr_t>(clear) & 15) return -3;
   GroupSpec g;
   g.pair = true;
   g.delta = delta;
+  g.clear = clear;
   return gemm_entry(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, 0, b_mn, EPI_STORE_DELTA, 1, 256, 0, 0, nullptr,
                     nullptr, nullptr, 0, status, stream, g);
 }

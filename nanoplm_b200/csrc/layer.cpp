@@ -24,7 +24,7 @@ struct Entry {   // in the order of `_native` in ops/layer.py
   decltype(&nplm_norm_fwd) norm_fwd;
   decltype(&nplm_norm_bwd) norm_bwd;
   decltype(&nplm_fa_fwd_ws) fa_fwd;
-  decltype(&nplm_fa_bwd_ws_mode) fa_bwd;
+  decltype(&nplm_fa_bwd_ws_zeroed) fa_bwd;
 };
 Entry fn;
 
@@ -226,9 +226,10 @@ extern "C" int nplm_layer_bwd(const long long* a, double scale) {
   TRY(fn.norm_bwd(d.dh, s.x1, nullptr, n2, rms ? nullptr : s.mean2, s.rstd2, dy, d.dx1, g_n2, nullptr, T, C, 0, rms,
                   k.stream));
   // attention
-  TRY(fn.delta(d.dx1, wo, d.d_o, s.o, d.delta, T, HD, C, C, HD, HD, HD, 1, k.status, k.stream));
+  float* dq = mode == 3 ? nullptr : d.dq;
+  TRY(fn.delta(d.dx1, wo, d.d_o, s.o, d.delta, dq, T, HD, C, C, HD, HD, HD, 1, k.status, k.stream));
   TRY(k.wgrad(d.dx1, s.o, g_o, T, C, HD, static_cast<int>(a[BWD_SPLITS_O])));
-  TRY(fn.fa_bwd(s.qkv, nullptr, d.d_o, s.lse, d.dqkv, mode == 3 ? nullptr : d.dq, d.delta, ss, se, T, H, 64, window,
+  TRY(fn.fa_bwd(s.qkv, nullptr, d.d_o, s.lse, d.dqkv, dq, d.delta, ss, se, T, H, 64, window,
                 static_cast<float>(scale), pos, cosp, sinp, 0, mode, k.status, k.stream));
   TRY(k.wgrad(d.dqkv, norm1 ? s.h1 : x, g_qkv, T, 3 * HD, C, static_cast<int>(a[BWD_SPLITS_QKV])));
   if (!norm1)   // the layer input enters the projection and the residual: both gradients in one epilogue

@@ -629,8 +629,8 @@ def gemm_dgrad_delta(dy: torch.Tensor, w: torch.Tensor, o: torch.Tensor, delta: 
     if N % 64 or tuple(o.shape) != (M, N) or tuple(delta.shape) != (N // 64, M) or not delta.is_contiguous():
         raise ValueError("o must be [M, N], delta [N / 64, M] contiguous, N a multiple of 64")
     out = torch.empty((M, N), dtype=_BF16, device=dy.device)
-    rc = typed("gemm_tcgen05", "nplm_gemm_bf16_delta", "ppppp" + "iiiiiiii" + "pp")(
-        dy.data_ptr(), w.data_ptr(), out.data_ptr(), o.data_ptr(), delta.data_ptr(), M, N, Kd, _rowmajor(dy, "dy"),
+    rc = typed("gemm_tcgen05", "nplm_gemm_bf16_delta", "pppppp" + "iiiiiiii" + "pp")(
+        dy.data_ptr(), w.data_ptr(), out.data_ptr(), o.data_ptr(), delta.data_ptr(), 0, M, N, Kd, _rowmajor(dy, "dy"),
         _rowmajor(w, "w"), N, _rowmajor(o, "o"), 1, status_word(dy.device).data_ptr(), raw_stream())
     check_rc(rc, "gemm_bf16_delta")
     count_launch()

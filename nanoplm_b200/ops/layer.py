@@ -32,7 +32,7 @@ def _native():
         fns = [("gemm_tcgen05", "nplm_gemm_bf16"), ("gemm_tcgen05", "nplm_gemm_bf16_pair"),
                ("gemm_tcgen05", "nplm_gemm_bf16_delta"), ("elementwise", "nplm_norm_fwd"),
                ("elementwise", "nplm_norm_bwd"), ("attention_ws", "nplm_fa_fwd_ws"),
-               ("attention_ws", "nplm_fa_bwd_ws_mode")]
+               ("attention_ws", "nplm_fa_bwd_ws_zeroed")]
         h.nplm_layer_init((ctypes.c_void_p * len(fns))(
             *[ctypes.cast(getattr(lib(l), f), ctypes.c_void_p).value for l, f in fns]))
         h.nplm_layer_bytes.argtypes = [ctypes.c_longlong] * 4 + [ctypes.c_int] * 3
