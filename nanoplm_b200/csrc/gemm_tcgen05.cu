@@ -823,9 +823,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               }
             } else if constexpr (EPI == EPI_AXPBY) {
               if (active) {
-                const int buf = (c - c0) & 1;
-                uint8_t* rb = stage + buf * 4096;
                 if (args.R != nullptr) {
+                  const int buf = (c - c0) & 1;
+                  uint8_t* rb = stage + buf * 4096;
                   if (!operand_wait(buf)) {
                     if (lane == 0) atomicExch(args.status, ST_TIMEOUT_MISC);
                   }
@@ -840,13 +840,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                                                       args.alpha * f[j * 8 + 2 * e + 1] + args.beta * t.y);
                     }
                   }
+                  stage_store_inplace(rb, &tmC, packed, x, y0, lane);
+                  if (c + 2 < c1 && chunk_in(c + 2)) operand_load(buf, x + 128, y0);
                 } else {
+                  // The buffers alternate from store to store and not with the chunk: a warp whose second chunk lies past the
+                  // last column stores one chunk an item, and by the chunk's number its next item would overwrite the buffer that
+                  // the newest store, which the wait leaves outstanding, may still be reading.
 #pragma unroll
                   for (int e = 0; e < 32; ++e) packed[e] = pack_bf16x2(args.alpha * f[2 * e], args.alpha * f[2 * e + 1]);
-                  if (elect_one()) tma_store_wait_read<1>();   // the store that read this buffer two chunks ago
+                  stage_store_bf16(stage, stage_toggle, &tmC, packed, x, y0, lane);
                 }
-                stage_store_inplace(rb, &tmC, packed, x, y0, lane);
-                if (args.R != nullptr && c + 2 < c1 && chunk_in(c + 2)) operand_load(buf, x + 128, y0);
                 const int m_tile = m0 - static_cast<int>(rank) * BM;
                 if (args.sym && it.b_row + n0 < m_tile) {
                   // the tile across the diagonal: column x + e of this row is row x + e there. Lanes 2i and 2i + 1 exchange

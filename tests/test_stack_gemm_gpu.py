@@ -39,6 +39,19 @@ def test_symmetric_products(B, m, k, cuda_status):
     assert torch.equal(P, P.transpose(1, 2))
 
 
+# half a pair of column chunks at the right edge, and several tiles for each of the 74 pairs
+@pytest.mark.parametrize("B,m,n,k", [(64, 512, 704, 64), (40, 256, 1088, 128)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_stack_of_many_ragged_tiles(B, m, n, k, b_mn, cuda_status):
+    """Bit for bit the products one by one: neither tiles nor buffers change the order of a sum."""
+    from nanoplm_b200.ops import kernels as K
+    torch.manual_seed(n)
+    a, b = _stack(B, m, k), _stack(B, k, n) if b_mn else _stack(B, n, k)
+    want = torch.stack([K.gemm(x, y, b_mn=b_mn) for x, y in zip(a, b)])
+    for _ in range(3):
+        assert torch.equal(K.gemm_stack(a, b, b_mn=b_mn), want)
+
+
 def test_stack_refusals(cuda_status):
     from nanoplm_b200.ops import kernels as K
     with pytest.raises(Exception):
