@@ -15,16 +15,15 @@ from torch.nn.modules.module import _has_any_global_hook
 
 from nanoplm_b200.config.schema import StudentConfig
 from nanoplm_b200.data.tokenizer import StudentTokenizer
-from nanoplm_b200.models.encoder import (BatchContext, EncoderModel, Linear, Norm,
+from nanoplm_b200.models.encoder import (Attention, BatchContext, EncoderLayer, EncoderModel, Linear, Norm,
                                          position_ids_from_cu_seqlens)
-from nanoplm_b200.ops import functional as ops
 from nanoplm_b200.ops import functional as ops
 from nanoplm_b200.ops import kernels as K
 
 
-# Tokens up to which embed_sequences joins batches: their activations (5 to 10 KB a token at 512 to 1024 channels) stay within
-# 350 MB, and longer runs gain nothing more (GEMMs of 32 768 rows fill 256 tiles of 128 rows a column of tiles).
-_EMBED_TOKENS = 32768
+# Tokens and bytes of activations up to which embed_sequences joins batches. Longer runs gain nothing more (GEMMs of 32 768 rows
+# fill 256 tiles of 128 rows a column of tiles).
+_EMBED_TOKENS, _EMBED_BYTES = 32768, 512 << 20
 
 
 class ProtX(EncoderModel):
@@ -133,6 +132,29 @@ class ProtX(EncoderModel):
                 and type(self).forward is ProtX.forward and "forward" not in self.__dict__
                 and not self._forward_hooks and not self._forward_pre_hooks and not _has_any_global_hook())
 
+    def _join_tokens(self) -> int:
+        """Tokens up to which embed_sequences may run several batches as one (0: not at all). Between them lies padding whose rows
+        have no keys: the attention kernel for 64-wide heads gives such rows zeros, the dense form that other widths take
+        gives NaN, which the next layer would spread, and needs scores of the square of the tokens. Experts see how many tokens
+        a call has, weights that are gathered on use want as many calls on every rank, and a hook on any part may count
+        them."""
+        cfg, walk = self.config, [self]
+        for l in self.layers:
+            if not (type(l) is EncoderLayer and type(l.attn) is Attention and l.attn.head_dim == 64 and not l.is_moe
+                    and type(l.attn.Wqkv) is Linear and l.attn.Wqkv.weight.dtype == torch.bfloat16):
+                return 0
+        while walk:         # (`modules()` also remembers whom it has met, which costs more than several layers' launches)
+            m = walk.pop()
+            if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+                return 0
+            if any(getattr(p, "_ag", None) is not None for p in m._parameters.values()):
+                return 0
+            walk += [c for c in m._modules.values() if c is not None]
+        # two copies of the streams and a layer's tensors beside them: 13.3 KB at 512 channels, 26.6 at 1024, 19.5 for four streams of
+        # 512, where the allocator's peak is 8.2, 16.5 and 16.5 a token
+        per_token = 2 * (cfg.hidden_size * (7 + 2 * cfg.mhc_streams) + 2 * cfg.intermediate_size)
+        return min(_EMBED_TOKENS, _EMBED_BYTES // per_token)
+
     def _pack_batches(self, batches: list[list[str]]) -> tuple[np.ndarray, np.ndarray, list[bool]]:
         """(ids, lengths, which of the sequences are real) of several batches one after the other. Every batch starts on a
         multiple of 256 tokens, behind padding: the attention's tiles then cut a batch where they cut it alone, and the
@@ -177,18 +199,32 @@ class ProtX(EncoderModel):
         h, _ = EncoderModel.forward(self, dev[:T], ctx)
         return h, cu_dev
 
+    def _embed_run(self, ids: np.ndarray, lens: np.ndarray, real: list[bool], per_token: bool, device):
+        """(device rows, how many of them each real sequence has; -1 for the mean of a stretch of padding) of a packed host
+        batch."""
+        h, cu = self._embed_packed(ids, lens, device, real)
+        if not per_token:
+            return K.segment_mean(h, cu, drop_last=1), [1 if r else -1 for r in real]
+        ends, lens = np.cumsum(lens).tolist(), lens.tolist()    # the residues' rows, without the trailing </s> of every sequence
+        keep = torch.cat([torch.arange(e - n, e - 1) for n, e, r in zip(lens, ends, real) if r])
+        return h[keep.to(device)], [n - 1 for n, r in zip(lens, real) if r]
+
     @torch.no_grad()
     def embed_sequences(self, sequences: list[str], batch_size: int = 16, per_token: bool = False,
                         device: Optional[torch.device] = None) -> list[torch.Tensor]:
-        """Mean-pooled (EOS excluded) or per-token embeddings for raw sequences."""
+        """Mean-pooled (EOS excluded) or per-token embeddings for raw sequences.
+
+        batch_size is the number of sequences that are padded to a common length where padding is needed, and what
+        bounds the memory there. A bf16 model with 64-wide heads on a GPU takes packed sequences: whole batches run together
+        up to 32 768 tokens and 512 MiB of activations, with the results that they have one by one, and one by one where
+        the memory for that is not there."""
         device = device or next(self.parameters()).device
         # (walking all modules to set a flag that is set already costs more than several layers' launches, and so does
         # looking at it through `modules()`, which remembers whom it has met)
-        was_training, watched, walk = False, False, [self]
+        was_training, walk = False, [self]
         while walk:
             m = walk.pop()
             was_training |= m.training
-            watched |= bool(m._forward_hooks) or bool(m._forward_pre_hooks) or "forward" in m.__dict__
             walk += [c for c in m._modules.values() if c is not None]
         restore = self.training
         if was_training:
@@ -210,47 +246,43 @@ class ProtX(EncoderModel):
 
         direct = packed and type(self.tokenizer) is StudentTokenizer and self.tokenizer.packs()
         plain = lambda b: type(b) is list and all(type(t) is str for t in b)
+        most = None                                                        # (tokens of joined batches, once there are two)
         i, end = 0, len(sequences) if range(0, 1, batch_size) else 0       # (a step of 0 is an error, a negative one no steps)
         while i < end:
-            batch, flat, real = sequences[i:i + batch_size], None, None
+            first, batch, flat, joined = i, sequences[i:i + batch_size], None, []
             i += batch_size
             if direct and plain(batch):
-                # Packed rows neither know their batch nor pad it: further batches join while they fit, unless a hook on some
-                # part may count them, and a layer's launches fill the chip. 91 proteins of 46 000 tokens at 512 channels took 36
-                # layers of 8 000 rows, one to two waves of tiles a GEMM.
+                # Packed rows neither know their batch nor pad it: further batches join while they fit, and a layer's launches
+                # fill the chip. 91 proteins of 46 000 tokens at 512 channels took 36 layers of 8 000 rows, one to two
+                # waves of tiles a GEMM.
                 joined = [batch]
                 tokens = sum(map(len, batch)) + len(batch)
-                while not watched and i < end:
+                while i < end:
+                    if most is None:
+                        most = self._join_tokens()
                     more = sequences[i:i + batch_size]
-                    if not plain(more):
-                        break
-                    tokens += 255 + sum(map(len, more)) + len(more)
-                    if tokens > _EMBED_TOKENS:
+                    tokens += 255 + sum(map(len, more)) + len(more) if most and plain(more) else most + 1
+                    if tokens > most:
                         break
                     joined.append(more)
                     i += batch_size
-                *flat, real = self._pack_batches(joined)
+                flat = self._pack_batches(joined)
             else:
                 enc = self.tokenizer(batch, padding=True, return_tensors="pt")
                 ids, mask = enc["input_ids"], enc["attention_mask"]
                 # the real tokens first, at least one, then padding
                 if (packed and not ids.is_cuda and bool(mask[:, 0].all())
                         and bool((mask[:, :-1] >= mask[:, 1:]).all())):
-                    flat = ids.numpy()[mask.numpy().astype(bool)], mask.sum(dim=1).numpy()
+                    flat = ids.numpy()[mask.numpy().astype(bool)], mask.sum(dim=1).numpy(), [True] * len(mask)
             if flat is not None:
-                ids, lens = flat
-                real = real or [True] * len(lens)
-                h, cu = self._embed_packed(ids, lens, device, real)
-                if per_token:       # the residues' rows, without the trailing </s> of every sequence
-                    ends = np.cumsum(lens).tolist()
-                    lens = lens.tolist()
-                    keep = torch.cat([torch.arange(e - n, e - 1) for n, e, r in zip(lens, ends, real) if r])
-                    h = h[keep.to(device)]
-                    waiting.append((h, [n - 1 for n, r in zip(lens, real) if r]))
-                else:
-                    h = K.segment_mean(h, cu, drop_last=1)
-                    waiting.append((h, [1 if r else -1 for r in real]))
-                rows += h.shape[0]
+                try:
+                    waiting.append(self._embed_run(*flat, per_token, device))
+                except torch.OutOfMemoryError:
+                    if len(joined) < 2:
+                        raise
+                    i, most = first, 0          # what fits one by one still runs
+                    continue
+                rows += waiting[-1][0].shape[0]
                 if rows >= 65536:   # bounds what waits on the device
                     collect()
                 continue
