@@ -234,7 +234,11 @@ def supported(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def addable(residual: torch.Tensor, x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the product's epilogue can add `residual`: bf16 rows of the output's shape on 16-byte boundaries."""
+    """Whether the product's epilogue can add `residual`: bf16 rows of the output's shape on 16-byte boundaries, and nobody
+    who has to see the sum itself (a tangent of the residual alone goes through a sum, but not through the product's node)."""
+    from .functional import functions_observed
+    if functions_observed():
+        return False
     if residual.dtype != _BF16 or not residual.is_cuda or residual.shape != (*x.shape[:-1], w.shape[0]):
         return False
     r = residual.reshape(-1, w.shape[0])
@@ -354,14 +358,14 @@ class _Fp8MlpFn(torch.autograd.Function):
         return dx, dw_in, dw_out, (dy if ctx.has_res else None)
 
 
-def mlp_fused(x: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor) -> bool:
-    """Whether `fp8_mlp` takes a call: both projections fit (`supported`, whole 128-column halves), whole 128-token blocks, and
-    a backward pass for both weights."""
+def mlp_fused(x: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor, residual: torch.Tensor | None = None) -> bool:
+    """Whether `fp8_mlp` takes a call: both projections fit (`supported`, whole 128-column halves), whole 128-token blocks, a
+    residual that the epilogue can add, and a backward pass for both weights."""
     from .functional import _keeps, functions_observed
     inter = w_out.shape[1]
-    return (not functions_observed() and supported(x, w_in) and supported(x, w_out) and w_in.shape[0] == 2 * inter and w_in.shape[1] == x.shape[-1]
-            and x.numel() > 0 and _dual_rows(x.numel() // x.shape[-1]) and _keeps() and w_in.requires_grad
-            and w_out.requires_grad)
+    return (not functions_observed() and supported(x, w_in) and supported(x, w_out) and w_in.shape[0] == 2 * inter
+            and w_in.shape[1] == x.shape[-1] and x.numel() > 0 and _dual_rows(x.numel() // x.shape[-1]) and _keeps()
+            and w_in.requires_grad and w_out.requires_grad and (residual is None or addable(residual, x, w_out)))
 
 
 def fp8_mlp(x, w_in, w_out, residual=None):

@@ -210,7 +210,7 @@ def mlp_swiglu(x, w_in, w_out, residual=None):
         return _call(_SwiGLUMLPFn, x, w_in, w_out, residual, _keeps())
     if x.is_cuda and _FP8_STATE["enabled"]:
         from . import fp8
-        if fp8.mlp_fused(x, w_in, w_out):
+        if fp8.mlp_fused(x, w_in, w_out, residual):
             return fp8.fp8_mlp(x, w_in, w_out, residual)
     return linear(linear(x, w_in, act="swiglu"), w_out, residual=residual)
 

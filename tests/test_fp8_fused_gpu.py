@@ -113,3 +113,46 @@ def test_mlp_node_is_the_composition(cuda_status):
     finally:
         F_.set_fp8(False)
         fp8.invalidate_weight_cache()
+
+
+def _residuals(T, C):
+    base = torch.randn(T * C + 8, device="cuda").to(BF)
+    return {"fp32": torch.randn(T, C, device="cuda"), "row": _randn(1, C), "off 16 bytes": base[1:T * C + 1].view(T, C),
+            "odd row stride": _randn(T, C + 1)[:, :C], "columns first": _randn(C, T).t()}
+
+
+@pytest.mark.parametrize("kind", ["fp32", "row", "off 16 bytes", "odd row stride", "columns first"])
+def test_residuals_that_the_epilogue_cannot_add(kind, cuda_status):
+    """They are added as a sum of its own, with its result type and its gradient."""
+    from nanoplm_b200.ops import fp8
+    from nanoplm_b200.ops import functional as F_
+    torch.manual_seed(1)
+    T, C, I = 256, 128, 256
+    x, wi, wo = _randn(T, C), _randn(2 * I, C, scale=C ** -0.5), _randn(C, I, scale=I ** -0.5)
+    wi.requires_grad_(True), wo.requires_grad_(True)
+    r = _residuals(T, C)[kind].requires_grad_(True)
+    F_.set_fp8(True)
+    try:
+        for call in (lambda res: F_.mlp_swiglu(x, wi, wo, res), lambda res: F_.linear(F_.mlp_swiglu(x, wi, wo), wo[:, :C], residual=res)):
+            y = call(r)
+            assert torch.equal(y, call(None) + r)
+            (g,) = torch.autograd.grad(y.float().sum(), r)
+            assert g.shape == r.shape and torch.equal(g, torch.full_like(g, T if kind == "row" else 1))
+    finally:
+        F_.set_fp8(False)
+        fp8.invalidate_weight_cache()
+
+
+def test_tangent_of_the_residual(cuda_status):
+    import torch.autograd.forward_ad as fwd
+    from nanoplm_b200.ops import fp8
+    from nanoplm_b200.ops import functional as F_
+    x, w, r, t = _randn(128, 128), _randn(128, 128), _randn(128, 128), _randn(128, 128)
+    F_.set_fp8(True)
+    try:
+        with fwd.dual_level():
+            y, dy = fwd.unpack_dual(F_.linear(x, w, residual=fwd.make_dual(r, t)))
+            assert torch.equal(dy, t) and torch.equal(y, F_.linear(x, w) + r)
+    finally:
+        F_.set_fp8(False)
+        fp8.invalidate_weight_cache()
