@@ -797,8 +797,10 @@ ce_fwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
 // Bound by its 2 x 32 fp32 multiply-adds an element of h. A thread owns two channels: W and the sums dW of all 32 entries
 // of the vocabulary stay in registers (128 of them, three blocks a multiprocessor), the dlogits of 16 rows are read as
 // broadcasts from shared memory, doubled for the packed multiply-adds. A block takes 256 channels of `rows` rows, so that
-// 1 300 rows already fill the chip: 1 300 x 1024 12.5 us, 8 300 x 1024 38, where a block a 32-row tile took 95 and 170.
+// 1 300 rows already fill the chip: 1 300 x 1024 11.5 us, 8 300 x 1024 42, where a block a 32-row tile took 95 and 170.
 // The 32 products of an element of dh are one chain in the vocabulary's order: its bits reach e4m3 training.
+// A row whose dlogits are all zero (an ignored label) has a zero gradient and its h is not read: an infinity or a NaN there
+// reaches nothing.
 constexpr int CE_ROWS = 16;
 
 __global__ void __launch_bounds__(128, 3)
@@ -808,6 +810,7 @@ ce_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
               int n, int C, int V, int rows) {
   grid_chain();
   __shared__ __align__(16) float2 sd[CE_ROWS][32];
+  __shared__ __align__(16) uint8_t live[CE_ROWS];
   const int tid = threadIdx.x;
   const int ch = blockIdx.x * 256 + tid * 2;
   const bool own = ch < C;
@@ -826,10 +829,16 @@ ce_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
 #pragma unroll
     for (int i = tid; i < CE_ROWS * 32; i += 128) {
       const int r = base + (i >> 5);
-      const float d = r < r1 ? dlogits[static_cast<size_t>(r) * 32 + (i & 31)] * g : 0.f;
+      const float d = r < r1 && (i & 31) < V ? dlogits[static_cast<size_t>(r) * 32 + (i & 31)] * g : 0.f;
       sd[i >> 5][i & 31] = make_float2(d, d);
+      const int any = __any_sync(0xffffffffu, d != 0.f);      // (a warp holds one row)
+      if ((i & 31) == 0) live[i >> 5] = any ? 1 : 0;
     }
     __syncthreads();
+    // bit r: row base + r has a gradient (four bytes of 0 or 1 gathered into the top nibble by each product)
+    const uint4 all = *reinterpret_cast<const uint4*>(live);
+    const uint32_t rows_on = (all.x * 0x10204080u >> 28) | (all.y * 0x10204080u >> 28 << 4) |
+                             (all.z * 0x10204080u >> 28 << 8) | (all.w * 0x10204080u >> 28 << 12);
     if (blockIdx.x == 0 && tid < 32) {
 #pragma unroll
       for (int r = 0; r < CE_ROWS; ++r) db += sd[r][tid].x;
@@ -839,7 +848,7 @@ ce_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
       float2 hv[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        hv[q] = own && base + r + q < r1
+        hv[q] = own && (rows_on >> (r + q) & 1u)
                     ? unpack_bf16x2(__ldg(reinterpret_cast<const uint32_t*>(h + static_cast<size_t>(base + r + q) * C + ch)))
                     : make_float2(0.f, 0.f);
 #pragma unroll
@@ -855,7 +864,8 @@ ce_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restri
           acc[v + 1] = fma2(d1, hv[q], acc[v + 1]);
         }
         if (own && base + r + q < r1)
-          *reinterpret_cast<uint32_t*>(dh + static_cast<size_t>(base + r + q) * C + ch) = pack_bf16x2(o.x, o.y);
+          *reinterpret_cast<uint32_t*>(dh + static_cast<size_t>(base + r + q) * C + ch) =
+              (rows_on >> (r + q) & 1u) ? pack_bf16x2(o.x, o.y) : 0u;
       }
     }
   }

@@ -66,3 +66,25 @@ def test_label_count(n, cuda_status):
     labels = torch.randint(-2, 3, (n,), device="cuda", dtype=torch.int32)
     inv, loss = k.ce_count(labels)
     assert inv.item() == (1.0 / (labels >= 0).sum().clamp(min=1).float()).item() and loss.item() == 0
+
+
+@pytest.mark.parametrize("C,V", [(256, 32), (1024, 31), (1032, 29), (2048, 32)])
+def test_decoder_backward_of_ignored_rows(C, V, cuda_status):
+    """Rows whose dlogits are all zero have a zero gradient whatever they hold."""
+    from nanoplm_b200.ops import kernels as k
+    n = 83
+    h, W = torch.randn(n, C, device="cuda").to(BF), (torch.randn(V, C, device="cuda") * 0.05).to(BF)
+    dl = torch.zeros(n, 32, device="cuda")
+    dl[:, :V] = torch.randn(n, V, device="cuda") / n
+    dl[::3] = 0
+    bad = h.clone()
+    bad[::6], bad[3::6] = float("inf"), float("nan")
+    gs = torch.full((1,), 0.5, device="cuda")
+    grads = []
+    for x in (bad, h):
+        dW, db = torch.zeros(V, C, device="cuda"), torch.zeros(V, device="cuda")
+        grads.append((k.ce_bwd(x, W, dl, gs, dW, db), dW, db))
+    (dh, dW, db), (dh_ref, dW_ref, db_ref) = grads
+    assert torch.equal(dh, dh_ref) and dh[::3].abs().max() == 0
+    # the blocks' sums are added in any order
+    assert (dW - dW_ref).abs().max() < 1e-6 and (db - db_ref).abs().max() < 1e-6
