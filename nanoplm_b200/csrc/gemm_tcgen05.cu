@@ -1127,7 +1127,8 @@ static int launch_impl(const GemmMaps& maps, const GemmArgs& args, int max_ctas,
     return static_cast<int>(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(grid),
                                                         dim3(S::THREADS), params, S::TOTAL, stream));
   }
-  launch_chained(kern, grid, S::THREADS, S::TOTAL, stream, tmA, tmB, maps.C, maps.R, args);
+  // (a grid that will wait for rows from other GPUs takes no room before its own turn)
+  launch_when(args.row_arrive == nullptr, kern, grid, S::THREADS, S::TOTAL, stream, tmA, tmB, maps.C, maps.R, args);
   return static_cast<int>(cudaGetLastError());
 }
 
