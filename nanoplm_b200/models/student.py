@@ -136,20 +136,16 @@ class ProtX(EncoderModel):
         """Tokens up to which embed_sequences may run several batches as one (0: not at all). Between them lies padding whose rows
         have no keys: the attention kernel for 64-wide heads gives such rows zeros, the dense form that other widths take
         gives NaN, which the next layer would spread, and needs scores of the square of the tokens. Experts see how many tokens
-        a call has, weights that are gathered on use want as many calls on every rank, and a hook on any part may count
-        them."""
-        cfg, walk = self.config, [self]
-        for l in self.layers:
-            if not (type(l) is EncoderLayer and type(l.attn) is Attention and l.attn.head_dim == 64 and not l.is_moe
-                    and type(l.attn.Wqkv) is Linear and l.attn.Wqkv.weight.dtype == torch.bfloat16):
+        a call has."""
+        cfg = self.config
+        for l in self.layers:       # (a dozen layers before the first launch: no look-ups through Module.__getattr__)
+            a = l._modules.get("attn")
+            if type(l) is not EncoderLayer or l.is_moe or type(a) is not Attention or a.head_dim != 64:
                 return 0
-        while walk:         # (`modules()` also remembers whom it has met, which costs more than several layers' launches)
-            m = walk.pop()
-            if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+            qkv = a._modules["Wqkv"]
+            w = qkv._parameters.get("weight")
+            if type(qkv) is not Linear or w is None or w.dtype != torch.bfloat16:
                 return 0
-            if any(getattr(p, "_ag", None) is not None for p in m._parameters.values()):
-                return 0
-            walk += [c for c in m._modules.values() if c is not None]
         # two copies of the streams and a layer's tensors beside them: 13.3 KB at 512 channels, 26.6 at 1024, 19.5 for four streams of
         # 512, where the allocator's peak is 8.2, 16.5 and 16.5 a token
         per_token = 2 * (cfg.hidden_size * (7 + 2 * cfg.mhc_streams) + 2 * cfg.intermediate_size)
@@ -221,10 +217,11 @@ class ProtX(EncoderModel):
         device = device or next(self.parameters()).device
         # (walking all modules to set a flag that is set already costs more than several layers' launches, and so does
         # looking at it through `modules()`, which remembers whom it has met)
-        was_training, walk = False, [self]
+        was_training, watched, walk = False, False, [self]
         while walk:
             m = walk.pop()
             was_training |= m.training
+            watched |= bool(m._forward_hooks) or bool(m._forward_pre_hooks) or "forward" in m.__dict__
             walk += [c for c in m._modules.values() if c is not None]
         restore = self.training
         if was_training:
@@ -246,7 +243,7 @@ class ProtX(EncoderModel):
 
         direct = packed and type(self.tokenizer) is StudentTokenizer and self.tokenizer.packs()
         plain = lambda b: type(b) is list and all(type(t) is str for t in b)
-        most = None                                                        # (tokens of joined batches, once there are two)
+        most = 0 if watched else None       # tokens of joined batches; a hook on some part may count them
         i, end = 0, len(sequences) if range(0, 1, batch_size) else 0       # (a step of 0 is an error, a negative one no steps)
         while i < end:
             first, batch, flat, joined = i, sequences[i:i + batch_size], None, []
