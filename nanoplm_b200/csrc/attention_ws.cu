@@ -1712,15 +1712,20 @@ static int ws_bwd_impl(const void* qkv, const void* out, const void* dout, const
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (grid > n_items) grid = n_items;
   if (mode == 2) {
-    launch_chained(fa_bwd_ws_kernel<2, BWD_KV_DQ>, grid, WsBwdCfg<2, true>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<2, BWD_KV_DQ>, grid, WsBwdCfg<2, true>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ,
+        tmOUT, a);
   } else if (mode == 0) {
-    launch_chained(fa_bwd_ws_kernel<4, BWD_KV>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_KV>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ,
+        tmOUT, a);
   } else if (mode == 3) {
-    launch_chained(fa_bwd_ws_kernel<4, BWD_KV>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
-    launch_chained(fa_bwd_ws_kernel<4, BWD_Q>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_KV>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ,
+        tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_Q>, grid, WsBwdCfg<4, false>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ,
+        tmOUT, a);
     return static_cast<int>(cudaGetLastError());
   } else {
-    launch_chained(fa_bwd_ws_kernel<4, BWD_KV_DQ>, grid, WsBwdCfg<4, true>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ, tmOUT, a);
+    launch_chained(fa_bwd_ws_kernel<4, BWD_KV_DQ>, grid, WsBwdCfg<4, true>::THREADS, WS_BWD_SMEM, st, tmQKV, tmDO, tmDQ,
+        tmOUT, a);
   }
   {
     const long long total = static_cast<long long>(T) * H * 4;

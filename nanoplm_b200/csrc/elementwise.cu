@@ -409,7 +409,7 @@ static int norm_bwd_ring(const __nv_bfloat16* dy, const __nv_bfloat16* x, const 
   int blocks = (T + NB_WARPS - 1) / NB_WARPS;
   if (blocks > 148 * 2) blocks = 148 * 2;   // more blocks only add contention on the dw atomics
   launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, kern, blocks, NB_WARPS * 32,
-              static_cast<size_t>(NB_WARPS) * NB_STAGES * (RES ? 3 : 2) * C * 2, st, dy, x, w, mean, rstd, dres, dx, dw, T, C);
+      static_cast<size_t>(NB_WARPS) * NB_STAGES * (RES ? 3 : 2) * C * 2, st, dy, x, w, mean, rstd, dres, dx, dw, T, C);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1143,7 +1143,8 @@ extern "C" int nplm_norm_fwd(const void* x, const int* ids, const void* w, void*
   if (C % 8) return -3;
   const int blocks = (T + 7) / 8 < 148 * 8 ? (T + 7) / 8 : 148 * 8;
 #define CALL(N_)                                                                               \
-  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, norm_fwd_kernel<N_>, blocks, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), ids,  \
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, norm_fwd_kernel<N_>, blocks, 256, 0, st,                       \
+      reinterpret_cast<const __nv_bfloat16*>(x), ids,                                                                         \
                                               reinterpret_cast<const __nv_bfloat16*>(w),       \
                                               reinterpret_cast<__nv_bfloat16*>(y), mean, rstd, \
                                               T, C, eps, rms)
@@ -1211,7 +1212,8 @@ extern "C" int nplm_embed_bwd(const void* dy, const void* table, const int* ids,
     NPLM_CUDA_CHECK(cudaFuncSetAttribute(embed_grad_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     configured_on[dev_slot] = true;
   }
-  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, embed_grad_sums_kernel, dim3(slices, by), 32 * warps, static_cast<size_t>(warps) * table_bytes, st,
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, embed_grad_sums_kernel, dim3(slices, by), 32 * warps,
+      static_cast<size_t>(warps) * table_bytes, st,
                  reinterpret_cast<const __nv_bfloat16*>(dy), ids, scratch, T, C, V);
   launch_chained(embed_grad_finish_kernel, V, 256, 0, st, scratch, reinterpret_cast<const __nv_bfloat16*>(table),
                  reinterpret_cast<const __nv_bfloat16*>(w), mean, rstd, dtable, dw, C, V, rms);
@@ -1223,8 +1225,8 @@ extern "C" int nplm_rope(void* qkv, const int* pos, const float* cos_t, const fl
   if (T <= 0) return 0;
   if (D % 16) return -3;
   const long long total = static_cast<long long>(T) * 2 * H * (D / 16);
-  launch_when(static_cast<long long>(T) * 2 * H * D <= CHAIN_ELEMENTS, rope_kernel, grid_for(total, 256), 256, 0, st, reinterpret_cast<__nv_bfloat16*>(qkv), pos,
-                                                    cos_t, sin_t, T, H, D, backward ? -1.f : 1.f);
+  launch_when(static_cast<long long>(T) * 2 * H * D <= CHAIN_ELEMENTS, rope_kernel, grid_for(total, 256), 256, 0, st,
+      reinterpret_cast<__nv_bfloat16*>(qkv), pos, cos_t, sin_t, T, H, D, backward ? -1.f : 1.f);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1355,8 +1357,8 @@ extern "C" int nplm_segment_mean(const void* x, const int* cu, float* out, int B
                                  cudaStream_t st) {
   if (B <= 0) return 0;
   if ((C % 8) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
-  launch_chained(nplm::segment_mean_kernel, dim3(B, (C + 63) / 64), 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), cu, out,
-                                                                    C, drop_last);
+  launch_chained(nplm::segment_mean_kernel, dim3(B, (C + 63) / 64), 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),
+      cu, out, C, drop_last);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1456,9 +1458,11 @@ static int unpad_fill(const void* mask, const void* ids, int id_bytes, const int
 // mask [B][S] (mask_bytes 1, 4 or 8: bool / integers, kept where not zero); counts: int [B] scratch, cu: int [B + 1].
 extern "C" int nplm_unpad_count(const void* mask, int mask_bytes, int B, int S, int* counts, int* cu, cudaStream_t st) {
   if (B <= 0 || S <= 0) return -3;
-  if (mask_bytes == 1) launch_chained(unpad_count_kernel<signed char>, B, 256, 0, st, static_cast<const signed char*>(mask), S, counts);
+  if (mask_bytes == 1) launch_chained(unpad_count_kernel<signed char>, B, 256, 0, st,
+      static_cast<const signed char*>(mask), S, counts);
   else if (mask_bytes == 4) launch_chained(unpad_count_kernel<int>, B, 256, 0, st, static_cast<const int*>(mask), S, counts);
-  else if (mask_bytes == 8) launch_chained(unpad_count_kernel<long long>, B, 256, 0, st, static_cast<const long long*>(mask), S, counts);
+  else if (mask_bytes == 8) launch_chained(unpad_count_kernel<long long>, B, 256, 0, st,
+      static_cast<const long long*>(mask), S, counts);
   else return -3;
   launch_chained(running_sum_kernel, 1, 1024, 0, st, counts, B, cu);
   return static_cast<int>(cudaGetLastError());
@@ -1478,7 +1482,8 @@ extern "C" int nplm_gather_rows(const void* src, const int* idx, void* dst, int 
                                 cudaStream_t st) {
   if (n <= 0) return 0;
   if (C % 8) return -3;
-  launch_when(static_cast<long long>(n) * C <= CHAIN_ELEMENTS, gather_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(n) * C <= CHAIN_ELEMENTS, gather_rows_kernel,
+      grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(src), idx, reinterpret_cast<__nv_bfloat16*>(dst), n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1487,7 +1492,8 @@ extern "C" int nplm_scatter_rows(const void* src, const int* idx, void* dst, int
                                  cudaStream_t st) {
   if (n <= 0) return 0;
   if (C % 8) return -3;
-  launch_when(static_cast<long long>(n) * C <= CHAIN_ELEMENTS, scatter_rows_kernel, grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(n) * C <= CHAIN_ELEMENTS, scatter_rows_kernel,
+      grid_for(static_cast<long long>(n) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(src), idx, reinterpret_cast<__nv_bfloat16*>(dst), n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -1550,8 +1556,8 @@ extern "C" int nplm_sumsq(const float* x, long long n, float* out, cudaStream_t 
 extern "C" int nplm_adamw(float* p, float* m, float* v, float* g, void* p_bf16, const float* hyper,
                           const float* sumsq, long long n, int zero_grad, cudaStream_t st) {
   if (n <= 0) return 0;
-  launch_when(n <= CHAIN_ELEMENTS, adamw_kernel, grid_for(n, 256), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p_bf16),
-                                                 hyper, sumsq, n, zero_grad);
+  launch_when(n <= CHAIN_ELEMENTS, adamw_kernel, grid_for(n, 256), 256, 0, st, p, m, v, g,
+      reinterpret_cast<__nv_bfloat16*>(p_bf16), hyper, sumsq, n, zero_grad);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1562,8 +1568,8 @@ extern "C" int nplm_muon_momentum(const float* g, float* m, const long long* off
   if (numel & 3) return -3;
   int bx = grid_for(numel / 4, 256);
   if (bx > 592) bx = 592;
-  launch_when(n_mat * numel <= CHAIN_ELEMENTS, muon_momentum_kernel, dim3(bx, n_mat), 256, 0, st, g, m, off, numel, reinterpret_cast<__nv_bfloat16*>(upd),
-                                                        usq, sumsq, gs, max_norm, mu, nesterov);
+  launch_when(n_mat * numel <= CHAIN_ELEMENTS, muon_momentum_kernel, dim3(bx, n_mat), 256, 0, st, g, m, off, numel,
+      reinterpret_cast<__nv_bfloat16*>(upd), usq, sumsq, gs, max_norm, mu, nesterov);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1573,8 +1579,8 @@ extern "C" int nplm_muon_apply(float* p, void* p16, const long long* off, int n_
   if (numel & 3) return -3;
   int bx = grid_for(numel / 4, 256);
   if (bx > 592) bx = 592;
-  launch_when(n_mat * numel <= CHAIN_ELEMENTS, muon_apply_kernel, dim3(bx, n_mat), 256, 0, st, p, reinterpret_cast<__nv_bfloat16*>(p16), off, numel,
-                                                     reinterpret_cast<const __nv_bfloat16*>(O), lr, wd, cautious);
+  launch_when(n_mat * numel <= CHAIN_ELEMENTS, muon_apply_kernel, dim3(bx, n_mat), 256, 0, st, p,
+      reinterpret_cast<__nv_bfloat16*>(p16), off, numel, reinterpret_cast<const __nv_bfloat16*>(O), lr, wd, cautious);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1585,15 +1591,15 @@ extern "C" int nplm_adamw_slots(float* p, float* m, float* v, const float* g, vo
   if (n_slots <= 0 || max_numel <= 0) return 0;
   int bx = grid_for(max_numel, 256);
   if (bx > 64) bx = 64;
-  launch_when(n_slots * max_numel <= CHAIN_ELEMENTS, adamw_slots_kernel, dim3(bx, n_slots), 256, 0, st, p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p16), off,
-                                                        numel, decay, sumsq, gs, max_norm, lr, b1, b2, eps, wd,
-                                                        bc1, bc2);
+  launch_when(n_slots * max_numel <= CHAIN_ELEMENTS, adamw_slots_kernel, dim3(bx, n_slots), 256, 0, st, p, m, v, g,
+      reinterpret_cast<__nv_bfloat16*>(p16), off, numel, decay, sumsq, gs, max_norm, lr, b1, b2, eps, wd, bc1, bc2);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int nplm_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
-  launch_when(n <= CHAIN_ELEMENTS, cast_f32_to_bf16_kernel, grid_for(n, 256), 256, 0, st, src, reinterpret_cast<__nv_bfloat16*>(dst), n);
+  launch_when(n <= CHAIN_ELEMENTS, cast_f32_to_bf16_kernel, grid_for(n, 256), 256, 0, st, src,
+      reinterpret_cast<__nv_bfloat16*>(dst), n);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1603,7 +1609,8 @@ extern "C" int nplm_masked_mse(const void* s, const void* t, const int* valid, c
                                cudaStream_t st) {
   if (T <= 0) return 0;
   if (C % 8) return -3;
-  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, masked_mse_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, masked_mse_kernel,
+      grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(s), reinterpret_cast<const __nv_bfloat16*>(t), valid,
       rows, inv_count, reinterpret_cast<__nv_bfloat16*>(ds), loss_sum, T, C);
   return static_cast<int>(cudaGetLastError());

@@ -89,10 +89,10 @@ dwconv_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 
 // Kernel size known at compile time: a warp owns 128 channels (a lane four: one 256-byte request a row) of a run of
 // consecutive tokens and slides over them, the KS rows around a token and the weights in registers, four rows loaded
-// ahead (eight: 17.5 us, fewer warps fit). Every row is read once but for KS - 1 at the ends of a run; tokens whose whole window lies inside their sequence (all
-// but KS - 1 of it) take no masks. 17 024 x 768, 7 taps: 24.8 -> 16.4 us; 55 424 x 1024 110 -> 83 (2.7 TB/s: bound by the latency of the
-// rows, 16 warps a multiprocessor). The form before, eight
-// channels x eight tokens a thread, read 14 rows for eight and ran one block of 243 registers a multiprocessor.
+// ahead (eight: 17.5 us, fewer warps fit). Every row is read once but for KS - 1 at the ends of a run; tokens whose whole
+// window lies inside their sequence (all but KS - 1 of it) take no masks. 17 024 x 768, 7 taps: 24.8 -> 16.4 us; 55 424 x
+// 1024 110 -> 83 (2.7 TB/s: bound by the latency of the rows, 16 warps a multiprocessor). The form before, eight channels x
+// eight tokens a thread, read 14 rows for eight and ran one block of 243 registers a multiprocessor.
 constexpr int DW_CH = 4, DW_AHEAD = 4;
 
 __device__ __forceinline__ void ld4(const __nv_bfloat16* p, float2 (&f)[2]) {
@@ -309,7 +309,8 @@ dwconv_bwd_w_run_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 }
 
 // Tokens a warp walks: as many as leave the two blocks of eight warps that a multiprocessor holds (more blocks wait for a
-// second round: 17 024 x 768 22 us with three), in whole batches of rows loaded ahead, 16 at least (a run reads KS - 1 rows more than it has) and 256 at most.
+// second round: 17 024 x 768 22 us with three), in whole batches of rows loaded ahead, 16 at least (a run reads KS - 1
+// rows more than it has) and 256 at most.
 static int dw_run(int T, int C) {
   const long long groups = (C + 127) / 128;
   long long run = (T * groups + 148 * 2 * 8 - 1) / (148 * 2 * 8);
@@ -628,7 +629,8 @@ extern "C" int nplm_dwconv(const void* x, const void* w, const void* bias, const
 #undef NPLM_DWCONV
     return static_cast<int>(cudaGetLastError());
   }
-  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, dwconv_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * C <= CHAIN_ELEMENTS, dwconv_kernel,
+      grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
       reinterpret_cast<const __nv_bfloat16*>(bias), s_start, s_end, reinterpret_cast<__nv_bfloat16*>(y), T, C,
       KS, flip, skip);
@@ -658,15 +660,15 @@ extern "C" int nplm_dwconv_bwd_w(const void* x, const void* dy, const int* s_sta
   const int tokens_per_block = 512;
   const dim3 grid((T + tokens_per_block - 1) / tokens_per_block, (C + 31) / 32);
   launch_chained(dwconv_bwd_w_kernel, grid, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),
-                                            reinterpret_cast<const __nv_bfloat16*>(dy), s_start, s_end, dw,
-                                            dbias, T, C, KS, tokens_per_block);
+      reinterpret_cast<const __nv_bfloat16*>(dy), s_start, s_end, dw, dbias, T, C, KS, tokens_per_block);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int nplm_mhc_read(const void* X, const float* alpha, void* h, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS) return -3;
-  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_read_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_read_kernel,
+      grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(X), alpha, reinterpret_cast<__nv_bfloat16*>(h), T, n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -674,7 +676,8 @@ extern "C" int nplm_mhc_read(const void* X, const float* alpha, void* h, int T, 
 extern "C" int nplm_mhc_mean(const void* X, void* z, int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS) return -3;
-  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_mean_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_mean_kernel,
+      grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<__nv_bfloat16*>(z), T, n, C);
   return static_cast<int>(cudaGetLastError());
 }
@@ -683,7 +686,8 @@ extern "C" int nplm_mhc_dx_combine(const void* g, const float* alpha, const void
                                    int T, int n, int C, cudaStream_t st) {
   if (T <= 0) return 0;
   if ((C % 8) || n < 1 || n > MAX_STREAMS || (dh != nullptr && alpha == nullptr)) return -3;
-  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_dx_combine_kernel, grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, mhc_dx_combine_kernel,
+      grid_for(static_cast<long long>(T) * (C / 8), 256), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(g), alpha, reinterpret_cast<const __nv_bfloat16*>(dh),
       reinterpret_cast<const __nv_bfloat16*>(dz), reinterpret_cast<__nv_bfloat16*>(dX), T, n, C);
   return static_cast<int>(cudaGetLastError());
@@ -696,8 +700,9 @@ extern "C" int nplm_mhc_write(const void* X, const void* y, const float* R, cons
   if ((C % 8) || n < 1 || n > 4) return -3;
   const int grid = grid_for(static_cast<long long>(T) * (C / 8), 256);
 #define NPLM_MHC_WRITE(N_)                                                                              \
-  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS, z != nullptr ? mhc_write_kernel<N_, true> : mhc_write_kernel<N_, false>, grid, 256, 0, st, \
-              reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, beta,   \
+  launch_when(static_cast<long long>(T) * n * C <= CHAIN_ELEMENTS,                                              \
+              z != nullptr ? mhc_write_kernel<N_, true> : mhc_write_kernel<N_, false>, grid, 256, 0, st,        \
+              reinterpret_cast<const __nv_bfloat16*>(X), reinterpret_cast<const __nv_bfloat16*>(y), R, beta,    \
               reinterpret_cast<__nv_bfloat16*>(Xn), reinterpret_cast<__nv_bfloat16*>(z), T, C)
   switch (n) {
     case 1: NPLM_MHC_WRITE(1); break;
@@ -1003,18 +1008,18 @@ namespace nplm {
 template <int N, typename P>
 static void mhc_coef_fwd_launch(const __nv_bfloat16* pre, const void* a, const void* b, const void* r, const void* s,
                                 int iters, int T, float* alpha, float* beta, float* R, int blocks, cudaStream_t st) {
-  launch_chained(mhc_coef_fwd_kernel<N, P>, blocks, 128, 0, st, pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
-                                                    reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters,
-                                                    T, alpha, beta, R);
+  launch_chained(mhc_coef_fwd_kernel<N, P>, blocks, 128, 0, st, pre, reinterpret_cast<const P*>(a),
+      reinterpret_cast<const P*>(b), reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters, T, alpha, beta,
+      R);
 }
 template <int N, typename P>
 static void mhc_coef_bwd_launch(const __nv_bfloat16* pre, const void* a, const void* b, const void* r, const void* s,
                                 int iters, int T, const float* dalpha, const float* dbeta, const float* dR,
                                 __nv_bfloat16* dpre, float* da, float* db, float* dr, float* ds, int blocks,
                                 cudaStream_t st) {
-  launch_chained(mhc_coef_bwd_kernel<N, P>, blocks, 128, 0, st, pre, reinterpret_cast<const P*>(a), reinterpret_cast<const P*>(b),
-                                                    reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters,
-                                                    T, dalpha, dbeta, dR, dpre, da, db, dr, ds);
+  launch_chained(mhc_coef_bwd_kernel<N, P>, blocks, 128, 0, st, pre, reinterpret_cast<const P*>(a),
+      reinterpret_cast<const P*>(b), reinterpret_cast<const P*>(r), reinterpret_cast<const P*>(s), iters, T, dalpha,
+      dbeta, dR, dpre, da, db, dr, ds);
 }
 }  // namespace nplm
 

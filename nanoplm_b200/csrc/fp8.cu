@@ -1058,9 +1058,9 @@ extern "C" int nplm_fp8_quant_dual(const void* x, int R, int K, int ldx, void* q
   if (R <= 0 || K <= 0) return 0;
   if ((K % 128) || (R % 128) || (ldx % 4) || (reinterpret_cast<uintptr_t>(x) & 7)) return -3;
   if (R / 128 > 65535) return -3;
-  launch_chained(quant_dual_kernel, dim3(K / 128, R / 128), DUAL_THREADS, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx,
-                                                                reinterpret_cast<uint8_t*>(qr), sr,
-                                                                reinterpret_cast<uint8_t*>(qt), st);
+  launch_chained(quant_dual_kernel, dim3(K / 128, R / 128), DUAL_THREADS, 0, stream,
+      reinterpret_cast<const __nv_bfloat16*>(x), R, K, ldx, reinterpret_cast<uint8_t*>(qr), sr,
+      reinterpret_cast<uint8_t*>(qt), st);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -1263,7 +1263,8 @@ static int gemm_entry(const void* A, const void* B, void* C, const void* R, int 
   if ((epi == EPI_AXPBY) != (grp.mode == 3)) return -9;
   if (grp.mode == 3 && (a_mn || direct_epilogue || !grp.pair || bn != 256 || max_ctas != 0 || grp.groups < 1 ||
                         grp.group_rows < 1 || (grp.group_rows % 256) || (K % BK) || (N % 64) || (ldc % 8) || (ldr % 8) ||
-                        (reinterpret_cast<uintptr_t>(R) & 15) || (grp.sym && (N != grp.group_rows || grp.b_group_rows != grp.group_rows)) || grp.ag_world > 1))
+                        (reinterpret_cast<uintptr_t>(R) & 15) || grp.ag_world > 1 ||
+                        (grp.sym && (N != grp.group_rows || grp.b_group_rows != grp.group_rows))))
     return -9;
   const int num_kb = (K + BK - 1) / BK;
   if (splits < 0) splits = 1;
@@ -1511,10 +1512,11 @@ extern "C" int nplm_gemm_bf16_delta(const void* A, const void* B, void* C, const
 // R_g (b_mn = 1, B_g [K][N]), all bf16 with fp32 accumulation and one rounding; A_g, C_g and R_g (may be null) are rows [g *
 // rows, (g + 1) * rows) of their matrices. rows a multiple of 256, K and N of 64. sym: every C_g is symmetric and square
 // (the caller's promise: A = B, or commuting symmetric operands), so only the tiles on and below the diagonal
-// are computed: 160 tiles of 256 x 256 for 16 matrices of 1024 x 1024 instead of 256. The symmetric products (K 1024 to
-// 4096) of a Newton-Schulz step over 64 matrices take 39.6 us a launch on average, 51 as full products on single CTAs;
-// the others 65, with the sum that they end in, 78 without. Bound by the tensor pipe and by the waves of 74 pairs (2.2 of
-// them round up to 3).
+// are computed: 160 tiles of 256 x 256 for 16 matrices of 1024 x 1024 instead of 256. Newton-Schulz calls it without alpha,
+// beta and R: few-token training wants the roundings of its sums between the products.
+// 16 matrices of 1024 rows, K = 1024 / 2048 / 3072 / 4096, us on a cold L2: Gram product 32.9 / 50.2 / 66.5 / 82.9, all its
+// tiles 37.0 / 58.4 / 78.8 / 99.2, on single CTAs 39.8 / 64.5 / 87.0 / 110.6; B X with as many columns 39.9 / 58.4 / 80.9 / 100.4
+// against 42.0 / 63.5 / 90.1 / 110.6. Bound by the tensor pipe and by the waves of 74 pairs (2.2 of them round up to 3).
 extern "C" int nplm_gemm_bf16_stack(const void* A, const void* B, void* C, const void* R, int groups, int rows, int N, int K,
                                     int lda, int ldb, int ldc, int ldr, int b_mn, float alpha, float beta, int sym,
                                     int* status, cudaStream_t stream) {

@@ -496,8 +496,8 @@ extern "C" int nplm_router_bwd(const float* probs, const float* gates, const int
                                void* dlogits, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (E < 1 || E > MOE_MAX_E || k < 1 || k > MOE_MAX_K) return -3;
-  launch_chained(router_bwd_kernel, grid_for(T, 8), 256, 0, stream, probs, gates, experts, d_gates, aux_grad, T, E,
-                                                        k, reinterpret_cast<__nv_bfloat16*>(dlogits));
+  launch_chained(router_bwd_kernel, grid_for(T, 8), 256, 0, stream, probs, gates, experts, d_gates, aux_grad, T, E, k,
+      reinterpret_cast<__nv_bfloat16*>(dlogits));
   return static_cast<int>(cudaGetLastError());
 }
 

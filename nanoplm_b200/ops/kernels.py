@@ -16,7 +16,7 @@ from ._lib import check_rc, count_launch, lib, ptr, raw_stream, status_word, str
 EPI_STORE, EPI_ADD, EPI_ATOMIC_F32, EPI_GELU, EPI_STORE_F32, EPI_SWIGLU, EPI_ROPE, EPI_RELU = 0, 1, 2, 3, 4, 5, 6, 7
 # acc = dL/dh of h = silu(gate) * value; aux = the [value | gate] pre-activations (2N wide);
 # out = their gradient (2N wide)
-EPI_SWIGLU_BWD = 8
+EPI_SWIGLU_BWD, EPI_STORE_DELTA = 8, 9
 
 _BF16 = torch.bfloat16
 
@@ -61,7 +61,7 @@ def pair_pays(M: int, N: int, K: int, epi: int) -> bool:
     """Whether a bf16-output GEMM on 256-wide tiles runs on CTA pairs by default: the rule of `gemm_pair_pays` in
     csrc/entry_points.h, which states the measurements on both sides of its lines."""
     tiles = (M + 127) // 128 * ((N + 255) // 256)
-    if epi in (EPI_SWIGLU_BWD, 9):       # 9: the delta epilogue, which has its own entry point
+    if epi in (EPI_SWIGLU_BWD, EPI_STORE_DELTA):
         return True
     if epi == EPI_ROPE:
         return tiles > 740 if K >= 1024 else K >= 768 and tiles > 2600
@@ -71,8 +71,8 @@ def pair_pays(M: int, N: int, K: int, epi: int) -> bool:
 def tile_width(M: int, N: int, epi: int) -> int:
     """Default tile width of a GEMM: the rule of `gemm_tile_width` in csrc/entry_points.h, which states the measurements on
     both sides of its lines."""
-    if epi in (EPI_SWIGLU_BWD, 9, EPI_ATOMIC_F32, EPI_STORE_F32):
-        return 256 if N >= 256 or epi in (EPI_SWIGLU_BWD, 9) else 128
+    if epi in (EPI_SWIGLU_BWD, EPI_STORE_DELTA, EPI_ATOMIC_F32, EPI_STORE_F32):
+        return 256 if N >= 256 or epi in (EPI_SWIGLU_BWD, EPI_STORE_DELTA) else 128
     rows = (M + 127) // 128
     if epi != EPI_SWIGLU and rows * ((N + 63) // 64) <= 148:
         return 64
