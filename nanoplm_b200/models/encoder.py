@@ -241,9 +241,17 @@ class EncoderLayer(nn.Module):
         return x, aux, (h, state)
 
 
+_LAYER_FORWARD = EncoderLayer.forward
+
+
+def _own_forward(layer) -> bool:
+    """A layer of this class, and with the class's own forward: a program that puts another one there expects it to be called."""
+    return type(layer) is EncoderLayer and EncoderLayer.forward is _LAYER_FORWARD
+
+
 def _stackable(layer) -> bool:
-    """A layer whose own call may be passed by: one of this class, nobody's hooks or forward on it."""
-    return (type(layer) is EncoderLayer and layer.mhc_attn is None and native_layer.unwatched(layer) and layer._plain())
+    """A layer whose own call may be passed by: nobody's hooks or forward on it."""
+    return _own_forward(layer) and layer.mhc_attn is None and native_layer.unwatched(layer) and layer._plain()
 
 
 class EncoderModel(nn.Module):
@@ -284,7 +292,7 @@ class EncoderModel(nn.Module):
                                              [rope[t] for t in types])
             layers = layers[done:]
         # on streams, a layer's last write and the next one's first read are one where nobody watches the layers' calls
-        own = [n > 1 and x.is_cuda and type(layer) is EncoderLayer and native_layer.unobserved((layer,)) for layer in layers]
+        own = [n > 1 and x.is_cuda and _own_forward(layer) and native_layer.unobserved((layer,)) for layer in layers]
         entry = None
         for i, layer in enumerate(layers):
             lt = layer.attention_type

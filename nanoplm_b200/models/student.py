@@ -15,7 +15,7 @@ from torch.nn.modules.module import _has_any_global_hook
 
 from nanoplm_b200.config.schema import StudentConfig
 from nanoplm_b200.data.tokenizer import StudentTokenizer
-from nanoplm_b200.models.encoder import (Attention, BatchContext, EncoderLayer, EncoderModel, Linear, Norm,
+from nanoplm_b200.models.encoder import (Attention, BatchContext, EncoderModel, Linear, Norm, _own_forward,
                                          position_ids_from_cu_seqlens)
 from nanoplm_b200.ops import functional as ops
 from nanoplm_b200.ops import kernels as K
@@ -94,7 +94,7 @@ class ProtX(EncoderModel):
     def packed_states(self, input_ids, attention_mask):
         """(states in the training mode [T, width], int64 indices of their rows among the B * S positions) of a padded batch
         on a GPU, for callers that need no padded output; None where somebody observes calls of this module."""
-        if not (type(self).forward is ProtX.forward and "forward" not in self.__dict__ and not self._forward_hooks
+        if not (type(self).forward is _FORWARD and "forward" not in self.__dict__ and not self._forward_hooks
                 and not self._forward_pre_hooks and not self._backward_hooks and not self._backward_pre_hooks
                 and not _has_any_global_hook() and self.final_norm.weight.dtype == torch.bfloat16
                 and input_ids.dim() == 2 and ops.unpad_takes(input_ids, attention_mask)):
@@ -126,10 +126,10 @@ class ProtX(EncoderModel):
 
     def _embeds_packed(self, device: torch.device) -> bool:
         """Whether embed_sequences may hand the model flat ids: bf16 on a GPU, and nothing that observes the padded
-        call (a forward of a subclass or of this instance, hooks on this module or on all modules)."""
+        call (a forward of a subclass, of this instance or put on the class, hooks on this module or on all modules)."""
         w = self.final_norm.weight
         return (device.type == "cuda" and w.dtype == torch.bfloat16 and w.shape[0] % 8 == 0
-                and type(self).forward is ProtX.forward and "forward" not in self.__dict__
+                and type(self).forward is _FORWARD and "forward" not in self.__dict__
                 and not self._forward_hooks and not self._forward_pre_hooks and not _has_any_global_hook())
 
     def _join_tokens(self) -> int:
@@ -140,7 +140,7 @@ class ProtX(EncoderModel):
         cfg = self.config
         for l in self.layers:       # (a dozen layers before the first launch: no look-ups through Module.__getattr__)
             a = l._modules.get("attn")
-            if type(l) is not EncoderLayer or l.is_moe or type(a) is not Attention or a.head_dim != 64:
+            if not _own_forward(l) or l.is_moe or type(a) is not Attention or a.head_dim != 64:
                 return 0
             qkv = a._modules["Wqkv"]
             w = qkv._parameters.get("weight")
@@ -293,6 +293,9 @@ class ProtX(EncoderModel):
         if was_training:
             self.train(restore)
         return out
+
+
+_FORWARD = ProtX.forward
 
 
 def inspect_checkpoint_architecture(path: str | Path) -> dict:
